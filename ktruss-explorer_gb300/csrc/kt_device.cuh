@@ -50,7 +50,7 @@ enum : uint32_t {
     kPWalk = 72,       // u64 (words 72..73): row entries queued for walks over the whole peel
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
-    kCtrlWords = 80,
+    kCtrlWords = 128,  // words 88-115: the list peel (kt_lists.cu)
 };
 
 // Schedule i of the autotuner's grid (kt_schedule_grid): support group {4, 8, 16} x chunk width

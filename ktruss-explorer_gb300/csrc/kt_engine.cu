@@ -117,6 +117,7 @@ void remember(kt_engine* e, const kt_engine::LastCall& c) {
     e->last = c;
     e->last.big_row = e->big_row;  // the build of the call being remembered set these
     e->last.tiny_row = e->tiny_row;
+    e->last.list_entries = e->list_entries;
 }
 
 void forget(kt_engine* e) {
@@ -378,6 +379,7 @@ int kt_engine_create(int device, kt_engine** out) {
     if ((rc = check_cuda(cudaSetDevice(device), "cudaSetDevice"))) return rc;
     kt_engine* e = new kt_engine();
     e->device = device;
+    e->lists_allowed = true;
     if ((rc = check_cuda(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device), "SM count")) ||
         (rc = check_cuda(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "create stream")) ||
         (rc = check_cuda(cudaEventCreate(&e->ev_start), "create event")) ||
@@ -409,6 +411,7 @@ int kt_engine_destroy(kt_engine* e) {
     if (e->arena) cudaFree(e->arena);
     if (e->aux) cudaFree(e->aux);
     if (e->tile_off) cudaFree(e->tile_off);
+    if (e->lists) cudaFree(e->lists);
     if (e->ctrl) cudaFree(e->ctrl);
     if (e->h_ctrl) cudaFreeHost(e->h_ctrl);
     if (e->ev_start) cudaEventDestroy(e->ev_start);

@@ -88,6 +88,10 @@ struct kt_engine {
     size_t aux_words = 0;
     uint32_t* tile_off = nullptr;  // tiled variant: first oriented position of each (vertex, column tile)
     size_t tile_off_words = 0;     //   (own allocation, made by the first tiled call)
+    uint2* lists = nullptr;        // triangle lists of a decomposition (own allocation, kt_lists.cu)
+    uint64_t list_cap = 0;         //   entries it holds
+    uint64_t list_entries = 0;     //   entries of the last call (three per triangle)
+    bool lists_allowed = false;    //   kt_engine_create sets it; the allocation-free path never does
 
     // Current graph.
     uint32_t n = 0;
@@ -123,6 +127,7 @@ struct kt_engine {
         uint32_t* k_max = nullptr;
         uint32_t k = 0;
         uint8_t* keep = nullptr;
+        uint64_t list_entries = 0;           // triangle list entries the call counted
         uint32_t big_row = 0, tiny_row = 0;  // read back by the call's build; a trusted build does not
     } last;
     cudaGraphExec_t replay = nullptr;
@@ -150,6 +155,8 @@ size_t carve(kt_engine* e, char* base, uint32_t n, uint64_t N, bool staging);
 
 // kt_sort.cu
 int exclusive_scan(kt_engine* e, const uint32_t* in, uint32_t* out, uint64_t n);
+// out[0, n] = cursor[0, n) = exclusive prefix sums of in[0, n) (out[n] is the total).
+int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* cursor);
 int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t n);
 // Sorts (keys, vals) by the low `bits` bits of the keys; ping-pongs between a and b buffers
 // and returns 0 if the result is in (key_a, val_a), 1 if in (key_b, val_b).  vals may be null.
@@ -174,6 +181,9 @@ int count_support(kt_engine* e);
 // kt_peel.cu
 int peel_decompose(kt_engine* e);
 int peel_single_k(kt_engine* e, uint32_t k);
+// kt_lists.cu: the decomposition from triangle lists (prepare_lists says whether it applies).
+int prepare_lists(kt_engine* e, bool* use);
+int peel_lists(kt_engine* e);
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max);
 int emit_keep(kt_engine* e, uint8_t* d_keep);
 int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, const uint32_t* d_offsets,

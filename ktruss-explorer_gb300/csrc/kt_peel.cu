@@ -951,7 +951,9 @@ int peel_decompose(kt_engine* e) {
     e->stats_ready = false;
     if ((rc = triangles(e))) return rc;
     if (e->m == 0) return KT_OK;
-    return launch_peel(e, 0);
+    bool lists = false;
+    if ((rc = prepare_lists(e, &lists))) return rc;
+    return lists ? peel_lists(e) : launch_peel(e, 0);
 }
 
 int peel_single_k(kt_engine* e, uint32_t k) {

@@ -44,8 +44,8 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* warp_sums, T* total) {
     return r;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const T* __restrict__ in, uint64_t n,
+template <class TI, class T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const TI* __restrict__ in, uint64_t n,
                                                                    T* __restrict__ sums) {
     __shared__ T ws[33];
     const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
@@ -60,17 +60,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const T* __rest
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// Exclusive scan of each tile, offset by the scanned tile sums (if given).
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T* in, T* out, uint64_t n,
-                                                               const T* __restrict__ tile_offsets) {
+// Exclusive scan of each tile, offset by the scanned tile sums (if given).  With `copy` the result is
+// written there too and out[n] is the total.
+template <class TI, class T>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const TI* in, T* out, uint64_t n,
+                                                               const T* __restrict__ tile_offsets, T* copy) {
     __shared__ T tile[kScanTile];
     __shared__ T ws[33];
     const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
         uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
-        tile[threadIdx.x + i * kScanThreads] = idx < n ? in[idx] : T(0);
+        tile[threadIdx.x + i * kScanThreads] = idx < n ? T(in[idx]) : T(0);
     }
     __syncthreads();
     T v[kScanItems], s = 0;
@@ -90,8 +91,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T* in, T* out
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
         uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
-        if (idx < n) out[idx] = tile[threadIdx.x + i * kScanThreads];
+        if (idx < n) {
+            out[idx] = tile[threadIdx.x + i * kScanThreads];
+            if (copy) copy[idx] = tile[threadIdx.x + i * kScanThreads];
+        }
     }
+    if (copy && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        out[n] = total + (tile_offsets ? tile_offsets[blockIdx.x] : T(0));
 }
 
 constexpr uint32_t kSortTile = 2048;  // keys per tile (one histogram column per tile and digit)
@@ -228,11 +234,12 @@ __global__ void __launch_bounds__(kScatterThreads) k_radix_scatter(const uint64_
 
 // Hierarchical scan: tile sums are scanned recursively in scratch (used as a stack from
 // word `tmp_off` on), then every tile is rescanned with its offset.
-template <class T>
-static int scan_level(kt_engine* e, const T* in, T* out, uint64_t n, T* tmp, uint64_t tmp_words, uint64_t tmp_off) {
+template <class TI, class T>
+static int scan_level(kt_engine* e, const TI* in, T* out, uint64_t n, T* tmp, uint64_t tmp_words, uint64_t tmp_off,
+                      T* copy = nullptr) {
     if (n == 0) return KT_OK;
     if (n <= kScanTile) {
-        k_scan_tiles<T><<<1, kScanThreads, 0, e->stream>>>(in, out, n, nullptr);
+        k_scan_tiles<TI, T><<<1, kScanThreads, 0, e->stream>>>(in, out, n, nullptr, copy);
         count_launch(e);
         return check_launch(e, "k_scan_tiles");
     }
@@ -241,23 +248,28 @@ static int scan_level(kt_engine* e, const T* in, T* out, uint64_t n, T* tmp, uin
     if (tmp_off + words > tmp_words)
         return fail(KT_ERR_INVALID_ARG, "scan scratch too small (%llu elements)", (unsigned long long)tmp_words);
     T* sums = tmp + tmp_off;
-    k_scan_tile_sums<T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, n, sums);
+    k_scan_tile_sums<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, n, sums);
     count_launch(e);
     int rc = check_launch(e, "k_scan_tile_sums");
     if (rc) return rc;
-    rc = scan_level<T>(e, sums, sums, nb, tmp, tmp_words, tmp_off + words);
+    rc = scan_level<T, T>(e, sums, sums, nb, tmp, tmp_words, tmp_off + words);
     if (rc) return rc;
-    k_scan_tiles<T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, out, n, sums);
+    k_scan_tiles<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, out, n, sums, copy);
     count_launch(e);
     return check_launch(e, "k_scan_tiles");
 }
 
 int exclusive_scan(kt_engine* e, const uint32_t* in, uint32_t* out, uint64_t n) {
-    return scan_level<uint32_t>(e, in, out, n, e->scan_tmp, e->scan_tmp_words, 0);
+    return scan_level<uint32_t, uint32_t>(e, in, out, n, e->scan_tmp, e->scan_tmp_words, 0);
 }
 
 int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t n) {
-    return scan_level<uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp), e->scan_tmp_words / 2, 0);
+    return scan_level<uint64_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp), e->scan_tmp_words / 2, 0);
+}
+
+int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* cursor) {
+    return scan_level<uint32_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp),
+                                          e->scan_tmp_words / 2, 0, cursor);
 }
 
 int radix_sort(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,
