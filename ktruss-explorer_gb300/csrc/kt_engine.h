@@ -155,8 +155,8 @@ size_t carve(kt_engine* e, char* base, uint32_t n, uint64_t N, bool staging);
 
 // kt_sort.cu
 int exclusive_scan(kt_engine* e, const uint32_t* in, uint32_t* out, uint64_t n);
-// out[0, n] = cursor[0, n) = exclusive prefix sums of in[0, n) (out[n] is the total).
-int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* cursor);
+// out[0, n] = exclusive prefix sums of in[0, n) (out[n] is the total); ends[i] = out[i + 1].
+int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* ends);
 int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t n);
 // Sorts (keys, vals) by the low `bits` bits of the keys; ping-pongs between a and b buffers
 // and returns 0 if the result is in (key_a, val_a), 1 if in (key_b, val_b).  vals may be null.
@@ -176,7 +176,12 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
                  uint32_t tiles_per_dim, uint32_t* d_tile_src_ptr, uint32_t* d_src_out, uint32_t* d_dst_out);
 
 // kt_support.cu: support of every edge (triangles through it) into e->sup.
+// The credits lie in two arrays until merge_support adds them up (and their sum into the control
+// block's triangle counter, which must be zero).
 int count_support(kt_engine* e);
+int merge_support(kt_engine* e);
+// Writes the triangle lists of the counted graph: list starts, and list ends (consumed).
+int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends);
 
 // kt_peel.cu
 int peel_decompose(kt_engine* e);

@@ -31,7 +31,7 @@
 // lists included / whole decomposition): R-MAT 20 of 15 M edges 61.0 -> 22.8 / 40.8 / 71.5 -> 51.4 ms,
 // R-MAT 22 of 60 M edges 246 -> 86 / 200 / 303 -> 257 ms, R-MAT 16 9.2 -> 5.1 / 5.6 / 10.1 -> 6.4 ms, a
 // Watts-Strogatz graph of 10 M edges 13.8 -> 2.6 / 4.0 / 17.2 -> 6.9 ms, a batch of 256 graphs (18 M
-// edges) 17.1 -> 4.3 / 5.9 / 22.4 -> 10.9 ms.
+// edges) 17.1 -> 4.3 / 5.9 / 22.4 -> 10.9 ms (the lists are written faster since, kt_support.cu).
 
 #include <algorithm>
 
@@ -42,7 +42,6 @@ namespace kt {
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kListThreads = 1024;        // one block per SM
 constexpr uint32_t kDead = 0xffffffffu;   // support of a removed edge (late decrements keep the top bit)
 constexpr uint32_t kQueue = 4096;         // edges a block queues in shared memory per round
@@ -519,54 +518,6 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
     }
 }
 
-// The lists: every triangle u < v < w found again from its lowest edge j = (u, v) as in the
-// support count, at positions x = (u, w) and y = (v, w).  The entries of j's own triangles fill
-// its list from the back (one group works on j, no atomics); those of triangles in which an edge
-// is x or y fill it from the front at its cursor.
-template <int G>
-__global__ void __launch_bounds__(kThreads) k_list_fill(const uint32_t* __restrict__ o_ptr,
-                                                        const uint32_t* __restrict__ o_col,
-                                                        const uint32_t* __restrict__ e_src, uint32_t m,
-                                                        const uint64_t* __restrict__ tptr,
-                                                        unsigned long long* __restrict__ cur, uint2* __restrict__ tri) {
-    const uint32_t lane = lane_id();
-    const uint32_t glane = lane & (G - 1), gshift = lane & ~(uint32_t)(G - 1);
-    const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << gshift);
-    const uint64_t gid = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const uint64_t ngroups = ((uint64_t)gridDim.x * blockDim.x) / G;
-    for (uint64_t j64 = gid; j64 < m; j64 += ngroups) {
-        const uint32_t j = (uint32_t)j64;
-        const uint32_t u = e_src[j], v = o_col[j];
-        const uint32_t a0 = j + 1, a1 = o_ptr[u + 1];
-        const uint32_t b0 = o_ptr[v], b1 = o_ptr[v + 1];
-        const uint32_t na = a1 - a0, nb = b1 - b0;
-        if (!na || !nb) continue;
-        uint64_t back = tptr[j + 1];
-        const bool iter_a = na <= nb;
-        const uint32_t i0 = iter_a ? a0 : b0, ni = iter_a ? na : nb;
-        const uint32_t s0 = iter_a ? b0 : a0, ns = iter_a ? nb : na;
-        for (uint32_t t0 = 0; t0 < ni; t0 += G) {
-            const uint32_t t = t0 + glane;
-            bool hit = false;
-            uint32_t x = 0, y = 0;
-            if (t < ni) {
-                x = i0 + t;
-                const uint32_t w = o_col[x];
-                const uint32_t idx = lower_bound_u32(o_col + s0, ns, w);
-                y = s0 + idx;
-                hit = idx < ns && o_col[y] == w;
-            }
-            const uint32_t hits = __ballot_sync(gmask, hit) & gmask;
-            if (hit) {
-                tri[back - 1 - __popc(hits & lanemask_lt())] = make_uint2(x, y);
-                tri[atomicAdd(&cur[x], 1ull)] = make_uint2(j, y);
-                tri[atomicAdd(&cur[y], 1ull)] = make_uint2(j, x);
-            }
-            back -= __popc(hits);
-        }
-    }
-}
-
 }  // namespace
 
 // Most list entries per edge on average (three per triangle) with which the lists are made.  Denser
@@ -624,16 +575,10 @@ int prepare_lists(kt_engine* e, bool* use) {
 int peel_lists(kt_engine* e) {
     int rc;
     const uint32_t m = e->m;
-    // the sort's key buffers are free after the build: list starts and fill cursors
+    // the sort's key buffers are free after the build: list starts, and ends for the fill
     uint64_t* tptr = e->key_a;
-    uint64_t* cur = e->key_b;
-    if ((rc = scan_offsets(e, e->sup, (uint64_t)m, tptr, cur))) return rc;
-    constexpr int G = 8;
-    const uint64_t blocks = std::min<uint64_t>(((uint64_t)m * G + kThreads - 1) / kThreads, (uint64_t)e->num_sms * 16);
-    k_list_fill<G><<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, m, tptr,
-                                                                 reinterpret_cast<unsigned long long*>(cur), e->lists);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_list_fill"))) return rc;
+    uint64_t* ends = e->key_b;
+    if ((rc = scan_offsets(e, e->sup, (uint64_t)m, tptr, ends)) || (rc = fill_lists(e, tptr, ends))) return rc;
     ListParams P;
     P.tri = e->lists;
     P.tptr = tptr;

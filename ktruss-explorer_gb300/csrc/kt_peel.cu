@@ -749,13 +749,6 @@ __global__ void k_init_peel_ctrl(uint32_t* ctrl) {
         ctrl[i] = (i >= kPLMin && i < kPLMin + 4) || (i >= kPLMinId && i < kPLMinId + 4) ? 0xffffffffu : 0u;
 }
 
-__global__ void k_sum_support(const uint32_t* __restrict__ sup, uint32_t m, unsigned long long* __restrict__ total) {
-    uint64_t s = 0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) s += sup[j];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
-    if (lane_id() == 0 && s) atomicAdd(total, (unsigned long long)s);
-}
-
 __global__ void k_emit_truss(const uint32_t* __restrict__ entry_eid, uint64_t entries, const uint32_t* __restrict__ tr,
                              uint32_t* __restrict__ out) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -934,12 +927,7 @@ int triangles(kt_engine* e) {
     unsigned long long* tot = reinterpret_cast<unsigned long long*>(e->ctrl + kCtrlTriLo);
     int rc = check_cuda(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), e->stream), "clear triangle counter");
     if (rc) return rc;
-    if (e->m) {
-        k_sum_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(e->sup, e->m, tot);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_sum_support"))) return rc;
-    }
-    return KT_OK;
+    return e->m ? merge_support(e) : KT_OK;
 }
 
 }  // namespace

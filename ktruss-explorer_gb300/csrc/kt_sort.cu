@@ -60,11 +60,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const TI* __res
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// Exclusive scan of each tile, offset by the scanned tile sums (if given).  With `copy` the result is
-// written there too and out[n] is the total.
+// Exclusive scan of each tile, offset by the scanned tile sums (if given).  With `ends` the inclusive
+// sums are written there and out[n] is the total.
 template <class TI, class T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const TI* in, T* out, uint64_t n,
-                                                               const T* __restrict__ tile_offsets, T* copy) {
+                                                               const T* __restrict__ tile_offsets, T* ends) {
     __shared__ T tile[kScanTile];
     __shared__ T ws[33];
     const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
@@ -93,11 +93,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const TI* in, T* ou
         uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
         if (idx < n) {
             out[idx] = tile[threadIdx.x + i * kScanThreads];
-            if (copy) copy[idx] = tile[threadIdx.x + i * kScanThreads];
+            if (ends && idx > 0) ends[idx - 1] = tile[threadIdx.x + i * kScanThreads];
         }
     }
-    if (copy && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-        out[n] = total + (tile_offsets ? tile_offsets[blockIdx.x] : T(0));
+    if (ends && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        out[n] = ends[n - 1] = total + (tile_offsets ? tile_offsets[blockIdx.x] : T(0));
 }
 
 constexpr uint32_t kSortTile = 2048;  // keys per tile (one histogram column per tile and digit)
@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(kScatterThreads) k_radix_scatter(const uint64_
 // word `tmp_off` on), then every tile is rescanned with its offset.
 template <class TI, class T>
 static int scan_level(kt_engine* e, const TI* in, T* out, uint64_t n, T* tmp, uint64_t tmp_words, uint64_t tmp_off,
-                      T* copy = nullptr) {
+                      T* ends = nullptr) {
     if (n == 0) return KT_OK;
     if (n <= kScanTile) {
-        k_scan_tiles<TI, T><<<1, kScanThreads, 0, e->stream>>>(in, out, n, nullptr, copy);
+        k_scan_tiles<TI, T><<<1, kScanThreads, 0, e->stream>>>(in, out, n, nullptr, ends);
         count_launch(e);
         return check_launch(e, "k_scan_tiles");
     }
@@ -254,7 +254,7 @@ static int scan_level(kt_engine* e, const TI* in, T* out, uint64_t n, T* tmp, ui
     if (rc) return rc;
     rc = scan_level<T, T>(e, sums, sums, nb, tmp, tmp_words, tmp_off + words);
     if (rc) return rc;
-    k_scan_tiles<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, out, n, sums, copy);
+    k_scan_tiles<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, out, n, sums, ends);
     count_launch(e);
     return check_launch(e, "k_scan_tiles");
 }
@@ -267,9 +267,9 @@ int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t
     return scan_level<uint64_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp), e->scan_tmp_words / 2, 0);
 }
 
-int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* cursor) {
+int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* ends) {
     return scan_level<uint32_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp),
-                                          e->scan_tmp_words / 2, 0, cursor);
+                                          e->scan_tmp_words / 2, 0, ends);
 }
 
 int radix_sort(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,

@@ -1,29 +1,37 @@
-// Edge support (triangle count per edge) on the degree-oriented CSR.
+// Edge support (triangle count per edge) on the degree-oriented CSR, and the triangle lists.
 //
 // Replaces count_triangles_kernel of the reference (kernel_ddc.cu:11-54): there one thread
-// merges the two out-lists of its edge and issues three atomics per triangle.  Two counts here,
-// chosen by the schedule's support_group:
+// merges the two out-lists of its edge and issues three atomics per triangle.  Every triangle
+// u < v < w (rank order) consists of the edges j = (u,v), x = (u,w) and y = (v,w).  Edge j's tail,
+// o_col[j+1 .. o_ptr[u+1]), holds u's neighbours above v; the triangles of j are the tail's members
+// that are also in v's row N+(v).  Two ways to test them, chosen by the middle vertex v:
 //
-// support_group 4, 8, 16, 32 - edge-centric: each oriented edge (u,v), u < v in rank order, is
-// handled by a group of G lanes.  Only the part of N+(u) above v can hold a common neighbour, and
-// it starts right after the edge itself in u's row, so the intersection is
-// S = o_col[j+1 .. o_ptr[u+1])  with  L = N+(v).  Lanes stride over the shorter list and
-// binary-search the longer one; for a triangle (u,v,w) found at positions x (in u's row) and y
-// (in v's row), the edges (u,w) = x and (v,w) = y gain one support each, and (u,v) gains the
-// group's match count once.  Bound: uncoalesced probes (about nine per search) through L1/L2.
+// Vertex-centric (k_middle): vertices with at least kMidIn in-edges and a row of at most kMidRow
+// entries.  A block hashes N+(v) into shared memory (key w -> row position, at most a quarter to a
+// half full) and streams the tails of a range of v's in-edges (the lower half of v's symmetric row)
+// through it, eight lanes to a tail: one shared-memory probe per entry instead of a binary search.
+// A triangle costs one global atomic (x); y is counted in shared memory and added once per item, j
+// once per tail.
 //
-// support_group 0 - vertex-centric with a shared-memory hash: every triangle u < v < w is found
-// from its middle vertex v.  The row N+(v) (at most a few thousand entries under degree
-// orientation) is hashed once into shared memory, key w -> position in the row; then the tails
-// S_uv = o_col[j+1 .. o_ptr[u+1]) of v's in-edges j = (u,v) (the lower part of v's symmetric row)
-// are streamed, coalesced, and each entry is one hash probe instead of a binary search.  A hit
-// at tail position x credits edge (u,w) = x with a global atomic, edge (v,w) with a shared-memory
-// counter at its row position (added to the support array once per row), and edge (u,v) with a
-// shared-memory counter per in-edge (added once per in-edge).  Lanes of a warp share the tails of
-// 32 in-edges at a time through a warp scan of the tail lengths, so short tails waste no lanes.
-// Scheduling by degree: a plan kernel sends vertices with short rows and few in-edges to single
-// warps (a warp-private table), all others as ranges of at most kHeavyIn in-edges to whole blocks
-// (a block table); rows longer than the block table are searched in HBM instead of hashed.
+// Edge-centric (k_support): all other edges, G lanes each (the schedule's support_group).  The
+// shorter of tail and row is walked, the longer binary-searched; x and y are credited with global
+// atomics, j once per group.
+//
+// The lists are written by a second pass over the triangles (kFill), in list order of locality:
+// scattered eight-byte writes into lists of many GB are bound by the DRAM's random accesses (R-MAT 20,
+// 1.1 G entries: 18.0 ms with the edge-centric pass alone, 24.6 ms with the vertex-centric one),
+// so three kernels write what is next to each other:
+//   k_middle  the entries of y for vertex-centric v: all in v's row.  An item's part of y's list was
+//             claimed by the count, whose addition to `sup` returned where it starts (bases); all
+//             other credits go to a second array (supx), so the claimed parts come first in a list;
+//   k_rows    the entries of j and x for the same v and rows u of at least kRowMin entries: all in
+//             u's row, after the claimed parts;
+//   k_support everything else, with a global cursor that fills each list from its end.
+//
+// Measured (GB300): count R-MAT 20 of 15 M edges 7.4 -> 3.8 ms, R-MAT 22 of 60 M edges 44.4 -> 23.7 ms
+// (k_support alone -> with k_middle; R-MAT 18: k_middle issues in 48 % of the cycles, L1 48 %, DRAM
+// 2 %); fill 18.0 -> 13.0 ms and 114 -> 77 ms, its DRAM writes on R-MAT 18 3.8 -> 2.1 GB for 1.8 GB of
+// entries.
 
 #include <algorithm>
 
@@ -36,338 +44,446 @@ namespace {
 
 constexpr int kThreads = 256;
 
-template <int G>
-__device__ __forceinline__ void support_body(const uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ o_col,
-                                             const uint32_t* __restrict__ e_src, uint32_t m,
-                                             uint32_t* __restrict__ sup) {
+constexpr int kMidThreads = 256;
+constexpr int kMidGroup = 8;                   // lanes per tail: R-MAT 22 count 23.3 ms, 24.0 with 16, 26.0 with 4
+constexpr uint32_t kMidSlots = 4096;           // hash slots (32 KB with positions and counters: 6 blocks an SM)
+constexpr uint32_t kMidRow = kMidSlots / 2;    // longest row that is hashed
+// A vertex is vertex-centric with at least kMidIn in-edges and kMidOut row entries: with fewer, a
+// table serves too few probes, or the search it replaces is short.  R-MAT 20 count 3.8 ms at 64
+// in-edges, 4.1 at 32, 3.8 at 128 (R-MAT 16: 0.21, 0.21, 0.23 ms); a batch of 256 graphs, whose hubs
+// have short rows, 1.08 ms at 32 row entries, 1.18 at 16, 1.35 at 1.
+constexpr uint32_t kMidIn = 64;
+constexpr uint32_t kMidOut = 32;
+constexpr uint32_t kMidItemIn = 256;           // in-edges per work item (more for longer rows)
+// Rows of kRowMin entries or more get a block of the fill: R-MAT 22 76.4 ms at 128, 79.8 at 64, 79.9
+// at 256; whole warps stream their rows (half warps: 81.0).
+constexpr uint32_t kRowMin = 128;
+constexpr int kRowGroup = 32;
+// A row is streamed through the table unless it is this many times longer than the tail that could
+// be searched in it instead (R-MAT 22: 76.4 ms at 6, 77.6 at 3, 78.8 at 12, 82.0 streaming always).
+constexpr uint32_t kRowFactor = 6;
+// Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save
+// (R-MAT 14 with 220,000 edges counts in 0.05 ms).
+constexpr uint32_t kMidMinEdges = 1u << 18;
+constexpr uint32_t kEmpty = 0xffffffffu;
+// control words of the plan, zero since the build
+constexpr uint32_t kMidItems = 21, kMidBases = 22, kMidCursor = 23;  // 23 count, 24 fill
+constexpr uint32_t kRowItems = 26, kRowCursor = 27;
+
+struct Graph {
+    const uint32_t* __restrict__ o_ptr;
+    const uint32_t* __restrict__ o_col;
+    const uint32_t* __restrict__ e_src;
+    const uint32_t* __restrict__ s_ptr;
+    const uint32_t* __restrict__ s_split;
+    const uint32_t* __restrict__ s_col;
+    const uint32_t* __restrict__ s_eid;
+    uint32_t n, m;
+    uint32_t mid_in;   // vertices with this many in-edges are vertex-centric (0: none) ...
+    uint32_t mid_out;  // ... if their row has this many entries
+};
+
+// Where counts go, and what the fill reads.
+struct Credits {
+    uint32_t* sup;                      // count: credits of y by vertex-centric items, claimed
+    uint32_t* supx;                     // count: all other credits
+    uint32_t* ycount;                   // fill: length of the part of each list that the items claimed
+    uint32_t* bases;                    // per item and row position: start of y's entries
+    const uint64_t* __restrict__ tptr;  // fill: list starts
+    unsigned long long* cur;            // fill: end of the free part of each list
+    uint2* tri;                         // fill: the lists
+};
+
+__device__ __forceinline__ bool vertex_centric(const Graph& g, uint32_t v, uint32_t row) {
+    return g.mid_in != 0 && row >= g.mid_out && row <= kMidRow && g.s_split[v] - g.s_ptr[v] >= g.mid_in;
+}
+
+// Rows long enough for a row block of the fill (k_rows).
+__device__ __forceinline__ bool row_block(uint32_t row) { return row >= kRowMin && row <= kMidRow; }
+
+template <int G, bool kFill>
+__device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
     const uint32_t lane = lane_id();
     const uint32_t glane = lane & (G - 1);
     const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << (lane & ~(uint32_t)(G - 1)));
     const uint64_t gid = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const uint64_t ngroups = ((uint64_t)gridDim.x * blockDim.x) / G;
-    for (uint64_t j64 = gid; j64 < m; j64 += ngroups) {
+    for (uint64_t j64 = gid; j64 < g.m; j64 += ngroups) {
         const uint32_t j = (uint32_t)j64;
-        const uint32_t u = e_src[j], v = o_col[j];
-        const uint32_t a0 = j + 1, a1 = o_ptr[u + 1];
-        const uint32_t b0 = o_ptr[v], b1 = o_ptr[v + 1];
+        const uint32_t u = g.e_src[j], v = g.o_col[j];
+        const uint32_t a0 = j + 1, a1 = g.o_ptr[u + 1];
+        const uint32_t b0 = g.o_ptr[v], b1 = g.o_ptr[v + 1];
         const uint32_t na = a1 - a0, nb = b1 - b0;
+        if (!na || !nb) continue;  // the same for the whole group
+        const bool middle = vertex_centric(g, v, nb);
+        if (middle && (!kFill || row_block(a1 - g.o_ptr[u]))) continue;
         uint32_t cnt = 0;
-        if (na && nb) {
-            // iterate the shorter list, search the longer
-            const bool iter_a = na <= nb;
-            const uint32_t i0 = iter_a ? a0 : b0, ni = iter_a ? na : nb;
-            const uint32_t s0 = iter_a ? b0 : a0, ns = iter_a ? nb : na;
-            for (uint32_t t = glane; t < ni; t += G) {
-                const uint32_t x = i0 + t;
-                const uint32_t w = o_col[x];
-                const uint32_t idx = lower_bound_u32(o_col + s0, ns, w);
-                if (idx < ns && o_col[s0 + idx] == w) {
+        // iterate the shorter list, search the longer
+        const bool iter_a = na <= nb;
+        const uint32_t i0 = iter_a ? a0 : b0, ni = iter_a ? na : nb;
+        const uint32_t s0 = iter_a ? b0 : a0, ns = iter_a ? nb : na;
+        for (uint32_t t0 = 0; t0 < ni; t0 += G) {
+            const uint32_t t = t0 + glane;
+            bool hit = false;
+            uint32_t x = 0, y = 0;
+            if (t < ni) {
+                x = i0 + t;
+                const uint32_t w = g.o_col[x];
+                const uint32_t idx = lower_bound_u32(g.o_col + s0, ns, w);
+                y = s0 + idx;
+                hit = idx < ns && g.o_col[y] == w;
+            }
+            if (!kFill) {
+                if (hit) {
                     ++cnt;
-                    atomicAdd(&sup[x], 1u);
-                    atomicAdd(&sup[s0 + idx], 1u);
+                    atomicAdd(&c.supx[x], 1u);
+                    atomicAdd(&c.supx[y], 1u);
+                }
+            } else {
+                const uint32_t hits = __ballot_sync(gmask, hit) & gmask;
+                if (hits) {
+                    const uint32_t first = __ffs(hits) - 1;
+                    unsigned long long own = 0;
+                    if (lane == first) own = atomicAdd(&c.cur[j], 0ull - __popc(hits));
+                    own = __shfl_sync(gmask, own, first);
+                    if (hit) {
+                        // walked and searched list in (u's row, v's row) or the other way round
+                        const uint32_t ex = iter_a ? x : y, ey = iter_a ? y : x;
+                        c.tri[own - 1 - __popc(hits & lanemask_lt())] = make_uint2(x, y);
+                        c.tri[atomicAdd(&c.cur[ex], ~0ull) - 1] = make_uint2(j, ey);
+                        if (!middle) c.tri[atomicAdd(&c.cur[ey], ~0ull) - 1] = make_uint2(j, ex);
+                    }
                 }
             }
         }
-        __syncwarp(gmask);
+        if (!kFill) {
+            __syncwarp(gmask);
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(gmask, cnt, o);
-        if (glane == 0 && cnt) atomicAdd(&sup[j], cnt);
+            for (int o = G / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(gmask, cnt, o);
+            if (glane == 0 && cnt) atomicAdd(&c.supx[j], cnt);
+        }
     }
 }
 
-template <int G>
-__global__ void __launch_bounds__(kThreads) k_support(const uint32_t* __restrict__ o_ptr,
-                                                      const uint32_t* __restrict__ o_col,
-                                                      const uint32_t* __restrict__ e_src, uint32_t m,
-                                                      uint32_t* __restrict__ sup) {
-    support_body<G>(o_ptr, o_col, e_src, m, sup);
+template <int G, bool kFill>
+__global__ void __launch_bounds__(kThreads) k_support(Graph g, Credits c) {
+    edge_body<G, kFill>(g, c);
 }
 
 // The same count with the lane group read from the control block, where the learned selector's
 // inference kernel wrote its choice: the schedule is chosen on the device, with no host read.
-__global__ void __launch_bounds__(kThreads) k_support_chosen(const uint32_t* __restrict__ o_ptr,
-                                                             const uint32_t* __restrict__ o_col,
-                                                             const uint32_t* __restrict__ e_src, uint32_t m,
-                                                             const uint32_t* __restrict__ sched,
-                                                             uint32_t* __restrict__ sup) {
+__global__ void __launch_bounds__(kThreads) k_support_chosen(Graph g, Credits c, const uint32_t* __restrict__ sched) {
     switch (sched[0]) {
-        case 4: support_body<4>(o_ptr, o_col, e_src, m, sup); break;
-        case 16: support_body<16>(o_ptr, o_col, e_src, m, sup); break;
-        case 32: support_body<32>(o_ptr, o_col, e_src, m, sup); break;
-        default: support_body<8>(o_ptr, o_col, e_src, m, sup); break;
+        case 4: edge_body<4, false>(g, c); break;
+        case 16: edge_body<16, false>(g, c); break;
+        case 32: edge_body<32, false>(g, c); break;
+        default: edge_body<8, false>(g, c); break;
     }
 }
 
-// ---- vertex-centric hashed count (support_group 0) --------------------------------------------
-
-constexpr int kHashThreads = 512;                 // 16 warps
-constexpr int kHashWarps = kHashThreads / 32;
-constexpr uint32_t kWarpSlots = 256;              // warp table: rows of at most 128 entries
-constexpr uint32_t kLightOut = kWarpSlots / 2;
-constexpr uint32_t kLightIn = 256;                // ... and at most this many in-edges
-constexpr uint32_t kBlockSlots = 4096;            // block table: rows of at most 2048 entries
-constexpr uint32_t kBlockOut = kBlockSlots / 2;
-constexpr uint32_t kHeavyIn = 1024;               // in-edges per block work item
-constexpr uint32_t kEmpty = 0xffffffffu;
-// control words of the plan (free during the support count)
-constexpr uint32_t kHLight = 21, kHHeavy = 22, kHLightCur = 23, kHHeavyCur = 24;
-
-struct HashSmem {
-    uint32_t wkey[kHashWarps][kWarpSlots];
-    uint16_t wval[kHashWarps][kWarpSlots];
-    uint32_t wcnt[kHashWarps][kLightOut];     // per row position of the warp's vertex
-    uint32_t jcnt[kHashWarps][32];            // per in-edge of the current batch
-    uint32_t bkey[kBlockSlots];
-    uint16_t bval[kBlockSlots];
-    uint32_t bcnt[kBlockOut];
-    uint32_t item;                            // the block's current heavy item
-};
-
-__device__ __forceinline__ uint32_t hash_slot(uint32_t w, uint32_t mask) { return (w * 0x9E3779B1u) >> 8 & mask; }
-
-// Plan: every vertex with in-edges and an out-row becomes a light vertex (one warp) or a list of
-// heavy items {v, first in-edge, end in-edge} (one block each).
-__global__ void k_support_plan(const uint32_t* __restrict__ s_ptr, const uint32_t* __restrict__ s_split,
-                               const uint32_t* __restrict__ o_ptr, uint32_t n, uint32_t* __restrict__ light,
-                               uint4* __restrict__ heavy, uint32_t* __restrict__ ctrl) {
+// Work items {v, first in-edge, end in-edge, first word of bases} of the vertex-centric vertices.
+// An item takes at least as many in-edges as v's row has entries, so all items together have at
+// most 2m words of bases.  Also lists the rows of the fill's row blocks.
+__global__ void k_middle_plan(Graph g, uint4* __restrict__ items, uint32_t* __restrict__ rows,
+                              uint32_t* __restrict__ ctrl) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t indeg = 0, outdeg = 0;
-    if (v < n) {
-        indeg = s_split[v] - s_ptr[v];
-        outdeg = o_ptr[v + 1] - o_ptr[v];
+    const uint32_t row = v < g.n ? g.o_ptr[v + 1] - g.o_ptr[v] : 0u;
+    const uint32_t listed = __ballot_sync(kFullMask, row_block(row));
+    if (listed) {
+        uint32_t base = 0;
+        if (lane_id() == 0) base = atomicAdd(ctrl + kRowItems, __popc(listed));
+        base = __shfl_sync(kFullMask, base, 0);
+        if (row_block(row)) rows[base + __popc(listed & lanemask_lt())] = v;
     }
-    const bool work = indeg && outdeg;
-    const bool is_light = work && outdeg <= kLightOut && indeg <= kLightIn;
-    const uint32_t lm = __ballot_sync(kFullMask, is_light);
-    uint32_t lb = 0;
-    if (lm && lane_id() == 0) lb = atomicAdd(ctrl + kHLight, __popc(lm));
-    lb = __shfl_sync(kFullMask, lb, 0);
-    if (is_light) light[lb + __popc(lm & lanemask_lt())] = v;
-    const uint32_t items = work && !is_light ? (indeg + kHeavyIn - 1) / kHeavyIn : 0u;
-    if (items) {
-        const uint32_t h0 = atomicAdd(ctrl + kHHeavy, items);
-        const uint32_t base = s_ptr[v];
-        for (uint32_t i = 0; i < items; ++i) {
-            const uint32_t a = base + i * kHeavyIn;
-            heavy[h0 + i] = make_uint4(v, a, min(a + kHeavyIn, base + indeg), 0u);
-        }
-    }
+    if (v >= g.n) return;
+    const uint32_t a = g.s_ptr[v], indeg = g.s_split[v] - a;
+    if (!row || !indeg || !vertex_centric(g, v, row)) return;
+    const uint32_t step = max(kMidItemIn, (row + kMidItemIn - 1) / kMidItemIn * kMidItemIn);
+    const uint32_t count = (indeg + step - 1) / step;
+    const uint32_t i0 = atomicAdd(ctrl + kMidItems, count), w0 = atomicAdd(ctrl + kMidBases, count * row);
+    for (uint32_t i = 0; i < count; ++i)
+        items[i0 + i] = make_uint4(v, a + i * step, a + min(indeg, (i + 1) * step), w0 + i * row);
 }
 
-// The tails of in-edges [a, b) (symmetric-row positions of v's lower neighbours), 32 in-edges at a
-// time per warp, starting at `first` and striding by `step` batches of 32.  `lookup(w)` returns the
-// row position of w in N+(v) or kEmpty; `credit_vw(pos)` records a triangle on edge (v,w).
-template <class Lookup, class Credit>
-__device__ __forceinline__ void stream_tails(const uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ o_col,
-                                             const uint32_t* __restrict__ s_col,
-                                             const uint32_t* __restrict__ s_eid, uint32_t* __restrict__ sup,
-                                             uint32_t a, uint32_t b, uint32_t first, uint32_t step,
-                                             uint32_t* jcnt, Lookup lookup, Credit credit_vw) {
-    const uint32_t lane = lane_id();
-    for (uint32_t base = a + first; base < b; base += step) {
-        const uint32_t p = base + lane;
-        uint32_t t0 = 0, len = 0, j = 0;
-        if (p < b) {
-            j = s_eid[p];
-            const uint32_t u = s_col[p];
-            t0 = j + 1;
-            len = o_ptr[u + 1] - t0;
+template <bool kFill>
+__global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Graph g, Credits c, const uint4* __restrict__ items,
+                                                           uint32_t* __restrict__ ctrl) {
+    __shared__ uint32_t key[kMidSlots];
+    __shared__ uint16_t at[kMidSlots];
+    __shared__ uint32_t cnt[kMidRow];  // count: triangles of y; fill: next list entry of y
+    __shared__ uint32_t s_item;
+    constexpr int G = kMidGroup;
+    const uint32_t lane = lane_id(), glane = lane & (G - 1);
+    const uint32_t gmask = ((1u << G) - 1) << (lane & ~(uint32_t)(G - 1));
+    const uint32_t group = threadIdx.x / G;
+    const uint32_t n_items = ctrl[kMidItems];
+    for (;;) {
+        if (threadIdx.x == 0) s_item = atomicAdd(ctrl + kMidCursor + (kFill ? 1 : 0), 1u);
+        __syncthreads();
+        const uint32_t it = s_item;
+        if (it >= n_items) return;
+        const uint4 d = items[it];
+        const uint32_t r0 = g.o_ptr[d.x], row = g.o_ptr[d.x + 1] - r0;
+        uint32_t bits = 6;  // at least four slots an entry, as far as the table goes
+        while (bits < 12 && (1u << bits) < 4 * row) ++bits;
+        const uint32_t mask = (1u << bits) - 1, shift = 32 - bits;
+        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = kEmpty;
+        // the fill counts list entries from the start of the row's lists (or, should they hold 2^32
+        // entries or more, from the start of each list)
+        uint64_t row_at = 0;
+        bool wide = false;
+        if (kFill) {
+            row_at = c.tptr[r0];
+            wide = c.tptr[r0 + row] - row_at >= 0xffffffffull;
         }
-        jcnt[lane] = 0;
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= (uint32_t)o) incl += t;
+        for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
+            cnt[i] = !kFill ? 0u : c.bases[d.w + i] + (wide ? 0u : (uint32_t)(c.tptr[r0 + i] - row_at));
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < row; i += kMidThreads) {
+            const uint32_t w = g.o_col[r0 + i];
+            uint32_t h = (w * 0x9E3779B1u) >> shift;
+            while (atomicCAS(&key[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
+            at[h] = (uint16_t)i;
         }
-        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-        __syncwarp();
-        for (uint32_t t = lane; t - lane < total; t += 32) {
-            // in-edge of flattened item t: the number of inclusive prefixes <= t
-            uint32_t i = 0;
-#pragma unroll
-            for (uint32_t s2 = 16; s2 > 0; s2 >>= 1) {
-                const uint32_t pv = __shfl_sync(kFullMask, incl, i + s2 - 1);
-                if (pv <= t) i += s2;
+        __syncthreads();
+        // eight in-edges at a time per group: their lanes load them together, then take the tails
+        // one after another
+        for (uint32_t p0 = d.y + group * G; p0 < d.z; p0 += kMidThreads) {
+            const uint32_t p = p0 + glane;
+            uint32_t j = 0, end = 0, mine = 0;
+            if (p < d.z) {
+                j = g.s_eid[p];
+                end = g.o_ptr[g.s_col[p] + 1];
             }
-            const uint32_t inc_i = __shfl_sync(kFullMask, incl, i & 31);
-            const uint32_t len_i = __shfl_sync(kFullMask, len, i & 31);
-            const uint32_t t0_i = __shfl_sync(kFullMask, t0, i & 31);
-            if (t < total) {
-                const uint32_t x = t0_i + (t - (inc_i - len_i));
-                const uint32_t pos = lookup(__ldg(o_col + x));
-                if (pos != kEmpty) {
-                    atomicAdd(&sup[x], 1u);
-                    credit_vw(pos);
-                    atomicAdd(&jcnt[i], 1u);
+            for (int q = 0; q < G; ++q) {
+                const uint32_t jq = __shfl_sync(gmask, j, q, G), eq = __shfl_sync(gmask, end, q, G);
+                uint32_t found = 0;
+                uint32_t w_next = jq + 1 + glane < eq ? g.o_col[jq + 1 + glane] : kEmpty;
+                for (uint32_t x = jq + 1 + glane; x < eq; x += G) {
+                    const uint32_t w = w_next;
+                    w_next = x + G < eq ? g.o_col[x + G] : kEmpty;
+                    uint32_t h = (w * 0x9E3779B1u) >> shift, k;
+                    while ((k = key[h]) != w && k != kEmpty) h = (h + 1) & mask;
+                    if (k == w) {
+                        const uint32_t pos = at[h];
+                        if (!kFill) {
+                            ++found;
+                            atomicAdd(&cnt[pos], 1u);
+                            atomicAdd(&c.supx[x], 1u);
+                        } else {
+                            c.tri[(wide ? __ldg(c.tptr + r0 + pos) : row_at) + atomicAdd(&cnt[pos], 1u)] =
+                                make_uint2(jq, x);
+                        }
+                    }
+                }
+                if (!kFill) {
+                    __syncwarp(gmask);
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) found += __shfl_xor_sync(gmask, found, o);
+                    if (glane == (uint32_t)q) mine = found;
                 }
             }
+            if (!kFill && mine) atomicAdd(&c.supx[j], mine);
         }
-        __syncwarp();
-        const uint32_t c = jcnt[lane];
-        if (p < b && c) atomicAdd(&sup[j], c);
-        __syncwarp();
+        __syncthreads();
+        if (!kFill)
+            for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
+                if (cnt[i]) c.bases[d.w + i] = atomicAdd(&c.sup[r0 + i], cnt[i]);
     }
 }
 
-__global__ void __launch_bounds__(kHashThreads) k_support_hash(const uint32_t* __restrict__ o_ptr,
-                                                               const uint32_t* __restrict__ o_col,
-                                                               const uint32_t* __restrict__ o_fence,
-                                                               const uint32_t* __restrict__ s_col,
-                                                               const uint32_t* __restrict__ s_eid,
-                                                               const uint32_t* __restrict__ s_ptr,
-                                                               const uint32_t* __restrict__ s_split,
-                                                               const uint32_t* __restrict__ light,
-                                                               const uint4* __restrict__ heavy,
-                                                               uint32_t* __restrict__ sup, uint32_t* __restrict__ ctrl) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    HashSmem& S = *reinterpret_cast<HashSmem*>(smem_raw);
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t n_heavy = ld_acquire(ctrl + kHHeavy), n_light = ld_acquire(ctrl + kHLight);
-
-    // heavy items: one block per item, the block table holds N+(v)
+// The fill's row blocks: for the rows u of kRowMin entries or more, the list entries of j and x of
+// the triangles whose middle vertex is vertex-centric (their y entries are k_middle's).  Both lie
+// in u's own row, so a block with the row hashed into shared memory and a cursor per row position
+// writes them without global atomics, into lists that are next to each other.  Groups of lanes
+// stream the rows N+(v) through the table - or, where v's row is much longer than u's tail above v,
+// search the tail's entries in it.
+__global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, const uint32_t* __restrict__ rows,
+                                                         uint32_t* __restrict__ ctrl) {
+    __shared__ uint32_t key[kMidSlots];
+    __shared__ uint16_t at[kMidSlots];
+    __shared__ uint32_t cur[kMidRow];  // next list entry, from the start of the row's lists
+    __shared__ uint32_t s_row;
+    constexpr int G = kRowGroup;
+    const uint32_t lane = lane_id(), glane = lane & (G - 1);
+    const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << (lane & ~(uint32_t)(G - 1)));
+    const uint32_t group = threadIdx.x / G, n_rows = ctrl[kRowItems];
     for (;;) {
-        if (threadIdx.x == 0) S.item = atomicAdd(ctrl + kHHeavyCur, 1u);
-        __syncthreads();
-        const uint32_t it = S.item;
-        if (it >= n_heavy) break;
-        const uint4 d = heavy[it];
-        const uint32_t v = d.x, r0 = o_ptr[v], outdeg = o_ptr[v + 1] - r0;
-        const bool hashed = outdeg <= kBlockOut;
-        uint32_t bits = 1;
-        while ((1u << bits) < 2 * outdeg) ++bits;
-        const uint32_t mask = (1u << bits) - 1;
-        if (hashed) {
-            for (uint32_t i = threadIdx.x; i <= mask; i += blockDim.x) S.bkey[i] = kEmpty;
-            for (uint32_t i = threadIdx.x; i < outdeg; i += blockDim.x) S.bcnt[i] = 0;
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < outdeg; i += blockDim.x) {
-                const uint32_t w = o_col[r0 + i];
-                uint32_t h = hash_slot(w, mask);
-                while (atomicCAS(&S.bkey[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
-                S.bval[h] = (uint16_t)i;
-            }
-            __syncthreads();
-            stream_tails(o_ptr, o_col, s_col, s_eid, sup, d.y, d.z, 32 * warp, 32 * kHashWarps, S.jcnt[warp],
-                         [&](uint32_t w) {
-                             uint32_t h = hash_slot(w, mask);
-                             for (;;) {
-                                 const uint32_t k = S.bkey[h];
-                                 if (k == w) return (uint32_t)S.bval[h];
-                                 if (k == kEmpty) return kEmpty;
-                                 h = (h + 1) & mask;
-                             }
-                         },
-                         [&](uint32_t pos) { atomicAdd(&S.bcnt[pos], 1u); });
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < outdeg; i += blockDim.x)
-                if (S.bcnt[i]) atomicAdd(&sup[r0 + i], S.bcnt[i]);
-        } else {
-            // a row too long for the table: binary search in HBM (through its fences), credits direct
-            stream_tails(o_ptr, o_col, s_col, s_eid, sup, d.y, d.z, 32 * warp, 32 * kHashWarps, S.jcnt[warp],
-                         [&](uint32_t w) {
-                             const uint32_t y = fenced_lower_bound(o_col, o_fence, r0, r0 + outdeg, w);
-                             return y < r0 + outdeg && __ldg(o_col + y) == w ? y - r0 : kEmpty;
-                         },
-                         [&](uint32_t pos) { atomicAdd(&sup[r0 + pos], 1u); });
+        if (threadIdx.x == 0) {
+            const uint32_t t = atomicAdd(ctrl + kRowCursor, 1u);
+            s_row = t < n_rows ? rows[t] : kEmpty;
         }
         __syncthreads();
-    }
-
-    // light vertices: one warp each, the warp's own table holds N+(v); batches of 32 vertices
-    uint32_t* wkey = S.wkey[warp];
-    uint16_t* wval = S.wval[warp];
-    uint32_t* wcnt = S.wcnt[warp];
-    for (;;) {
-        uint32_t b0 = 0;
-        if (lane == 0) b0 = atomicAdd(ctrl + kHLightCur, 32u);
-        b0 = __shfl_sync(kFullMask, b0, 0);
-        if (b0 >= n_light) break;
-        const uint32_t b1 = min(b0 + 32u, n_light);
-        for (uint32_t li = b0; li < b1; ++li) {
-            const uint32_t v = light[li], r0 = o_ptr[v], outdeg = o_ptr[v + 1] - r0;
-            uint32_t bits = 1;
-            while ((1u << bits) < 2 * outdeg) ++bits;
-            const uint32_t mask = (1u << bits) - 1;
-            for (uint32_t i = lane; i <= mask; i += 32) wkey[i] = kEmpty;
-            for (uint32_t i = lane; i < outdeg; i += 32) wcnt[i] = 0;
-            __syncwarp();
-            for (uint32_t i = lane; i < outdeg; i += 32) {
-                const uint32_t w = o_col[r0 + i];
-                uint32_t h = hash_slot(w, mask);
-                while (atomicCAS(&wkey[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
-                wval[h] = (uint16_t)i;
-            }
-            __syncwarp();
-            stream_tails(o_ptr, o_col, s_col, s_eid, sup, s_ptr[v], s_split[v], 0u, 32u, S.jcnt[warp],
-                         [&](uint32_t w) {
-                             uint32_t h = hash_slot(w, mask);
-                             for (;;) {
-                                 const uint32_t k = wkey[h];
-                                 if (k == w) return (uint32_t)wval[h];
-                                 if (k == kEmpty) return kEmpty;
-                                 h = (h + 1) & mask;
-                             }
-                         },
-                         [&](uint32_t pos) { atomicAdd(&wcnt[pos], 1u); });
-            __syncwarp();
-            for (uint32_t i = lane; i < outdeg; i += 32)
-                if (wcnt[i]) atomicAdd(&sup[r0 + i], wcnt[i]);
-            __syncwarp();
+        const uint32_t u = s_row;
+        if (u == kEmpty) return;
+        const uint32_t r0 = g.o_ptr[u], row = g.o_ptr[u + 1] - r0;
+        uint32_t bits = 6;
+        while (bits < 12 && (1u << bits) < 4 * row) ++bits;
+        const uint32_t mask = (1u << bits) - 1, shift = 32 - bits;
+        const uint64_t row_at = c.tptr[r0];
+        const bool wide = c.tptr[r0 + row] - row_at >= 0xffffffffull;
+        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = kEmpty;
+        for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
+            cur[i] = c.ycount[r0 + i] + (wide ? 0u : (uint32_t)(c.tptr[r0 + i] - row_at));
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < row; i += kMidThreads) {
+            const uint32_t w = g.o_col[r0 + i];
+            uint32_t h = (w * 0x9E3779B1u) >> shift;
+            while (atomicCAS(&key[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
+            at[h] = (uint16_t)i;
         }
+        __syncthreads();
+        // positions group, group + groups, ...: the group's lanes load the rows of the next G together
+        constexpr uint32_t kGroups = kMidThreads / G;
+        for (uint32_t i0 = group; i0 + 1 < row; i0 += kGroups * G) {
+            uint32_t lb0 = 0, lb1 = 0;
+            if (i0 + glane * kGroups + 1 < row) {
+            const uint32_t v = g.o_col[r0 + i0 + glane * kGroups];
+            lb0 = g.o_ptr[v];
+            lb1 = g.o_ptr[v + 1];
+            if (lb0 != lb1 && !vertex_centric(g, v, lb1 - lb0)) lb1 = lb0;
+            }
+            for (int l = 0; l < G; ++l) {
+            const uint32_t i = i0 + l * kGroups;
+            const uint32_t b0 = __shfl_sync(gmask, lb0, l, G), b1 = __shfl_sync(gmask, lb1, l, G), tail = row - 1 - i;
+            if (b0 == b1) continue;
+            const bool stream = b1 - b0 <= kRowFactor * tail;
+            const uint32_t p0 = stream ? b0 : r0 + i + 1, p1 = stream ? b1 : r0 + row;
+            uint32_t w_next = p0 + glane < p1 ? g.o_col[p0 + glane] : kEmpty;
+            for (uint32_t q0 = p0; q0 < p1; q0 += G) {
+                const uint32_t p = q0 + glane, w = w_next;
+                w_next = p + G < p1 ? g.o_col[p + G] : kEmpty;
+                uint32_t pos = kEmpty, y = p;  // x = r0 + pos
+                if (w != kEmpty) {
+                    if (stream) {
+                        uint32_t h = (w * 0x9E3779B1u) >> shift, k;
+                        while ((k = key[h]) != w && k != kEmpty) h = (h + 1) & mask;
+                        if (k == w) pos = at[h];
+                    } else {
+                        y = b0 + lower_bound_u32(g.o_col + b0, b1 - b0, w);
+                        if (y < b1 && g.o_col[y] == w) pos = p - r0;
+                    }
+                }
+                const uint32_t hits = __ballot_sync(gmask, pos != kEmpty) & gmask;
+                if (hits) {
+                    const uint32_t first = __ffs(hits) - 1;
+                    uint32_t own = 0;
+                    if (lane == first) own = atomicAdd(&cur[i], __popc(hits));
+                    own = __shfl_sync(gmask, own, first);
+                    if (pos != kEmpty) {
+                        c.tri[(wide ? __ldg(c.tptr + r0 + i) : row_at) + own + __popc(hits & lanemask_lt())] =
+                            make_uint2(r0 + pos, y);
+                        c.tri[(wide ? __ldg(c.tptr + r0 + pos) : row_at) + atomicAdd(&cur[pos], 1u)] =
+                            make_uint2(r0 + i, y);
+                    }
+                }
+            }
+          }
+        }
+        __syncthreads();
     }
 }
 
-int count_support_hash(kt_engine* e) {
-    int rc;
-    if ((rc = check_cuda(cudaMemsetAsync(e->ctrl + kHLight, 0, 4 * sizeof(uint32_t), e->stream), "clear plan")))
+// sup += supx, what it was into ycount, and the sum of all supports (three per triangle).
+__global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __restrict__ supx,
+                                uint32_t* __restrict__ ycount, uint32_t m, unsigned long long* __restrict__ total) {
+    uint64_t s = 0;
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t y = sup[j], v = y + supx[j];
+        ycount[j] = y;
+        sup[j] = v;
+        s += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
+    if (lane_id() == 0 && s) atomicAdd(total, (unsigned long long)s);
+}
+
+Graph graph_of(const kt_engine* e) {
+    // the choice must be the same in the count and in the fill of one call
+    const bool hash_all = !e->sched_on_device && e->sched.support_group == 0;
+    const uint32_t mid_in = hash_all ? 1u : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? 1u : kMidOut;
+    return Graph{e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out};
+}
+
+// The items lie in the first chunk buffer, the claims in the second, the rows in the first queue:
+// all free until the peel.
+uint4* items_of(const kt_engine* e) { return e->chunks0; }
+uint32_t* rows_of(const kt_engine* e) { return e->q0; }
+Credits credits_of(const kt_engine* e) {
+    return Credits{e->sup, e->rnd, e->tr, reinterpret_cast<uint32_t*>(e->chunks1), nullptr, nullptr, nullptr};
+}
+
+template <bool kFill>
+int launch_middle(kt_engine* e, const Graph& g, const Credits& c) {
+    int rc, per_sm = 0;
+    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_middle<kFill>, kMidThreads, 0),
+                         "occupancy of k_middle")))
         return rc;
-    k_support_plan<<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(e->s_ptr, e->s_split, e->o_ptr, e->n,
-                                                                                  e->q0, e->chunks0, e->ctrl);
+    if (per_sm < 1) return fail(KT_ERR_CUDA, "k_middle cannot be resident");
+    k_middle<kFill><<<(uint32_t)(e->num_sms * per_sm), kMidThreads, 0, e->stream>>>(g, c, items_of(e), e->ctrl);
     count_launch(e);
-    if ((rc = check_launch(e, "k_support_plan"))) return rc;
-    const int smem = (int)sizeof(HashSmem);
-    if ((rc = check_cuda(cudaFuncSetAttribute(k_support_hash, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                         "shared memory of k_support_hash")))
-        return rc;
-    int per_sm = 0;
-    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_support_hash, kHashThreads, smem),
-                         "occupancy of k_support_hash")))
-        return rc;
-    if (per_sm < 1) return fail(KT_ERR_CUDA, "k_support_hash cannot be resident");
-    k_support_hash<<<e->num_sms * per_sm, kHashThreads, smem, e->stream>>>(e->o_ptr, e->o_col, e->o_fence, e->s_col,
-                                                                           e->s_eid, e->s_ptr, e->s_split, e->q0,
-                                                                           e->chunks0, e->sup, e->ctrl);
-    count_launch(e);
-    return check_launch(e, "k_support_hash");
+    return check_launch(e, "k_middle");
+}
+
+uint32_t edge_blocks(const kt_engine* e, uint32_t G) {
+    return (uint32_t)std::min<uint64_t>(((uint64_t)e->m * G + kThreads - 1) / kThreads, (uint64_t)e->num_sms * 16);
 }
 
 }  // namespace
 
 int count_support(kt_engine* e) {
     if (e->m == 0) return KT_OK;
-    int rc = check_cuda(cudaMemsetAsync(e->sup, 0, sizeof(uint32_t) * e->m, e->stream), "clear support");
-    if (rc) return rc;
+    int rc;
+    const Graph g = graph_of(e);
+    const Credits c = credits_of(e);
+    if ((rc = check_cuda(cudaMemsetAsync(c.sup, 0, sizeof(uint32_t) * e->m, e->stream), "clear support")) ||
+        (rc = check_cuda(cudaMemsetAsync(c.supx, 0, sizeof(uint32_t) * e->m, e->stream), "clear support")))
+        return rc;
+    if (g.mid_in) {
+        k_middle_plan<<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), rows_of(e),
+                                                                                    e->ctrl);
+        count_launch(e);
+        if ((rc = check_launch(e, "k_middle_plan")) || (rc = launch_middle<false>(e, g, c))) return rc;
+    }
     if (e->sched_on_device) {
         // any group the selector may choose (4, 8 or 16 lanes per edge) fits this grid
-        const uint64_t blocks = std::min<uint64_t>(((uint64_t)e->m * 16 + kThreads - 1) / kThreads,
-                                                   (uint64_t)e->num_sms * 16);
-        k_support_chosen<<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, e->m,
-                                                                       e->ctrl + kPSched, e->sup);
+        k_support_chosen<<<edge_blocks(e, 16), kThreads, 0, e->stream>>>(g, c, e->ctrl + kPSched);
         count_launch(e);
         return check_launch(e, "k_support_chosen");
     }
-    const uint32_t G = e->sched.support_group;
-    if (G == 0) return count_support_hash(e);
-    uint64_t blocks = ((uint64_t)e->m * G + kThreads - 1) / kThreads;
-    const uint64_t max_blocks = (uint64_t)e->num_sms * 16;
-    if (blocks > max_blocks) blocks = max_blocks;
+    const uint32_t G = e->sched.support_group ? e->sched.support_group : 8;
+    const uint32_t blocks = edge_blocks(e, G);
     switch (G) {
-        case 4: k_support<4><<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, e->m, e->sup); break;
-        case 16: k_support<16><<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, e->m, e->sup); break;
-        case 32: k_support<32><<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, e->m, e->sup); break;
-        default: k_support<8><<<(uint32_t)blocks, kThreads, 0, e->stream>>>(e->o_ptr, e->o_col, e->e_src, e->m, e->sup); break;
+        case 4: k_support<4, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
+        case 16: k_support<16, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
+        case 32: k_support<32, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
+        default: k_support<8, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
     }
+    count_launch(e);
+    return check_launch(e, "k_support");
+}
+
+int merge_support(kt_engine* e) {
+    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(
+        e->sup, e->rnd, e->tr, e->m, reinterpret_cast<unsigned long long*>(e->ctrl + kCtrlTriLo));
+    count_launch(e);
+    return check_launch(e, "k_merge_support");
+}
+
+int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends) {
+    int rc;
+    const Graph g = graph_of(e);
+    Credits c = credits_of(e);
+    c.tptr = tptr;
+    c.cur = reinterpret_cast<unsigned long long*>(ends);
+    c.tri = e->lists;
+    if (g.mid_in) {
+        if ((rc = launch_middle<true>(e, g, c))) return rc;
+        k_rows<<<(uint32_t)e->num_sms * 6, kMidThreads, 0, e->stream>>>(g, c, rows_of(e), e->ctrl);
+        count_launch(e);
+        if ((rc = check_launch(e, "k_rows"))) return rc;
+    }
+    k_support<8, true><<<edge_blocks(e, 8), kThreads, 0, e->stream>>>(g, c);
     count_launch(e);
     return check_launch(e, "k_support");
 }

@@ -38,6 +38,14 @@ def _copies(part, count):
     return int(n) * count, (u + at).ravel(), (v + at).ravel()
 
 
+def _core(r, c):
+    """A complete bipartite graph of r + r vertices whose first c left vertices form a clique."""
+    c = min(c, r)
+    left, right = np.divmod(np.arange(r * r), r)
+    cu, cv = np.triu_indices(c, 1)
+    return 2 * r, np.concatenate([left, cu]), np.concatenate([right + r, cv])
+
+
 GRAPHS = {
     "one_edge": lambda: (2, np.array([0], np.uint32), np.array([1], np.uint32)),
     "one_triangle": lambda: _union([_clique(3)]),
@@ -47,6 +55,13 @@ GRAPHS = {
     "many_strips": lambda: _union([_copies(_strip(9), 220000), _clique(5)]),     # 900,000 edges queued in a round
     "chunk_overflow": lambda: _union([_copies(_clique(100), 25), _clique(120)]),  # four chunks an edge
     "rmat12_odd": lambda: kt.gen_rmat(12, 13, 0.57, 0.19, 0.19, 77),
+    # the vertex-centric count and the three kernels of the fill: graphs of 2^18 edges and more
+    "rmat15": lambda: kt.gen_rmat(15, 16, 0.57, 0.19, 0.19, 80),
+    "rmat15_cliques": lambda: kt.plant_cliques(*kt.gen_rmat(15, 12, 0.45, 0.22, 0.22, 81), 12, 60, 200, 82),
+    "rows_of_2000": lambda: _core(2000, 100),   # the longest rows that are hashed ...
+    "rows_of_2100": lambda: _core(2100, 100),   # ... and rows that are not
+    "rows_at_the_lines": lambda: _union([_core(r, c) for r in (31, 32, 127, 128, 129) for c in (20, 66)] +
+                                        [_core(500, 70)]),
     "hubs": lambda: kt.plant_cliques(*kt.gen_ba(20000, 12, 78), 6, 30, 90, 79),
 }
 
