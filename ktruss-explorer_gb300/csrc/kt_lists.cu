@@ -19,19 +19,25 @@
 //
 // A round is one phase and one grid barrier:
 //   1. warps take chunks (descriptors of up to 32 list entries) of the round's frontier; a decrement
-//      that takes an edge from k-2 to k-3 appends it to the block's queue in shared memory;
-//   2. the block flushes its queue: every queued edge is stamped, gets its truss number, and its
-//      list is cut into chunks for the next round (one global atomic per 32 edges);
-//   3. the barrier's arrival adds the block's queued edges to the arrival word, so the poll that
-//      ends the wait also delivers the size of the next frontier.
+//      that takes an edge from k-2 to k-3 stamps it, writes its truss number and appends it to the
+//      block's queue in shared memory;
+//   2. the block flushes its queue: the edges' lists are cut into chunks for the next round, in a
+//      buffer that all blocks share;
+//   3. the barrier's arrival adds the block's queued edges to the arrival word, next to which lies
+//      the count of chunks, so the 16-byte poll that ends the wait also delivers the size of the
+//      next frontier.
 //
-// Bound by latency: a round of up to 512 frontier edges takes 5 us (8.5 us when walking rows: barrier,
-// chunk, row entry, stamp, search, stamp, decrement, two pushes one after the other), larger ones by
-// the two gathers an entry.  Measured against the walking peel (GB300, peel kernel / writing the
-// lists included / whole decomposition): R-MAT 20 of 15 M edges 61.0 -> 22.8 / 40.8 / 71.5 -> 51.4 ms,
-// R-MAT 22 of 60 M edges 246 -> 86 / 200 / 303 -> 257 ms, R-MAT 16 9.2 -> 5.1 / 5.6 / 10.1 -> 6.4 ms, a
-// Watts-Strogatz graph of 10 M edges 13.8 -> 2.6 / 4.0 / 17.2 -> 6.9 ms, a batch of 256 graphs (18 M
-// edges) 17.1 -> 4.3 / 5.9 / 22.4 -> 10.9 ms (the lists are written faster since, kt_support.cu).
+// Bound: small rounds by one chain - chunk, entries, states, decrements, queue, claim of the next
+// chunks, barrier - of about 8,000 cycles (3.6 us; 8.5 us when walking rows), large ones by the
+// gathers in flight.  Measured against the walking peel (GB300, peel kernel / whole decomposition when
+// the lists came in): R-MAT 20 of 15 M edges 61.0 -> 22.8 / 71.5 -> 51.4 ms, R-MAT 22 of 60 M edges
+// 246 -> 86 / 303 -> 257 ms, R-MAT 16 9.2 -> 5.1 / 10.1 -> 6.4 ms, a Watts-Strogatz graph of 10 M edges
+// 13.8 -> 2.6 / 17.2 -> 6.9 ms, a batch of 256 graphs (18 M edges) 17.1 -> 4.3 / 22.4 -> 10.9 ms (the lists
+// are written faster since, kt_support.cu).  Chunks dealt to the blocks in turn, the frontier's size
+// delivered by the barrier's own poll, list bounds loaded while the decrements are under way, entries
+// prefetched across the barrier and four entries a lane under way in large rounds: peel kernel on
+// R-MAT 20 22.4 -> 18.3 ms, R-MAT 22 83.4 -> 67.8, R-MAT 16 4.7 -> 4.0, Watts-Strogatz 2.5 -> 2.2, the batch
+// 4.2 -> 3.5.
 
 #include <algorithm>
 
@@ -48,12 +54,17 @@ constexpr uint32_t kQueue = 4096;         // edges a block queues in shared memo
 constexpr uint32_t kStampPeriod = 254;    // round stamps 1..254
 constexpr uint32_t kOld = 255;            // state of edges removed before the last sweep
 constexpr uint32_t kChunk = 32;           // list entries per chunk
+constexpr uint32_t kAhead = 1024;         // queue entries whose list bounds may be loaded ahead
+constexpr uint32_t kNotLoaded = 0xffffffffu;
+constexpr uint32_t kPrefetch = 1u << 16;  // chunks of a frontier whose entries are prefetched to L2 (16 MB):
+                                          // R-MAT 20 peel kernel 20.9 -> 20.3 ms
 
-// Control words of this kernel (beyond the words it shares with the walking peel).
-constexpr uint32_t kLBar = 88;    // u64 [2]: arrivals << 32 | edges queued, by barrier parity
-constexpr uint32_t kLSlot = 96;   // [4] x {u64 chunks, u32 overflowed edges, u32 minimum support}
-constexpr uint32_t kLMinId = 112; // [4] smallest alive edge id of a level scan
-static_assert(kLMinId + 4 <= kCtrlWords, "control block holds the list peel's words");
+// Control words of this kernel (beyond the words it shares with the walking peel): a ring of four
+// barrier slots, each {u64 arrivals << 32 | edges queued, u64 global chunks, overflowed edges,
+// minimum support, smallest alive edge id, unused}.
+constexpr uint32_t kLRing = 96, kLSlotWords = 8;
+constexpr uint32_t kLChunks = 2, kLBig = 4, kLMin = 5, kLMinId = 6;
+static_assert(kLRing + 4 * kLSlotWords <= kCtrlWords, "control block holds the list peel's words");
 
 struct ListParams {
     const uint2* __restrict__ tri;       // per list entry: the triangle's other two edges
@@ -86,32 +97,40 @@ struct Front {
 
 struct ListShared {
     uint32_t queue[kQueue];
+    uint64_t start[kAhead];       // list start and length of the first queue entries, where loaded
+    uint32_t len[kAhead];
     uint32_t queued;              // edges queued since the last barrier (may exceed kQueue)
-    uint32_t bar_edges[2];        // the arrival words' edge sums when they last completed
-    uint32_t bar_arrivals[2];     // ... and their arrivals
     Front front;
     uint32_t ok;
     uint32_t min_sup, min_id;     // a level scan's block minima
-    unsigned long long walk;      // list entries queued (a statistic)
+    uint32_t walk;                // list entries queued in the level, and before it (a statistic)
+    unsigned long long walked;
     unsigned long long ns[9];     // block 0: phase clock
 };
 
-// Stamps the edges of a warp's lanes for the next round and cuts their lists into chunks.  All 32
-// lanes call it together; `slot` is the ring slot of the barrier that closes the current phase.
-__device__ __forceinline__ void push_lists(const ListParams& P, ListShared& S, uint32_t e, bool take, uint32_t rr,
-                                           uint32_t k, uint32_t slot, uint32_t parity) {
-    uint64_t t0 = 0;
-    uint32_t len = 0;
+// List bounds of edge e.  An edge removed at level 3 has no triangle left whose other edges are
+// alive or in its round: nothing to walk.
+__device__ __forceinline__ void list_of(const ListParams& P, uint32_t e, bool take, uint32_t k, uint64_t* t0,
+                                        uint32_t* len) {
+    *t0 = 0;
+    *len = 0;
+    if (take && k != 3) {
+        *t0 = __ldg(P.tptr + e);
+        *len = (uint32_t)(__ldg(P.tptr + e + 1) - *t0);
+    }
+}
+
+// Removes a warp's edges in round rr - stamp, truss number - and cuts their lists (len entries from
+// t0 on; kNotLoaded: still to be looked up) into chunks of the next frontier.  All 32 lanes call it
+// together; `slot` is the ring slot of the barrier that closes the current phase.
+__device__ __forceinline__ void push_lists(const ListParams& P, ListShared& S, uint32_t e, bool take, uint64_t t0,
+                                           uint32_t len, uint32_t rr, uint32_t k, uint32_t slot, uint32_t parity) {
     if (take) {
         P.st[e] = (uint8_t)stamp_of(rr);
         P.tr[e] = k - 1;
         P.sup[e] = kDead;
-        // an edge removed at level 3 has no triangle left whose other edges are alive or in its round
-        if (k != 3) {
-            t0 = __ldg(P.tptr + e);
-            len = (uint32_t)(__ldg(P.tptr + e + 1) - t0);
-        }
     }
+    if (len == kNotLoaded) list_of(P, e, take, k, &t0, &len);
     const uint32_t nch = (len + kChunk - 1) / kChunk;
     const uint32_t lane = lane_id();
     uint32_t incl = nch;
@@ -125,45 +144,61 @@ __device__ __forceinline__ void push_lists(const ListParams& P, ListShared& S, u
     const uint32_t walked = __reduce_add_sync(kFullMask, len);
     unsigned long long cb = 0;
     if (lane == 0) {
-        cb = atomicAdd(reinterpret_cast<unsigned long long*>(P.ctrl + kLSlot + 4 * slot), (unsigned long long)total);
-        atomicAdd(&S.walk, (unsigned long long)walked);
+        cb = atomicAdd(reinterpret_cast<unsigned long long*>(P.ctrl + kLRing + kLSlotWords * slot + kLChunks),
+                       (unsigned long long)total);
+        atomicAdd(&S.walk, walked);
     }
     cb = __shfl_sync(kFullMask, cb, 0);
     uint4* ch = P.ch[parity];
-    if (cb + total <= P.cap_chunks) {
-        // lanes write the chunks in turn, whichever lane's edge they belong to
-        const uint32_t lo = (uint32_t)t0, hi = (uint32_t)(t0 >> 32);
-        for (uint32_t i0 = 0; i0 < total; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            uint32_t own = 0;  // the number of inclusive prefixes <= i
-#pragma unroll
-            for (uint32_t s = 16; s > 0; s >>= 1) {
-                const uint32_t v = __shfl_sync(kFullMask, incl, own + s - 1);
-                if (v <= i) own += s;
-            }
-            own &= 31u;
-            const uint32_t oe = __shfl_sync(kFullMask, e, own), ol = __shfl_sync(kFullMask, len, own);
-            const uint32_t oi = __shfl_sync(kFullMask, incl, own), on = __shfl_sync(kFullMask, nch, own);
-            const uint64_t op = (uint64_t)__shfl_sync(kFullMask, hi, own) << 32 | __shfl_sync(kFullMask, lo, own);
-            if (i < total) {
-                const uint32_t off = (i - (oi - on)) * kChunk;
-                const uint64_t p = op + off;
-                ch[cb + i] = make_uint4(oe, (uint32_t)p, (uint32_t)(p >> 32), min(kChunk, ol - off));
-            }
-        }
-    } else {
+    if (cb + total > P.cap_chunks) {
+        // the claimed slots stay empty; the edges go to the overflow queue
         const uint64_t stop = cb + total < P.cap_chunks ? cb + total : P.cap_chunks;
+#pragma unroll 1
         for (uint64_t i = cb + lane; i < stop; i += 32) ch[i] = make_uint4(0, 0, 0, 0);
-        const bool mine = len != 0;
+        const bool mine = nch != 0;
         const uint32_t mb = __ballot_sync(kFullMask, mine);
         uint32_t bb = 0;
-        if (lane == 0) bb = atomicAdd(P.ctrl + kLSlot + 4 * slot + 2, __popc(mb));
+        if (lane == 0) bb = atomicAdd(P.ctrl + kLRing + kLSlotWords * slot + kLBig, __popc(mb));
         bb = __shfl_sync(kFullMask, bb, 0);
         if (mine) P.big[parity][bb + __popc(mb & lanemask_lt())] = e;
+        return;
+    }
+    // lanes write the chunks in turn, whichever lane's edge they belong to
+    const uint32_t lo = (uint32_t)t0, hi = (uint32_t)(t0 >> 32);
+#pragma unroll 1
+    for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        uint32_t at = 0;  // the number of inclusive prefixes <= i
+#pragma unroll
+        for (uint32_t s = 16; s > 0; s >>= 1) {
+            const uint32_t v = __shfl_sync(kFullMask, incl, at + s - 1);
+            if (v <= i) at += s;
+        }
+        at &= 31u;
+        const uint32_t oe = __shfl_sync(kFullMask, e, at), ol = __shfl_sync(kFullMask, len, at);
+        const uint32_t oi = __shfl_sync(kFullMask, incl, at), on = __shfl_sync(kFullMask, nch, at);
+        const uint64_t op = (uint64_t)__shfl_sync(kFullMask, hi, at) << 32 | __shfl_sync(kFullMask, lo, at);
+        if (i < total) {
+            const uint32_t off = (i - (oi - on)) * kChunk;
+            const uint64_t p = op + off;
+            const uint32_t cnt = min(kChunk, ol - off);
+            ch[cb + i] = make_uint4(oe, (uint32_t)p, (uint32_t)(p >> 32), cnt);
+            if (cb < kPrefetch) {  // on their way while the blocks meet at the barrier
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(P.tri + p));
+                if (cnt > 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(P.tri + p + 16));
+            }
+        }
     }
 }
 
-// Queues the taken edges of a warp in the block's queue (a full queue: straight to chunks).
+// The rare push of edges that did not fit the queue, kept out of the callers' code.
+__device__ __noinline__ void push_overflow(const ListParams& P, ListShared& S, uint32_t e, bool take, uint32_t rr,
+                                           uint32_t k, uint32_t slot, uint32_t parity) {
+    push_lists(P, S, e, take, 0, take ? kNotLoaded : 0u, rr, k, slot, parity);
+}
+
+// Queues the taken edges of a warp, to be removed in round rr, in the block's queue (a full queue:
+// straight to chunks).
 __device__ __forceinline__ void enqueue(const ListParams& P, ListShared& S, uint32_t e, bool take, uint32_t rr,
                                         uint32_t k, uint32_t slot, uint32_t parity) {
     const uint32_t mt = __ballot_sync(kFullMask, take);
@@ -172,9 +207,41 @@ __device__ __forceinline__ void enqueue(const ListParams& P, ListShared& S, uint
     if (lane_id() == 0) base = atomicAdd(&S.queued, __popc(mt));
     base = __shfl_sync(kFullMask, base, 0);
     const uint32_t pos = base + __popc(mt & lanemask_lt());
-    const bool fits = pos < kQueue;
-    if (take && fits) S.queue[pos] = e;
-    if (base + __popc(mt) > kQueue) push_lists(P, S, e, take && !fits, rr, k, slot, parity);
+    if (take && pos < kQueue) {
+        S.queue[pos] = e;
+        if (pos < kAhead) S.len[pos] = kNotLoaded;
+    }
+    if (base + __popc(mt) > kQueue) push_overflow(P, S, e, take && pos >= kQueue, rr, k, slot, parity);
+}
+
+// The same for two edges a lane, with the list bounds of the first kAhead queue entries.
+__device__ __forceinline__ void enqueue_two(const ListParams& P, ListShared& S, uint2 e, bool qf, bool qg, uint32_t rr,
+                                            uint32_t k, uint32_t slot, uint32_t parity, uint64_t f0, uint32_t flen,
+                                            uint64_t g0, uint32_t glen) {
+    const uint32_t mf = __ballot_sync(kFullMask, qf), mg = __ballot_sync(kFullMask, qg);
+    if (!(mf | mg)) return;
+    uint32_t base = 0;
+    if (lane_id() == 0) base = atomicAdd(&S.queued, __popc(mf) + __popc(mg));
+    base = __shfl_sync(kFullMask, base, 0);
+    const uint32_t pf = base + __popc(mf & lanemask_lt()), pg = base + __popc(mf) + __popc(mg & lanemask_lt());
+    if (qf && pf < kQueue) {
+        S.queue[pf] = e.x;
+        if (pf < kAhead) {
+            S.start[pf] = f0;
+            S.len[pf] = flen;
+        }
+    }
+    if (qg && pg < kQueue) {
+        S.queue[pg] = e.y;
+        if (pg < kAhead) {
+            S.start[pg] = g0;
+            S.len[pg] = glen;
+        }
+    }
+    if (base + __popc(mf) + __popc(mg) > kQueue) {
+        push_overflow(P, S, e.x, qf && pf >= kQueue, rr, k, slot, parity);
+        push_overflow(P, S, e.y, qg && pg >= kQueue, rr, k, slot, parity);
+    }
 }
 
 // The block's queue becomes chunks of the next round.  Called by the whole block after a
@@ -182,47 +249,57 @@ __device__ __forceinline__ void enqueue(const ListParams& P, ListShared& S, uint
 __device__ __forceinline__ void flush(const ListParams& P, ListShared& S, uint32_t rr, uint32_t k, uint32_t slot,
                                       uint32_t parity) {
     const uint32_t n = min(S.queued, kQueue);
+#pragma unroll 1
     for (uint32_t b = threadIdx.x & ~31u; b < n; b += blockDim.x) {
         const uint32_t i = b + lane_id();
-        push_lists(P, S, i < n ? S.queue[i] : 0u, i < n, rr, k, slot, parity);
+        uint32_t e = 0, len = 0;
+        uint64_t t0 = 0;
+        if (i < n) {
+            e = S.queue[i];
+            len = i < kAhead ? S.len[i] : kNotLoaded;
+            if (i < kAhead) t0 = S.start[i];
+        }
+        push_lists(P, S, e, i < n, t0, len, rr, k, slot, parity);
     }
 }
 
-// Grid barrier `epoch` (counted from 0): the block's queued edges are added to the arrival word of
-// the epoch's parity together with its arrival.  Two words, so that a word read after its barrier
-// completed stays still until every block has read it and arrived at the next barrier.  Bounded
-// like grid_barrier.  Delivers the phase's frontier in S.front.
-__device__ __forceinline__ bool list_barrier(const ListParams& P, ListShared& S, uint32_t epoch, uint64_t wait_ns) {
+// Grid barrier `epoch` (counted from 0) on ring slot epoch & 3, which was zero when the epoch
+// began: the block's queued edges are added to the slot's first word together with its arrival.
+// Bounded like grid_barrier (`units`: the work it covers).  Delivers the phase's frontier in S.front (kScan: and the minima).
+template <bool kScan>
+__device__ __forceinline__ bool list_barrier(const ListParams& P, ListShared& S, uint32_t epoch, uint64_t units) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned long long* word = reinterpret_cast<unsigned long long*>(P.ctrl + kLBar) + (epoch & 1);
-        const unsigned long long add = 1ull << 32 | S.queued;
-        const uint32_t target = S.bar_arrivals[epoch & 1] + gridDim.x;
-        unsigned long long v = atom_add_acq_rel_u64(word, add) + add;
-        uint32_t ok = 1;
-        if ((uint32_t)(v >> 32) != target) {
-            const uint64_t t0 = global_ns();
-            uint32_t spins = 0;
-            while ((uint32_t)((v = ld_acquire_u64(word)) >> 32) != target) {
-                if ((++spins & 31u) == 0) {
-                    if (ld_acquire(P.ctrl + kCtrlError) & kErrTimeout) { ok = 0; break; }
-                    if (global_ns() - t0 > wait_ns) {
-                        atomicOr(P.ctrl + kCtrlError, kErrTimeout);
-                        ok = 0;
-                        break;
-                    }
-                    if (spins > 256) __nanosleep(64);
+        uint32_t* slot = P.ctrl + kLRing + kLSlotWords * (epoch & 3);
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(slot), "l"(1ull << 32 | S.queued) : "memory");
+        uint64_t bar, chunks, t0 = 0;
+        uint32_t ok = 1, spins = 0;
+        for (;;) {
+            // one 16-byte access: the count of chunks is final once every block has arrived
+            asm volatile(
+                "{\n\t.reg .b128 q;\n\tld.acquire.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+                : "=l"(bar), "=l"(chunks)
+                : "l"(slot)
+                : "memory");
+            if ((uint32_t)(bar >> 32) == gridDim.x) break;
+            if ((++spins & 31u) == 0) {
+                if (spins == 32) t0 = global_ns();
+                if (ld_acquire(P.ctrl + kCtrlError) & kErrTimeout) { ok = 0; break; }
+                if (global_ns() - t0 > P.wait_base_ns + P.wait_ns_per_unit * units) {
+                    atomicOr(P.ctrl + kCtrlError, kErrTimeout);
+                    ok = 0;
+                    break;
                 }
+                if (spins > 256) __nanosleep(64);
             }
         }
-        const uint4 s = __ldcg(reinterpret_cast<const uint4*>(P.ctrl + kLSlot) + (epoch & 3));
-        S.front.min_id = __ldcg(P.ctrl + kLMinId + (epoch & 3));
-        S.front.edges = (uint32_t)v - S.bar_edges[epoch & 1];
-        S.front.chunks = (uint32_t)min((unsigned long long)s.y << 32 | s.x, (unsigned long long)P.cap_chunks);
-        S.front.big = s.z;
-        S.front.min_sup = s.w;
-        S.bar_edges[epoch & 1] = (uint32_t)v;
-        S.bar_arrivals[epoch & 1] = target;
+        S.front.edges = (uint32_t)bar;
+        S.front.chunks = (uint32_t)min(chunks, (uint64_t)P.cap_chunks);
+        S.front.big = chunks > P.cap_chunks ? __ldcg(slot + kLBig) : 0u;
+        if (kScan) {
+            S.front.min_sup = __ldcg(slot + kLMin);
+            S.front.min_id = __ldcg(slot + kLMinId);
+        }
         S.queued = 0;
         S.ok = ok;
     }
@@ -230,23 +307,76 @@ __device__ __forceinline__ bool list_barrier(const ListParams& P, ListShared& S,
     return S.ok != 0;
 }
 
-// One list entry (f, g) of the edge e removed in round r: returns which of the two lose a support
-// and reach k-3.  States seen: 0 alive, `nxt` alive but queued for the next round (its support no
-// longer matters), `cur` removed in this round, anything else removed earlier.
-__device__ __forceinline__ void destroy(const ListParams& P, uint32_t e, uint2 t, bool act, uint32_t cur, uint32_t nxt,
-                                        uint32_t km2, bool* qf, bool* qg) {
-    *qf = *qg = false;
-    if (act) {
-        const uint32_t sf = __ldcg(P.st + t.x), sg = __ldcg(P.st + t.y);
-        const bool okf = sf == 0 || sf == nxt || (sf == cur && e < t.x);
-        const bool okg = sg == 0 || sg == nxt || (sg == cur && e < t.y);
+// N list entries t = (f, g) a lane of edges e removed in round r: the two edges that survive it lose
+// a support; those that reach k-3 are removed in the next round.  States seen: 0 alive, `nxt` alive
+// but queued for the next round (its support no longer matters), `cur` removed in this round,
+// anything else removed earlier.  With kAheadLoads the list bounds of f and g are loaded while their
+// decrements are under way (for rounds bound by latency).
+template <int N, bool kAheadLoads>
+__device__ __forceinline__ void destroy(const ListParams& P, ListShared& S, const uint32_t (&e)[N], const uint2 (&t)[N],
+                                        const bool (&act)[N], uint32_t cur, uint32_t nxt, uint32_t r, uint32_t k,
+                                        uint32_t slot, uint32_t parity) {
+    uint32_t sf[N], sg[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        sf[i] = act[i] ? __ldcg(P.st + t[i].x) : kOld;
+        sg[i] = act[i] ? __ldcg(P.st + t[i].y) : kOld;
+    }
+    uint32_t of[N], og[N];
+    uint64_t f0[N], f1[N], g0[N], g1[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        of[i] = og[i] = 0;
+        f0[i] = g0[i] = 0;
+        f1[i] = g1[i] = kNotLoaded;
+        const bool okf = sf[i] == 0 || sf[i] == nxt || (sf[i] == cur && e[i] < t[i].x);
+        const bool okg = sg[i] == 0 || sg[i] == nxt || (sg[i] == cur && e[i] < t[i].y);
         if (okf && okg) {
-            uint32_t of = 0, og = 0;
-            if (sf == 0) of = atomicSub(&P.sup[t.x], 1u);
-            if (sg == 0) og = atomicSub(&P.sup[t.y], 1u);
-            *qf = of == km2;
-            *qg = og == km2;
+            if (sf[i] == 0) {
+                of[i] = atomicSub(&P.sup[t[i].x], 1u);
+                if (kAheadLoads) {
+                    f0[i] = __ldg(P.tptr + t[i].x);
+                    f1[i] = __ldg(P.tptr + t[i].x + 1);
+                }
+            }
+            if (sg[i] == 0) {
+                og[i] = atomicSub(&P.sup[t[i].y], 1u);
+                if (kAheadLoads) {
+                    g0[i] = __ldg(P.tptr + t[i].y);
+                    g1[i] = __ldg(P.tptr + t[i].y + 1);
+                }
+            }
         }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        enqueue_two(P, S, t[i], of[i] == k - 2, og[i] == k - 2, r + 1, k, slot, parity, f0[i],
+                    (uint32_t)(f1[i] - f0[i]), g0[i], (uint32_t)(g1[i] - g0[i]));
+}
+
+// N of the chunks c, c + step, ... < C a warp at once.
+template <int N>
+__device__ __forceinline__ void whole_chunks(const ListParams& P, ListShared& S, const uint4* __restrict__ ch,
+                                             uint32_t C, uint32_t first, uint32_t step, uint32_t cur, uint32_t nxt,
+                                             uint32_t r, uint32_t k, uint32_t slot, uint32_t parity) {
+    const uint32_t lane = lane_id();
+#pragma unroll 1
+    for (uint32_t c = first; c < C; c += N * step) {
+        uint4 d[N];
+        uint32_t e[N];
+        uint2 t[N];
+        bool act[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            d[i] = i == 0 || c + i * step < C ? __ldcg(ch + c + i * step) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            e[i] = d[i].x;
+            act[i] = lane < d[i].w;
+            t[i] = make_uint2(0, 0);
+            if (act[i]) t[i] = __ldcs(P.tri + ((uint64_t)d[i].z << 32 | d[i].y) + lane);
+        }
+        destroy<N, true>(P, S, e, t, act, cur, nxt, r, k, slot, parity);
     }
 }
 
@@ -254,24 +384,22 @@ __device__ __forceinline__ void destroy(const ListParams& P, uint32_t e, uint2 t
 __device__ __forceinline__ void run_chunks(const ListParams& P, ListShared& S, const uint4* __restrict__ ch, uint32_t C,
                                            uint32_t gw, uint32_t nw, uint32_t r, uint32_t k, uint32_t slot,
                                            uint32_t parity) {
-    const uint32_t lane = lane_id(), cur = stamp_of(r), nxt = stamp_of(r + 1), km2 = k - 2;
-    bool qf, qg;
-    if (C <= 4 * nw) {
-        // few chunks: one at a time, for the shortest chain
-        for (uint32_t c = gw; c < C; c += nw) {
-            const uint4 d = __ldcg(ch + c);
-            const bool act = lane < d.w;
-            uint2 t = make_uint2(0, 0);
-            if (act) t = __ldcs(P.tri + ((uint64_t)d.z << 32 | d.y) + lane);
-            destroy(P, d.x, t, act, cur, nxt, km2, &qf, &qg);
-            enqueue(P, S, t.x, qf, r + 1, k, slot, parity);
-            enqueue(P, S, t.y, qg, r + 1, k, slot, parity);
-        }
+    const uint32_t lane = lane_id(), cur = stamp_of(r), nxt = stamp_of(r + 1);
+    if (C <= nw) {
+        // a chunk a warp: the shortest chain
+        whole_chunks<1>(P, S, ch, C, gw, nw, cur, nxt, r, k, slot, parity);
         return;
     }
-    // many chunks: 32 (or the warp's share) at a time, their entries flattened over the lanes, the
-    // next step's entries loaded before the current step's are used
+    if (C <= 4 * nw) {
+        whole_chunks<2>(P, S, ch, C, gw, nw, cur, nxt, r, k, slot, parity);
+        return;
+    }
+    // many chunks: 32 (or the warp's share) at a time, their entries flattened over the lanes, kFlat
+    // entries a lane under way at once (R-MAT 22 peel kernel: 84.7 ms with one, 74.7 with two, 67.8
+    // with four, 69.4 with eight, which spills)
+    constexpr int kFlat = 4;
     const uint32_t D = min(32u, (C + nw - 1) / nw);
+#pragma unroll 1
     for (uint64_t c0 = (uint64_t)gw * D; c0 < C; c0 += (uint64_t)nw * D) {
         uint4 d = make_uint4(0, 0, 0, 0);
         if (lane < D && c0 + lane < C) d = __ldcg(ch + c0 + lane);
@@ -285,61 +413,62 @@ __device__ __forceinline__ void run_chunks(const ListParams& P, ListShared& S, c
         // position of flattened entry i of chunk `own`: p_own + i with p_own = start - prefix
         const uint64_t p0 = ((uint64_t)d.z << 32 | d.y) - (incl - d.w);
         const uint32_t plo = (uint32_t)p0, phi = (uint32_t)(p0 >> 32);
-        uint32_t e_next = 0;
-        uint2 t_next = make_uint2(0, 0);
-        bool a_next = false;
-        auto fetch = [&](uint32_t i) {
-            uint32_t own = 0;
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < total; i0 += 32 * kFlat) {
+            uint32_t e[kFlat];
+            uint2 t[kFlat];
+            bool act[kFlat];
 #pragma unroll
-            for (uint32_t s = 16; s > 0; s >>= 1) {
-                const uint32_t v = __shfl_sync(kFullMask, incl, own + s - 1);
-                if (v <= i) own += s;
+            for (int q = 0; q < kFlat; ++q) {
+                const uint32_t i = i0 + 32 * q + lane;
+                uint32_t own = 0;
+#pragma unroll
+                for (uint32_t s = 16; s > 0; s >>= 1) {
+                    const uint32_t v = __shfl_sync(kFullMask, incl, own + s - 1);
+                    if (v <= i) own += s;
+                }
+                own &= 31u;
+                e[q] = __shfl_sync(kFullMask, d.x, own);
+                const uint64_t p =
+                    ((uint64_t)__shfl_sync(kFullMask, phi, own) << 32 | __shfl_sync(kFullMask, plo, own)) + i;
+                act[q] = i < total;
+                t[q] = make_uint2(0, 0);
+                if (act[q]) t[q] = __ldcs(P.tri + p);
             }
-            own &= 31u;
-            e_next = __shfl_sync(kFullMask, d.x, own);
-            const uint64_t p = ((uint64_t)__shfl_sync(kFullMask, phi, own) << 32 | __shfl_sync(kFullMask, plo, own)) + i;
-            a_next = i < total;
-            if (a_next) t_next = __ldcs(P.tri + p);
-        };
-        fetch(lane);
-        for (uint32_t i0 = 0; i0 < total; i0 += 32) {
-            const uint32_t e = e_next;
-            const uint2 t = t_next;
-            const bool act = a_next;
-            if (i0 + 32 < total) fetch(i0 + 32 + lane);
-            destroy(P, e, t, act, cur, nxt, km2, &qf, &qg);
-            enqueue(P, S, t.x, qf, r + 1, k, slot, parity);
-            enqueue(P, S, t.y, qg, r + 1, k, slot, parity);
+            destroy<kFlat, false>(P, S, e, t, act, cur, nxt, r, k, slot, parity);
         }
     }
 }
 
-__global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
+__global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_constant__ ListParams P) {
     __shared__ ListShared S;
     uint32_t* ctrl = P.ctrl;
     const uint32_t lane = lane_id();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nthreads = gridDim.x * blockDim.x;
-    const uint32_t gwarp = tid >> 5, nwarps = nthreads >> 5;
+    // chunks go to the blocks in turn: few chunks do not crowd on few SMs (R-MAT 16: peel kernel
+    // 4.96 -> 4.29 ms)
+    const uint32_t nwarps = nthreads >> 5, gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     // the clock and the logs belong to a thread that is not the barrier's
     const bool scribe = blockIdx.x == 0 && threadIdx.x == blockDim.x - 1;
     if (threadIdx.x == 0) {
         S.queued = 0;
-        S.bar_edges[0] = S.bar_edges[1] = S.bar_arrivals[0] = S.bar_arrivals[1] = 0;
         S.min_sup = S.min_id = kDead;
         S.walk = 0;
+        S.walked = 0;
     }
     if (scribe) {
         for (int i = 0; i < 6; ++i) S.ns[i] = 0;
         S.ns[6] = global_ns();
     }
     __syncthreads();
-    // ring slot s of the phase that barrier `epoch` closes is s = epoch & 3; slot (epoch + 2) & 3
-    // is cleared meanwhile (its last readers arrived at barrier epoch - 1)
+    // the phase that barrier `epoch` closes uses ring slot epoch & 3; slot (epoch + 2) & 3 is cleared
+    // meanwhile (its last readers arrived at barrier epoch - 1)
     auto clear_slot = [&](uint32_t epoch) {
         if (scribe) {
-            *reinterpret_cast<uint4*>(ctrl + kLSlot + 4 * (epoch & 3)) = make_uint4(0, 0, 0, kDead);
-            ctrl[kLMinId + (epoch & 3)] = kDead;
+            uint4* slot = reinterpret_cast<uint4*>(ctrl + kLRing + kLSlotWords * (epoch & 3));
+            slot[0] = make_uint4(0, 0, 0, 0);
+            slot[1] = make_uint4(0, kDead, kDead, 0);
         }
     };
     auto phase = [&](int kind) {
@@ -349,22 +478,27 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
             S.ns[6] = now;
         }
     };
-    const uint64_t phase_wait = P.wait_base_ns + P.wait_ns_per_unit * 2ull * P.m;
+    const uint64_t phase_units = 2ull * P.m;  // work that a level phase's barrier covers
     uint32_t epoch = 0, parity = 0;  // parity: the chunk buffer the next frontier is written to
     clear_slot(1);
     clear_slot(2);
     {
         uint4* st4 = reinterpret_cast<uint4*>(P.st);
         const uint64_t n16 = ((uint64_t)P.m + 15) / 16;
+#pragma unroll 1
         for (uint64_t i = tid; i < n16; i += nthreads) st4[i] = make_uint4(0, 0, 0, 0);
     }
-    if (!list_barrier(P, S, epoch, phase_wait)) return;
+    if (!list_barrier<false>(P, S, epoch, phase_units)) return;
     phase(0);
     ++epoch;
 
     uint32_t r = 0, level = 0, k_last = 2, live = P.m, start = 0, swept = 0;
     while (live) {
         if (scribe) S.ns[7] = S.ns[6];
+        if (threadIdx.x == 0) {
+            S.walked += S.walk;
+            S.walk = 0;
+        }
         // level start: stream the supports (removed edges have the top bit) from the smallest id
         // alive at the last scan; collect the frontier of level k_last+1 and the minimum support
         uint32_t k = k_last + 1;
@@ -374,6 +508,7 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
             const uint4* sup4 = reinterpret_cast<const uint4*>(P.sup);
             const uint64_t m4 = ((uint64_t)P.m + 3) / 4;
             constexpr int kScan = 2;  // 16-byte loads in flight per lane
+#pragma unroll 1
             for (uint64_t i0 = (start >> 2) + tid - lane; i0 < m4; i0 += (uint64_t)nthreads * kScan) {
                 uint4 q4[kScan];
 #pragma unroll
@@ -384,16 +519,23 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
 #pragma unroll
                 for (int u = 0; u < kScan; ++u) {
                     const uint64_t i = i0 + (uint64_t)u * nthreads + lane;
-                    const uint32_t sv[4] = {q4[u].x, q4[u].y, q4[u].z, q4[u].w};
+                    uint32_t sv[4] = {q4[u].x, q4[u].y, q4[u].z, q4[u].w};
+                    bool low = false;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const uint64_t j = 4 * i + c;
-                        const uint32_t sj = j < P.m ? sv[c] : kDead;
-                        if (sj < 0x80000000u) {
-                            mn = min(mn, sj);
+                        if (j >= P.m) sv[c] = kDead;
+                        if (sv[c] < 0x80000000u) {
+                            mn = min(mn, sv[c]);
                             mid = min(mid, (uint32_t)j);
                         }
-                        enqueue(P, S, (uint32_t)j, sj <= k - 3, r + 1, k, epoch & 3, parity);
+                        low = low || sv[c] <= k - 3;
+                    }
+                    if (!__any_sync(kFullMask, low)) continue;
+#pragma unroll 1
+                    for (uint32_t c = 0; c < 4; ++c) {
+                        const uint32_t sj = c == 0 ? sv[0] : c == 1 ? sv[1] : c == 2 ? sv[2] : sv[3];
+                        enqueue(P, S, (uint32_t)(4 * i) + c, sj <= k - 3, r + 1, k, epoch & 3, parity);
                     }
                 }
             }
@@ -405,13 +547,14 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
             }
             __syncthreads();
             if (threadIdx.x == 0 && S.min_id != kDead) {
-                atomicMin(ctrl + kLSlot + 4 * (epoch & 3) + 3, S.min_sup);
-                atomicMin(ctrl + kLMinId + (epoch & 3), S.min_id);
+                uint32_t* slot = ctrl + kLRing + kLSlotWords * (epoch & 3);
+                atomicMin(slot + kLMin, S.min_sup);
+                atomicMin(slot + kLMinId, S.min_id);
                 S.min_sup = S.min_id = kDead;
             }
             flush(P, S, r + 1, k, epoch & 3, parity);
         }
-        if (!list_barrier(P, S, epoch, phase_wait)) return;
+        if (!list_barrier<true>(P, S, epoch, phase_units)) return;
         phase(1);
         ++epoch;
         start = S.front.min_id;
@@ -419,6 +562,7 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
             // level k_last+1 is empty: the next non-empty level is the minimum support + 3
             k = S.front.min_sup + 3;
             clear_slot(epoch + 2);
+#pragma unroll 1
             for (uint64_t j0 = start + tid - lane; j0 < P.m; j0 += nthreads) {
                 const uint64_t j = j0 + lane;
                 const uint32_t sj = j < P.m ? __ldcg(P.sup + j) : kDead;
@@ -426,7 +570,7 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
             }
             __syncthreads();
             flush(P, S, r + 1, k, epoch & 3, parity);
-            if (!list_barrier(P, S, epoch, phase_wait)) return;
+            if (!list_barrier<false>(P, S, epoch, phase_units)) return;
             phase(2);
             ++epoch;
         }
@@ -450,7 +594,7 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
                 S.ns[8] = S.ns[6];
             }
             const uint32_t from = parity;
-            if (E == live || (C == 0 && B == 0)) {
+            if (E == live || k == 3) {
                 // nothing left to decrement, or nothing to walk: the round is done
                 live -= E;
                 if (log) P.round_ns[r] = 0;
@@ -462,37 +606,34 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
                 // old stamps become 255 before they could be taken for this or the next round's
                 const uint32_t keep = stamp_of(r);
                 clear_slot(epoch + 2);
+#pragma unroll 1
                 for (uint64_t i = tid; i < P.m; i += nthreads) {
                     const uint32_t s = __ldcg(P.st + i);
                     if (s != 0 && s != keep && s != kOld) P.st[i] = (uint8_t)kOld;
                 }
-                if (!list_barrier(P, S, epoch, phase_wait)) return;
+                if (!list_barrier<false>(P, S, epoch, phase_units)) return;
                 phase(4);
                 ++epoch;
                 swept = r - 1;
             }
             clear_slot(epoch + 2);
-            const uint64_t round_wait =
-                P.wait_base_ns + P.wait_ns_per_unit * ((uint64_t)C * kChunk + (B ? 2ull * P.m : 0ull));
             run_chunks(P, S, P.ch[from], C, gwarp, nwarps, r, k, epoch & 3, parity);
             // edges whose chunks did not fit the buffer: one warp per edge
+#pragma unroll 1
             for (uint32_t i = gwarp; i < B; i += nwarps) {
                 const uint32_t e = __ldcg(P.big[from] + i);
                 const uint64_t t0 = P.tptr[e], t1 = P.tptr[e + 1];
-                const uint32_t cur = stamp_of(r), nxt = stamp_of(r + 1);
+#pragma unroll 1
                 for (uint64_t p0 = t0; p0 < t1; p0 += 32) {
-                    const bool act = p0 + lane < t1;
-                    uint2 t = make_uint2(0, 0);
-                    if (act) t = __ldcs(P.tri + p0 + lane);
-                    bool qf, qg;
-                    destroy(P, e, t, act, cur, nxt, k - 2, &qf, &qg);
-                    enqueue(P, S, t.x, qf, r + 1, k, epoch & 3, parity);
-                    enqueue(P, S, t.y, qg, r + 1, k, epoch & 3, parity);
+                    const uint32_t ea[1] = {e};
+                    const bool act[1] = {p0 + lane < t1};
+                    const uint2 t[1] = {act[0] ? __ldcs(P.tri + p0 + lane) : make_uint2(0, 0)};
+                    destroy<1, false>(P, S, ea, t, act, stamp_of(r), stamp_of(r + 1), r, k, epoch & 3, parity);
                 }
             }
             __syncthreads();
             flush(P, S, r + 1, k, epoch & 3, parity);
-            if (!list_barrier(P, S, epoch, round_wait)) return;
+            if (!list_barrier<false>(P, S, epoch, (uint64_t)C * kChunk + (B ? phase_units : 0ull))) return;
             phase(5);
             ++epoch;
             if (log) P.round_ns[r] = (uint32_t)(S.ns[6] - S.ns[8]);
@@ -505,7 +646,8 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(ListParams P) {
         k_last = k;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && S.walk) atomicAdd(reinterpret_cast<unsigned long long*>(ctrl + kPWalk), S.walk);
+    if (threadIdx.x == 0 && S.walked + S.walk)
+        atomicAdd(reinterpret_cast<unsigned long long*>(ctrl + kPWalk), S.walked + S.walk);
     if (scribe) {
         ctrl[kPKmax] = k_last - 1;
         ctrl[kPRounds] = r;
