@@ -4,12 +4,18 @@
 // every adjacency list on the CPU between two PCIe copies; here everything stays in HBM:
 //
 //   1. degree histogram of the input entries (with id, self-loop checks);
-//   2. vertex rank = position in ascending (degree, id) order (radix sort of n keys);
+//   2. vertex rank = position in ascending (degree, id) order: a stable radix sort of the ids by the
+//      digits of their degrees; ranks, row lengths and row starts in one scan (k_rank_rows);
 //   3. every entry becomes the key (rank[src] << vb | rank[dst]) carrying its entry index;
 //      one radix sort of the 2m keys yields the symmetric CSR with rows sorted by rank;
 //   4. each row splits at its own rank: the part above it is the row of the degree-oriented
-//      CSR (edge id = position in the oriented array); the part below gets its edge id by a
-//      binary search in the neighbour's oriented row, which also proves the input symmetric.
+//      CSR (edge id = position in the oriented array), numbered by a scan of the sorted entries
+//      that writes both CSRs at once (k_csr); the part below gets its edge id by a binary search in
+//      the neighbour's oriented row, which also proves the input symmetric (k_entry_eid).
+//
+// Scans and radix passes are one kernel each (kt_look.cuh).  A small graph's build is bound by its
+// launches: G(4096, 16/4095) takes 17 instead of 43, 0.098 ms instead of 0.238; R-MAT 16 0.26 instead of
+// 0.42 ms, R-MAT 20 2.9 instead of 3.05 ms (the sort's five passes 1.6 ms of it).
 //
 // Layout in HBM (n vertices, m undirected edges, all uint32):
 //   s_ptr[n+1], s_len[n], s_split[n]   symmetric rows (lower ranks, then higher ranks)
@@ -17,8 +23,10 @@
 //   o_ptr[n+1], o_col[m], e_src[m]     oriented CSR/COO; edge id = index
 //   sorted_entry[2m]                   input entry index of each symmetric entry
 
-#include "kt_device.cuh"
+#include <algorithm>
+
 #include "kt_engine.h"
+#include "kt_look.cuh"
 
 namespace kt {
 
@@ -55,164 +63,228 @@ __global__ void k_degree(const uint32_t* __restrict__ src, const uint32_t* __res
     if (err && lane_id() == 0) atomicOr(&ctrl[kCtrlError], err);
 }
 
-__global__ void k_rank_keys(const uint32_t* __restrict__ deg, uint32_t n, unsigned vb, uint64_t* __restrict__ keys) {
-    uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) keys[v] = ((uint64_t)deg[v] << vb) | v;
+// Rank keys (degree << vb | id), listed by id: the sort is stable, so it needs the degree's digits
+// only.  A simple graph's degrees are below n; a degree that is not (the input has duplicates and
+// will be refused) is sorted by its low digits.
+__global__ void __launch_bounds__(kThreads) k_rank_keys(const uint32_t* __restrict__ deg, uint32_t n, unsigned vb,
+                                                        unsigned passes, uint64_t* __restrict__ keys,
+                                                        uint32_t* __restrict__ counts) {
+    __shared__ uint32_t h[4 * 256];
+    digit_counts_clear(h, passes);
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kThreads; v0 < n; v0 += (uint64_t)gridDim.x * kThreads) {
+        const uint64_t v = v0 + threadIdx.x;
+        const uint64_t d = v < n ? deg[v] : 0u;
+        if (v < n) keys[v] = d << vb | v;
+        digit_counts_add(h, d, v < n, passes);
+    }
+    digit_counts_flush(h, passes, counts);
 }
 
-// Orientation by vertex id (KT_DIRECTED_BY_INDEX, graph.cu:194-207 without the relabel of
-// kernel.cu:13-20): rank[v] = v; row_len[v] = degree.
-__global__ void k_rank_identity(const uint32_t* __restrict__ deg, uint32_t n, uint32_t* __restrict__ rank,
-                                uint32_t* __restrict__ row_len) {
-    uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) {
-        rank[v] = v;
-        row_len[v] = deg[v];
-    } else if (v == n) {
-        row_len[n] = 0;
+// Ranks and row starts in one pass over the sorted rank keys: rank[v] = sorted position p (or v, when
+// orienting by vertex id, KT_DIRECTED_BY_INDEX, graph.cu:194-207 without the relabel of
+// kernel.cu:13-20), row lengths, and their exclusive scan.  Empty rows get their split and oriented
+// start here (by degree they come first), the marks of the first long and first not tiny row too.
+template <bool kByIndex>
+__global__ void __launch_bounds__(kScanThreads) k_rank_rows(const uint64_t* __restrict__ sorted,
+                                                            const uint32_t* __restrict__ deg, uint32_t n, unsigned vb,
+                                                            uint32_t* __restrict__ rank, uint32_t* __restrict__ s_len,
+                                                            uint32_t* __restrict__ s_ptr,
+                                                            uint32_t* __restrict__ s_split,
+                                                            uint32_t* __restrict__ o_ptr, Look L) {
+    __shared__ uint64_t ws[33], s_prefix;
+    __shared__ uint32_t s_tile;
+    const uint32_t tile = look_tile(L, &s_tile);
+    if (tile == kNoTile) return;
+    const uint64_t p0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    const uint64_t mask = (1ull << vb) - 1;
+    uint32_t len[kScanItems];
+    uint64_t sum = 0;
+    uint32_t before = !kByIndex && p0 > 0 && p0 < n ? (uint32_t)(sorted[p0 - 1] >> vb) : 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < kScanItems; ++i) {
+        const uint64_t p = p0 + i;
+        len[i] = 0;
+        if (p < n) {
+            const uint64_t key = kByIndex ? (uint64_t)deg[p] << vb | p : sorted[p];
+            len[i] = (uint32_t)(key >> vb);
+            rank[key & mask] = (uint32_t)p;
+            s_len[p] = len[i];
+            if (kByIndex && p == 0) L.ctrl[kCtrlTinyRow] = 0;  // rows in no order: a warp for each
+            if (!kByIndex) {
+                if (len[i] >= kBigRow && (p == 0 || before < kBigRow)) L.ctrl[kCtrlBigRow] = (uint32_t)p;
+                if (len[i] > kTinyRow && (p == 0 || before <= kTinyRow)) L.ctrl[kCtrlTinyRow] = (uint32_t)p;
+                before = len[i];
+            }
+        }
+        sum += len[i];
+    }
+    uint64_t end;
+    uint64_t at = tile_scan<uint64_t>(L, tile, sum, ws, &s_prefix, &end);
+#pragma unroll
+    for (uint32_t i = 0; i < kScanItems; ++i) {
+        const uint64_t p = p0 + i;
+        if (p < n) {
+            s_ptr[p] = (uint32_t)at;
+            if (len[i] == 0) {
+                s_split[p] = (uint32_t)at;
+                if (!kByIndex) o_ptr[p] = 0;
+            }
+            if (p == n - 1) {
+                s_ptr[n] = (uint32_t)(at + len[i]);
+                if (len[i] == 0 && at == 0) o_ptr[n] = 0;  // no entries at all
+            }
+        }
+        at += len[i];
     }
 }
 
-// rank[v] = sorted position; row_len[rank] = degree (row lengths of the symmetric CSR).
-__global__ void k_rank_scatter(const uint64_t* __restrict__ sorted, uint32_t n, unsigned vb,
-                               uint32_t* __restrict__ rank, uint32_t* __restrict__ row_len) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) {
-        uint64_t key = sorted[p];
-        rank[(uint32_t)(key & ((1ull << vb) - 1))] = p;
-        row_len[p] = (uint32_t)(key >> vb);
-    } else if (p == n) {
-        row_len[n] = 0;
+// Entry keys (rank of the source << vb | rank of the destination) and their digit counts.  An id >= n
+// (already flagged by k_degree; the call fails at the end of the build) is read as vertex 0, so that
+// every kernel up to that check indexes inside its arrays.
+__global__ void __launch_bounds__(kThreads) k_edge_keys(const uint32_t* __restrict__ src,
+                                                        const uint32_t* __restrict__ dst, uint64_t entries, uint32_t n,
+                                                        const uint32_t* __restrict__ rank, unsigned vb, unsigned passes,
+                                                        uint64_t* __restrict__ keys, uint32_t* __restrict__ counts,
+                                                        const uint32_t* __restrict__ ctrl) {
+    __shared__ uint32_t h[kMaxDigitPasses * 256];
+    if (__syncthreads_or(timed_out(ctrl))) return;
+    digit_counts_clear(h, passes);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kThreads; i0 < entries; i0 += (uint64_t)gridDim.x * kThreads) {
+        const uint64_t i = i0 + threadIdx.x;
+        uint64_t key = 0;
+        if (i < entries) {
+            const uint32_t s = src[i], d = dst[i];
+            key = ((uint64_t)rank[s < n ? s : 0] << vb) | rank[d < n ? d : 0];
+            keys[i] = key;
+        }
+        digit_counts_add(h, key, i < entries, passes);
     }
+    digit_counts_flush(h, passes, counts);
 }
 
-// An id >= n (already flagged by k_degree; the call fails at the end of the build) is read as
-// vertex 0, so that every kernel up to that check indexes inside its arrays.
-__global__ void k_edge_keys(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t entries,
-                            uint32_t n, const uint32_t* __restrict__ rank, unsigned vb, uint64_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < entries) {
-        const uint32_t s = src[i], d = dst[i];
-        keys[i] = ((uint64_t)rank[s < n ? s : 0] << vb) | rank[d < n ? d : 0];
-        vals[i] = (uint32_t)i;
+// One pass over the sorted entry keys builds both CSRs: columns, the duplicate check, where each
+// row's higher-rank part starts, and - by a scan of the higher-rank entries - their oriented
+// positions, which are the edge ids.  A row's oriented start is the scan at its first entry.
+__global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
+                                                      uint32_t n, uint32_t m, uint32_t* __restrict__ s_col,
+                                                      uint32_t* __restrict__ s_eid, uint32_t* __restrict__ s_split,
+                                                      uint32_t* __restrict__ o_ptr, uint32_t* __restrict__ o_col,
+                                                      uint32_t* __restrict__ e_src, uint32_t* __restrict__ fence,
+                                                      Look L) {
+    __shared__ FlagSmem S;
+    const uint32_t tile = look_tile(L, &S.tile);
+    if (tile == kNoTile) return;
+    const uint64_t p0 = (uint64_t)tile * kFlagTile + threadIdx.x;
+    const uint64_t mask = (1ull << vb) - 1;
+    const uint32_t warp = threadIdx.x >> 5;
+    uint64_t key[kFlagSteps];
+    uint32_t fwd = 0;  // bit s: the entry of step s is a higher-rank one
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint64_t p = p0 + s * kFlagThreads;
+        key[s] = p < entries ? keys[p] : 0ull;
     }
-}
-
-__global__ void k_split_init(const uint32_t* __restrict__ s_ptr, uint32_t n, uint32_t* __restrict__ s_split,
-                             uint32_t* __restrict__ s_len) {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) {
-        s_split[r] = s_ptr[r + 1];
-        s_len[r] = s_ptr[r + 1] - s_ptr[r];
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const bool f = (uint32_t)(key[s] & mask) > (uint32_t)(key[s] >> vb);
+        fwd |= (uint32_t)f << s;
+        const uint32_t b = __ballot_sync(kFullMask, f);
+        if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
     }
-}
-
-// Neighbour column, duplicate check and the start of each row's higher-rank part.
-__global__ void k_csr_fill(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
-                           const uint32_t* __restrict__ s_ptr, uint32_t* __restrict__ s_col,
-                           uint32_t* __restrict__ s_split, uint32_t* __restrict__ ctrl) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    __syncthreads();
+    flag_sums<true>(S, L, tile);
     uint32_t err = 0;
-    if (p < entries) {
-        const uint64_t mask = (1ull << vb) - 1;
-        uint64_t key = keys[p];
-        uint32_t row = (uint32_t)(key >> vb), col = (uint32_t)(key & mask);
-        s_col[p] = col;
-        uint64_t prev = p > 0 ? keys[p - 1] : ~0ull;
-        if (p > 0 && prev == key) err = kErrDuplicate;
-        if (col > row && (p == s_ptr[row] || (uint32_t)(prev >> vb) != row || (uint32_t)(prev & mask) < row))
-            s_split[row] = (uint32_t)p;
-    }
-    err = __reduce_or_sync(kFullMask, err);
-    if (err && lane_id() == 0) atomicOr(&ctrl[kCtrlError], err);
-}
-
-__global__ void k_out_len(const uint32_t* __restrict__ s_ptr, const uint32_t* __restrict__ s_split, uint32_t n,
-                          uint32_t* __restrict__ out_len) {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n) out_len[r] = s_ptr[r + 1] - s_split[r];
-    else if (r == n) out_len[n] = 0;
-}
-
-// Higher-rank entries become oriented edges; their edge id is their oriented position.
-__global__ void k_orient(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
-                         const uint32_t* __restrict__ s_split, const uint32_t* __restrict__ o_ptr,
-                         uint32_t* __restrict__ o_col, uint32_t* __restrict__ e_src, uint32_t* __restrict__ s_eid,
-                         uint32_t m) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < entries) {
-        uint64_t key = keys[p];
-        uint32_t row = (uint32_t)(key >> vb), col = (uint32_t)(key & ((1ull << vb) - 1));
-        if (col > row) {
-            uint32_t j = o_ptr[row] + (uint32_t)(p - s_split[row]);
-            if (j < m) {
-                o_col[j] = col;
-                e_src[j] = row;
-                s_eid[p] = j;
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint64_t p = p0 + s * kFlagThreads;
+        const bool f = fwd >> s & 1u;
+        const uint64_t j = S.prefix + S.before[s * kFlagWarps + warp] +
+                           __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
+        if (p < entries) {
+            const uint64_t k = key[s];
+            const uint64_t prev = p > 0 ? keys[p - 1] : ~0ull, next = p + 1 < entries ? keys[p + 1] : ~0ull;
+            const uint32_t row = (uint32_t)(k >> vb), col = (uint32_t)(k & mask);
+            const bool first = p == 0 || (uint32_t)(prev >> vb) != row;
+            const bool last = p + 1 == entries || (uint32_t)(next >> vb) != row;
+            s_col[p] = col;
+            if (p > 0 && prev == k) err |= kErrDuplicate;
+            if (first) o_ptr[row] = (uint32_t)(j < m ? j : m);
+            if (f) {
+                if (first || (uint32_t)(prev & mask) < row) s_split[row] = (uint32_t)p;
+                if (j < m) {
+                    o_col[j] = col;
+                    e_src[j] = row;
+                    s_eid[p] = (uint32_t)j;
+                    if ((j & 31) == 0) fence[j >> 5] = col;  // every 32nd oriented column
+                }
+            } else if (last) {
+                s_split[row] = (uint32_t)p + 1;
+            }
+            if (p + 1 == entries) {
+                const uint64_t end = j + f;
+                o_ptr[n] = (uint32_t)(end < m ? end : m);
+                if (end != m) err |= kErrAsymmetric;
             }
         }
     }
+    err = __reduce_or_sync(kFullMask, err);
+    if (err && lane_id() == 0) atomicOr(&L.ctrl[kCtrlError], err);
 }
 
-// fence[f] = o_col[32 f]: the first level of every search in an oriented row (fenced_lower_bound).
-__global__ void k_fences(const uint32_t* __restrict__ o_col, uint32_t m, uint32_t* __restrict__ fence) {
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((uint64_t)f * 32 < m) fence[f] = o_col[(uint64_t)f * 32];
+// Oriented starts of empty rows when orienting by vertex id (by degree they come first, at 0): the
+// start of the next row that has entries.
+__global__ void k_empty_rows(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb, uint32_t n,
+                             const uint32_t* __restrict__ s_ptr, const uint32_t* __restrict__ s_len,
+                             uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ ctrl) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n || s_len[r] || timed_out(ctrl)) return;
+    const uint32_t p = s_ptr[r];
+    o_ptr[r] = p < entries ? o_ptr[(uint32_t)(keys[p] >> vb)] : o_ptr[n];
 }
 
-// Lower-rank entries (row r, column c < r) take the id of edge (c, r) from c's oriented row.
-// The oriented CSR must hold exactly m = entries / 2 edges; an input that is not symmetric can
-// leave rows that do not nest in [0, m): they are flagged, never searched.
-__global__ void k_in_eid(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb, uint32_t n, uint32_t m,
-                         const uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ o_col,
-                         const uint32_t* __restrict__ fence, uint32_t* __restrict__ s_eid,
-                         uint32_t* __restrict__ ctrl) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Edge ids of all entries: higher-rank entries have theirs; lower-rank entries (row r, column c < r)
+// take the id of edge (c, r) from c's oriented row.  Written per sorted entry (compacted while
+// peeling) and per input entry (outputs are gathered by it).  An input that is not symmetric has
+// entries whose edge is not there: flagged.  The supports are cleared on the way.
+__global__ void __launch_bounds__(kThreads) k_entry_eid(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
+                                                        uint32_t m, const uint32_t* __restrict__ o_ptr,
+                                                        const uint32_t* __restrict__ o_col,
+                                                        const uint32_t* __restrict__ fence,
+                                                        const uint32_t* __restrict__ sorted_entry,
+                                                        uint32_t* __restrict__ s_eid, uint32_t* __restrict__ entry_eid,
+                                                        uint32_t* __restrict__ sup, uint32_t* __restrict__ supx,
+                                                        uint32_t* __restrict__ ctrl) {
+    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (__any_sync(kFullMask, timed_out(ctrl))) return;
     uint32_t err = 0;
-    if (p == 0 && o_ptr[n] != m) err = kErrAsymmetric;
+    if (p < m) sup[p] = supx[p] = 0;
     if (p < entries) {
-        uint64_t key = keys[p];
-        uint32_t row = (uint32_t)(key >> vb), col = (uint32_t)(key & ((1ull << vb) - 1));
-        if (col < row) {
+        const uint64_t key = keys[p];
+        const uint32_t row = (uint32_t)(key >> vb), col = (uint32_t)(key & ((1ull << vb) - 1));
+        uint32_t eid = 0;
+        if (col > row) {
+            eid = s_eid[p];
+        } else {
             const uint32_t lo = o_ptr[col], hi = o_ptr[col + 1];
             uint32_t idx = 0xffffffffu;
-            if (lo <= hi && hi <= m) {
-                const uint32_t len = hi - lo;
-                idx = fenced_lower_bound(o_col, fence, lo, hi, row) - lo;
-                if (idx >= len || o_col[lo + idx] != row) idx = 0xffffffffu;
+            if (col < row && lo <= hi && hi <= m) {
+                idx = fenced_lower_bound(o_col, fence, lo, hi, row);
+                if (idx >= hi || o_col[idx] != row) idx = 0xffffffffu;
             }
-            if (idx != 0xffffffffu) s_eid[p] = lo + idx;
-            else { s_eid[p] = 0; err = kErrAsymmetric; }
+            if (idx != 0xffffffffu) eid = idx;
+            else err = kErrAsymmetric;
+            s_eid[p] = eid;
         }
+        entry_eid[sorted_entry[p]] = eid;
     }
     err = __reduce_or_sync(kFullMask, err);
     if (err && lane_id() == 0) atomicOr(&ctrl[kCtrlError], err);
 }
 
-// Edge id of each input entry, kept apart from s_eid because peeling compacts the rows.
-__global__ void k_entry_eid(const uint32_t* __restrict__ sorted_entry, const uint32_t* __restrict__ s_eid,
-                            uint64_t entries, uint32_t* __restrict__ entry_eid) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < entries) entry_eid[sorted_entry[p]] = s_eid[p];
-}
-
-// First rank whose symmetric row has at least `thr` entries (rows grow with rank: ranks are
-// ascending degree), written to ctrl[slot].
-__global__ void k_find_big_row(const uint32_t* __restrict__ s_ptr, uint32_t n, uint32_t thr,
-                               uint32_t* __restrict__ ctrl, uint32_t slot) {
-    uint32_t lo = 0, len = n;
-    while (len > 0) {
-        uint32_t half = len >> 1;
-        uint32_t r = lo + half;
-        if (s_ptr[r + 1] - s_ptr[r] < thr) {
-            lo = r + 1;
-            len -= half + 1;
-        } else {
-            len = half;
-        }
-    }
-    ctrl[slot] = lo;
+// Blocks of a kernel that makes sort keys: four keys a thread at least, at most eight blocks an SM
+// (each adds its digit counts to the global ones).
+uint32_t key_blocks(const kt_engine* e, uint64_t keys) {
+    return (uint32_t)std::min<uint64_t>((keys + 4 * kThreads - 1) / (4 * kThreads), (uint64_t)e->num_sms * 8);
 }
 
 unsigned bits_for(uint64_t n) {
@@ -294,51 +366,95 @@ __global__ void k_tile_ptr(const uint64_t* __restrict__ keys, uint64_t entries, 
 
 // Symmetrize and deduplicate: entry i becomes the undirected key (min << vb | max); ids >= n
 // set kErrBadVertex (key 0, a self loop, dropped).
-__global__ void k_canon_keys(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t entries,
-                             uint32_t n, unsigned vb, uint64_t* __restrict__ keys, uint32_t* __restrict__ ctrl) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kThreads) k_canon_keys(const uint32_t* __restrict__ src,
+                                                         const uint32_t* __restrict__ dst, uint64_t entries, uint32_t n,
+                                                         unsigned vb, unsigned passes, uint64_t* __restrict__ keys,
+                                                         uint32_t* __restrict__ counts, uint32_t* __restrict__ ctrl) {
+    __shared__ uint32_t h[kMaxDigitPasses * 256];
+    digit_counts_clear(h, passes);
     uint32_t err = 0;
-    if (i < entries) {
-        const uint32_t s = src[i], d = dst[i];
-        if (s >= n || d >= n) {
-            err = kErrBadVertex;
-            keys[i] = 0;
-        } else {
-            keys[i] = ((uint64_t)(s < d ? s : d) << vb) | (s < d ? d : s);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kThreads; i0 < entries; i0 += (uint64_t)gridDim.x * kThreads) {
+        const uint64_t i = i0 + threadIdx.x;
+        uint64_t key = 0;
+        if (i < entries) {
+            const uint32_t s = src[i], d = dst[i];
+            if (s >= n || d >= n) err = kErrBadVertex;
+            else key = ((uint64_t)(s < d ? s : d) << vb) | (s < d ? d : s);
+            keys[i] = key;
         }
+        digit_counts_add(h, key, i < entries, passes);
     }
+    digit_counts_flush(h, passes, counts);
     err = __reduce_or_sync(kFullMask, err);
     if (err && lane_id() == 0) atomicOr(&ctrl[kCtrlError], err);
 }
 
-// flag[p] = 1 for the first copy of each sorted key that is not a self loop; flag[entries] = 0.
-__device__ __forceinline__ bool canon_first(const uint64_t* keys, uint64_t p, unsigned vb) {
-    const uint64_t key = keys[p];
-    return (key >> vb) != (key & ((1ull << vb) - 1)) && (p == 0 || keys[p - 1] != key);
+// The first copy of each sorted key that is not a self loop.
+__device__ __forceinline__ bool canon_first(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
+                                            uint64_t p, uint64_t* key) {
+    if (p >= entries) return false;
+    *key = keys[p];
+    return (*key >> vb) != (*key & ((1ull << vb) - 1)) && (p == 0 || keys[p - 1] != *key);
 }
 
-__global__ void k_canon_flags(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
-                              uint32_t* __restrict__ flag) {
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < entries) flag[p] = canon_first(keys, p, vb) ? 1u : 0u;
-    else if (p == entries) flag[p] = 0;
+// Unique edges before each tile, and all of them into the control block.
+__global__ void __launch_bounds__(kFlagThreads) k_canon_count(const uint64_t* __restrict__ keys, uint64_t entries,
+                                                              unsigned vb, uint32_t* __restrict__ tile_start, Look L) {
+    __shared__ FlagSmem S;
+    const uint32_t tile = look_tile(L, &S.tile);
+    if (tile == kNoTile) return;
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        uint64_t key;
+        const bool f =
+            canon_first(keys, entries, vb, (uint64_t)tile * kFlagTile + s * kFlagThreads + threadIdx.x, &key);
+        const uint32_t b = __ballot_sync(kFullMask, f);
+        if (lane_id() == 0) S.before[s * kFlagWarps + (threadIdx.x >> 5)] = __popc(b);
+    }
+    __syncthreads();
+    flag_sums<true>(S, L, tile);
+    if (threadIdx.x == 0) {
+        tile_start[tile] = (uint32_t)S.prefix;
+        if (tile == gridDim.x - 1) L.ctrl[kCtrlTriLo] = (uint32_t)(S.prefix + S.total);
+    }
 }
 
-// Unique edge j (pos[p] after the scan) goes to j as (lo, hi) and to u + j as (hi, lo), where
-// u = pos[entries]; nothing is written unless all 2u entries fit.
-__global__ void k_canon_emit(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
-                             const uint32_t* __restrict__ pos, uint64_t capacity, uint32_t* __restrict__ src_out,
-                             uint32_t* __restrict__ dst_out) {
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t u = pos[entries];
-    if (p >= entries || 2 * u > capacity || !canon_first(keys, p, vb)) return;
-    const uint64_t key = keys[p];
-    const uint32_t lo = (uint32_t)(key >> vb), hi = (uint32_t)(key & ((1ull << vb) - 1));
-    const uint64_t j = pos[p];
-    src_out[j] = lo;
-    dst_out[j] = hi;
-    src_out[u + j] = hi;
-    dst_out[u + j] = lo;
+// Unique edge j goes to j as (lo, hi) and to u + j as (hi, lo), where u is their number; nothing is
+// written unless all 2u entries fit.
+__global__ void __launch_bounds__(kFlagThreads) k_canon_emit(const uint64_t* __restrict__ keys, uint64_t entries,
+                                                             unsigned vb, const uint32_t* __restrict__ tile_start,
+                                                             uint64_t capacity, uint32_t* __restrict__ src_out,
+                                                             uint32_t* __restrict__ dst_out, Look L) {
+    __shared__ FlagSmem S;
+    const uint64_t u = L.ctrl[kCtrlTriLo];
+    if (__syncthreads_or(2 * u > capacity || timed_out(L.ctrl))) return;
+    const uint32_t warp = threadIdx.x >> 5;
+    uint64_t key[kFlagSteps];
+    uint32_t first = 0;
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const bool f = canon_first(keys, entries, vb, (uint64_t)blockIdx.x * kFlagTile + s * kFlagThreads + threadIdx.x,
+                                   &key[s]);
+        first |= (uint32_t)f << s;
+        const uint32_t b = __ballot_sync(kFullMask, f);
+        if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
+    }
+    __syncthreads();
+    flag_sums<false>(S, L, blockIdx.x);
+    const uint32_t start = tile_start[blockIdx.x];
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const bool f = first >> s & 1u;
+        const uint64_t j =
+            start + S.before[s * kFlagWarps + warp] + __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
+        if (f) {
+            const uint32_t lo = (uint32_t)(key[s] >> vb), hi = (uint32_t)(key[s] & ((1ull << vb) - 1));
+            src_out[j] = lo;
+            dst_out[j] = hi;
+            src_out[u + j] = hi;
+            dst_out[u + j] = lo;
+        }
+    }
 }
 
 }  // namespace
@@ -354,28 +470,26 @@ int symmetrize(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
         (rc = reserve(e, n > e->cap_nodes ? n : e->cap_nodes, entries > e->cap_entries ? entries : e->cap_entries)))
         return rc;
     cudaStream_t st = e->stream;
-    const unsigned vb = bits_for(n > 1 ? n : 2);
-    if ((rc = check_cuda(cudaMemsetAsync(e->ctrl, 0, sizeof(uint32_t) * kCtrlWords, st), "clear control block")))
-        return rc;
-    k_canon_keys<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, vb, e->key_a, e->ctrl);
+    const unsigned vb = bits_for(n > 1 ? n : 2), passes = (2 * vb + 7) / 8;
+    if ((rc = begin_session(e, n, 0, look_words(entries)))) return rc;
+    uint32_t* counts = next_counts(e, passes);
+    k_canon_keys<<<key_blocks(e, entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, vb, passes, e->key_a, counts,
+                                                              e->ctrl);
     count_launch(e);
     if ((rc = check_launch(e, "k_canon_keys"))) return rc;
     int in_b = 0;
-    if ((rc = radix_sort(e, e->key_a, nullptr, e->key_b, nullptr, entries, 2 * vb, &in_b))) return rc;
+    if ((rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, entries, 0, passes, counts, &in_b))) return rc;
     const uint64_t* keys = in_b ? e->key_b : e->key_a;
-    // the other key buffer (2 * entries words) holds the flags and, scanned in place, the positions
-    uint32_t* pos = reinterpret_cast<uint32_t*>(in_b ? e->key_a : e->key_b);
-    k_canon_flags<<<grid_for(entries + 1), kThreads, 0, st>>>(keys, entries, vb, pos);
+    uint32_t* tile_start = reinterpret_cast<uint32_t*>(in_b ? e->key_a : e->key_b);  // the sort's other buffer
+    const uint32_t tiles = ceil_div(entries, kFlagTile);
+    k_canon_count<<<tiles, kFlagThreads, 0, st>>>(keys, entries, vb, tile_start, next_look(e));
     count_launch(e);
-    if ((rc = check_launch(e, "k_canon_flags")) || (rc = exclusive_scan(e, pos, pos, entries + 1))) return rc;
-    k_canon_emit<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, pos, capacity, d_src_out, d_dst_out);
+    if ((rc = check_launch(e, "k_canon_count"))) return rc;
+    k_canon_emit<<<tiles, kFlagThreads, 0, st>>>(keys, entries, vb, tile_start, capacity, d_src_out, d_dst_out,
+                                                 next_look(e));
     count_launch(e);
-    if ((rc = check_launch(e, "k_canon_emit"))) return rc;
-    uint32_t u = 0;
-    if ((rc = check_cuda(cudaMemcpyAsync(&u, pos + entries, sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
-                         "read edge count")) ||
-        (rc = sync_and_check(e)))
-        return rc;
+    if ((rc = check_launch(e, "k_canon_emit")) || (rc = sync_and_check(e))) return rc;
+    const uint32_t u = e->h_ctrl[kCtrlTriLo];
     *num_out = 2ull * u;
     if (2ull * u > capacity)
         return fail(KT_ERR_CAPACITY, "symmetrized graph has %llu entries, capacity %llu", 2ull * u,
@@ -398,14 +512,17 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
         (rc = reserve(e, n > e->cap_nodes ? n : e->cap_nodes, entries > e->cap_entries ? entries : e->cap_entries)))
         return rc;
     cudaStream_t st = e->stream;
-    if ((rc = check_cuda(cudaMemsetAsync(e->ctrl, 0, sizeof(uint32_t) * kCtrlWords, st), "clear control block")))
-        return rc;
+    if ((rc = begin_session(e, n, 0, look_words(entries)))) return rc;
     int in_b = 0;
     if (entries) {
         k_tile_keys<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, T, ts, vb, e->key_a, e->ctrl);
         count_launch(e);
         if ((rc = check_launch(e, "k_tile_keys")) || (rc = sync_and_check(e))) return rc;
-        if ((rc = radix_sort(e, e->key_a, nullptr, e->key_b, nullptr, entries, rb + vb, &in_b))) return rc;
+        const unsigned passes = (rb + vb + 7) / 8;
+        uint32_t* counts = next_counts(e, passes);
+        if ((rc = count_digits(e, e->key_a, entries, 0, passes, counts)) ||
+            (rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, entries, 0, passes, counts, &in_b)))
+            return rc;
         k_tile_entries<<<grid_for(entries), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, entries, T, ts, vb,
                                                               d_src_out, d_dst_out);
         count_launch(e);
@@ -414,7 +531,7 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
     k_tile_ptr<<<grid_for(rows + 1), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, entries, vb, rows, d_tile_src_ptr);
     count_launch(e);
     if ((rc = check_launch(e, "k_tile_ptr"))) return rc;
-    return check_cuda(cudaStreamSynchronize(st), "synchronize");
+    return sync_and_check(e);
 }
 
 int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n) {
@@ -432,13 +549,11 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     e->vb = bits_for(n > 1 ? n : 2);
     const unsigned vb = e->vb;
     cudaStream_t st = e->stream;
-    int rc = check_cuda(cudaMemsetAsync(e->ctrl, 0, sizeof(uint32_t) * kCtrlWords, st), "clear control block");
+    int rc = begin_session(e, n, n, std::max(look_words(n), look_words(entries)));
     if (rc) return rc;
     if (n == 0) return entries ? fail(KT_ERR_INVALID_ARG, "entries given for a graph with 0 vertices") : KT_OK;
 
     // 1. degrees (and id / self-loop checks)
-    rc = check_cuda(cudaMemsetAsync(e->deg, 0, sizeof(uint32_t) * n, st), "clear degrees");
-    if (rc) return rc;
     if (entries) {
         k_degree<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, e->deg, e->ctrl);
         count_launch(e);
@@ -447,77 +562,55 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     // (input errors are read back once, at the end of the build: every kernel before that
     // check indexes inside its arrays whatever the input)
 
-    // 2. ranks: ascending (degree, id), or the ids themselves when orienting by index
+    // 2. ranks - ascending (degree, id), or the ids themselves when orienting by index - and the row
+    // starts of the symmetric CSR (row r holds the neighbours of the rank-r vertex)
     int in_b = 0;
     if (e->orient_by_index) {
-        k_rank_identity<<<grid_for((uint64_t)n + 1), kThreads, 0, st>>>(e->deg, n, e->rank, e->s_len);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_rank_identity"))) return rc;
+        k_rank_rows<true><<<ceil_div(n, kScanTile), kScanThreads, 0, st>>>(nullptr, e->deg, n, vb, e->rank, e->s_len,
+                                                                          e->s_ptr, e->s_split, e->o_ptr, next_look(e));
     } else {
-        k_rank_keys<<<grid_for(n), kThreads, 0, st>>>(e->deg, n, vb, e->key_a);
+        const unsigned passes = (vb + 7) / 8;
+        uint32_t* counts = next_counts(e, passes);
+        k_rank_keys<<<key_blocks(e, n), kThreads, 0, st>>>(e->deg, n, vb, passes, e->key_a, counts);
         count_launch(e);
-        if ((rc = check_launch(e, "k_rank_keys"))) return rc;
-        if ((rc = radix_sort(e, e->key_a, nullptr, e->key_b, nullptr, n, vb + bits_for(entries + 2), &in_b)))
+        if ((rc = check_launch(e, "k_rank_keys")) ||
+            (rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, n, vb, passes, counts, &in_b)))
             return rc;
-        k_rank_scatter<<<grid_for((uint64_t)n + 1), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, n, vb, e->rank,
-                                                                       e->s_len);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_rank_scatter"))) return rc;
+        k_rank_rows<false><<<ceil_div(n, kScanTile), kScanThreads, 0, st>>>(in_b ? e->key_b : e->key_a, e->deg, n, vb,
+                                                                           e->rank, e->s_len, e->s_ptr, e->s_split,
+                                                                           e->o_ptr, next_look(e));
     }
-    // row starts of the symmetric CSR (row r holds the neighbours of the rank-r vertex)
-    if ((rc = exclusive_scan(e, e->s_len, e->s_ptr, (uint64_t)n + 1))) return rc;
+    count_launch(e);
+    if ((rc = check_launch(e, "k_rank_rows"))) return rc;
 
-    // 3. sort entries by (rank[src], rank[dst])
+    // 3. sort entries by (rank[src], rank[dst]); 4. both CSRs and the edge ids
     if (entries) {
-        k_edge_keys<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, e->rank, vb, e->key_a,
-                                                            e->val_a);
+        const unsigned passes = (2 * vb + 7) / 8;
+        uint32_t* counts = next_counts(e, passes);
+        k_edge_keys<<<key_blocks(e, entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, e->rank, vb, passes, e->key_a,
+                                                                 counts, e->ctrl);
         count_launch(e);
         if ((rc = check_launch(e, "k_edge_keys"))) return rc;
-        if ((rc = radix_sort(e, e->key_a, e->val_a, e->key_b, e->val_b, entries, 2 * vb, &in_b))) return rc;
-    }
-    const uint64_t* keys = in_b ? e->key_b : e->key_a;
-    e->sorted_entry = in_b ? e->val_b : e->val_a;
-    e->entry_eid = in_b ? e->val_a : e->val_b;  // the sort's other value buffer is free now
-
-    // 4. columns, split points, oriented CSR, edge ids
-    k_split_init<<<grid_for(n), kThreads, 0, st>>>(e->s_ptr, n, e->s_split, e->s_len);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_split_init"))) return rc;
-    if (entries) {
-        k_csr_fill<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, e->s_ptr, e->s_col, e->s_split, e->ctrl);
+        if ((rc = radix_passes(e, e->key_a, e->val_a, e->key_b, e->val_b, entries, 0, passes, counts, &in_b))) return rc;
+        const uint64_t* keys = in_b ? e->key_b : e->key_a;
+        e->sorted_entry = in_b ? e->val_b : e->val_a;
+        e->entry_eid = in_b ? e->val_a : e->val_b;  // the sort's other value buffer is free now
+        k_csr<<<ceil_div(entries, kFlagTile), kFlagThreads, 0, st>>>(keys, entries, vb, n, e->m, e->s_col, e->s_eid,
+                                                                    e->s_split, e->o_ptr, e->o_col, e->e_src,
+                                                                    e->o_fence, next_look(e));
         count_launch(e);
-        if ((rc = check_launch(e, "k_csr_fill"))) return rc;
-    }
-    k_out_len<<<grid_for((uint64_t)n + 1), kThreads, 0, st>>>(e->s_ptr, e->s_split, n, e->o_ptr);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_out_len"))) return rc;
-    if ((rc = exclusive_scan(e, e->o_ptr, e->o_ptr, (uint64_t)n + 1))) return rc;
-    if (entries) {
-        k_orient<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, e->s_split, e->o_ptr, e->o_col, e->e_src,
-                                                         e->s_eid, e->m);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_orient"))) return rc;
-    }
-    if (e->m) {
-        k_fences<<<grid_for((e->m + 31) / 32), kThreads, 0, st>>>(e->o_col, e->m, e->o_fence);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_fences"))) return rc;
-    }
-    if (entries) {
-        k_in_eid<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, n, e->m, e->o_ptr, e->o_col, e->o_fence,
-                                                         e->s_eid, e->ctrl);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_in_eid"))) return rc;
-        k_entry_eid<<<grid_for(entries), kThreads, 0, st>>>(e->sorted_entry, e->s_eid, entries, e->entry_eid);
+        if ((rc = check_launch(e, "k_csr"))) return rc;
+        if (e->orient_by_index) {
+            k_empty_rows<<<grid_for(n), kThreads, 0, st>>>(keys, entries, vb, n, e->s_ptr, e->s_len, e->o_ptr, e->ctrl);
+            count_launch(e);
+            if ((rc = check_launch(e, "k_empty_rows"))) return rc;
+        }
+        k_entry_eid<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, e->m, e->o_ptr, e->o_col, e->o_fence,
+                                                            e->sorted_entry, e->s_eid, e->entry_eid, e->sup, e->rnd,
+                                                            e->ctrl);
         count_launch(e);
         if ((rc = check_launch(e, "k_entry_eid"))) return rc;
     }
-    k_find_big_row<<<1, 1, 0, st>>>(e->s_ptr, n, kBigRow, e->ctrl, kCtrlBigRow);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_find_big_row"))) return rc;
-    k_find_big_row<<<1, 1, 0, st>>>(e->s_ptr, n, kTinyRow + 1, e->ctrl, kCtrlTinyRow);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_find_big_row"))) return rc;
     if (e->trusted) return KT_OK;  // same input: big_row and tiny_row as read before
     if ((rc = sync_and_check(e))) return rc;
     e->big_row = e->h_ctrl[kCtrlBigRow];

@@ -47,10 +47,8 @@ struct Carver {
 size_t carve(kt_engine* e, char* base, uint32_t n, uint64_t N, bool staging) {
     const uint64_t m = N / 2 + 1;
     const uint64_t keys = std::max<uint64_t>(N, n);
-    const uint64_t sort_blocks = (keys + 2047) / 2048;
-    const uint64_t hist_words = 256 * sort_blocks;
-    const uint64_t scan_max = std::max<uint64_t>(std::max<uint64_t>((uint64_t)n, N) + 1, hist_words);
-    const uint64_t scan_words = scan_max / 4096 + 4096;
+    // look-back words for sorts of any size up to the capacity
+    const uint64_t look_cap = std::max(look_words(keys), look_words(std::min(keys, kSmallSort)));
     Carver c{base};
     e->key_a = c.take<uint64_t>(keys);
     e->key_b = c.take<uint64_t>(keys);
@@ -88,10 +86,9 @@ size_t carve(kt_engine* e, char* base, uint32_t n, uint64_t N, bool staging) {
     e->sel_part = c.take<uint64_t>((size_t)kSelMaxBlocks * 10);
     e->sel_feat = c.take<float>(KT_SELECTOR_FEATURES);
     e->sel_choice = c.take<uint32_t>(1);
-    e->hist = c.take<uint32_t>(hist_words);
-    e->hist_words = hist_words;
-    e->scan_tmp = c.take<uint32_t>(scan_words);
-    e->scan_tmp_words = scan_words;
+    e->look = c.take<unsigned long long>(look_cap);
+    e->look_cap = look_cap;
+    e->digit_counts = c.take<uint32_t>(kCountWords);
     if (staging) {
         e->in_src = c.take<uint32_t>(N);
         e->in_dst = c.take<uint32_t>(N);

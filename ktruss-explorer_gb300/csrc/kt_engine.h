@@ -61,11 +61,12 @@ struct kt_engine {
     uint32_t cap_chunks = 0;
     uint32_t big_row = 0;         // ranks >= big_row have rows of kBigRow entries or more
     uint32_t tiny_row = 0;        // ranks < tiny_row have rows of at most 8 entries
-    // Scratch for scans and sort histograms.
-    uint32_t* scan_tmp = nullptr;
-    size_t scan_tmp_words = 0;
-    uint32_t* hist = nullptr;
-    size_t hist_words = 0;
+    // Scratch of the one-pass scans and radix passes (kt_look.cuh): look-back words, digit counts
+    // and tickets, cleared by begin_session; the current session's tag and count blocks in use.
+    unsigned long long* look = nullptr;
+    uint64_t look_cap = 0;
+    uint32_t* digit_counts = nullptr;
+    uint32_t look_tag = 0, look_count = 0;
     // Control block (device) and its pinned host mirror.
     uint32_t* ctrl = nullptr;
     uint32_t* h_ctrl = nullptr;
@@ -153,15 +154,26 @@ void remember(kt_engine* e, const kt_engine::LastCall& c);
 void forget(kt_engine* e);
 size_t carve(kt_engine* e, char* base, uint32_t n, uint64_t N, bool staging);
 
-// kt_sort.cu
-int exclusive_scan(kt_engine* e, const uint32_t* in, uint32_t* out, uint64_t n);
-// out[0, n] = exclusive prefix sums of in[0, n) (out[n] is the total); ends[i] = out[i + 1].
-int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* ends);
-int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t n);
-// Sorts (keys, vals) by the low `bits` bits of the keys; ping-pongs between a and b buffers
-// and returns 0 if the result is in (key_a, val_a), 1 if in (key_b, val_b).  vals may be null.
-int radix_sort(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b,
-               uint64_t n, unsigned bits, int* result_in_b);
+struct Look;  // kt_look.cuh
+
+// kt_sort.cu.  Sorts of up to kSmallSort keys take small tiles (enough blocks for every SM).
+constexpr uint64_t kSmallSort = 1u << 18;
+constexpr uint64_t kSmallTile = 1024, kLargeTile = 4096;
+constexpr uint32_t kCountWords = 32 * 256 + 64;  // digit count blocks and tickets of a session
+inline uint64_t look_words(uint64_t keys) {
+    return 256 * (keys <= kSmallSort ? (keys + kSmallTile - 1) / kSmallTile : (keys + kLargeTile - 1) / kLargeTile);
+}
+// A session clears the control block, deg[0, deg_words) and the look-back scratch for sorts of up to
+// `words` (look_words) and sets the row marks to n; each launch that looks back takes a tag of it.
+int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words);
+Look next_look(kt_engine* e);
+uint32_t* next_counts(kt_engine* e, unsigned passes);  // zeroed digit counts, 256 words a pass
+int count_digits(kt_engine* e, const uint64_t* keys, uint64_t n, unsigned shift, unsigned passes, uint32_t* counts);
+// Sorts keys by `passes` 8-bit digits from bit `shift` on, whose counts are in `counts`; ping-pongs
+// between the a and b buffers and says in *result_in_b where the result is.  With value buffers the
+// values are the keys' positions before the sort (not read, only written).
+int radix_passes(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,
+                 unsigned shift, unsigned passes, const uint32_t* counts, int* result_in_b);
 
 // kt_build.cu: relabel by degree, orient, sort, symmetric + oriented CSR, edge ids.
 int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n);

@@ -41,8 +41,8 @@
 
 #include <algorithm>
 
-#include "kt_device.cuh"
 #include "kt_engine.h"
+#include "kt_look.cuh"
 
 namespace kt {
 
@@ -660,6 +660,34 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
     }
 }
 
+// List starts (tptr[m] is the total) and ends: exclusive and inclusive prefix sums of the supports.
+__global__ void __launch_bounds__(kScanThreads) k_list_bounds(const uint32_t* __restrict__ sup, uint32_t m,
+                                                              uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
+                                                              Look L) {
+    __shared__ uint64_t ws[33], s_prefix;
+    __shared__ uint32_t s_tile;
+    const uint32_t tile = look_tile(L, &s_tile);
+    if (tile == kNoTile) return;
+    const uint64_t j0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    uint64_t sum = 0, end;
+#pragma unroll
+    for (uint32_t i = 0; i < kScanItems; ++i) {
+        v[i] = j0 + i < m ? sup[j0 + i] : 0u;
+        sum += v[i];
+    }
+    uint64_t at = tile_scan<uint64_t>(L, tile, sum, ws, &s_prefix, &end);
+#pragma unroll
+    for (uint32_t i = 0; i < kScanItems; ++i) {
+        if (j0 + i < m) {
+            tptr[j0 + i] = at;
+            at += v[i];
+            ends[j0 + i] = at;
+            if (j0 + i == m - 1) tptr[m] = at;
+        }
+    }
+}
+
 }  // namespace
 
 // Most list entries per edge on average (three per triangle) with which the lists are made.  Denser
@@ -720,7 +748,9 @@ int peel_lists(kt_engine* e) {
     // the sort's key buffers are free after the build: list starts, and ends for the fill
     uint64_t* tptr = e->key_a;
     uint64_t* ends = e->key_b;
-    if ((rc = scan_offsets(e, e->sup, (uint64_t)m, tptr, ends)) || (rc = fill_lists(e, tptr, ends))) return rc;
+    k_list_bounds<<<ceil_div(m, kScanTile), kScanThreads, 0, e->stream>>>(e->sup, m, tptr, ends, next_look(e));
+    count_launch(e);
+    if ((rc = check_launch(e, "k_list_bounds")) || (rc = fill_lists(e, tptr, ends))) return rc;
     ListParams P;
     P.tri = e->lists;
     P.tptr = tptr;

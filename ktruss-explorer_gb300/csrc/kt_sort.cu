@@ -1,299 +1,289 @@
-// Device primitives for the CSR build: exclusive scan and a stable LSD radix sort.
+// A stable LSD radix sort for the CSR build, one kernel a digit.
 //
-// These replace the Thrust scan and the per-row CPU quicksort of the reference build
-// (graph.cu:457 thrust::exclusive_scan, graph.cu:462-476 "Sort outgoing edges ... on CPU").
+// It replaces the per-row CPU quicksort of the reference build (graph.cu:462-476 "Sort outgoing
+// edges ... on CPU").  Every digit's histogram is counted by the kernel that makes the keys (or by
+// k_digit_counts), so a pass reads the keys once: a tile ranks its keys by warp matches, learns where
+// its digits' runs start from its predecessors (decoupled look-back, one word a digit), arranges
+// itself in digit order in shared memory and writes runs of consecutive positions.  The first pass
+// can make the values (entry indices) itself.
+//
+// Bound: the serial chain of a tile (ticket, loads, ranks, look-back, runs) at half occupancy - 64
+// registers, issue active 44 %, DRAM 28 % - and for small inputs the launches.  A pass over 31.4 M keys
+// with values takes 0.31 ms (histogram, scan and scatter kernels: 0.34 ms); a pass over 64,000 entries
+// is one launch instead of four.
 
-#include "kt_device.cuh"
+#include <algorithm>
+#include <utility>
+
 #include "kt_engine.h"
+#include "kt_look.cuh"
 
 namespace kt {
 
 namespace {
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // 4096
+constexpr int kDigits = 256;
+// Large tiles: 512 threads of 8 keys, two blocks an SM.  512 of 4 keys (four blocks) and 256 of 8 measured
+// within 4 %, 1024 of 4 keys 17 % slower (build of R-MAT 20).
+constexpr int kLargeThreads = 512, kLargeItems = (int)kLargeTile / kLargeThreads;
+constexpr int kSmallThreads = 256, kSmallItems = (int)kSmallTile / kSmallThreads;
 
-// Block-wide exclusive scan of one value per thread; returns the block total in *total.
-template <class T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T* warp_sums, T* total) {
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    T x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        T y = __shfl_up_sync(kFullMask, x, o);
-        if (lane >= (uint32_t)o) x += y;
+// Digit counts of all passes for keys that are there already.
+__global__ void __launch_bounds__(256) k_digit_counts(const uint64_t* __restrict__ keys, uint64_t n, unsigned shift,
+                                                      unsigned passes, uint32_t* __restrict__ counts) {
+    __shared__ uint32_t h[kMaxDigitPasses * kDigits];
+    digit_counts_clear(h, passes);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = i0 + threadIdx.x;
+        digit_counts_add(h, i < n ? keys[i] >> shift : 0, i < n, passes);
     }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        T w = lane < nwarps ? warp_sums[lane] : T(0);
-        T s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            T y = __shfl_up_sync(kFullMask, s, o);
-            if (lane >= (uint32_t)o) s += y;
-        }
-        if (lane < nwarps) warp_sums[lane] = s - w;
-        if (lane == 31) warp_sums[32] = s;
-    }
-    __syncthreads();
-    T r = warp_sums[warp] + x - v;
-    *total = warp_sums[32];
-    __syncthreads();
-    return r;
+    digit_counts_flush(h, passes, counts);
 }
 
-template <class TI, class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const TI* __restrict__ in, uint64_t n,
-                                                                   T* __restrict__ sums) {
-    __shared__ T ws[33];
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-    T s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
-        if (idx < n) s += in[idx];
-    }
-    T total;
-    block_exclusive_scan<T>(s, ws, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
+// Shared memory of a pass, by tile shape.
+template <int kThreads, int kItems>
+struct PassSmem {
+    uint32_t wh[kThreads / 32][kDigits];  // per warp: keys of each digit, then their offset in the tile's run
+    uint64_t key[kThreads * kItems];
+    uint32_t val[kThreads * kItems];
+    uint32_t goff[kDigits];  // where the tile's run of each digit goes, less its start in the tile
+    uint32_t toff[kDigits];
+    uint32_t ws[2][kDigits / 32];
+    uint32_t tile, ok;
+};
 
-// Exclusive scan of each tile, offset by the scanned tile sums (if given).  With `ends` the inclusive
-// sums are written there and out[n] is the total.
-template <class TI, class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const TI* in, T* out, uint64_t n,
-                                                               const T* __restrict__ tile_offsets, T* ends) {
-    __shared__ T tile[kScanTile];
-    __shared__ T ws[33];
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
-        tile[threadIdx.x + i * kScanThreads] = idx < n ? T(in[idx]) : T(0);
-    }
-    __syncthreads();
-    T v[kScanItems], s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        v[i] = tile[threadIdx.x * kScanItems + i];
-        s += v[i];
-    }
-    T total;
-    T run = block_exclusive_scan<T>(s, ws, &total) + (tile_offsets ? tile_offsets[blockIdx.x] : T(0));
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        tile[threadIdx.x * kScanItems + i] = run;
-        run += v[i];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        uint64_t idx = base + threadIdx.x + (uint64_t)i * kScanThreads;
-        if (idx < n) {
-            out[idx] = tile[threadIdx.x + i * kScanThreads];
-            if (ends && idx > 0) ends[idx - 1] = tile[threadIdx.x + i * kScanThreads];
-        }
-    }
-    if (ends && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-        out[n] = ends[n - 1] = total + (tile_offsets ? tile_offsets[blockIdx.x] : T(0));
-}
-
-constexpr uint32_t kSortTile = 2048;  // keys per tile (one histogram column per tile and digit)
-constexpr int kDigits = 256;          // 8-bit digits
-constexpr int kSortThreads = kDigits; // the histogram kernel: one digit per thread
-// The scatter: kScatterThreads threads a block, each warp ranking kScatterSteps 32-key steps.
-// 512 threads of 4 steps hold 32 registers a thread (4 blocks, all 64 warps of a SM); 256
-// threads of 8 steps needed 64 (32 warps a SM) and ran at 40 % of DRAM bandwidth.  Measured on
-// GB300: batch4096 build 69.7 -> 69.1 ms, R-MAT 24 build 128.7 -> 128.3 ms.
-constexpr int kScatterThreads = 512;
-constexpr int kScatterWarps = kScatterThreads / 32;
-constexpr int kScatterSteps = 4;
-constexpr uint32_t kScatterWarpKeys = 32 * kScatterSteps;
-static_assert(kScatterWarps * kScatterWarpKeys == kSortTile, "a scatter block covers one tile");
-static_assert(kScatterThreads >= kDigits, "the first kDigits threads own one digit each");
-
-__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint64_t* __restrict__ keys, uint64_t n,
-                                                               unsigned shift, uint32_t* __restrict__ hist,
-                                                               uint32_t num_blocks) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-    for (uint32_t i = threadIdx.x; i < kSortTile; i += kSortThreads) {
-        uint64_t idx = base + i;
-        if (idx < n) atomicAdd(&h[(uint32_t)(keys[idx] >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    hist[(uint64_t)threadIdx.x * num_blocks + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter of one 2048-key tile: each warp ranks its kScatterWarpKeys consecutive keys in
-// 32-key steps with __match_any_sync; warps are then offset by the counts of earlier warps (the
-// first kDigits threads own one digit each for the tile's counts and offsets).  The tile is first
-// arranged in digit order in shared memory, then written out so that consecutive threads store
-// consecutive positions of each digit's run (coalesced stores).
-__global__ void __launch_bounds__(kScatterThreads) k_radix_scatter(const uint64_t* __restrict__ kin,
-                                                                  const uint32_t* __restrict__ vin,
-                                                                  uint64_t* __restrict__ kout,
-                                                                  uint32_t* __restrict__ vout, uint64_t n,
-                                                                  unsigned shift,
-                                                                  const uint32_t* __restrict__ hist,
-                                                                  uint32_t num_blocks) {
-    __shared__ uint32_t wh[kScatterWarps][kDigits];
-    __shared__ uint32_t goff[kDigits];   // global start of each digit's run for this tile
-    __shared__ uint32_t toff[kDigits];   // start of each digit's run inside the tile
-    __shared__ uint32_t ws[33];
-    __shared__ uint64_t skey[kSortTile];
-    __shared__ uint32_t sval[kSortTile];
+template <int kThreads, int kItems, bool kVals>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const uint64_t* __restrict__ kin,
+                                                         const uint32_t* __restrict__ vin,
+                                                         uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                         uint64_t n, unsigned shift,
+                                                         const uint32_t* __restrict__ counts, Look L) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    PassSmem<kThreads, kItems>& S = *reinterpret_cast<PassSmem<kThreads, kItems>*>(raw);
+    constexpr int kWarps = kThreads / 32;
+    static_assert(kThreads >= kDigits, "the first kDigits threads own one digit each");
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const bool owner = threadIdx.x < (uint32_t)kDigits;  // digit threadIdx.x (whole warps)
-    for (uint32_t i = threadIdx.x; i < kScatterWarps * kDigits; i += kScatterThreads) (&wh[0][0])[i] = 0;
-    if (owner) goff[threadIdx.x] = hist[(uint64_t)threadIdx.x * num_blocks + blockIdx.x];
-    __syncthreads();
-    const uint64_t tbase = (uint64_t)blockIdx.x * kSortTile;
-    const uint64_t wbase = tbase + (uint64_t)warp * kScatterWarpKeys;
-    uint64_t key[kScatterSteps];
-    uint32_t val[kScatterSteps], dig[kScatterSteps], rk[kScatterSteps];
+    const bool owner = threadIdx.x < (uint32_t)kDigits;  // of digit threadIdx.x (whole warps)
+    for (uint32_t i = threadIdx.x; i < kWarps * kDigits; i += kThreads) (&S.wh[0][0])[i] = 0;
+    if (threadIdx.x == 0) S.ok = 1;
+    const uint32_t tile = look_tile(L, &S.tile);
+    if (tile == kNoTile) return;
+    const uint64_t tbase = (uint64_t)tile * (kThreads * kItems);
+    const uint64_t wbase = tbase + (uint64_t)warp * (32 * kItems);
+    uint64_t key[kItems];
+    uint32_t rk[kItems];
 #pragma unroll
-    for (int s = 0; s < kScatterSteps; ++s) {
-        uint64_t idx = wbase + (uint32_t)s * 32 + lane;
-        bool valid = idx < n;
-        key[s] = valid ? kin[idx] : 0ull;
-        val[s] = (valid && vin) ? vin[idx] : 0u;
-        uint32_t d = valid ? ((uint32_t)(key[s] >> shift) & 255u) : 256u;
-        dig[s] = d;
-        uint32_t peers = __match_any_sync(kFullMask, d);
-        uint32_t base = d < 256 ? wh[warp][d] : 0u;
+    for (int s = 0; s < kItems; ++s) {
+        const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
+        key[s] = idx < n ? kin[idx] : 0ull;
+    }
+    // the leader of each set of equal digits claims its ranks, step after step, without waiting for
+    // the atomics' results in between
+    uint32_t first[kItems];
+#pragma unroll
+    for (int s = 0; s < kItems; ++s) {
+        const bool valid = wbase + (uint32_t)s * 32 + lane < n;
+        const uint32_t d = valid ? ((uint32_t)(key[s] >> shift) & 255u) : 256u;
+        // lanes with the same digit, bit by bit (match.any instead of the eight ballots made the warps
+        // wait on its result: short-scoreboard stalls 11 against 2 cycles an instruction)
+        uint32_t peers = __ballot_sync(kFullMask, valid);
+        peers = valid ? peers : 0u;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const uint32_t ones = __ballot_sync(kFullMask, d >> b & 1u);
+            peers &= (d >> b & 1u) ? ones : ~ones;
+        }
+        const uint32_t leader = __ffs(peers) - 1;
+        first[s] = 0;
+        if (valid && lane == leader) first[s] = atomicAdd(&S.wh[warp][d], __popc(peers));
         __syncwarp();
-        if (d < 256 && lane == (uint32_t)(__ffs(peers) - 1)) wh[warp][d] = base + __popc(peers);
-        __syncwarp();
-        rk[s] = base + __popc(peers & lanemask_lt());
+        rk[s] = leader << 8 | __popc(peers & lanemask_lt());
+    }
+#pragma unroll
+    for (int s = 0; s < kItems; ++s) rk[s] = __shfl_sync(kFullMask, first[s], rk[s] >> 8) + (rk[s] & 255u);
+    uint32_t val[kItems];
+#pragma unroll
+    for (int s = 0; s < kItems; ++s) {
+        const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
+        val[s] = kVals ? (vin ? (idx < n ? vin[idx] : 0u) : (uint32_t)idx) : 0u;
     }
     __syncthreads();
-    uint32_t count = 0;  // keys of digit threadIdx.x in the tile
+    uint32_t count = 0, all = 0;  // keys of digit threadIdx.x in the tile, and in all tiles
     if (owner) {
         uint32_t run = 0;
 #pragma unroll
-        for (int w = 0; w < kScatterWarps; ++w) {
-            uint32_t c = wh[w][threadIdx.x];
-            wh[w][threadIdx.x] = run;
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t c = S.wh[w][threadIdx.x];
+            S.wh[w][threadIdx.x] = run;
             run += c;
         }
         count = run;
+        all = counts[threadIdx.x];
+        st_relaxed_u64(L.words + (uint64_t)tile * kDigits + threadIdx.x,
+                       look_word(tile ? kLookAggregate : kLookInclusive, L.tag, count));
     }
-    // exclusive scan of the tile's digit counts (one digit per owner thread)
-    {
-        constexpr int kDigitWarps = kDigits / 32;
-        uint32_t x = count;
-        if (owner) {
+    // exclusive scans over the digits: starts in the tile and in the output
+    uint32_t x = count, y = all;
+    if (owner) {
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFullMask, x, o);
-                if (lane >= (uint32_t)o) x += y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(kFullMask, x, o), b = __shfl_up_sync(kFullMask, y, o);
+            if (lane >= (uint32_t)o) {
+                x += a;
+                y += b;
             }
-            if (lane == 31) ws[warp] = x;
         }
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t w = lane < kDigitWarps ? ws[lane] : 0u;
-            uint32_t t = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFullMask, t, o);
-                if (lane >= (uint32_t)o) t += y;
-            }
-            if (lane < kDigitWarps) ws[lane] = t - w;
-        }
-        __syncthreads();
-        if (owner) toff[threadIdx.x] = ws[warp] + x - count;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < kScatterSteps; ++s) {
-        const uint32_t d = dig[s];
-        if (d < 256) {
-            const uint32_t lp = toff[d] + wh[warp][d] + rk[s];
-            skey[lp] = key[s];
-            sval[lp] = val[s];
+        if (lane == 31) {
+            S.ws[0][warp] = x;
+            S.ws[1][warp] = y;
         }
     }
     __syncthreads();
-    const uint32_t valid = (uint32_t)min((uint64_t)kSortTile, n - tbase);
-    for (uint32_t i = threadIdx.x; i < valid; i += kScatterThreads) {
-        const uint64_t k = skey[i];
-        const uint32_t d = (uint32_t)(k >> shift) & 255u;
-        const uint32_t pos = goff[d] + (i - toff[d]);
-        kout[pos] = k;
-        if (vin) vout[pos] = sval[i];
+    uint32_t start = 0;
+    if (owner) {
+        uint32_t bx = 0, by = 0;
+#pragma unroll
+        for (int w = 0; w < kDigits / 32; ++w) {
+            bx += w < (int)warp ? S.ws[0][w] : 0u;
+            by += w < (int)warp ? S.ws[1][w] : 0u;
+        }
+        S.toff[threadIdx.x] = bx + x - count;
+        start = by + y - all;
     }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kItems; ++s) {
+        if (wbase + (uint32_t)s * 32 + lane < n) {
+            const uint32_t d = (uint32_t)(key[s] >> shift) & 255u;
+            const uint32_t lp = S.toff[d] + S.wh[warp][d] + rk[s];
+            S.key[lp] = key[s];
+            if (kVals) S.val[lp] = val[s];
+        }
+    }
+    // the owners look back, four predecessors at a time
+    if (owner) {
+        uint64_t prefix = 0;
+        if (tile) {
+            LookWait wait;
+            int64_t t = (int64_t)tile - 1;
+            bool done = false;
+            while (!done) {
+                unsigned long long w[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    w[q] = t - q >= 0 ? ld_relaxed_u64(L.words + (uint64_t)(t - q) * kDigits + threadIdx.x)
+                                      : look_word(kLookInclusive, L.tag, 0);
+                int used = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!done && used == q && look_valid(w[q], L.tag)) {
+                        prefix += (uint64_t)w[q] & kLookValue;
+                        done = (w[q] >> 62) == kLookInclusive;
+                        ++used;
+                    }
+                }
+                t -= used;
+                if (!done && used == 0 && !wait.again(L.ctrl)) {
+                    S.ok = 0;
+                    break;
+                }
+            }
+            st_relaxed_u64(L.words + (uint64_t)tile * kDigits + threadIdx.x,
+                           look_word(kLookInclusive, L.tag, prefix + count));
+        }
+        S.goff[threadIdx.x] = start + (uint32_t)prefix - S.toff[threadIdx.x];
+    }
+    __syncthreads();
+    if (!S.ok) return;
+    const uint32_t valid = (uint32_t)min((uint64_t)(kThreads * kItems), n - tbase);
+    for (uint32_t i = threadIdx.x; i < valid; i += kThreads) {
+        const uint64_t k = S.key[i];
+        const uint64_t pos = S.goff[(uint32_t)(k >> shift) & 255u] + i;  // modulo 2^32
+        if ((uint32_t)pos < n) {
+            kout[(uint32_t)pos] = k;
+            if (kVals) vout[(uint32_t)pos] = S.val[i];
+        }
+    }
+}
+
+// Starts a session: clears the control block (if asked to), the degrees, the look-back words and
+// the digit counts and tickets; the row marks start at n.
+__global__ void k_session(uint32_t* __restrict__ ctrl, uint32_t ctrl_words, uint32_t n, uint32_t* __restrict__ deg,
+                          uint32_t deg_words, uint4* __restrict__ words, uint64_t quads, uint32_t* __restrict__ counts,
+                          uint32_t count_words) {
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = tid; i < ctrl_words; i += step) ctrl[i] = i == kCtrlBigRow || i == kCtrlTinyRow ? n : 0u;
+    for (uint64_t i = tid; i < deg_words; i += step) deg[i] = 0;
+    for (uint64_t i = tid; i < quads; i += step) words[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = tid; i < count_words; i += step) counts[i] = 0;
+}
+
+template <int kThreads, int kItems, bool kVals>
+int launch_pass(kt_engine* e, const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, uint64_t n,
+                unsigned shift, const uint32_t* counts, const Look& L) {
+    const int smem = (int)sizeof(PassSmem<kThreads, kItems>);
+    int rc = check_cuda(cudaFuncSetAttribute(k_radix_pass<kThreads, kItems, kVals>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                        "shared memory of k_radix_pass");
+    if (rc) return rc;
+    const uint64_t tiles = (n + kThreads * kItems - 1) / (kThreads * kItems);
+    k_radix_pass<kThreads, kItems, kVals><<<(uint32_t)tiles, kThreads, smem, e->stream>>>(kin, vin, kout, vout, n, shift,
+                                                                                         counts, L);
+    count_launch(e);
+    return check_launch(e, "k_radix_pass");
 }
 
 }  // namespace
 
-// Hierarchical scan: tile sums are scanned recursively in scratch (used as a stack from
-// word `tmp_off` on), then every tile is rescanned with its offset.
-template <class TI, class T>
-static int scan_level(kt_engine* e, const TI* in, T* out, uint64_t n, T* tmp, uint64_t tmp_words, uint64_t tmp_off,
-                      T* ends = nullptr) {
-    if (n == 0) return KT_OK;
-    if (n <= kScanTile) {
-        k_scan_tiles<TI, T><<<1, kScanThreads, 0, e->stream>>>(in, out, n, nullptr, ends);
-        count_launch(e);
-        return check_launch(e, "k_scan_tiles");
-    }
-    const uint64_t nb = (n + kScanTile - 1) / kScanTile;
-    const uint64_t words = (nb + 63) & ~63ull;
-    if (tmp_off + words > tmp_words)
-        return fail(KT_ERR_INVALID_ARG, "scan scratch too small (%llu elements)", (unsigned long long)tmp_words);
-    T* sums = tmp + tmp_off;
-    k_scan_tile_sums<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, n, sums);
+int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words) {
+    if (words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
+    e->look_tag = e->look_count = 0;
+    const uint64_t work = std::max<uint64_t>(words / 2, std::max<uint32_t>(deg_words, kCountWords));
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((work + 255) / 256, (uint64_t)e->num_sms * 8);
+    k_session<<<blocks, 256, 0, e->stream>>>(e->ctrl, kCtrlWords, n, e->deg, deg_words,
+                                             reinterpret_cast<uint4*>(e->look), words / 2, e->digit_counts, kCountWords);
     count_launch(e);
-    int rc = check_launch(e, "k_scan_tile_sums");
-    if (rc) return rc;
-    rc = scan_level<T, T>(e, sums, sums, nb, tmp, tmp_words, tmp_off + words);
-    if (rc) return rc;
-    k_scan_tiles<TI, T><<<(uint32_t)nb, kScanThreads, 0, e->stream>>>(in, out, n, sums, ends);
+    return check_launch(e, "k_session");
+}
+
+Look next_look(kt_engine* e) {
+    ++e->look_tag;
+    return Look{e->look, e->digit_counts + kLookTags * 256, e->ctrl, e->look_tag};
+}
+
+uint32_t* next_counts(kt_engine* e, unsigned passes) {
+    uint32_t* c = e->digit_counts + 256 * e->look_count;
+    e->look_count += passes;
+    return c;
+}
+
+int count_digits(kt_engine* e, const uint64_t* keys, uint64_t n, unsigned shift, unsigned passes, uint32_t* counts) {
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((n + 1023) / 1024, (uint64_t)e->num_sms * 8);
+    k_digit_counts<<<blocks, 256, 0, e->stream>>>(keys, n, shift, passes, counts);
     count_launch(e);
-    return check_launch(e, "k_scan_tiles");
+    return check_launch(e, "k_digit_counts");
 }
 
-int exclusive_scan(kt_engine* e, const uint32_t* in, uint32_t* out, uint64_t n) {
-    return scan_level<uint32_t, uint32_t>(e, in, out, n, e->scan_tmp, e->scan_tmp_words, 0);
-}
-
-int exclusive_scan_u64(kt_engine* e, const uint64_t* in, uint64_t* out, uint64_t n) {
-    return scan_level<uint64_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp), e->scan_tmp_words / 2, 0);
-}
-
-int scan_offsets(kt_engine* e, const uint32_t* in, uint64_t n, uint64_t* out, uint64_t* ends) {
-    return scan_level<uint32_t, uint64_t>(e, in, out, n, reinterpret_cast<uint64_t*>(e->scan_tmp),
-                                          e->scan_tmp_words / 2, 0, ends);
-}
-
-int radix_sort(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,
-               unsigned bits, int* result_in_b) {
+int radix_passes(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,
+                 unsigned shift, unsigned passes, const uint32_t* counts, int* result_in_b) {
     *result_in_b = 0;
-    if (n <= 1 || bits == 0) return KT_OK;
-    const uint64_t nb64 = (n + kSortTile - 1) / kSortTile;
-    if (nb64 * 256 > e->hist_words) return fail(KT_ERR_INVALID_ARG, "sort histogram scratch too small");
-    const uint32_t nb = (uint32_t)nb64;
     uint64_t *kin = key_a, *kout = key_b;
-    uint32_t *vin = val_a, *vout = val_b;
-    for (unsigned shift = 0; shift < bits; shift += 8) {
-        k_radix_hist<<<nb, kSortThreads, 0, e->stream>>>(kin, n, shift, e->hist, nb);
-        count_launch(e);
-        int rc = check_launch(e, "k_radix_hist");
+    uint32_t *vin = nullptr, *vout = val_b;  // the first pass numbers the keys
+    for (unsigned p = 0; p < passes; ++p) {
+        const Look L = next_look(e);
+        int rc;
+        if (n <= kSmallSort)
+            rc = val_a ? launch_pass<kSmallThreads, kSmallItems, true>(e, kin, vin, kout, vout, n, shift + 8 * p, counts + 256 * p, L)
+                       : launch_pass<kSmallThreads, kSmallItems, false>(e, kin, vin, kout, vout, n, shift + 8 * p, counts + 256 * p, L);
+        else
+            rc = val_a ? launch_pass<kLargeThreads, kLargeItems, true>(e, kin, vin, kout, vout, n, shift + 8 * p, counts + 256 * p, L)
+                       : launch_pass<kLargeThreads, kLargeItems, false>(e, kin, vin, kout, vout, n, shift + 8 * p, counts + 256 * p, L);
         if (rc) return rc;
-        rc = exclusive_scan(e, e->hist, e->hist, (uint64_t)nb * 256);
-        if (rc) return rc;
-        k_radix_scatter<<<nb, kScatterThreads, 0, e->stream>>>(kin, vin, kout, vout, n, shift, e->hist, nb);
-        count_launch(e);
-        rc = check_launch(e, "k_radix_scatter");
-        if (rc) return rc;
-        uint64_t* tk = kin; kin = kout; kout = tk;
-        uint32_t* tv = vin; vin = vout; vout = tv;
+        std::swap(kin, kout);
+        if (val_a) {
+            vin = vout;
+            vout = vin == val_b ? val_a : val_b;
+        }
         *result_in_b ^= 1;
     }
     return KT_OK;

@@ -435,10 +435,7 @@ int count_support(kt_engine* e) {
     if (e->m == 0) return KT_OK;
     int rc;
     const Graph g = graph_of(e);
-    const Credits c = credits_of(e);
-    if ((rc = check_cuda(cudaMemsetAsync(c.sup, 0, sizeof(uint32_t) * e->m, e->stream), "clear support")) ||
-        (rc = check_cuda(cudaMemsetAsync(c.supx, 0, sizeof(uint32_t) * e->m, e->stream), "clear support")))
-        return rc;
+    const Credits c = credits_of(e);  // cleared by the build
     if (g.mid_in) {
         k_middle_plan<<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), rows_of(e),
                                                                                     e->ctrl);
