@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kScanThreads) k_rank_rows(const uint64_t* __re
 }
 
 // Entry keys (rank of the source << vb | rank of the destination) and their digit counts.  An id >= n
-// (already flagged by k_degree; the call fails at the end of the build) is read as vertex 0, so that
+// (already flagged by k_degree; the call fails) is read as vertex 0, so that
 // every kernel up to that check indexes inside its arrays.
 __global__ void __launch_bounds__(kThreads) k_edge_keys(const uint32_t* __restrict__ src,
                                                         const uint32_t* __restrict__ dst, uint64_t entries, uint32_t n,
@@ -293,7 +293,9 @@ unsigned bits_for(uint64_t n) {
     return b;
 }
 
-int error_status(uint32_t err) {
+}  // namespace
+
+int input_status(uint32_t err) {
     if (err & kErrBadVertex) return fail(KT_ERR_INVALID_ARG, "an entry names a vertex id >= num_nodes");
     if (err & kErrSelfLoop) return fail(KT_ERR_SELF_LOOP, "Edges from a vertex to itself are not allowed!");
     if (err & kErrDuplicate) return fail(KT_ERR_NOT_SYMMETRIC, "duplicate entry in the input edge list");
@@ -309,8 +311,10 @@ int sync_and_check(kt_engine* e) {
     if (rc) return rc;
     rc = check_cuda(cudaStreamSynchronize(e->stream), "build synchronize");
     if (rc) return rc;
-    return error_status(e->h_ctrl[kCtrlError]);
+    return input_status(e->h_ctrl[kCtrlError]);
 }
+
+namespace {
 
 // Tiled COO/CSR (coo2tiledcoocsr, graph.cu:641-706): key = row << vb | dst with row =
 // (src / ts * T + dst / ts) * ts + src % ts; the entry index rides along as the value.
@@ -534,7 +538,8 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
     return sync_and_check(e);
 }
 
-int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n) {
+int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n,
+                bool check) {
     if (entries & 1) return fail(KT_ERR_NOT_SYMMETRIC, "odd number of entries (%llu): every edge needs both directions",
                                  (unsigned long long)entries);
     if (entries >= 0xffffffffull) return fail(KT_ERR_TOO_LARGE, "more than 2^32-2 entries");
@@ -559,8 +564,8 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
         count_launch(e);
         if ((rc = check_launch(e, "k_degree"))) return rc;
     }
-    // (input errors are read back once, at the end of the build: every kernel before that
-    // check indexes inside its arrays whatever the input)
+    // (input errors are read back once, after the build: every kernel up to its end indexes inside its
+    // arrays whatever the input, and the kernels after it return at once when the error word is set)
 
     // 2. ranks - ascending (degree, id), or the ids themselves when orienting by index - and the row
     // starts of the symmetric CSR (row r holds the neighbours of the rank-r vertex)
@@ -611,11 +616,7 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
         count_launch(e);
         if ((rc = check_launch(e, "k_entry_eid"))) return rc;
     }
-    if (e->trusted) return KT_OK;  // same input: big_row and tiny_row as read before
-    if ((rc = sync_and_check(e))) return rc;
-    e->big_row = e->h_ctrl[kCtrlBigRow];
-    e->tiny_row = e->h_ctrl[kCtrlTinyRow];
-    return KT_OK;
+    return check && !e->trusted ? sync_and_check(e) : KT_OK;
 }
 
 }  // namespace kt

@@ -48,6 +48,8 @@ enum : uint32_t {
     kPChunks = 64,     // [4] u64 (words 64..71): work chunks claimed for the round; 64 bits
                        //     because a frontier of most edges can need more than 2^32 chunks
     kPWalk = 72,       // u64 (words 72..73): row entries queued for walks over the whole peel
+    kPPasses = 80,     // passes of the reference's chained schedule for the same decomposition, and
+    kPAliveSum = 82,   // u64 (words 82..83): the alive edges they see
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
     kCtrlWords = 128,  // words 88-115: the list peel (kt_lists.cu)
@@ -125,6 +127,14 @@ __host__ __device__ __forceinline__ uint32_t fenced_lower_bound(const uint32_t* 
         hi = e;
     }
     return lo + lower_bound_u32(a + lo, hi - lo, t);
+}
+
+// An error of the call so far: kernels that index by what the build made return at once (the host
+// reads the word only once a call).
+__device__ __forceinline__ bool failed(const uint32_t* ctrl) {
+    uint32_t v;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(ctrl + kCtrlError) : "memory");
+    return v != 0;
 }
 
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }

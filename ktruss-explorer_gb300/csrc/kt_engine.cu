@@ -112,8 +112,6 @@ void remember(kt_engine* e, const kt_engine::LastCall& c) {
         l.truss != c.truss || l.k_max != c.k_max || l.k != c.k || l.keep != c.keep)
         drop_replay(e);
     e->last = c;
-    e->last.big_row = e->big_row;  // the build of the call being remembered set these
-    e->last.tiny_row = e->tiny_row;
     e->last.list_entries = e->list_entries;
 }
 
@@ -150,6 +148,7 @@ int reserve(kt_engine* e, uint32_t max_nodes, uint64_t max_entries) {
         return rc;
     e->cap_nodes = max_nodes;
     e->cap_entries = max_entries;
+    reserve_small_lists(e, max_entries / 2);
     return KT_OK;
 }
 
@@ -185,10 +184,14 @@ int record_start(kt_engine* e) {
 
 int record(kt_engine* e, cudaEvent_t ev) { return check_cuda(cudaEventRecord(ev, e->stream), "record event"); }
 
+// Ends a call: the stop event, then the control block to the host (the call's one read, unless its
+// triangle count was needed); waits for both and returns an input error.
 int record_stop(kt_engine* e) {
     int rc = check_cuda(cudaEventRecord(e->ev_stop, e->stream), "record stop");
     if (rc) return rc;
-    if ((rc = check_cuda(cudaEventSynchronize(e->ev_stop), "synchronize stop"))) return rc;
+    e->ctrl_fresh = false;
+    if ((rc = kt::sync_and_check(e))) return rc;
+    e->ctrl_fresh = true;
     float a = 0, b = 0, c = 0, d = 0;
     if ((rc = check_cuda(cudaEventElapsedTime(&a, e->ev_start, e->ev_select), "elapsed time")) ||
         (rc = check_cuda(cudaEventElapsedTime(&d, e->ev_select, e->ev_built), "elapsed time")) ||
@@ -223,12 +226,20 @@ int fill_graph_stats(kt_engine* e) {
     return KT_OK;
 }
 
+// A batch's vertex ranges and where its graphs' k_max go.
+struct Batch {
+    const uint32_t* offsets;
+    uint32_t graphs;
+    uint32_t* k_max;
+};
+
 // Device pipeline for the decomposition (inputs on the device).
 int run_decompose(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n,
-                  uint32_t* d_truss, uint32_t* d_k_max) {
+                  uint32_t* d_truss, uint32_t* d_k_max, const Batch* batch = nullptr) {
     int rc;
     if ((rc = record_start(e))) return rc;
-    if ((rc = kt::build_graph(e, d_src, d_dst, entries, n))) return rc;
+    // (the selector's statistics need a checked graph)
+    if ((rc = kt::build_graph(e, d_src, d_dst, entries, n, e->selector != nullptr))) return rc;
     if ((rc = record(e, e->ev_select))) return rc;
     if ((rc = kt::select_schedule(e))) return rc;
     if ((rc = record(e, e->ev_built))) return rc;
@@ -238,6 +249,8 @@ int run_decompose(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, ui
     if ((rc = record(e, e->ev_peeled))) return rc;
     e->emit_timed = true;
     if ((rc = kt::emit_truss_per_entry(e, d_truss, d_k_max))) return rc;
+    if (batch && (rc = kt::emit_graph_kmax(e, d_src, d_dst, batch->offsets, batch->graphs, d_truss, batch->k_max)))
+        return rc;
     if ((rc = record_stop(e))) return rc;
     return fill_graph_stats(e);
 }
@@ -270,7 +283,7 @@ int run_ktruss(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
     int rc;
     if ((rc = record_start(e))) return rc;
     e->orient_by_index = e->variant.directedness == KT_DIRECTED_BY_INDEX;
-    rc = kt::build_graph(e, d_src, d_dst, entries, n);
+    rc = kt::build_graph(e, d_src, d_dst, entries, n, !single_k_capturable(e));
     e->orient_by_index = false;
     if (rc) return rc;
     if ((rc = record(e, e->ev_select))) return rc;
@@ -286,10 +299,8 @@ int run_ktruss(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
 // of the call itself): no host reads, so it can be captured into a CUDA graph.
 int replay_pipeline(kt_engine* e) {
     const kt_engine::LastCall& c = e->last;
-    e->big_row = c.big_row;  // other calls since may have built other graphs
-    e->tiny_row = c.tiny_row;
     int rc;
-    if (c.kind == 1 && (rc = kt::build_graph(e, c.src, c.dst, c.entries, c.n))) return rc;
+    if (c.kind == 1 && (rc = kt::build_graph(e, c.src, c.dst, c.entries, c.n, false))) return rc;
     if (c.kind == 1 && (rc = kt::select_schedule(e))) return rc;  // on the device: capturable
     if (c.kind == 1)
         return (rc = kt::count_support(e)) || (rc = kt::peel_decompose(e)) ||
@@ -297,7 +308,7 @@ int replay_pipeline(kt_engine* e) {
                    ? rc
                    : KT_OK;
     e->orient_by_index = e->variant.directedness == KT_DIRECTED_BY_INDEX;
-    rc = kt::build_graph(e, c.src, c.dst, c.entries, c.n);
+    rc = kt::build_graph(e, c.src, c.dst, c.entries, c.n, false);
     e->orient_by_index = false;
     if (rc || (rc = single_k_body(e, c.k)) || (rc = kt::emit_keep(e, c.keep))) return rc;
     return KT_OK;
@@ -346,6 +357,7 @@ int replay(kt_engine* e, int sync) {
     }
     if ((rc = check_cuda(cudaEventRecord(e->ev_stop, e->stream), "record stop"))) return rc;
     e->peel_mode = e->replay_peel_mode;
+    e->ctrl_fresh = false;
     e->peel_timed = false;
     e->stats_ready = false;
     e->stats.build_ms = e->stats.select_ms = e->stats.support_ms = e->stats.peel_ms = 0;
@@ -620,7 +632,7 @@ int autotune(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_
         float t_min = 0;
         for (uint32_t r = 0; r < repeats && !rc; ++r) {
             // the rows are compacted in place while peeling, so every run builds the CSR again
-            if ((rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes)) || (rc = record(e, e->ev_built)) ||
+            if ((rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes, true)) || (rc = record(e, e->ev_built)) ||
                 (rc = kt::count_support(e)) || (rc = kt::peel_decompose(e)) || (rc = record(e, e->ev_stop)) ||
                 (rc = check_cuda(cudaEventSynchronize(e->ev_stop), "synchronize")))
                 break;
@@ -698,7 +710,7 @@ int kt_engine_features(kt_engine* e, const uint32_t* d_src, const uint32_t* d_ds
     if (!e || !features) return fail(KT_ERR_INVALID_ARG, "kt_engine_features: null argument");
     if (num_entries && (!d_src || !d_dst)) return fail(KT_ERR_INVALID_ARG, "kt_engine_features: null buffer");
     int rc = check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
-    if (rc || (rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes)) ||
+    if (rc || (rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes, true)) ||
         (rc = kt::graph_features(e, nullptr)) ||
         (rc = check_cuda(cudaMemcpyAsync(features, e->sel_feat, sizeof(float) * KT_SELECTOR_FEATURES,
                                          cudaMemcpyDeviceToHost, e->stream), "read features")))
@@ -777,15 +789,12 @@ int kt_engine_decompose_batch(kt_engine* e, const uint32_t* d_src, const uint32_
     // the union of disjoint graphs: its truss numbers are each graph's own
     kt::forget(e);
     e->batch_call = true;
-    rc = run_decompose(e, d_src, d_dst, num_entries, num_nodes, d_truss_per_entry, nullptr);
+    const Batch batch{d_vertex_offsets, num_graphs, d_k_max_per_graph};
+    rc = run_decompose(e, d_src, d_dst, num_entries, num_nodes, d_truss_per_entry, nullptr, &batch);
     e->batch_call = false;
     if (rc) return rc;
-    if ((rc = kt::emit_graph_kmax(e, d_src, d_dst, d_vertex_offsets, num_graphs, d_truss_per_entry,
-                                  d_k_max_per_graph)))
-        return rc;
     if (sync) {
         if ((rc = check_cuda(cudaStreamSynchronize(e->stream), "synchronize"))) return rc;
-        e->stats_ready = false;
         return kt::finish_stats(e);
     }
     return KT_OK;
@@ -831,10 +840,10 @@ int kt_decompose_batch(const uint32_t* src, const uint32_t* dst, uint64_t num_en
         return rc;
     if ((rc = record(e, e->ev_copy[1]))) return rc;
     e->batch_call = true;
-    rc = run_decompose(e, e->in_src, e->in_dst, N, num_nodes, e->out_u32, nullptr);
+    const Batch batch{d_off, num_graphs, d_kmax};
+    rc = run_decompose(e, e->in_src, e->in_dst, N, num_nodes, e->out_u32, nullptr, &batch);
     e->batch_call = false;
     if (rc) return rc;
-    if ((rc = kt::emit_graph_kmax(e, e->in_src, e->in_dst, d_off, num_graphs, e->out_u32, d_kmax))) return rc;
     if ((rc = record(e, e->ev_copy[2]))) return rc;
     if (N && (rc = check_cuda(cudaMemcpyAsync(truss_per_entry, e->out_u32, N * 4, cudaMemcpyDeviceToHost, e->stream),
                               "D2H")))
@@ -843,7 +852,6 @@ int kt_decompose_batch(const uint32_t* src, const uint32_t* dst, uint64_t num_en
                                          cudaMemcpyDeviceToHost, e->stream), "D2H")) ||
         (rc = record(e, e->ev_copy[3])) || (rc = check_cuda(cudaStreamSynchronize(e->stream), "synchronize")))
         return rc;
-    e->stats_ready = false;
     if ((rc = kt::finish_stats(e))) return rc;
     return copy_times(e);
 }

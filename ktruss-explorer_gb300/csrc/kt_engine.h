@@ -59,8 +59,6 @@ struct kt_engine {
     uint4* chunks0 = nullptr;     // peel work chunks, by round parity
     uint4* chunks1 = nullptr;
     uint32_t cap_chunks = 0;
-    uint32_t big_row = 0;         // ranks >= big_row have rows of kBigRow entries or more
-    uint32_t tiny_row = 0;        // ranks < tiny_row have rows of at most 8 entries
     // Scratch of the one-pass scans and radix passes (kt_look.cuh): look-back words, digit counts
     // and tickets, cleared by begin_session; the current session's tag and count blocks in use.
     unsigned long long* look = nullptr;
@@ -129,7 +127,6 @@ struct kt_engine {
         uint32_t k = 0;
         uint8_t* keep = nullptr;
         uint64_t list_entries = 0;           // triangle list entries the call counted
-        uint32_t big_row = 0, tiny_row = 0;  // read back by the call's build; a trusted build does not
     } last;
     cudaGraphExec_t replay = nullptr;
     bool replay_direct = false;      // the pipeline could not be captured: replays launch it directly
@@ -138,6 +135,7 @@ struct kt_engine {
     bool trusted = false;
     bool replay_timing = false;      // last_ms of a replay is read when the stream has drained
     bool stats_ready = false;   // stats already read back from the device
+    bool ctrl_fresh = false;    // h_ctrl holds the control block as the last call left it
 };
 
 namespace kt {
@@ -175,8 +173,14 @@ int count_digits(kt_engine* e, const uint64_t* keys, uint64_t n, unsigned shift,
 int radix_passes(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,
                  unsigned shift, unsigned passes, const uint32_t* counts, int* result_in_b);
 
-// kt_build.cu: relabel by degree, orient, sort, symmetric + oriented CSR, edge ids.
-int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n);
+// kt_build.cu: relabel by degree, orient, sort, symmetric + oriented CSR, edge ids.  With `check` it
+// waits and returns an input error as a status; without, the error stays in the control block, the
+// kernels after the build return at once, and the caller reads it (input_status).
+int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t entries, uint32_t n,
+                bool check);
+int input_status(uint32_t err);
+// Reads the control block back and waits for it; returns an input error or an expired wait.
+int sync_and_check(kt_engine* e);
 
 // Symmetric simple graph of an arbitrary entry list (directions merged, duplicates and self loops
 // dropped): (lo, hi) pairs in sorted order, then the same pairs reversed; synchronous.
@@ -188,8 +192,8 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
                  uint32_t tiles_per_dim, uint32_t* d_tile_src_ptr, uint32_t* d_src_out, uint32_t* d_dst_out);
 
 // kt_support.cu: support of every edge (triangles through it) into e->sup.
-// The credits lie in two arrays until merge_support adds them up (and their sum into the control
-// block's triangle counter, which must be zero).
+// The credits lie in two arrays until merge_support (or the list peel's bounds) adds them up, and their
+// sum into the control block's triangle counter, which the build cleared.
 int count_support(kt_engine* e);
 int merge_support(kt_engine* e);
 // Writes the triangle lists of the counted graph: list starts, and list ends (consumed).
@@ -198,9 +202,10 @@ int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends);
 // kt_peel.cu
 int peel_decompose(kt_engine* e);
 int peel_single_k(kt_engine* e, uint32_t k);
-// kt_lists.cu: the decomposition from triangle lists (prepare_lists says whether it applies).
-int prepare_lists(kt_engine* e, bool* use);
-int peel_lists(kt_engine* e);
+// kt_lists.cu: adds up the supports and decomposes from triangle lists where they apply (*done).
+int peel_lists(kt_engine* e, bool* done);
+// A list buffer for graphs of up to max_edges whose lists are made without reading the triangle count.
+void reserve_small_lists(kt_engine* e, uint64_t max_edges);
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max);
 int emit_keep(kt_engine* e, uint8_t* d_keep);
 int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, const uint32_t* d_offsets,

@@ -40,6 +40,7 @@
 // 4.2 -> 3.5.
 
 #include <algorithm>
+#include <cmath>
 
 #include "kt_engine.h"
 #include "kt_look.cuh"
@@ -443,6 +444,7 @@ __device__ __forceinline__ void run_chunks(const ListParams& P, ListShared& S, c
 __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_constant__ ListParams P) {
     __shared__ ListShared S;
     uint32_t* ctrl = P.ctrl;
+    if (__syncthreads_or(failed(ctrl))) return;  // the same for all blocks: set, if at all, by earlier kernels
     const uint32_t lane = lane_id();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nthreads = gridDim.x * blockDim.x;
@@ -660,30 +662,53 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
     }
 }
 
-// List starts (tptr[m] is the total) and ends: exclusive and inclusive prefix sums of the supports.
-__global__ void __launch_bounds__(kScanThreads) k_list_bounds(const uint32_t* __restrict__ sup, uint32_t m,
+// sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
+// total, three per triangle) and ends.
+__global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restrict__ sup,
+                                                              const uint32_t* __restrict__ supx,
+                                                              uint32_t* __restrict__ ycount, uint32_t m,
                                                               uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
                                                               Look L) {
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
+    if (__syncthreads_or(failed(L.ctrl))) return;
     const uint32_t tile = look_tile(L, &s_tile);
     if (tile == kNoTile) return;
     const uint64_t j0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint64_t sum = 0, end;
+    uint32_t y[kScanItems], v[kScanItems];
+    const bool whole = j0 + kScanItems <= m;
+    if (whole) {
+        const uint4 a = *reinterpret_cast<const uint4*>(sup + j0), b = *reinterpret_cast<const uint4*>(supx + j0);
+        y[0] = a.x, y[1] = a.y, y[2] = a.z, y[3] = a.w;
+        v[0] = a.x + b.x, v[1] = a.y + b.y, v[2] = a.z + b.z, v[3] = a.w + b.w;
+        *reinterpret_cast<uint4*>(ycount + j0) = a;
+        *reinterpret_cast<uint4*>(sup + j0) = make_uint4(v[0], v[1], v[2], v[3]);
+    } else {
 #pragma unroll
-    for (uint32_t i = 0; i < kScanItems; ++i) {
-        v[i] = j0 + i < m ? sup[j0 + i] : 0u;
-        sum += v[i];
+        for (uint32_t i = 0; i < kScanItems; ++i) {
+            y[i] = v[i] = 0;
+            if (j0 + i < m) {
+                y[i] = sup[j0 + i];
+                v[i] = y[i] + supx[j0 + i];
+                ycount[j0 + i] = y[i];
+                sup[j0 + i] = v[i];
+            }
+        }
     }
-    uint64_t at = tile_scan<uint64_t>(L, tile, sum, ws, &s_prefix, &end);
+    static_assert(kScanItems == 4, "four supports a thread");
+    uint64_t end;
+    uint64_t at = tile_scan<uint64_t>(L, tile, (uint64_t)v[0] + v[1] + v[2] + v[3], ws, &s_prefix, &end);
 #pragma unroll
     for (uint32_t i = 0; i < kScanItems; ++i) {
         if (j0 + i < m) {
             tptr[j0 + i] = at;
             at += v[i];
             ends[j0 + i] = at;
-            if (j0 + i == m - 1) tptr[m] = at;
+            if (j0 + i == m - 1) {
+                tptr[m] = at;
+                L.ctrl[kCtrlTriLo] = (uint32_t)at;
+                L.ctrl[kCtrlTriHi] = (uint32_t)(at >> 32);
+            }
         }
     }
 }
@@ -702,55 +727,78 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(const uint32_t* __
 #endif
 constexpr uint64_t kMaxListPerEdge = KT_LIST_PER_EDGE;
 
-// Whether the current graph's decomposition takes triangle lists; reads the triangle count (the
-// supports must be counted and summed on e->stream) and sizes the list buffer.
-int prepare_lists(kt_engine* e, bool* use) {
+// Graphs of up to this many edges take lists whatever their density: m edges have at most
+// (sqrt(2) / 3) m^1.5 triangles, so a buffer of 8.4 M entries (67 MB) holds their lists and the call
+// need not wait for the triangle count.
+constexpr uint32_t kSmallLists = 1u << 15;
+
+namespace {
+
+// At least three times the triangles that m edges can form.
+uint64_t most_entries(uint64_t m) { return (uint64_t)(1.41422 * (double)m * std::sqrt((double)m)) + 64; }
+
+bool grow_lists(kt_engine* e, uint64_t entries) {
+    if (e->lists) cudaFree(e->lists);
+    e->lists = nullptr;
+    e->list_cap = 0;
+    void* p = nullptr;
+    if (cudaMalloc(&p, entries * sizeof(uint2)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    e->lists = static_cast<uint2*>(p);
+    e->list_cap = entries;
+    return true;
+}
+
+// Whether the current graph takes lists; waits for its triangle count unless it is small, and sizes the
+// list buffer.
+int want_lists(kt_engine* e, bool* use) {
     *use = false;
-    if (!e->lists_allowed || e->m == 0) return KT_OK;
     int rc;
+    if (e->m <= kSmallLists && most_entries(e->m) <= e->list_cap) {
+        *use = true;
+        return KT_OK;
+    }
     uint64_t total = e->last.list_entries;  // a trusted run repeats a call that counted them
     if (!e->trusted) {
-        if ((rc = check_cuda(cudaMemcpyAsync(e->h_ctrl + kCtrlTriLo, e->ctrl + kCtrlTriLo, sizeof(uint64_t),
-                                             cudaMemcpyDeviceToHost, e->stream), "read triangle count")) ||
-            (rc = check_cuda(cudaStreamSynchronize(e->stream), "synchronize")))
-            return rc;
+        if ((rc = sync_and_check(e))) return rc;
         total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
         e->list_entries = total;
     }
     if (total > kMaxListPerEdge * e->m) return KT_OK;
     if (total > e->list_cap) {
         if (e->trusted) return KT_OK;
-        const uint64_t want = std::max<uint64_t>(total + total / 16, 1u << 20);
-        if ((rc = check_cuda(cudaStreamSynchronize(e->stream), "synchronize before resize"))) return rc;
+        const uint64_t want = total + total / 16;
         drop_replay(e);
-        if (e->lists) cudaFree(e->lists);
-        e->lists = nullptr;
-        e->list_cap = 0;
         size_t free_bytes = 0, all_bytes = 0;
         if ((rc = check_cuda(cudaMemGetInfo(&free_bytes, &all_bytes), "free device memory"))) return rc;
-        if (want * sizeof(uint2) > free_bytes / 2) return KT_OK;  // the rows are walked instead
-        void* p = nullptr;
-        if (cudaMalloc(&p, want * sizeof(uint2)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return KT_OK;
-        }
-        e->lists = static_cast<uint2*>(p);
-        e->list_cap = want;
+        if (want * sizeof(uint2) > (free_bytes + e->list_cap * sizeof(uint2)) / 2) return KT_OK;  // walk rows instead
+        if (!grow_lists(e, want)) return KT_OK;
     }
     *use = true;
     return KT_OK;
 }
 
-// Builds the lists of the current graph and peels it from them.
-int peel_lists(kt_engine* e) {
+}  // namespace
+
+void reserve_small_lists(kt_engine* e, uint64_t max_edges) {
+    const uint64_t want = most_entries(std::min<uint64_t>(max_edges, kSmallLists));
+    if (e->lists_allowed && want > e->list_cap) grow_lists(e, want);
+}
+
+int peel_lists(kt_engine* e, bool* done) {
     int rc;
     const uint32_t m = e->m;
     // the sort's key buffers are free after the build: list starts, and ends for the fill
     uint64_t* tptr = e->key_a;
     uint64_t* ends = e->key_b;
-    k_list_bounds<<<ceil_div(m, kScanTile), kScanThreads, 0, e->stream>>>(e->sup, m, tptr, ends, next_look(e));
+    k_list_bounds<<<ceil_div(m, kScanTile), kScanThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, m, tptr, ends,
+                                                                         next_look(e));
     count_launch(e);
-    if ((rc = check_launch(e, "k_list_bounds")) || (rc = fill_lists(e, tptr, ends))) return rc;
+    if ((rc = check_launch(e, "k_list_bounds")) || (rc = want_lists(e, done)) || !*done ||
+        (rc = fill_lists(e, tptr, ends)))
+        return rc;
     ListParams P;
     P.tri = e->lists;
     P.tptr = tptr;

@@ -42,7 +42,7 @@ __device__ __forceinline__ bool look_valid(unsigned long long w, uint32_t tag) {
     return (w >> 62) != 0 && ((uint32_t)(w >> 56) & 63u) == tag;
 }
 
-__device__ __forceinline__ bool timed_out(const uint32_t* ctrl) { return __ldcg(ctrl + kCtrlError) & kErrTimeout; }
+__device__ __forceinline__ bool timed_out(const uint32_t* ctrl) { return __ldca(ctrl + kCtrlError) & kErrTimeout; }
 
 // A waiting thread's bound: false when the wait should be given up.
 struct LookWait {

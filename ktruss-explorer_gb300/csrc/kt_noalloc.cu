@@ -104,16 +104,12 @@ extern "C" int kt_decompose_noalloc(const uint32_t* d_src, const uint32_t* d_dst
     kt_engine& e = d.engine;
     e.stream = static_cast<cudaStream_t>(stream);
     e.stats_ready = false;
-    if ((rc = kt::build_graph(&e, d_src, d_dst, num_entries, num_nodes)) || (rc = kt::count_support(&e)) ||
+    if ((rc = kt::build_graph(&e, d_src, d_dst, num_entries, num_nodes, false)) || (rc = kt::count_support(&e)) ||
         (rc = kt::peel_decompose(&e)) || (rc = kt::emit_truss_per_entry(&e, d_truss_per_entry, d_k_max)))
         return rc;
     // the call ends only when its GPU work has: then a peel wait that ran out is reported
-    if ((rc = kt::check_cuda(cudaMemcpyAsync(d.h_ctrl, e.ctrl, sizeof(uint32_t), cudaMemcpyDeviceToHost, e.stream),
-                             "read control word")) ||
-        (rc = kt::check_cuda(cudaStreamSynchronize(e.stream), "synchronize")))
-        return rc;
-    if (d.h_ctrl[kt::kCtrlError] & kt::kErrTimeout)
-        return kt::fail(KT_ERR_TIMEOUT, "a grid barrier wait of the peel kernel expired");
+    // (and an input error)
+    if ((rc = kt::sync_and_check(&e))) return rc;
     if (d.h_ctrl[kt::kCtrlError] & kt::kErrRunaway)
         return kt::fail(KT_ERR_INTERNAL, "the peel kernel exceeded its round or level bound");
     return KT_OK;

@@ -41,7 +41,6 @@
 
 #include <algorithm>
 #include <cstdlib>
-#include <vector>
 
 #include "kt_device.cuh"
 #include "kt_engine.h"
@@ -99,7 +98,7 @@ struct PeelParams {
     uint32_t* level_front;
     uint32_t cap_rounds;
     uint32_t cap_levels;
-    uint32_t n, m, big_row, tiny_row;
+    uint32_t n, m;
     uint32_t cw_shift;  // log2 of the chunk width (row entries per work chunk): 3, 4 or 5
     uint32_t compact_num;  // rows are compacted once alive edges < compact_num/100 of the count
                            // at the last compaction (0: never)
@@ -338,8 +337,7 @@ __device__ void compact_rows(const PeelParams& P, uint32_t r_done, uint32_t* war
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t big = P.big_row < P.n ? P.big_row : P.n;
-    const uint32_t tiny = P.tiny_row < big ? P.tiny_row : big;
+    const uint32_t big = min(__ldcg(P.ctrl + kCtrlBigRow), P.n), tiny = min(__ldcg(P.ctrl + kCtrlTinyRow), big);
     for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < tiny; row += gridDim.x * blockDim.x) {
         const uint32_t base = P.s_ptr[row], len = P.s_len[row];
         uint32_t w = 0;
@@ -451,6 +449,7 @@ template <int kBlocksPerSm>
 __global__ void __launch_bounds__(peel_threads<kBlocksPerSm>(), kBlocksPerSm) k_peel(PeelParams P) {
     __shared__ uint32_t warp_cnt[peel_threads<kBlocksPerSm>() / 32];
     uint32_t* ctrl = P.ctrl;
+    if (__syncthreads_or(failed(ctrl))) return;  // the same for all blocks: set, if at all, by earlier kernels
     if (threadIdx.x == 0) {
         if (P.d_sched) {
             const uint32_t w = P.d_sched[1];
@@ -484,6 +483,8 @@ __global__ void __launch_bounds__(peel_threads<kBlocksPerSm>(), kBlocksPerSm) k_
     if (leader) {
         for (int i = 0; i < 6; ++i) phase_ns[i] = 0;
         phase_ns[6] = global_ns();
+        // the build cleared the control block; the rings of minima start high
+        for (int i = 0; i < 4; ++i) ctrl[kPLMin + i] = ctrl[kPLMinId + i] = 0xffffffffu;
     }
     uint32_t compactions = 0;
 #define KT_PHASE(kind)                                   \
@@ -743,25 +744,69 @@ __global__ void k_barrier_probe(uint32_t* ctrl, uint64_t timeout_ns) {
     grid_barrier(ctrl, gridDim.x + 1, timeout_ns);
 }
 
-__global__ void k_init_peel_ctrl(uint32_t* ctrl) {
-    const uint32_t i = threadIdx.x;
-    if (i >= kPBarCount && i < kPSched)
-        ctrl[i] = (i >= kPLMin && i < kPLMin + 4) || (i >= kPLMinId && i < kPLMinId + 4) ? 0xffffffffu : 0u;
+// The passes that the reference's chained schedule takes for the decomposition in the round log, and
+// the alive edges they see: level 3 is one pass over all m edges; each level k >= 4 up to k_max+1
+// takes one pass per removing round plus a final one, each seeing the edges alive at its start;
+// levels that remove nothing take one pass each.  One block; counting along in the peel kernels
+// instead cost their rounds 1-3 %.
+__device__ void count_passes(const uint32_t* __restrict__ size, const uint32_t* __restrict__ level, uint32_t rounds,
+                             uint32_t m, uint32_t* __restrict__ ctrl) {
+    __shared__ uint32_t removed[kThreads];
+    __shared__ unsigned long long sums[2];
+    const uint32_t per = (rounds + kThreads - 1) / kThreads;
+    const uint32_t a = 1 + threadIdx.x * per, b = min(a + per, rounds + 1);  // rounds are logged from 1 on
+    uint32_t sum = 0;
+    for (uint32_t i = a; i < b; ++i) sum += size[i];
+    removed[threadIdx.x] = sum;
+    if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t alive = m;
+    for (uint32_t t = 0; t < threadIdx.x; ++t) alive -= removed[t];
+    unsigned long long passes = threadIdx.x == 0 ? 1 : 0, seen = threadIdx.x == 0 ? m : 0;
+    for (uint32_t i = a; i < b; ++i) {
+        const uint32_t k = level[i], before = i > 1 ? level[i - 1] : 2u;
+        const uint32_t next = before + 1 > 4 ? before + 1 : 4u;  // the first level after the last one
+        if (before != k && k > next) {
+            passes += k - next;
+            seen += (unsigned long long)(k - next) * alive;
+        }
+        const bool last = i == rounds || level[i + 1] != k;
+        if (k >= 4) {
+            passes += last ? 2 : 1;
+            seen += (unsigned long long)alive + (last ? alive - size[i] : 0u);
+        }
+        alive -= size[i];
+    }
+    atomicAdd(&sums[0], passes);
+    atomicAdd(&sums[1], seen);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ctrl[kPPasses] = (uint32_t)sums[0];
+        ctrl[kPAliveSum] = (uint32_t)sums[1];
+        ctrl[kPAliveSum + 1] = (uint32_t)(sums[1] >> 32);
+    }
 }
 
-__global__ void k_emit_truss(const uint32_t* __restrict__ entry_eid, uint64_t entries, const uint32_t* __restrict__ tr,
-                             uint32_t* __restrict__ out) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kThreads) k_emit_truss(const uint32_t* __restrict__ entry_eid, uint64_t entries,
+                                                         const uint32_t* __restrict__ tr, uint32_t* __restrict__ out,
+                                                         uint32_t* __restrict__ k_max,
+                                                         const uint32_t* __restrict__ round_size,
+                                                         const uint32_t* __restrict__ round_level, uint32_t cap_rounds,
+                                                         uint32_t m, uint32_t* __restrict__ ctrl) {
+    if (failed(ctrl)) return;  // the same for the whole launch
+    if (blockIdx.x == 0 && ctrl[kPRounds] < cap_rounds)
+        count_passes(round_size, round_level, ctrl[kPRounds], m, ctrl);
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < entries) out[i] = tr[entry_eid[i]];
+    if (i == 0 && k_max) *k_max = ctrl[kPKmax];
 }
 
 __global__ void k_emit_keep(const uint32_t* __restrict__ entry_eid, uint64_t entries, const uint32_t* __restrict__ rnd,
-                            uint8_t* __restrict__ out) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                            uint8_t* __restrict__ out, const uint32_t* __restrict__ ctrl) {
+    if (failed(ctrl)) return;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < entries) out[i] = rnd[entry_eid[i]] == 0 ? 1 : 0;
 }
-
-__global__ void k_copy_u32(uint32_t* dst, const uint32_t* src) { *dst = *src; }
 
 // Graph of vertex s: the last g with offsets[g] <= s (num_graphs when s is past the last range,
 // 0xffffffff when it is below the first).
@@ -792,6 +837,7 @@ __global__ void k_graph_kmax(const uint32_t* __restrict__ src, const uint32_t* _
                              const uint32_t* __restrict__ offsets, uint32_t num_graphs,
                              const uint32_t* __restrict__ truss, uint32_t* __restrict__ kmax,
                              uint32_t* __restrict__ ctrl) {
+    if (__ldca(ctrl + kCtrlError) & ~kErrCrossGraph) return;  // bits that this kernel does not set
     const uint32_t lane = lane_id();
     const uint64_t gwarp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -854,9 +900,6 @@ __global__ void k_fill_edges(uint32_t m, uint32_t value, uint32_t* __restrict__ 
 
 int launch_peel(kt_engine* e, uint32_t single_k) {
     int rc;
-    k_init_peel_ctrl<<<1, kCtrlWords, 0, e->stream>>>(e->ctrl);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_init_peel_ctrl"))) return rc;
     int l2 = 0;
     if ((rc = check_cuda(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, e->device), "L2 size"))) return rc;
     // automatic choice: two blocks per SM when the oriented CSR outgrows L2 - but not for a batch,
@@ -900,8 +943,6 @@ int launch_peel(kt_engine* e, uint32_t single_k) {
     P.cap_levels = e->cap_levels;
     P.n = e->n;
     P.m = e->m;
-    P.big_row = e->big_row;
-    P.tiny_row = e->tiny_row < e->big_row ? e->tiny_row : e->big_row;
     P.cw_shift = e->sched.chunk_width == 8 ? 3u : e->sched.chunk_width == 16 ? 4u : 5u;
     P.compact_num = e->sched.compact_percent;
     P.recount_num = e->sched.recount_percent;
@@ -923,13 +964,6 @@ int launch_peel(kt_engine* e, uint32_t single_k) {
     return check_cuda(cudaEventRecord(e->ev_peel1, e->stream), "record event");
 }
 
-int triangles(kt_engine* e) {
-    unsigned long long* tot = reinterpret_cast<unsigned long long*>(e->ctrl + kCtrlTriLo);
-    int rc = check_cuda(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), e->stream), "clear triangle counter");
-    if (rc) return rc;
-    return e->m ? merge_support(e) : KT_OK;
-}
-
 }  // namespace
 
 int peel_decompose(kt_engine* e) {
@@ -937,11 +971,14 @@ int peel_decompose(kt_engine* e) {
     e->peel_timed = false;
     e->peel_mode = 0;
     e->stats_ready = false;
-    if ((rc = triangles(e))) return rc;
     if (e->m == 0) return KT_OK;
-    bool lists = false;
-    if ((rc = prepare_lists(e, &lists))) return rc;
-    return lists ? peel_lists(e) : launch_peel(e, 0);
+    bool done = false;
+    if (e->lists_allowed) {
+        if ((rc = peel_lists(e, &done)) || done) return rc;
+    } else if ((rc = merge_support(e))) {
+        return rc;
+    }
+    return launch_peel(e, 0);
 }
 
 int peel_single_k(kt_engine* e, uint32_t k) {
@@ -949,8 +986,8 @@ int peel_single_k(kt_engine* e, uint32_t k) {
     e->peel_timed = false;
     e->peel_mode = 1;
     e->stats_ready = false;
-    if (k >= 3 && (rc = triangles(e))) return rc;
     if (e->m == 0) return KT_OK;
+    if (k >= 3 && (rc = merge_support(e))) return rc;
     if (k < 3) {
         // k = 2 keeps every edge; k < 2 removes every edge (k-2 wraps as unsigned, as in
         // mark_deleted_edges_kernel, kernel_ddc.cu:64)
@@ -965,19 +1002,12 @@ int peel_single_k(kt_engine* e, uint32_t k) {
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max) {
     int rc;
     if (e->entries) {
-        k_emit_truss<<<grid_for(e->entries), kThreads, 0, e->stream>>>(e->entry_eid, e->entries, e->tr, d_out);
+        k_emit_truss<<<grid_for(e->entries), kThreads, 0, e->stream>>>(
+            e->entry_eid, e->entries, e->tr, d_out, d_k_max, e->round_size, e->round_level, e->cap_rounds, e->m, e->ctrl);
         count_launch(e);
-        if ((rc = check_launch(e, "k_emit_truss"))) return rc;
+        return check_launch(e, "k_emit_truss");
     }
-    if (d_k_max) {
-        if (e->m) {
-            k_copy_u32<<<1, 1, 0, e->stream>>>(d_k_max, e->ctrl + kPKmax);
-        } else {
-            if ((rc = check_cuda(cudaMemsetAsync(d_k_max, 0, sizeof(uint32_t), e->stream), "clear k_max"))) return rc;
-        }
-        count_launch(e);
-        if ((rc = check_launch(e, "k_copy_u32"))) return rc;
-    }
+    if (d_k_max && (rc = check_cuda(cudaMemsetAsync(d_k_max, 0, sizeof(uint32_t), e->stream), "clear k_max"))) return rc;
     return KT_OK;
 }
 
@@ -995,16 +1025,13 @@ int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, 
 
 int emit_keep(kt_engine* e, uint8_t* d_keep) {
     if (!e->entries) return KT_OK;
-    k_emit_keep<<<grid_for(e->entries), kThreads, 0, e->stream>>>(e->entry_eid, e->entries, e->rnd, d_keep);
+    k_emit_keep<<<grid_for(e->entries), kThreads, 0, e->stream>>>(e->entry_eid, e->entries, e->rnd, d_keep, e->ctrl);
     count_launch(e);
     return check_launch(e, "k_emit_keep");
 }
 
-// Reads the control block and the round log after the stream has drained; fills the peel
-// statistics, including the pass statistics of the reference's chained schedule: level 3 is
-// one pass over all m edges; each level k >= 4 up to k_max+1 takes one pass per removing round
-// plus a final pass, each seeing the edges alive at its start; levels that remove nothing take
-// one pass each.
+// Reads the control block (unless the call left it in h_ctrl) after the stream has drained; fills the
+// peel statistics.
 int finish_stats(kt_engine* e) {
     if (e->stats_ready) return KT_OK;
     if (e->replay_timing) {  // the stream has drained: the replay's events are complete
@@ -1025,9 +1052,11 @@ int finish_stats(kt_engine* e) {
         e->stats_ready = true;
         return KT_OK;
     }
-    int rc = check_cuda(cudaMemcpy(e->h_ctrl, e->ctrl, sizeof(uint32_t) * kCtrlWords, cudaMemcpyDeviceToHost),
-                        "read control block");
-    if (rc) return rc;
+    int rc;
+    if (!e->ctrl_fresh && (rc = check_cuda(cudaMemcpy(e->h_ctrl, e->ctrl, sizeof(uint32_t) * kCtrlWords,
+                                                      cudaMemcpyDeviceToHost), "read control block")))
+        return rc;
+    e->ctrl_fresh = true;
     const uint32_t err = e->h_ctrl[kCtrlError];
     if (err & kErrTimeout) return fail(KT_ERR_TIMEOUT, "a grid barrier wait of the peel kernel expired");
     if (err & kErrRunaway) return fail(KT_ERR_INTERNAL, "the peel kernel exceeded its round or level bound");
@@ -1052,38 +1081,15 @@ int finish_stats(kt_engine* e) {
     for (int i = 0; i < 6; ++i)
         e->stats.peel_phase_ms[i] =
             (float)(((uint64_t)e->h_ctrl[kPPhaseNs + 2 * i + 1] << 32 | e->h_ctrl[kPPhaseNs + 2 * i]) * 1e-6);
-    e->stats.plain_passes = 0;
-    e->stats.plain_alive_sum = 0;
-    const uint32_t R = e->stats.num_rounds;
-    if (e->peel_mode == 0 && m && R < e->cap_rounds) {
-        std::vector<uint32_t> size(R + 1), lvl(R + 1);
-        if (R && ((rc = check_cuda(cudaMemcpy(size.data(), e->round_size, sizeof(uint32_t) * (R + 1),
-                                              cudaMemcpyDeviceToHost), "read round log")) ||
-                  (rc = check_cuda(cudaMemcpy(lvl.data(), e->round_level, sizeof(uint32_t) * (R + 1),
-                                              cudaMemcpyDeviceToHost), "read round log"))))
-            return rc;
-        uint64_t alive = m, passes = 1, alive_sum = m;
-        uint32_t next_k = 3;
-        for (uint32_t r = 1; r <= R;) {
-            const uint32_t k = lvl[r];
-            if (k < next_k || k > e->stats.k_max + 1) return fail(KT_ERR_INTERNAL, "inconsistent round log");
-            for (uint32_t kk = next_k > 4 ? next_k : 4; kk < k; ++kk) { passes++; alive_sum += alive; }
-            while (r <= R && lvl[r] == k) {
-                if (k >= 4) { passes++; alive_sum += alive; }
-                alive -= size[r];
-                ++r;
-            }
-            if (k >= 4) { passes++; alive_sum += alive; }
-            next_k = k + 1;
-        }
-        e->stats.plain_passes = (uint32_t)passes;
-        e->stats.plain_alive_sum = alive_sum;
-    }
+    const bool full = e->peel_mode == 0 && m;
+    e->stats.plain_passes = full ? e->h_ctrl[kPPasses] : 0;
+    e->stats.plain_alive_sum = full ? (uint64_t)e->h_ctrl[kPAliveSum + 1] << 32 | e->h_ctrl[kPAliveSum] : 0;
     e->stats_ready = true;
     return KT_OK;
 }
 
 int barrier_timeout_probe(kt_engine* e, uint64_t timeout_ns) {
+    e->ctrl_fresh = false;
     int rc = check_cuda(cudaMemsetAsync(e->ctrl, 0, sizeof(uint32_t) * kCtrlWords, e->stream), "clear control block");
     if (rc) return rc;
     uint32_t* ctrl = e->ctrl;

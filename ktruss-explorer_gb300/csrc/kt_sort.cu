@@ -238,6 +238,7 @@ int launch_pass(kt_engine* e, const uint64_t* kin, const uint32_t* vin, uint64_t
 int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words) {
     if (words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
     e->look_tag = e->look_count = 0;
+    e->ctrl_fresh = false;
     const uint64_t work = std::max<uint64_t>(words / 2, std::max<uint32_t>(deg_words, kCountWords));
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((work + 255) / 256, (uint64_t)e->num_sms * 8);
     k_session<<<blocks, 256, 0, e->stream>>>(e->ctrl, kCtrlWords, n, e->deg, deg_words,

@@ -71,6 +71,7 @@ constexpr uint32_t kMidItems = 21, kMidBases = 22, kMidCursor = 23;  // 23 count
 constexpr uint32_t kRowItems = 26, kRowCursor = 27;
 
 struct Graph {
+    const uint32_t* ctrl;
     const uint32_t* __restrict__ o_ptr;
     const uint32_t* __restrict__ o_col;
     const uint32_t* __restrict__ e_src;
@@ -167,12 +168,14 @@ __device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
 
 template <int G, bool kFill>
 __global__ void __launch_bounds__(kThreads) k_support(Graph g, Credits c) {
+    if (failed(g.ctrl)) return;
     edge_body<G, kFill>(g, c);
 }
 
 // The same count with the lane group read from the control block, where the learned selector's
 // inference kernel wrote its choice: the schedule is chosen on the device, with no host read.
 __global__ void __launch_bounds__(kThreads) k_support_chosen(Graph g, Credits c, const uint32_t* __restrict__ sched) {
+    if (failed(g.ctrl)) return;
     switch (sched[0]) {
         case 4: edge_body<4, false>(g, c); break;
         case 16: edge_body<16, false>(g, c); break;
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(kThreads) k_support_chosen(Graph g, Credits c,
 // most 2m words of bases.  Also lists the rows of the fill's row blocks.
 __global__ void k_middle_plan(Graph g, uint4* __restrict__ items, uint32_t* __restrict__ rows,
                               uint32_t* __restrict__ ctrl) {
+    if (failed(ctrl)) return;
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t row = v < g.n ? g.o_ptr[v + 1] - g.o_ptr[v] : 0u;
     const uint32_t listed = __ballot_sync(kFullMask, row_block(row));
@@ -216,7 +220,7 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
     const uint32_t lane = lane_id(), glane = lane & (G - 1);
     const uint32_t gmask = ((1u << G) - 1) << (lane & ~(uint32_t)(G - 1));
     const uint32_t group = threadIdx.x / G;
-    const uint32_t n_items = ctrl[kMidItems];
+    const uint32_t n_items = failed(ctrl) ? 0u : ctrl[kMidItems];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(ctrl + kMidCursor + (kFill ? 1 : 0), 1u);
         __syncthreads();
@@ -307,7 +311,7 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
     constexpr int G = kRowGroup;
     const uint32_t lane = lane_id(), glane = lane & (G - 1);
     const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << (lane & ~(uint32_t)(G - 1)));
-    const uint32_t group = threadIdx.x / G, n_rows = ctrl[kRowItems];
+    const uint32_t group = threadIdx.x / G, n_rows = failed(ctrl) ? 0u : ctrl[kRowItems];
     for (;;) {
         if (threadIdx.x == 0) {
             const uint32_t t = atomicAdd(ctrl + kRowCursor, 1u);
@@ -386,7 +390,8 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
 
 // sup += supx, what it was into ycount, and the sum of all supports (three per triangle).
 __global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __restrict__ supx,
-                                uint32_t* __restrict__ ycount, uint32_t m, unsigned long long* __restrict__ total) {
+                                uint32_t* __restrict__ ycount, uint32_t m, uint32_t* __restrict__ ctrl) {
+    if (failed(ctrl)) return;
     uint64_t s = 0;
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t y = sup[j], v = y + supx[j];
@@ -395,14 +400,15 @@ __global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __re
         s += v;
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
-    if (lane_id() == 0 && s) atomicAdd(total, (unsigned long long)s);
+    if (lane_id() == 0 && s)
+        atomicAdd(reinterpret_cast<unsigned long long*>(ctrl + kCtrlTriLo), (unsigned long long)s);
 }
 
 Graph graph_of(const kt_engine* e) {
     // the choice must be the same in the count and in the fill of one call
     const bool hash_all = !e->sched_on_device && e->sched.support_group == 0;
     const uint32_t mid_in = hash_all ? 1u : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? 1u : kMidOut;
-    return Graph{e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out};
+    return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out};
 }
 
 // The items lie in the first chunk buffer, the claims in the second, the rows in the first queue:
@@ -461,8 +467,7 @@ int count_support(kt_engine* e) {
 }
 
 int merge_support(kt_engine* e) {
-    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(
-        e->sup, e->rnd, e->tr, e->m, reinterpret_cast<unsigned long long*>(e->ctrl + kCtrlTriLo));
+    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, e->m, e->ctrl);
     count_launch(e);
     return check_launch(e, "k_merge_support");
 }

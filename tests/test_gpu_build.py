@@ -67,3 +67,52 @@ def test_rows_without_entries(factor, size):
             eng.ktruss(d_src.data_ptr(), d_dst.data_ptr(), len(src), n, k, keep.data_ptr())
             assert np.array_equal(keep.cpu().numpy().astype(bool), ref["truss"] >= k), (directedness, k)
     eng.close()
+
+
+def _broken(src, dst, n, what):
+    src, dst = src.copy(), dst.copy()
+    i = len(src) // 3
+    if what == "bad vertex":
+        dst[i] = n + 7
+    elif what == "self loop":
+        src[i] = dst[i]
+    elif what == "duplicate":  # both directions of an edge twice, another edge gone
+        half = len(src) // 2
+        src[0], dst[0], src[half], dst[half] = src[i], dst[i], dst[i], src[i]
+    else:  # one direction missing, its slot filled with a new edge's one direction
+        dst[i] = (dst[i] + 1) % n if (dst[i] + 1) % n != src[i] else (dst[i] + 2) % n
+    return src, dst
+
+
+@pytest.mark.parametrize("size", [300, 6000, 40000])
+@pytest.mark.parametrize("what,status", [("bad vertex", 1), ("self loop", 2), ("duplicate", 3), ("asymmetric", 3)])
+def test_refused_inputs(size, what, status):
+    """Input errors are read once a call, after the kernels behind the build were launched: they are
+    still the call's status, nothing is written, and the engine keeps working."""
+    torch = pytest.importorskip("torch")
+    n, u, v = kt.gen_ba(size, 8, 9)
+    src, dst = both_directions(u, v)
+    b_src, b_dst = _broken(src, dst, n, what)
+    eng = kt.Engine(0)
+    good = [_cuda(torch, x) for x in (src, dst)]
+    bad = [_cuda(torch, x) for x in (b_src, b_dst)]
+    truss = torch.full((len(src),), 77, dtype=torch.int32, device="cuda")
+    keep = torch.full((len(src),), 77, dtype=torch.uint8, device="cuda")
+    k_max = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    off = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    s, d = (x.data_ptr() for x in bad)
+    calls = [lambda: eng.decompose(s, d, len(src), n, truss.data_ptr(), k_max.data_ptr()),
+             lambda: eng.ktruss(s, d, len(src), n, 4, keep.data_ptr()),
+             lambda: eng.decompose_batch(s, d, len(src), n, off.data_ptr(), 1, truss.data_ptr(), k_max.data_ptr())]
+    if len(src) <= 1 << 19:
+        calls.append(lambda: kt.decompose_noalloc(s, d, len(src), n, truss.data_ptr(), k_max.data_ptr()))
+    for i, call in enumerate(calls):
+        with pytest.raises(kt.KtrussError) as ei:
+            call()
+        assert ei.value.status == status, i
+        assert bool((truss == 77).all()) and bool((keep == 77).all())
+    eng.decompose(good[0].data_ptr(), good[1].data_ptr(), len(src), n, truss.data_ptr(), k_max.data_ptr())
+    ref = oracle.decompose(n, src, dst, method="peel")
+    assert np.array_equal(truss.cpu().numpy().view(np.uint32), ref["truss"]) and int(k_max.item()) == ref["k_max"]
+    eng.close()
