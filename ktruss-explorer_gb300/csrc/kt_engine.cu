@@ -420,6 +420,7 @@ int kt_engine_destroy(kt_engine* e) {
     if (e->arena) cudaFree(e->arena);
     if (e->aux) cudaFree(e->aux);
     if (e->tile_off) cudaFree(e->tile_off);
+    if (e->ingest) cudaFree(e->ingest);
     if (e->lists) cudaFree(e->lists);
     if (e->ctrl) cudaFree(e->ctrl);
     if (e->h_ctrl) cudaFreeHost(e->h_ctrl);

@@ -87,6 +87,8 @@ struct kt_engine {
     size_t aux_words = 0;
     uint32_t* tile_off = nullptr;  // tiled variant: first oriented position of each (vertex, column tile)
     size_t tile_off_words = 0;     //   (own allocation, made by the first tiled call)
+    unsigned long long* ingest = nullptr;  // TSV ingest: outcome, tokens before each tile
+    uint64_t ingest_words = 0;             //   (own allocation, made by the first ingest)
     uint2* lists = nullptr;        // triangle lists of a decomposition (own allocation, kt_lists.cu)
     uint64_t list_cap = 0;         //   entries it holds
     uint64_t list_entries = 0;     //   entries of the last call (three per triangle)
