@@ -52,8 +52,20 @@ enum : uint32_t {
     kPAliveSum = 82,   // u64 (words 82..83): the alive edges they see
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
-    kCtrlWords = 128,  // words 88-115: the list peel (kt_lists.cu)
+    // words 88-115: the list peel (kt_lists.cu)
+    kPruneFront = 116,  // single-k: edges whose counted support is too small (the first round's frontier)
+    kPruneLeft = 117,   //   the others, when these were counted again (recount_pruned)
+    kPruneT0 = 118,     //   u64 (words 118..119): when that began
+    kPrunePlan = 120,   //   items, bases and cursor of its plan
+    kCtrlWords = 128,
 };
+
+// Whether a single-k call's first round is run by recount_pruned instead of the peel kernel: the
+// frontier holds at least `percent` (0: never) of the m edges.  The word is final before the kernels that
+// ask start, so it may come from L1 (every thread of a large grid reads it).
+__device__ __forceinline__ bool pruned_first(const uint32_t* ctrl, uint32_t m, uint32_t percent) {
+    return percent != 0 && (uint64_t)__ldca(ctrl + kPruneFront) * 100 >= (uint64_t)percent * m;
+}
 
 // Schedule i of the autotuner's grid (kt_schedule_grid): support group {4, 8, 16} x chunk width
 // {8, 16, 32} x compaction {0, 85} x recount {0, 50}, the last varying fastest.  Shared by the host

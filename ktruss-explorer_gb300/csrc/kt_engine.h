@@ -197,7 +197,17 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
 // The credits lie in two arrays until merge_support (or the list peel's bounds) adds them up, and their
 // sum into the control block's triangle counter, which the build cleared.
 int count_support(kt_engine* e);
-int merge_support(kt_engine* e);
+int merge_support(kt_engine* e, uint32_t limit);
+
+// Counts the edges left by a single-k call's first round again if that round removes `percent` or more
+// of them (decided on the device; percent 0 in *out: never).  new_id: the edge's number among those
+// left, or its top bit; count: their supports.
+struct PrunedCount {
+    uint32_t percent;
+    const uint32_t* new_id;
+    const uint32_t* count;
+};
+int recount_pruned(kt_engine* e, uint32_t limit, uint32_t percent, PrunedCount* out);
 // Writes the triangle lists of the counted graph: list starts, and list ends (consumed).
 int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends);
 

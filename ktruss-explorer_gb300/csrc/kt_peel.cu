@@ -26,7 +26,9 @@
 // fences (every 32nd column, an array that stays in L2), then in one block of at most 32 entries,
 // so a search misses L2 once or twice however long the row.  A round whose
 // frontier holds at least the schedule's recount share of the alive edges instead removes the
-// frontier at once and recounts the survivors' support (the reference's full recount).  A removed
+// frontier at once and recounts the survivors' support (the reference's full recount); where that is
+// the first round of a single-k call on a large graph, the support count's kernels have done it before
+// this kernel starts (recount_pruned), and the rows are compacted first.  A removed
 // edge's support is set to kDead, so a level's scan of the alive list reads one array; that scan
 // also collects the frontier of level k_last+1, and only when that level turns out to be empty
 // does a second pass collect the frontier of the next non-empty level.
@@ -104,6 +106,7 @@ struct PeelParams {
                            // at the last compaction (0: never)
     uint32_t recount_num;  // a round whose frontier holds >= recount_num % of the alive edges
                            // recounts the survivors' support instead of decrementing (0: never)
+    PrunedCount pruned;  // the first round of a single-k call may have been run before this kernel
     uint32_t single_k;  // 0: full decomposition; >= 3: the k of a single-k truss
     const uint32_t* d_sched;  // non-null: chunk width, compaction and recount from these control
                               // words (the selector's on-device choice) instead of the three above
@@ -498,9 +501,13 @@ __global__ void __launch_bounds__(peel_threads<kBlocksPerSm>(), kBlocksPerSm) k_
     // a round's closing barrier covers the round's queued chunks, each of at most 1 << cw_shift row
     // entries (read at its start; the count includes chunks that overflowed to the block queue)
     const uint64_t phase_wait = P.wait_base_ns + P.wait_ns_per_unit * 2ull * P.m;
+    const bool pre = P.single_k != 0 && pruned_first(ctrl, P.m, P.pruned.percent);
     for (uint64_t j = tid; j < P.m; j += nthreads) {
-        P.rnd[j] = 0;
-        P.tr[j] = 0;
+        const uint32_t id = pre ? P.pruned.new_id[j] : 0u;  // (in the place of tr[j])
+        const bool gone = id >> 31;
+        P.rnd[j] = gone ? 1u : 0u;
+        P.tr[j] = gone ? P.single_k - 1 : 0u;
+        if (pre) P.sup[j] = gone ? kDead : P.pruned.count[id];
     }
     if (!peel_barrier(ctrl, nblocks, phase_wait)) return;
     KT_PHASE(0)
@@ -510,6 +517,20 @@ __global__ void __launch_bounds__(peel_threads<kBlocksPerSm>(), kBlocksPerSm) k_
     // first frontier goes to slot (r+2) & 3.  `rounds` counts the rounds actually run.
     uint32_t r = 0, rounds = 0, level = 0, k = 3, k_last = 2;
     uint32_t live = P.m, live_at_compaction = P.m;  // alive edges now and at the last compaction
+    if (pre) {  // round 1, stamp 1: the frontier is removed and the others are counted
+        const uint32_t E = __ldcg(ctrl + kPruneFront);
+        rounds = 1;
+        live -= E;
+        if (leader) {
+            const uint64_t took = phase_ns[6] - ld_acquire_u64(reinterpret_cast<const unsigned long long*>(ctrl + kPruneT0));
+            phase_ns[4] += took - phase_ns[0];
+            if (P.cap_rounds > 1) {
+                P.round_size[1] = E;
+                P.round_level[1] = P.single_k;
+                P.round_ns[1] = (uint32_t)took;
+            }
+        }
+    }
 #define KT_MAX_STAMP (2ull * P.m + 8)
     for (;;) {
         const uint32_t ls = level & 3;
@@ -613,7 +634,7 @@ __global__ void __launch_bounds__(peel_threads<kBlocksPerSm>(), kBlocksPerSm) k_
             P.level_k[level] = k;
             P.level_alive[level] = P.single_k ? P.m : ld_acquire(ctrl + kPLAlive + ls);
             P.level_ns[level] = (uint32_t)(global_ns() - phase_ns[7]);
-            P.level_front[level] = E;
+            P.level_front[level] = pre ? P.m - live : E;
         }
         uint32_t C = (uint32_t)min(ld_acquire_u64(chunk_ctr + (rr & 3)), (unsigned long long)P.cap_chunks);
         while (E) {
@@ -898,7 +919,7 @@ __global__ void k_fill_edges(uint32_t m, uint32_t value, uint32_t* __restrict__ 
     if (j < m) rnd[j] = value;
 }
 
-int launch_peel(kt_engine* e, uint32_t single_k) {
+int launch_peel(kt_engine* e, uint32_t single_k, const PrunedCount& pruned = {}) {
     int rc;
     int l2 = 0;
     if ((rc = check_cuda(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, e->device), "L2 size"))) return rc;
@@ -947,6 +968,7 @@ int launch_peel(kt_engine* e, uint32_t single_k) {
     P.compact_num = e->sched.compact_percent;
     P.recount_num = e->sched.recount_percent;
     P.single_k = single_k;
+    P.pruned = pruned;
     P.d_sched = e->sched_on_device ? e->ctrl + kPSched : nullptr;
     P.wait_base_ns = e->wait_base_ns;
     P.wait_ns_per_unit = e->wait_ns_per_unit;
@@ -975,7 +997,7 @@ int peel_decompose(kt_engine* e) {
     bool done = false;
     if (e->lists_allowed) {
         if ((rc = peel_lists(e, &done)) || done) return rc;
-    } else if ((rc = merge_support(e))) {
+    } else if ((rc = merge_support(e, 0))) {
         return rc;
     }
     return launch_peel(e, 0);
@@ -987,7 +1009,7 @@ int peel_single_k(kt_engine* e, uint32_t k) {
     e->peel_mode = 1;
     e->stats_ready = false;
     if (e->m == 0) return KT_OK;
-    if (k >= 3 && (rc = merge_support(e))) return rc;
+    if (k >= 3 && (rc = merge_support(e, k - 2))) return rc;
     if (k < 3) {
         // k = 2 keeps every edge; k < 2 removes every edge (k-2 wraps as unsigned, as in
         // mark_deleted_edges_kernel, kernel_ddc.cu:64)
@@ -996,7 +1018,10 @@ int peel_single_k(kt_engine* e, uint32_t k) {
         count_launch(e);
         return check_launch(e, "k_fill_edges");
     }
-    return launch_peel(e, k);
+    // (at k = 3 the frontier's edges are in no triangle, so nothing has to be counted again)
+    PrunedCount pruned;
+    if ((rc = recount_pruned(e, k - 2, k > 3 ? e->sched.recount_percent : 0, &pruned))) return rc;
+    return launch_peel(e, k, pruned);
 }
 
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max) {

@@ -35,8 +35,8 @@
 
 #include <algorithm>
 
-#include "kt_device.cuh"
 #include "kt_engine.h"
+#include "kt_look.cuh"
 
 namespace kt {
 
@@ -65,9 +65,11 @@ constexpr uint32_t kRowFactor = 6;
 // Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save
 // (R-MAT 14 with 220,000 edges counts in 0.05 ms).
 constexpr uint32_t kMidMinEdges = 1u << 18;
+constexpr uint32_t kPruneMin = 1u << 19, kPruneEarly = 1u << 20;  // edges (see recount_pruned)
 constexpr uint32_t kEmpty = 0xffffffffu;
 // control words of the plan, zero since the build
-constexpr uint32_t kMidItems = 21, kMidBases = 22, kMidCursor = 23;  // 23 count, 24 fill
+constexpr uint32_t kMidPlan = 21;  // items, bases, count cursor, fill cursor
+constexpr uint32_t kPlanBases = 1, kPlanCursor = 2;
 constexpr uint32_t kRowItems = 26, kRowCursor = 27;
 
 struct Graph {
@@ -82,6 +84,11 @@ struct Graph {
     uint32_t n, m;
     uint32_t mid_in;   // vertices with this many in-edges are vertex-centric (0: none) ...
     uint32_t mid_out;  // ... if their row has this many entries
+    uint32_t plan;     // first control word of the plan
+    // The edges left by a first round (recount_pruned): o_ptr, o_col and e_src are theirs, m is the
+    // edges of the whole graph, which s_ptr .. s_eid describe; new_id[j] is what became of edge j.
+    uint32_t percent;
+    const uint32_t* __restrict__ new_id;
 };
 
 // Where counts go, and what the fill reads.
@@ -99,17 +106,26 @@ __device__ __forceinline__ bool vertex_centric(const Graph& g, uint32_t v, uint3
     return g.mid_in != 0 && row >= g.mid_out && row <= kMidRow && g.s_split[v] - g.s_ptr[v] >= g.mid_in;
 }
 
+constexpr uint32_t kGone = 0x80000000u;  // in new_id: removed (the low bits number the edges left before it)
+
+// Nothing to do: the input was refused, or the first round is the peel's (kPruned).
+template <bool kPruned>
+__device__ __forceinline__ bool skip(const Graph& g) {
+    return failed(g.ctrl) || (kPruned && !pruned_first(g.ctrl, g.m, g.percent));
+}
+
 // Rows long enough for a row block of the fill (k_rows).
 __device__ __forceinline__ bool row_block(uint32_t row) { return row >= kRowMin && row <= kMidRow; }
 
-template <int G, bool kFill>
+template <int G, bool kFill, bool kPruned = false>
 __device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
     const uint32_t lane = lane_id();
     const uint32_t glane = lane & (G - 1);
     const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << (lane & ~(uint32_t)(G - 1)));
     const uint64_t gid = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const uint64_t ngroups = ((uint64_t)gridDim.x * blockDim.x) / G;
-    for (uint64_t j64 = gid; j64 < g.m; j64 += ngroups) {
+    const uint32_t m = kPruned ? __ldcg(g.ctrl + kPruneLeft) : g.m;
+    for (uint64_t j64 = gid; j64 < m; j64 += ngroups) {
         const uint32_t j = (uint32_t)j64;
         const uint32_t u = g.e_src[j], v = g.o_col[j];
         const uint32_t a0 = j + 1, a1 = g.o_ptr[u + 1];
@@ -166,10 +182,10 @@ __device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
     }
 }
 
-template <int G, bool kFill>
+template <int G, bool kFill, bool kPruned = false>
 __global__ void __launch_bounds__(kThreads) k_support(Graph g, Credits c) {
-    if (failed(g.ctrl)) return;
-    edge_body<G, kFill>(g, c);
+    if (skip<kPruned>(g)) return;
+    edge_body<G, kFill, kPruned>(g, c);
 }
 
 // The same count with the lane group read from the control block, where the learned selector's
@@ -187,12 +203,13 @@ __global__ void __launch_bounds__(kThreads) k_support_chosen(Graph g, Credits c,
 // Work items {v, first in-edge, end in-edge, first word of bases} of the vertex-centric vertices.
 // An item takes at least as many in-edges as v's row has entries, so all items together have at
 // most 2m words of bases.  Also lists the rows of the fill's row blocks.
+template <bool kPruned>
 __global__ void k_middle_plan(Graph g, uint4* __restrict__ items, uint32_t* __restrict__ rows,
                               uint32_t* __restrict__ ctrl) {
-    if (failed(ctrl)) return;
+    if (skip<kPruned>(g)) return;
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t row = v < g.n ? g.o_ptr[v + 1] - g.o_ptr[v] : 0u;
-    const uint32_t listed = __ballot_sync(kFullMask, row_block(row));
+    const uint32_t listed = kPruned ? 0u : __ballot_sync(kFullMask, row_block(row));
     if (listed) {
         uint32_t base = 0;
         if (lane_id() == 0) base = atomicAdd(ctrl + kRowItems, __popc(listed));
@@ -204,12 +221,12 @@ __global__ void k_middle_plan(Graph g, uint4* __restrict__ items, uint32_t* __re
     if (!row || !indeg || !vertex_centric(g, v, row)) return;
     const uint32_t step = max(kMidItemIn, (row + kMidItemIn - 1) / kMidItemIn * kMidItemIn);
     const uint32_t count = (indeg + step - 1) / step;
-    const uint32_t i0 = atomicAdd(ctrl + kMidItems, count), w0 = atomicAdd(ctrl + kMidBases, count * row);
+    const uint32_t i0 = atomicAdd(ctrl + g.plan, count), w0 = atomicAdd(ctrl + g.plan + kPlanBases, count * row);
     for (uint32_t i = 0; i < count; ++i)
         items[i0 + i] = make_uint4(v, a + i * step, a + min(indeg, (i + 1) * step), w0 + i * row);
 }
 
-template <bool kFill>
+template <bool kFill, bool kPruned = false>
 __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Graph g, Credits c, const uint4* __restrict__ items,
                                                            uint32_t* __restrict__ ctrl) {
     __shared__ uint32_t key[kMidSlots];
@@ -220,9 +237,9 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
     const uint32_t lane = lane_id(), glane = lane & (G - 1);
     const uint32_t gmask = ((1u << G) - 1) << (lane & ~(uint32_t)(G - 1));
     const uint32_t group = threadIdx.x / G;
-    const uint32_t n_items = failed(ctrl) ? 0u : ctrl[kMidItems];
+    const uint32_t n_items = skip<kPruned>(g) ? 0u : ctrl[g.plan];
     for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(ctrl + kMidCursor + (kFill ? 1 : 0), 1u);
+        if (threadIdx.x == 0) s_item = atomicAdd(ctrl + g.plan + kPlanCursor + (kFill ? 1 : 0), 1u);
         __syncthreads();
         const uint32_t it = s_item;
         if (it >= n_items) return;
@@ -257,7 +274,8 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
             uint32_t j = 0, end = 0, mine = 0;
             if (p < d.z) {
                 j = g.s_eid[p];
-                end = g.o_ptr[g.s_col[p] + 1];
+                if (kPruned) j = g.new_id[j];
+                if (!kPruned || !(j & kGone)) end = g.o_ptr[g.s_col[p] + 1];  // (else no tail)
             }
             for (int q = 0; q < G; ++q) {
                 const uint32_t jq = __shfl_sync(gmask, j, q, G), eq = __shfl_sync(gmask, end, q, G);
@@ -292,7 +310,10 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
         __syncthreads();
         if (!kFill)
             for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
-                if (cnt[i]) c.bases[d.w + i] = atomicAdd(&c.sup[r0 + i], cnt[i]);
+                if (cnt[i]) {
+                    if (kPruned) atomicAdd(&c.supx[r0 + i], cnt[i]);
+                    else c.bases[d.w + i] = atomicAdd(&c.sup[r0 + i], cnt[i]);
+                }
     }
 }
 
@@ -388,27 +409,86 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
     }
 }
 
-// sup += supx, what it was into ycount, and the sum of all supports (three per triangle).
+// sup += supx, what it was into ycount, the sum of all supports (three per triangle), and the number of
+// supports below `limit` (a single-k call's first frontier).
 __global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __restrict__ supx,
-                                uint32_t* __restrict__ ycount, uint32_t m, uint32_t* __restrict__ ctrl) {
+                                uint32_t* __restrict__ ycount, uint32_t m, uint32_t limit, uint32_t* __restrict__ ctrl) {
     if (failed(ctrl)) return;
     uint64_t s = 0;
+    uint32_t low = 0;
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t y = sup[j], v = y + supx[j];
         ycount[j] = y;
         sup[j] = v;
         s += v;
+        low += v < limit;
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
     if (lane_id() == 0 && s)
         atomicAdd(reinterpret_cast<unsigned long long*>(ctrl + kCtrlTriLo), (unsigned long long)s);
+    low = __reduce_add_sync(kFullMask, low);
+    if (lane_id() == 0 && low) atomicAdd(ctrl + kPruneFront, low);
+}
+
+// A single-k call's first round that removes many of the edges (pruned_first): the edges left are
+// numbered in order (new_id) and their oriented CSR is written next to the old one, so that the
+// kernels of the support count can count them again ...
+__global__ void __launch_bounds__(kFlagThreads) k_prune(Graph whole, const uint32_t* __restrict__ sup, uint32_t limit,
+                                                        uint32_t percent, uint32_t* __restrict__ new_id,
+                                                        uint32_t* __restrict__ o_col, uint32_t* __restrict__ e_src,
+                                                        uint32_t* __restrict__ count, Look L) {
+    __shared__ FlagSmem S;
+    if (__syncthreads_or(failed(L.ctrl) || !pruned_first(L.ctrl, whole.m, percent))) return;
+    const uint32_t tile = look_tile(L, &S.tile);
+    if (tile == kNoTile) return;
+    const uint64_t j0 = (uint64_t)tile * kFlagTile + threadIdx.x;
+    const uint32_t warp = threadIdx.x >> 5, m = whole.m;
+    if (j0 == 0) *reinterpret_cast<unsigned long long*>(L.ctrl + kPruneT0) = global_ns();
+    uint32_t left = 0;  // bit s: the edge of step s is left
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint64_t j = j0 + s * kFlagThreads;
+        left |= (uint32_t)(j < m && sup[j] >= limit) << s;
+    }
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint32_t b = __ballot_sync(kFullMask, left >> s & 1u);
+        if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
+    }
+    __syncthreads();
+    flag_sums<true>(S, L, tile);
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint64_t j = j0 + s * kFlagThreads;
+        const bool f = left >> s & 1u;
+        const uint32_t id = (uint32_t)S.prefix + S.before[s * kFlagWarps + warp] +
+                            __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
+        if (j >= m) continue;
+        new_id[j] = f ? id : id | kGone;
+        if (f) {
+            o_col[id] = whole.o_col[j];
+            e_src[id] = whole.e_src[j];
+            count[id] = 0;
+        }
+        if (j == m - 1) L.ctrl[kPruneLeft] = id + f;
+    }
+}
+
+// ... and the starts of their rows.
+__global__ void k_prune_rows(Graph whole, uint32_t percent, const uint32_t* __restrict__ new_id,
+                             uint32_t* __restrict__ o_ptr) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > whole.n || failed(whole.ctrl) || !pruned_first(whole.ctrl, whole.m, percent)) return;
+    const uint32_t j = whole.o_ptr[r];
+    o_ptr[r] = j < whole.m ? new_id[j] & ~kGone : whole.ctrl[kPruneLeft];
 }
 
 Graph graph_of(const kt_engine* e) {
     // the choice must be the same in the count and in the fill of one call
     const bool hash_all = !e->sched_on_device && e->sched.support_group == 0;
     const uint32_t mid_in = hash_all ? 1u : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? 1u : kMidOut;
-    return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out};
+    return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out,
+                 kMidPlan, 0, nullptr};
 }
 
 // The items lie in the first chunk buffer, the claims in the second, the rows in the first queue:
@@ -419,14 +499,14 @@ Credits credits_of(const kt_engine* e) {
     return Credits{e->sup, e->rnd, e->tr, reinterpret_cast<uint32_t*>(e->chunks1), nullptr, nullptr, nullptr};
 }
 
-template <bool kFill>
+template <bool kFill, bool kPruned = false>
 int launch_middle(kt_engine* e, const Graph& g, const Credits& c) {
     int rc, per_sm = 0;
-    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_middle<kFill>, kMidThreads, 0),
+    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_middle<kFill, kPruned>, kMidThreads, 0),
                          "occupancy of k_middle")))
         return rc;
     if (per_sm < 1) return fail(KT_ERR_CUDA, "k_middle cannot be resident");
-    k_middle<kFill><<<(uint32_t)(e->num_sms * per_sm), kMidThreads, 0, e->stream>>>(g, c, items_of(e), e->ctrl);
+    k_middle<kFill, kPruned><<<(uint32_t)(e->num_sms * per_sm), kMidThreads, 0, e->stream>>>(g, c, items_of(e), e->ctrl);
     count_launch(e);
     return check_launch(e, "k_middle");
 }
@@ -443,7 +523,7 @@ int count_support(kt_engine* e) {
     const Graph g = graph_of(e);
     const Credits c = credits_of(e);  // cleared by the build
     if (g.mid_in) {
-        k_middle_plan<<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), rows_of(e),
+        k_middle_plan<false><<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), rows_of(e),
                                                                                     e->ctrl);
         count_launch(e);
         if ((rc = check_launch(e, "k_middle_plan")) || (rc = launch_middle<false>(e, g, c))) return rc;
@@ -466,10 +546,59 @@ int count_support(kt_engine* e) {
     return check_launch(e, "k_support");
 }
 
-int merge_support(kt_engine* e) {
-    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, e->m, e->ctrl);
+int merge_support(kt_engine* e, uint32_t limit) {
+    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, e->m, limit, e->ctrl);
     count_launch(e);
     return check_launch(e, "k_merge_support");
+}
+
+// The first round of a single-k call whose frontier (supports below `limit`) is a recount round: the
+// peel kernel's recount searches every surviving edge's rows among the removed entries; here the edges
+// left are packed and counted like a graph of their own.  All kernels return at once when the
+// frontier is smaller.
+// Measured: R-MAT 18 (3.7 M edges), k = 32, the first round 2.4 ms walked, 2.0 recounted by the peel
+// kernel, 0.62 here (the call 4.81 -> 3.06 ms); R-MAT 20, k = 32: 10.8 -> 2.4 ms; G(40000) with 6 M edges,
+// k = 5: 16.7 walked, 0.86 here.
+// The line lies at 7/10 of the schedule's recount share, as this recount costs less than the peel's: a
+// frontier of 30-32 % of an R-MAT graph's edges takes 3.9 ms walked and 3.7 here (15 M edges), 0.80 and
+// 0.81 (3.7 M); 26 %: 2.8 and 3.9, 0.55 and 0.88; 41 %: 7.5 and 3.5, 1.2 and 0.73.  Below 2^20 edges it is the
+// share itself (400,000 edges: 40 % 0.10 and 0.14 ms, 48 % 0.135 and 0.125), and below 2^19 the peel's: the five
+// launches that return cost a call 0.02 ms, 4 % of one on 400,000 edges whose frontier is smaller.
+// The peel finds new ids in e->tr and the new counts in key_b (3 m words on); the sort keys are free
+// after the build.
+int recount_pruned(kt_engine* e, uint32_t limit, uint32_t percent, PrunedCount* out) {
+    *out = PrunedCount{0, nullptr, nullptr};
+    if (percent == 0 || e->m < kPruneMin || e->sched_on_device) return KT_OK;
+    if (e->m >= kPruneEarly) percent = std::max(1u, percent * 7 / 10);
+    int rc;
+    const Graph whole = graph_of(e);
+    uint32_t* o_ptr = reinterpret_cast<uint32_t*>(e->key_a);  // n + 1 words of 2 max(n, entries)
+    uint32_t* o_col = reinterpret_cast<uint32_t*>(e->key_b);  // 3 m words of 4 m
+    uint32_t *e_src = o_col + e->m, *count = e_src + e->m, *new_id = e->tr;
+    const uint32_t tiles = (e->m + kFlagTile - 1) / kFlagTile;
+    k_prune<<<tiles, kFlagThreads, 0, e->stream>>>(whole, e->sup, limit, percent, new_id, o_col, e_src, count,
+                                                   next_look(e));
+    count_launch(e);
+    if ((rc = check_launch(e, "k_prune"))) return rc;
+    k_prune_rows<<<(uint32_t)(((uint64_t)e->n + kThreads) / kThreads), kThreads, 0, e->stream>>>(whole, percent, new_id, o_ptr);
+    count_launch(e);
+    if ((rc = check_launch(e, "k_prune_rows"))) return rc;
+    Graph g = whole;
+    g.o_ptr = o_ptr;
+    g.o_col = o_col;
+    g.e_src = e_src;
+    g.plan = kPrunePlan;
+    g.percent = percent;
+    g.new_id = new_id;
+    Credits c = credits_of(e);
+    c.sup = c.supx = count;
+    k_middle_plan<true><<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), nullptr, e->ctrl);
+    count_launch(e);
+    if ((rc = check_launch(e, "k_middle_plan")) || (rc = launch_middle<false, true>(e, g, c))) return rc;
+    k_support<8, false, true><<<edge_blocks(e, 8), kThreads, 0, e->stream>>>(g, c);
+    count_launch(e);
+    *out = PrunedCount{percent, new_id, count};
+    return check_launch(e, "k_support");
 }
 
 int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends) {
