@@ -7,11 +7,12 @@
 // that are also in v's row N+(v).  Two ways to test them, chosen by the middle vertex v:
 //
 // Vertex-centric (k_middle): vertices with at least kMidIn in-edges and a row of at most kMidRow
-// entries.  A block hashes N+(v) into shared memory (key w -> row position, at most a quarter to a
-// half full) and streams the tails of a range of v's in-edges (the lower half of v's symmetric row)
-// through it, eight lanes to a tail: one shared-memory probe per entry instead of a binary search.
-// A triangle costs one global atomic (x); y is counted in shared memory and added once per item, j
-// once per tail.
+// entries.  A block hashes N+(v) into shared memory (column -> row position, in buckets of two, at most a
+// quarter to a half full) and streams the tails of a range of v's in-edges (the lower half of v's
+// symmetric row) through it: one or two shared-memory probes per entry instead of a binary search.  The
+// tails of 256 in-edges at a time are laid end to end and dealt evenly over the warps, however
+// different their lengths.  A triangle costs one global atomic (x); y is counted in shared memory and
+// added once per item, j once per tail.
 //
 // Edge-centric (k_support): all other edges, G lanes each (the schedule's support_group).  The
 // shorter of tail and row is walked, the longer binary-searched; x and y are credited with global
@@ -28,10 +29,12 @@
 //             u's row, after the claimed parts;
 //   k_support everything else, with a global cursor that fills each list from its end.
 //
-// Measured (GB300): count R-MAT 20 of 15 M edges 7.4 -> 3.8 ms, R-MAT 22 of 60 M edges 44.4 -> 23.7 ms
-// (k_support alone -> with k_middle; R-MAT 18: k_middle issues in 48 % of the cycles, L1 48 %, DRAM
-// 2 %); fill 18.0 -> 13.0 ms and 114 -> 77 ms, its DRAM writes on R-MAT 18 3.8 -> 2.1 GB for 1.8 GB of
-// entries.
+// Measured (GB300): count R-MAT 20 of 15 M edges 7.4 -> 3.5 ms, R-MAT 22 of 60 M edges 44.4 -> 18.6 ms
+// (k_support alone -> with k_middle; 3.7 and 23.0 ms with eight lanes to a tail, half of whose stalls were
+// waits for the longest tail).  k_middle issues in 84 % of the cycles, L1 70 % (bank conflicts of the
+// probes), DRAM 5 %.  A filter of the row's columns in front of the table: 3.9-4.2 ms; lookups queued up
+// to full warps, by binary search in the row: 5.0 ms.  Fill 18.0 -> 13.0 ms and 114 -> 76 ms, its DRAM
+// writes on R-MAT 18 3.8 -> 2.1 GB for 1.8 GB of entries.
 
 #include <algorithm>
 
@@ -45,13 +48,12 @@ namespace {
 constexpr int kThreads = 256;
 
 constexpr int kMidThreads = 256;
-constexpr int kMidGroup = 8;                   // lanes per tail: R-MAT 22 count 23.3 ms, 24.0 with 16, 26.0 with 4
 constexpr uint32_t kMidSlots = 4096;           // hash slots (32 KB with positions and counters: 6 blocks an SM)
 constexpr uint32_t kMidRow = kMidSlots / 2;    // longest row that is hashed
 // A vertex is vertex-centric with at least kMidIn in-edges and kMidOut row entries: with fewer, a
-// table serves too few probes, or the search it replaces is short.  R-MAT 20 count 3.8 ms at 64
-// in-edges, 4.1 at 32, 3.8 at 128 (R-MAT 16: 0.21, 0.21, 0.23 ms); a batch of 256 graphs, whose hubs
-// have short rows, 1.08 ms at 32 row entries, 1.18 at 16, 1.35 at 1.
+// table serves too few probes, or the search it replaces is short.  R-MAT 22 count 18.6 ms at 64
+// in-edges, 18.7 at 32, 19.3 at 96 (R-MAT 16: 0.18, 0.19, 0.21 ms); a batch of 256 graphs, whose hubs
+// have short rows, 1.01 ms at 32 row entries, 1.07 at 16.
 constexpr uint32_t kMidIn = 64;
 constexpr uint32_t kMidOut = 32;
 constexpr uint32_t kMidItemIn = 256;           // in-edges per work item (more for longer rows)
@@ -229,14 +231,14 @@ __global__ void k_middle_plan(Graph g, uint4* __restrict__ items, uint32_t* __re
 template <bool kFill, bool kPruned = false>
 __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Graph g, Credits c, const uint4* __restrict__ items,
                                                            uint32_t* __restrict__ ctrl) {
-    __shared__ uint32_t key[kMidSlots];
+    __shared__ uint2 key[kMidSlots / 2];  // buckets of two, filled in order
     __shared__ uint16_t at[kMidSlots];
     __shared__ uint32_t cnt[kMidRow];  // count: triangles of y; fill: next list entry of y
     __shared__ uint32_t s_item;
-    constexpr int G = kMidGroup;
-    const uint32_t lane = lane_id(), glane = lane & (G - 1);
-    const uint32_t gmask = ((1u << G) - 1) << (lane & ~(uint32_t)(G - 1));
-    const uint32_t group = threadIdx.x / G;
+    // a batch of in-edges, one a thread: tail entries before its tail, its tail's start less these, and
+    // its triangles (count) or edge id (fill)
+    __shared__ uint32_t before[kMidThreads + 1], start[kMidThreads], tag[kMidThreads], wsum[kMidThreads / 32];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t n_items = skip<kPruned>(g) ? 0u : ctrl[g.plan];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(ctrl + g.plan + kPlanCursor + (kFill ? 1 : 0), 1u);
@@ -245,10 +247,10 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
         if (it >= n_items) return;
         const uint4 d = items[it];
         const uint32_t r0 = g.o_ptr[d.x], row = g.o_ptr[d.x + 1] - r0;
-        uint32_t bits = 6;  // at least four slots an entry, as far as the table goes
-        while (bits < 12 && (1u << bits) < 4 * row) ++bits;
+        uint32_t bits = 5;  // at least four slots an entry, as far as the table goes
+        while (bits < 11 && (1u << bits) < 2 * row) ++bits;
         const uint32_t mask = (1u << bits) - 1, shift = 32 - bits;
-        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = kEmpty;
+        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = make_uint2(kEmpty, kEmpty);
         // the fill counts list entries from the start of the row's lists (or, should they hold 2^32
         // entries or more, from the start of each list)
         uint64_t row_at = 0;
@@ -263,51 +265,96 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
         for (uint32_t i = threadIdx.x; i < row; i += kMidThreads) {
             const uint32_t w = g.o_col[r0 + i];
             uint32_t h = (w * 0x9E3779B1u) >> shift;
-            while (atomicCAS(&key[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
-            at[h] = (uint16_t)i;
+            for (;; h = (h + 1) & mask) {
+                if (atomicCAS(&key[h].x, kEmpty, w) == kEmpty) {
+                    at[2 * h] = (uint16_t)i;
+                    break;
+                }
+                if (atomicCAS(&key[h].y, kEmpty, w) == kEmpty) {
+                    at[2 * h + 1] = (uint16_t)i;
+                    break;
+                }
+            }
         }
-        __syncthreads();
-        // eight in-edges at a time per group: their lanes load them together, then take the tails
-        // one after another
-        for (uint32_t p0 = d.y + group * G; p0 < d.z; p0 += kMidThreads) {
-            const uint32_t p = p0 + glane;
-            uint32_t j = 0, end = 0, mine = 0;
+        for (uint32_t p0 = d.y; p0 < d.z; p0 += kMidThreads) {
+            const uint32_t p = p0 + threadIdx.x;
+            uint32_t j = 0, len = 0;
             if (p < d.z) {
                 j = g.s_eid[p];
                 if (kPruned) j = g.new_id[j];
-                if (!kPruned || !(j & kGone)) end = g.o_ptr[g.s_col[p] + 1];  // (else no tail)
+                if (!kPruned || !(j & kGone)) len = g.o_ptr[g.s_col[p] + 1] - (j + 1);  // (else no tail)
             }
-            for (int q = 0; q < G; ++q) {
-                const uint32_t jq = __shfl_sync(gmask, j, q, G), eq = __shfl_sync(gmask, end, q, G);
-                uint32_t found = 0;
-                uint32_t w_next = jq + 1 + glane < eq ? g.o_col[jq + 1 + glane] : kEmpty;
-                for (uint32_t x = jq + 1 + glane; x < eq; x += G) {
-                    const uint32_t w = w_next;
-                    w_next = x + G < eq ? g.o_col[x + G] : kEmpty;
-                    uint32_t h = (w * 0x9E3779B1u) >> shift, k;
-                    while ((k = key[h]) != w && k != kEmpty) h = (h + 1) & mask;
-                    if (k == w) {
-                        const uint32_t pos = at[h];
+            uint32_t incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= (uint32_t)o) incl += t;
+            }
+            if (lane == 31) wsum[warp] = incl;
+            __syncthreads();  // (for the table too)
+            uint32_t total = 0, at0 = incl - len;
+#pragma unroll
+            for (int q = 0; q < kMidThreads / 32; ++q) {
+                const uint32_t t = wsum[q];
+                at0 += q < (int)warp ? t : 0u;
+                total += t;
+            }
+            before[threadIdx.x] = at0;
+            start[threadIdx.x] = j + 1 - at0;
+            tag[threadIdx.x] = kFill ? j : 0u;
+            if (threadIdx.x == 0) before[kMidThreads] = total;
+            __syncthreads();
+            // the warps share the entries of all tails evenly
+            const uint32_t share = (total + kMidThreads - 1) / kMidThreads * 32;
+            const uint32_t end = min(total, (warp + 1) * share);
+            uint32_t t = warp * share + lane;
+            if (t < end) {
+                uint32_t own = 0;  // the last tail that starts at or before entry t
+#pragma unroll
+                for (uint32_t b = kMidThreads / 2; b > 0; b >>= 1)
+                    if (before[own + b] <= t) own += b;
+                uint32_t next = before[own + 1], off = start[own], found = 0;
+                uint32_t j_own = kFill ? tag[own] : 0u;
+                uint32_t x = t + off, w = g.o_col[x];
+                while (t < end) {
+                    const uint32_t x_now = x, w_now = w, j_now = j_own;
+                    uint32_t* const tag_now = &tag[own];
+                    const bool moves = t + 32 >= next;
+                    t += 32;
+                    if (t < end) {
+                        if (moves) {
+                            do next = before[++own + 1];
+                            while (t >= next);
+                            off = start[own];
+                            if (kFill) j_own = tag[own];
+                        }
+                        x = t + off;
+                        w = g.o_col[x];
+                    }
+                    uint32_t h = (w_now * 0x9E3779B1u) >> shift;
+                    uint2 k = key[h];
+                    while (k.x != w_now && k.y != w_now && k.y != kEmpty) k = key[h = (h + 1) & mask];
+                    if (k.x == w_now || k.y == w_now) {
+                        const uint32_t pos = at[2 * h + (k.y == w_now)];
                         if (!kFill) {
                             ++found;
                             atomicAdd(&cnt[pos], 1u);
-                            atomicAdd(&c.supx[x], 1u);
+                            atomicAdd(&c.supx[x_now], 1u);
                         } else {
                             c.tri[(wide ? __ldg(c.tptr + r0 + pos) : row_at) + atomicAdd(&cnt[pos], 1u)] =
-                                make_uint2(jq, x);
+                                make_uint2(j_now, x_now);
                         }
                     }
+                    if (!kFill && moves && found) {
+                        atomicAdd(tag_now, found);
+                        found = 0;
+                    }
                 }
-                if (!kFill) {
-                    __syncwarp(gmask);
-#pragma unroll
-                    for (int o = G / 2; o > 0; o >>= 1) found += __shfl_xor_sync(gmask, found, o);
-                    if (glane == (uint32_t)q) mine = found;
-                }
+                if (!kFill && found) atomicAdd(&tag[own], found);
             }
-            if (!kFill && mine) atomicAdd(&c.supx[j], mine);
+            __syncthreads();
+            if (!kFill && tag[threadIdx.x]) atomicAdd(&c.supx[j], tag[threadIdx.x]);
         }
-        __syncthreads();
         if (!kFill)
             for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
                 if (cnt[i]) {
@@ -325,7 +372,7 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
 // search the tail's entries in it.
 __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, const uint32_t* __restrict__ rows,
                                                          uint32_t* __restrict__ ctrl) {
-    __shared__ uint32_t key[kMidSlots];
+    __shared__ uint2 key[kMidSlots / 2];  // (as in k_middle)
     __shared__ uint16_t at[kMidSlots];
     __shared__ uint32_t cur[kMidRow];  // next list entry, from the start of the row's lists
     __shared__ uint32_t s_row;
@@ -342,20 +389,28 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
         const uint32_t u = s_row;
         if (u == kEmpty) return;
         const uint32_t r0 = g.o_ptr[u], row = g.o_ptr[u + 1] - r0;
-        uint32_t bits = 6;
-        while (bits < 12 && (1u << bits) < 4 * row) ++bits;
+        uint32_t bits = 5;
+        while (bits < 11 && (1u << bits) < 2 * row) ++bits;
         const uint32_t mask = (1u << bits) - 1, shift = 32 - bits;
         const uint64_t row_at = c.tptr[r0];
         const bool wide = c.tptr[r0 + row] - row_at >= 0xffffffffull;
-        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = kEmpty;
+        for (uint32_t i = threadIdx.x; i <= mask; i += kMidThreads) key[i] = make_uint2(kEmpty, kEmpty);
         for (uint32_t i = threadIdx.x; i < row; i += kMidThreads)
             cur[i] = c.ycount[r0 + i] + (wide ? 0u : (uint32_t)(c.tptr[r0 + i] - row_at));
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < row; i += kMidThreads) {
             const uint32_t w = g.o_col[r0 + i];
             uint32_t h = (w * 0x9E3779B1u) >> shift;
-            while (atomicCAS(&key[h], kEmpty, w) != kEmpty) h = (h + 1) & mask;
-            at[h] = (uint16_t)i;
+            for (;; h = (h + 1) & mask) {
+                if (atomicCAS(&key[h].x, kEmpty, w) == kEmpty) {
+                    at[2 * h] = (uint16_t)i;
+                    break;
+                }
+                if (atomicCAS(&key[h].y, kEmpty, w) == kEmpty) {
+                    at[2 * h + 1] = (uint16_t)i;
+                    break;
+                }
+            }
         }
         __syncthreads();
         // positions group, group + groups, ...: the group's lanes load the rows of the next G together
@@ -381,9 +436,10 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
                 uint32_t pos = kEmpty, y = p;  // x = r0 + pos
                 if (w != kEmpty) {
                     if (stream) {
-                        uint32_t h = (w * 0x9E3779B1u) >> shift, k;
-                        while ((k = key[h]) != w && k != kEmpty) h = (h + 1) & mask;
-                        if (k == w) pos = at[h];
+                        uint32_t h = (w * 0x9E3779B1u) >> shift;
+                        uint2 k = key[h];
+                        while (k.x != w && k.y != w && k.y != kEmpty) k = key[h = (h + 1) & mask];
+                        if (k.x == w || k.y == w) pos = at[2 * h + (k.y == w)];
                     } else {
                         y = b0 + lower_bound_u32(g.o_col + b0, b1 - b0, w);
                         if (y < b1 && g.o_col[y] == w) pos = p - r0;
@@ -557,7 +613,7 @@ int merge_support(kt_engine* e, uint32_t limit) {
 // left are packed and counted like a graph of their own.  All kernels return at once when the
 // frontier is smaller.
 // Measured: R-MAT 18 (3.7 M edges), k = 32, the first round 2.4 ms walked, 2.0 recounted by the peel
-// kernel, 0.62 here (the call 4.81 -> 3.06 ms); R-MAT 20, k = 32: 10.8 -> 2.4 ms; G(40000) with 6 M edges,
+// kernel, 0.53 here (the call 4.81 -> 2.88 ms); R-MAT 20, k = 32: 10.8 -> 2.4 ms; G(40000) with 6 M edges,
 // k = 5: 16.7 walked, 0.86 here.
 // The line lies at 7/10 of the schedule's recount share, as this recount costs less than the peel's: a
 // frontier of 30-32 % of an R-MAT graph's edges takes 3.9 ms walked and 3.7 here (15 M edges), 0.80 and
