@@ -14,8 +14,8 @@
 //      the neighbour's oriented row, which also proves the input symmetric (k_entry_eid).
 //
 // Scans and radix passes are one kernel each (kt_look.cuh).  A small graph's build is bound by its
-// launches: G(4096, 16/4095) takes 17 instead of 43, 0.098 ms instead of 0.238; R-MAT 16 0.26 instead of
-// 0.42 ms, R-MAT 20 2.9 instead of 3.05 ms (the sort's five passes 1.6 ms of it).
+// launches: G(4096, 16/4095) takes 17 instead of 43, 0.083 ms instead of 0.238; R-MAT 16 0.21 instead of
+// 0.42 ms, R-MAT 20 2.6 instead of 3.05 ms (the sort's five passes 1.3 ms of it).
 //
 // Layout in HBM (n vertices, m undirected edges, all uint32):
 //   s_ptr[n+1], s_len[n], s_split[n]   symmetric rows (lower ranks, then higher ranks)

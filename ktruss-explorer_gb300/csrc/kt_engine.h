@@ -158,7 +158,7 @@ struct Look;  // kt_look.cuh
 
 // kt_sort.cu.  Sorts of up to kSmallSort keys take small tiles (enough blocks for every SM).
 constexpr uint64_t kSmallSort = 1u << 18;
-constexpr uint64_t kSmallTile = 1024, kLargeTile = 4096;
+constexpr uint64_t kSmallTile = 1024, kLargeTile = 6144;
 constexpr uint32_t kCountWords = 32 * 256 + 64;  // digit count blocks and tickets of a session
 inline uint64_t look_words(uint64_t keys) {
     return 256 * (keys <= kSmallSort ? (keys + kSmallTile - 1) / kSmallTile : (keys + kLargeTile - 1) / kLargeTile);

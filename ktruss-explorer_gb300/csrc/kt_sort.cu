@@ -2,15 +2,16 @@
 //
 // It replaces the per-row CPU quicksort of the reference build (graph.cu:462-476 "Sort outgoing
 // edges ... on CPU").  Every digit's histogram is counted by the kernel that makes the keys (or by
-// k_digit_counts), so a pass reads the keys once: a tile ranks its keys by warp matches, learns where
-// its digits' runs start from its predecessors (decoupled look-back, one word a digit), arranges
-// itself in digit order in shared memory and writes runs of consecutive positions.  The first pass
-// can make the values (entry indices) itself.
+// k_digit_counts), so a pass reads the keys once: a tile counts its digits and publishes the counts, then
+// ranks its keys by warp ballots, arranges itself in digit order in shared memory, learns where its
+// digits' runs start from its predecessors (decoupled look-back, one word a digit), and writes runs of
+// consecutive positions.  The first pass can make the values (entry indices) itself.
 //
-// Bound: the serial chain of a tile (ticket, loads, ranks, look-back, runs) at half occupancy - 64
-// registers, issue active 44 %, DRAM 28 % - and for small inputs the launches.  A pass over 31.4 M keys
-// with values takes 0.31 ms (histogram, scan and scatter kernels: 0.34 ms); a pass over 64,000 entries
-// is one launch instead of four.
+// Bound: the serial chain of a tile (ticket, loads, counts, ranks, look-back, runs) at half occupancy, 64
+// registers, issue active 47 % - and for small inputs the launches.  A pass over 30 M keys with values
+// takes 0.26 ms, 2.8 TB/s of keys and values (0.31 ms when the counts were published after the ranks
+// and a tile's places were added up from three tables; histogram, scan and scatter kernels: 0.33 ms); a
+// pass over 64,000 entries is one launch instead of four.
 
 #include <algorithm>
 #include <utility>
@@ -23,8 +24,9 @@ namespace kt {
 namespace {
 
 constexpr int kDigits = 256;
-// Large tiles: 512 threads of 8 keys, two blocks an SM.  512 of 4 keys (four blocks) and 256 of 8 measured
-// within 4 %, 1024 of 4 keys 17 % slower (build of R-MAT 20).
+// Large tiles: 512 threads of 12 keys, two blocks an SM.  Build of R-MAT 20 / symmetrize of 16.8 M edges:
+// 2.61 / 0.96 ms with 12 keys, 2.63 / 0.97 with 10, 2.67 / 1.00 with 8, 2.68 / 1.02 with 14; three blocks of 6
+// keys 2.66 / 1.04, 256 threads of 8 keys 2.75 / 1.12.
 constexpr int kLargeThreads = 512, kLargeItems = (int)kLargeTile / kLargeThreads;
 constexpr int kSmallThreads = 256, kSmallItems = (int)kSmallTile / kSmallThreads;
 
@@ -43,11 +45,10 @@ __global__ void __launch_bounds__(256) k_digit_counts(const uint64_t* __restrict
 // Shared memory of a pass, by tile shape.
 template <int kThreads, int kItems>
 struct PassSmem {
-    uint32_t wh[kThreads / 32][kDigits];  // per warp: keys of each digit, then their offset in the tile's run
+    uint32_t wh[kThreads / 32][kDigits];  // per warp: keys of each digit, then the place of the next one in the tile
     uint64_t key[kThreads * kItems];
     uint32_t val[kThreads * kItems];
     uint32_t goff[kDigits];  // where the tile's run of each digit goes, less its start in the tile
-    uint32_t toff[kDigits];
     uint32_t ws[2][kDigits / 32];
     uint32_t tile, ok;
 };
@@ -71,15 +72,63 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
     const uint64_t tbase = (uint64_t)tile * (kThreads * kItems);
     const uint64_t wbase = tbase + (uint64_t)warp * (32 * kItems);
     uint64_t key[kItems];
-    uint32_t rk[kItems];
 #pragma unroll
     for (int s = 0; s < kItems; ++s) {
         const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
         key[s] = idx < n ? kin[idx] : 0ull;
     }
-    // the leader of each set of equal digits claims its ranks, step after step, without waiting for
+    // the counts first: the tile's successors wait for them, not for its ranks
+#pragma unroll
+    for (int s = 0; s < kItems; ++s)
+        if (wbase + (uint32_t)s * 32 + lane < n) atomicAdd(&S.wh[warp][(uint32_t)(key[s] >> shift) & 255u], 1u);
+    __syncthreads();
+    uint32_t count = 0, all = 0;  // keys of digit threadIdx.x in the tile, and in all tiles
+    uint32_t x = 0, y = 0;
+    if (owner) {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) count += S.wh[w][threadIdx.x];
+        all = counts[threadIdx.x];
+        st_relaxed_u64(L.words + (uint64_t)tile * kDigits + threadIdx.x,
+                       look_word(tile ? kLookAggregate : kLookInclusive, L.tag, count));
+        // exclusive scans over the digits: starts in the tile and in the output
+        x = count;
+        y = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(kFullMask, x, o), b = __shfl_up_sync(kFullMask, y, o);
+            if (lane >= (uint32_t)o) {
+                x += a;
+                y += b;
+            }
+        }
+        if (lane == 31) {
+            S.ws[0][warp] = x;
+            S.ws[1][warp] = y;
+        }
+    }
+    __syncthreads();
+    uint32_t start = 0, toff = 0;
+    if (owner) {
+        uint32_t bx = 0, by = 0;
+#pragma unroll
+        for (int w = 0; w < kDigits / 32; ++w) {
+            bx += w < (int)warp ? S.ws[0][w] : 0u;
+            by += w < (int)warp ? S.ws[1][w] : 0u;
+        }
+        toff = bx + x - count;
+        start = by + y - all;
+        uint32_t run = toff;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t c = S.wh[w][threadIdx.x];
+            S.wh[w][threadIdx.x] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+    // the leader of each set of equal digits claims its places, step after step, without waiting for
     // the atomics' results in between
-    uint32_t first[kItems];
+    uint32_t first[kItems], rk[kItems];
 #pragma unroll
     for (int s = 0; s < kItems; ++s) {
         const bool valid = wbase + (uint32_t)s * 32 + lane < n;
@@ -101,63 +150,12 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
     }
 #pragma unroll
     for (int s = 0; s < kItems; ++s) rk[s] = __shfl_sync(kFullMask, first[s], rk[s] >> 8) + (rk[s] & 255u);
-    uint32_t val[kItems];
 #pragma unroll
     for (int s = 0; s < kItems; ++s) {
         const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
-        val[s] = kVals ? (vin ? (idx < n ? vin[idx] : 0u) : (uint32_t)idx) : 0u;
-    }
-    __syncthreads();
-    uint32_t count = 0, all = 0;  // keys of digit threadIdx.x in the tile, and in all tiles
-    if (owner) {
-        uint32_t run = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = S.wh[w][threadIdx.x];
-            S.wh[w][threadIdx.x] = run;
-            run += c;
-        }
-        count = run;
-        all = counts[threadIdx.x];
-        st_relaxed_u64(L.words + (uint64_t)tile * kDigits + threadIdx.x,
-                       look_word(tile ? kLookAggregate : kLookInclusive, L.tag, count));
-    }
-    // exclusive scans over the digits: starts in the tile and in the output
-    uint32_t x = count, y = all;
-    if (owner) {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t a = __shfl_up_sync(kFullMask, x, o), b = __shfl_up_sync(kFullMask, y, o);
-            if (lane >= (uint32_t)o) {
-                x += a;
-                y += b;
-            }
-        }
-        if (lane == 31) {
-            S.ws[0][warp] = x;
-            S.ws[1][warp] = y;
-        }
-    }
-    __syncthreads();
-    uint32_t start = 0;
-    if (owner) {
-        uint32_t bx = 0, by = 0;
-#pragma unroll
-        for (int w = 0; w < kDigits / 32; ++w) {
-            bx += w < (int)warp ? S.ws[0][w] : 0u;
-            by += w < (int)warp ? S.ws[1][w] : 0u;
-        }
-        S.toff[threadIdx.x] = bx + x - count;
-        start = by + y - all;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < kItems; ++s) {
-        if (wbase + (uint32_t)s * 32 + lane < n) {
-            const uint32_t d = (uint32_t)(key[s] >> shift) & 255u;
-            const uint32_t lp = S.toff[d] + S.wh[warp][d] + rk[s];
-            S.key[lp] = key[s];
-            if (kVals) S.val[lp] = val[s];
+        if (idx < n) {
+            S.key[rk[s]] = key[s];
+            if (kVals) S.val[rk[s]] = vin ? vin[idx] : (uint32_t)idx;
         }
     }
     // the owners look back, four predecessors at a time
@@ -191,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
             st_relaxed_u64(L.words + (uint64_t)tile * kDigits + threadIdx.x,
                            look_word(kLookInclusive, L.tag, prefix + count));
         }
-        S.goff[threadIdx.x] = start + (uint32_t)prefix - S.toff[threadIdx.x];
+        S.goff[threadIdx.x] = start + (uint32_t)prefix - toff;
     }
     __syncthreads();
     if (!S.ok) return;
