@@ -199,6 +199,8 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
 int count_support(kt_engine* e);
 int merge_support(kt_engine* e, uint32_t limit);
 
+int truss3(kt_engine* e);  // merge_support and the 3-truss: rnd 0 for the edges that stay
+
 // Counts the edges left by a single-k call's first round again if that round removes `percent` or more
 // of them (decided on the device; percent 0 in *out: never).  new_id: the edge's number among those
 // left, or its top bit; count: their supports.

@@ -1009,7 +1009,8 @@ int peel_single_k(kt_engine* e, uint32_t k) {
     e->peel_mode = 1;
     e->stats_ready = false;
     if (e->m == 0) return KT_OK;
-    if (k >= 3 && (rc = merge_support(e, k - 2))) return rc;
+    if (k == 3) return truss3(e);
+    if (k > 3 && (rc = merge_support(e, k - 2))) return rc;
     if (k < 3) {
         // k = 2 keeps every edge; k < 2 removes every edge (k-2 wraps as unsigned, as in
         // mark_deleted_edges_kernel, kernel_ddc.cu:64)
@@ -1018,9 +1019,8 @@ int peel_single_k(kt_engine* e, uint32_t k) {
         count_launch(e);
         return check_launch(e, "k_fill_edges");
     }
-    // (at k = 3 the frontier's edges are in no triangle, so nothing has to be counted again)
     PrunedCount pruned;
-    if ((rc = recount_pruned(e, k - 2, k > 3 ? e->sched.recount_percent : 0, &pruned))) return rc;
+    if ((rc = recount_pruned(e, k - 2, e->sched.recount_percent, &pruned))) return rc;
     return launch_peel(e, k, pruned);
 }
 
