@@ -14,7 +14,7 @@
 //      the neighbour's oriented row, which also proves the input symmetric (k_entry_eid).
 //
 // Scans and radix passes are one kernel each (kt_look.cuh).  A small graph's build is bound by its
-// launches: G(4096, 16/4095) takes 17 instead of 43, 0.083 ms instead of 0.238; R-MAT 16 0.21 instead of
+// launches: G(4096, 16/4095) takes 12 instead of 43, chained, 0.064 ms instead of 0.238; R-MAT 16 0.21 instead of
 // 0.42 ms, R-MAT 20 2.6 instead of 3.05 ms (the sort's five passes 1.3 ms of it).
 //
 // Layout in HBM (n vertices, m undirected edges, all uint32):
@@ -43,8 +43,10 @@ inline uint32_t grid_for(uint64_t n, int threads = kThreads) {
 
 // Degree histogram with per-warp aggregation: lanes holding the same source add once (inputs
 // listed row by row put a hub's many entries in the same warps).
+template <bool kChained>
 __global__ void k_degree(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t entries,
                          uint32_t n, uint32_t* __restrict__ deg, uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(src, dst, deg, ctrl);
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t err = 0, s = 0xffffffffu;
     if (i < entries) {
@@ -66,9 +68,11 @@ __global__ void k_degree(const uint32_t* __restrict__ src, const uint32_t* __res
 // Rank keys (degree << vb | id), listed by id: the sort is stable, so it needs the degree's digits
 // only.  A simple graph's degrees are below n; a degree that is not (the input has duplicates and
 // will be refused) is sorted by its low digits.
+template <bool kChained>
 __global__ void __launch_bounds__(kThreads) k_rank_keys(const uint32_t* __restrict__ deg, uint32_t n, unsigned vb,
                                                         unsigned passes, uint64_t* __restrict__ keys,
                                                         uint32_t* __restrict__ counts) {
+    if (kChained) after_previous(deg, keys, counts);
     __shared__ uint32_t h[4 * 256];
     digit_counts_clear(h, passes);
     for (uint64_t v0 = (uint64_t)blockIdx.x * kThreads; v0 < n; v0 += (uint64_t)gridDim.x * kThreads) {
@@ -84,13 +88,14 @@ __global__ void __launch_bounds__(kThreads) k_rank_keys(const uint32_t* __restri
 // orienting by vertex id, KT_DIRECTED_BY_INDEX, graph.cu:194-207 without the relabel of
 // kernel.cu:13-20), row lengths, and their exclusive scan.  Empty rows get their split and oriented
 // start here (by degree they come first), the marks of the first long and first not tiny row too.
-template <bool kByIndex>
+template <bool kByIndex, bool kChained>
 __global__ void __launch_bounds__(kScanThreads) k_rank_rows(const uint64_t* __restrict__ sorted,
                                                             const uint32_t* __restrict__ deg, uint32_t n, unsigned vb,
                                                             uint32_t* __restrict__ rank, uint32_t* __restrict__ s_len,
                                                             uint32_t* __restrict__ s_ptr,
                                                             uint32_t* __restrict__ s_split,
                                                             uint32_t* __restrict__ o_ptr, Look L) {
+    if (kChained) after_previous(sorted, deg, rank, s_len, s_ptr, s_split, o_ptr);
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
     const uint32_t tile = look_tile(L, &s_tile);
@@ -141,11 +146,13 @@ __global__ void __launch_bounds__(kScanThreads) k_rank_rows(const uint64_t* __re
 // Entry keys (rank of the source << vb | rank of the destination) and their digit counts.  An id >= n
 // (already flagged by k_degree; the call fails) is read as vertex 0, so that
 // every kernel up to that check indexes inside its arrays.
+template <bool kChained>
 __global__ void __launch_bounds__(kThreads) k_edge_keys(const uint32_t* __restrict__ src,
                                                         const uint32_t* __restrict__ dst, uint64_t entries, uint32_t n,
                                                         const uint32_t* __restrict__ rank, unsigned vb, unsigned passes,
                                                         uint64_t* __restrict__ keys, uint32_t* __restrict__ counts,
                                                         const uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(src, dst, rank, keys, counts, ctrl);
     __shared__ uint32_t h[kMaxDigitPasses * 256];
     if (__syncthreads_or(timed_out(ctrl))) return;
     digit_counts_clear(h, passes);
@@ -165,12 +172,14 @@ __global__ void __launch_bounds__(kThreads) k_edge_keys(const uint32_t* __restri
 // One pass over the sorted entry keys builds both CSRs: columns, the duplicate check, where each
 // row's higher-rank part starts, and - by a scan of the higher-rank entries - their oriented
 // positions, which are the edge ids.  A row's oriented start is the scan at its first entry.
+template <bool kChained>
 __global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
                                                       uint32_t n, uint32_t m, uint32_t* __restrict__ s_col,
                                                       uint32_t* __restrict__ s_eid, uint32_t* __restrict__ s_split,
                                                       uint32_t* __restrict__ o_ptr, uint32_t* __restrict__ o_col,
                                                       uint32_t* __restrict__ e_src, uint32_t* __restrict__ fence,
                                                       Look L) {
+    if (kChained) after_previous(keys, s_col, s_eid, s_split, o_ptr, o_col, e_src, fence);
     __shared__ FlagSmem S;
     const uint32_t tile = look_tile(L, &S.tile);
     if (tile == kNoTile) return;
@@ -236,6 +245,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict
 __global__ void k_empty_rows(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb, uint32_t n,
                              const uint32_t* __restrict__ s_ptr, const uint32_t* __restrict__ s_len,
                              uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ ctrl) {
+    after_previous(keys, s_ptr, s_len, o_ptr, ctrl);
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n || s_len[r] || timed_out(ctrl)) return;
     const uint32_t p = s_ptr[r];
@@ -246,6 +256,7 @@ __global__ void k_empty_rows(const uint64_t* __restrict__ keys, uint64_t entries
 // take the id of edge (c, r) from c's oriented row.  Written per sorted entry (compacted while
 // peeling) and per input entry (outputs are gathered by it).  An input that is not symmetric has
 // entries whose edge is not there: flagged.  The supports are cleared on the way.
+template <bool kChained>
 __global__ void __launch_bounds__(kThreads) k_entry_eid(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
                                                         uint32_t m, const uint32_t* __restrict__ o_ptr,
                                                         const uint32_t* __restrict__ o_col,
@@ -254,6 +265,7 @@ __global__ void __launch_bounds__(kThreads) k_entry_eid(const uint64_t* __restri
                                                         uint32_t* __restrict__ s_eid, uint32_t* __restrict__ entry_eid,
                                                         uint32_t* __restrict__ sup, uint32_t* __restrict__ supx,
                                                         uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(keys, o_ptr, o_col, fence, sorted_entry, s_eid, entry_eid, sup, supx, ctrl);
     const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (__any_sync(kFullMask, timed_out(ctrl))) return;
     uint32_t err = 0;
@@ -374,6 +386,7 @@ __global__ void __launch_bounds__(kThreads) k_canon_keys(const uint32_t* __restr
                                                          const uint32_t* __restrict__ dst, uint64_t entries, uint32_t n,
                                                          unsigned vb, unsigned passes, uint64_t* __restrict__ keys,
                                                          uint32_t* __restrict__ counts, uint32_t* __restrict__ ctrl) {
+    after_previous(src, dst, keys, counts, ctrl);
     __shared__ uint32_t h[kMaxDigitPasses * 256];
     digit_counts_clear(h, passes);
     uint32_t err = 0;
@@ -404,6 +417,7 @@ __device__ __forceinline__ bool canon_first(const uint64_t* __restrict__ keys, u
 // Unique edges before each tile, and all of them into the control block.
 __global__ void __launch_bounds__(kFlagThreads) k_canon_count(const uint64_t* __restrict__ keys, uint64_t entries,
                                                               unsigned vb, uint32_t* __restrict__ tile_start, Look L) {
+    after_previous(keys, tile_start);
     __shared__ FlagSmem S;
     const uint32_t tile = look_tile(L, &S.tile);
     if (tile == kNoTile) return;
@@ -429,6 +443,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_canon_emit(const uint64_t* __r
                                                              unsigned vb, const uint32_t* __restrict__ tile_start,
                                                              uint64_t capacity, uint32_t* __restrict__ src_out,
                                                              uint32_t* __restrict__ dst_out, Look L) {
+    after_previous(keys, tile_start, src_out, dst_out);
     __shared__ FlagSmem S;
     const uint64_t u = L.ctrl[kCtrlTriLo];
     if (__syncthreads_or(2 * u > capacity || timed_out(L.ctrl))) return;
@@ -475,24 +490,19 @@ int symmetrize(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
         return rc;
     cudaStream_t st = e->stream;
     const unsigned vb = bits_for(n > 1 ? n : 2), passes = (2 * vb + 7) / 8;
-    if ((rc = begin_session(e, n, 0, look_words(entries)))) return rc;
+    if ((rc = begin_session(e, n, 0, look_words(entries), entries))) return rc;
     uint32_t* counts = next_counts(e, passes);
-    k_canon_keys<<<key_blocks(e, entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, vb, passes, e->key_a, counts,
-                                                              e->ctrl);
-    count_launch(e);
-    if ((rc = check_launch(e, "k_canon_keys"))) return rc;
+    if ((rc = launch_chained(e, "k_canon_keys", k_canon_keys, key_blocks(e, entries), kThreads, 0, d_src, d_dst,
+                             entries, n, vb, passes, e->key_a, counts, e->ctrl))) return rc;
     int in_b = 0;
     if ((rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, entries, 0, passes, counts, &in_b))) return rc;
     const uint64_t* keys = in_b ? e->key_b : e->key_a;
     uint32_t* tile_start = reinterpret_cast<uint32_t*>(in_b ? e->key_a : e->key_b);  // the sort's other buffer
     const uint32_t tiles = ceil_div(entries, kFlagTile);
-    k_canon_count<<<tiles, kFlagThreads, 0, st>>>(keys, entries, vb, tile_start, next_look(e));
-    count_launch(e);
-    if ((rc = check_launch(e, "k_canon_count"))) return rc;
-    k_canon_emit<<<tiles, kFlagThreads, 0, st>>>(keys, entries, vb, tile_start, capacity, d_src_out, d_dst_out,
-                                                 next_look(e));
-    count_launch(e);
-    if ((rc = check_launch(e, "k_canon_emit")) || (rc = sync_and_check(e))) return rc;
+    if ((rc = launch_chained(e, "k_canon_count", k_canon_count, tiles, kFlagThreads, 0, keys, entries, vb,
+                             tile_start, next_look(e)))) return rc;
+    if ((rc = launch_chained(e, "k_canon_emit", k_canon_emit, tiles, kFlagThreads, 0, keys, entries, vb, tile_start,
+                             capacity, d_src_out, d_dst_out, next_look(e))) || (rc = sync_and_check(e))) return rc;
     const uint32_t u = e->h_ctrl[kCtrlTriLo];
     *num_out = 2ull * u;
     if (2ull * u > capacity)
@@ -516,7 +526,7 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
         (rc = reserve(e, n > e->cap_nodes ? n : e->cap_nodes, entries > e->cap_entries ? entries : e->cap_entries)))
         return rc;
     cudaStream_t st = e->stream;
-    if ((rc = begin_session(e, n, 0, look_words(entries)))) return rc;
+    if ((rc = begin_session(e, n, 0, look_words(entries), entries))) return rc;
     int in_b = 0;
     if (entries) {
         k_tile_keys<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, T, ts, vb, e->key_a, e->ctrl);
@@ -554,15 +564,14 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     e->vb = bits_for(n > 1 ? n : 2);
     const unsigned vb = e->vb;
     cudaStream_t st = e->stream;
-    int rc = begin_session(e, n, n, std::max(look_words(n), look_words(entries)));
+    int rc = begin_session(e, n, n, std::max(look_words(n), look_words(entries)), entries);
     if (rc) return rc;
     if (n == 0) return entries ? fail(KT_ERR_INVALID_ARG, "entries given for a graph with 0 vertices") : KT_OK;
 
     // 1. degrees (and id / self-loop checks)
     if (entries) {
-        k_degree<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, e->deg, e->ctrl);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_degree"))) return rc;
+        if ((rc = launch_chained(e, "k_degree", e->chained ? k_degree<true> : k_degree<false>, grid_for(entries),
+                                 kThreads, 0, d_src, d_dst, entries, n, e->deg, e->ctrl))) return rc;
     }
     // (input errors are read back once, after the build: every kernel up to its end indexes inside its
     // arrays whatever the input, and the kernels after it return at once when the error word is set)
@@ -571,50 +580,43 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     // starts of the symmetric CSR (row r holds the neighbours of the rank-r vertex)
     int in_b = 0;
     if (e->orient_by_index) {
-        k_rank_rows<true><<<ceil_div(n, kScanTile), kScanThreads, 0, st>>>(nullptr, e->deg, n, vb, e->rank, e->s_len,
-                                                                          e->s_ptr, e->s_split, e->o_ptr, next_look(e));
+        rc = launch_chained(e, "k_rank_rows", e->chained ? k_rank_rows<true, true> : k_rank_rows<true, false>,
+                            ceil_div(n, kScanTile), kScanThreads, 0, nullptr, e->deg, n, vb, e->rank, e->s_len,
+                            e->s_ptr, e->s_split, e->o_ptr, next_look(e));
     } else {
         const unsigned passes = (vb + 7) / 8;
         uint32_t* counts = next_counts(e, passes);
-        k_rank_keys<<<key_blocks(e, n), kThreads, 0, st>>>(e->deg, n, vb, passes, e->key_a, counts);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_rank_keys")) ||
+        if ((rc = launch_chained(e, "k_rank_keys", e->chained ? k_rank_keys<true> : k_rank_keys<false>,
+                                 key_blocks(e, n), kThreads, 0, e->deg, n, vb, passes, e->key_a, counts)) ||
             (rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, n, vb, passes, counts, &in_b)))
             return rc;
-        k_rank_rows<false><<<ceil_div(n, kScanTile), kScanThreads, 0, st>>>(in_b ? e->key_b : e->key_a, e->deg, n, vb,
-                                                                           e->rank, e->s_len, e->s_ptr, e->s_split,
-                                                                           e->o_ptr, next_look(e));
+        rc = launch_chained(e, "k_rank_rows", e->chained ? k_rank_rows<false, true> : k_rank_rows<false, false>,
+                            ceil_div(n, kScanTile), kScanThreads, 0, in_b ? e->key_b : e->key_a, e->deg, n, vb,
+                            e->rank, e->s_len, e->s_ptr, e->s_split, e->o_ptr, next_look(e));
     }
-    count_launch(e);
-    if ((rc = check_launch(e, "k_rank_rows"))) return rc;
+    if (rc) return rc;
 
     // 3. sort entries by (rank[src], rank[dst]); 4. both CSRs and the edge ids
     if (entries) {
         const unsigned passes = (2 * vb + 7) / 8;
         uint32_t* counts = next_counts(e, passes);
-        k_edge_keys<<<key_blocks(e, entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, e->rank, vb, passes, e->key_a,
-                                                                 counts, e->ctrl);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_edge_keys"))) return rc;
+        if ((rc = launch_chained(e, "k_edge_keys", e->chained ? k_edge_keys<true> : k_edge_keys<false>,
+                                 key_blocks(e, entries), kThreads, 0, d_src, d_dst, entries, n, e->rank, vb, passes,
+                                 e->key_a, counts, e->ctrl))) return rc;
         if ((rc = radix_passes(e, e->key_a, e->val_a, e->key_b, e->val_b, entries, 0, passes, counts, &in_b))) return rc;
         const uint64_t* keys = in_b ? e->key_b : e->key_a;
         e->sorted_entry = in_b ? e->val_b : e->val_a;
         e->entry_eid = in_b ? e->val_a : e->val_b;  // the sort's other value buffer is free now
-        k_csr<<<ceil_div(entries, kFlagTile), kFlagThreads, 0, st>>>(keys, entries, vb, n, e->m, e->s_col, e->s_eid,
-                                                                    e->s_split, e->o_ptr, e->o_col, e->e_src,
-                                                                    e->o_fence, next_look(e));
-        count_launch(e);
-        if ((rc = check_launch(e, "k_csr"))) return rc;
+        if ((rc = launch_chained(e, "k_csr", e->chained ? k_csr<true> : k_csr<false>, ceil_div(entries, kFlagTile),
+                                 kFlagThreads, 0, keys, entries, vb, n, e->m, e->s_col, e->s_eid, e->s_split,
+                                 e->o_ptr, e->o_col, e->e_src, e->o_fence, next_look(e)))) return rc;
         if (e->orient_by_index) {
-            k_empty_rows<<<grid_for(n), kThreads, 0, st>>>(keys, entries, vb, n, e->s_ptr, e->s_len, e->o_ptr, e->ctrl);
-            count_launch(e);
-            if ((rc = check_launch(e, "k_empty_rows"))) return rc;
+            if ((rc = launch_chained(e, "k_empty_rows", k_empty_rows, grid_for(n), kThreads, 0, keys, entries, vb, n,
+                                     e->s_ptr, e->s_len, e->o_ptr, e->ctrl))) return rc;
         }
-        k_entry_eid<<<grid_for(entries), kThreads, 0, st>>>(keys, entries, vb, e->m, e->o_ptr, e->o_col, e->o_fence,
-                                                            e->sorted_entry, e->s_eid, e->entry_eid, e->sup, e->rnd,
-                                                            e->ctrl);
-        count_launch(e);
-        if ((rc = check_launch(e, "k_entry_eid"))) return rc;
+        if ((rc = launch_chained(e, "k_entry_eid", e->chained ? k_entry_eid<true> : k_entry_eid<false>,
+                                 grid_for(entries), kThreads, 0, keys, entries, vb, e->m, e->o_ptr, e->o_col,
+                                 e->o_fence, e->sorted_entry, e->s_eid, e->entry_eid, e->sup, e->rnd, e->ctrl))) return rc;
     }
     return check && !e->trusted ? sync_and_check(e) : KT_OK;
 }

@@ -60,6 +60,27 @@ enum : uint32_t {
     kCtrlWords = 128,
 };
 
+// Kernels that the host chains (launch_chained) start while their predecessor still runs: its tail hides
+// their launch.  They wait here, before they touch memory, until it is done and its writes are visible;
+// what follows may then start in their own tail.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The pointer as the compiler sees it after the wait: loads through it are not moved before it.
+template <class T>
+__device__ __forceinline__ void anew(T& p) {
+    asm volatile("" : "+l"(p)::"memory");
+}
+
+template <class T, class... U>
+__device__ __forceinline__ void after_previous(T& p, U&... more) {
+    after_previous();
+    anew(p);
+    (anew(more), ...);
+}
+
 // Whether a single-k call's first round is run by recount_pruned instead of the peel kernel: the
 // frontier holds at least `percent` (0: never) of the m edges.  The word is final before the kernels that
 // ask start, so it may come from L1 (every thread of a large grid reads it).

@@ -87,6 +87,7 @@ struct kt_engine {
     size_t aux_words = 0;
     uint32_t* tile_off = nullptr;  // tiled variant: first oriented position of each (vertex, column tile)
     size_t tile_off_words = 0;     //   (own allocation, made by the first tiled call)
+    bool chained = false;  // the session's kernels start in their predecessors' tails (launch_chained)
     unsigned long long* ingest = nullptr;  // TSV ingest: outcome, tokens before each tile
     uint64_t ingest_words = 0;             //   (own allocation, made by the first ingest)
     uint2* lists = nullptr;        // triangle lists of a decomposition (own allocation, kt_lists.cu)
@@ -147,6 +148,26 @@ inline void count_launch(kt_engine* e, uint64_t n = 1) { e->launches += n; }
 int check_cuda(cudaError_t err, const char* what);
 int check_launch(kt_engine* e, const char* what);
 
+// Launches a kernel that begins with after_previous().  In a chained session it may start before its
+// predecessor in the stream has finished, whose tail then hides the launch: building a graph of 15,000
+// or 32,000 edges, 12 launches, takes 58 and 64 us instead of 81 and 87.
+template <class... P, class... A>
+int launch_chained(kt_engine* e, const char* what, void (*kernel)(P...), uint32_t blocks, int threads, int smem,
+                   A&&... args) {
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = e->stream;
+    c.attrs = &a;
+    c.numAttrs = e->chained ? 1 : 0;
+    count_launch(e);
+    return check_cuda(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...), what);
+}
+
 int reserve(kt_engine* e, uint32_t max_nodes, uint64_t max_entries);
 // kt_engine_replay bookkeeping (kt_engine.cu)
 void drop_replay(kt_engine* e);
@@ -165,7 +186,7 @@ inline uint64_t look_words(uint64_t keys) {
 }
 // A session clears the control block, deg[0, deg_words) and the look-back scratch for sorts of up to
 // `words` (look_words) and sets the row marks to n; each launch that looks back takes a tag of it.
-int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words);
+int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words, uint64_t keys);
 Look next_look(kt_engine* e);
 uint32_t* next_counts(kt_engine* e, unsigned passes);  // zeroed digit counts, 256 words a pass
 int count_digits(kt_engine* e, const uint64_t* keys, uint64_t n, unsigned shift, unsigned passes, uint32_t* counts);

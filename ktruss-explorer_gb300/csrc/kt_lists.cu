@@ -664,11 +664,13 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.
+template <bool kChained>
 __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restrict__ sup,
                                                               const uint32_t* __restrict__ supx,
                                                               uint32_t* __restrict__ ycount, uint32_t m,
                                                               uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
                                                               Look L) {
+    if (kChained) after_previous(sup, supx, ycount, tptr, ends);
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
     if (__syncthreads_or(failed(L.ctrl))) return;
@@ -793,10 +795,9 @@ int peel_lists(kt_engine* e, bool* done) {
     // the sort's key buffers are free after the build: list starts, and ends for the fill
     uint64_t* tptr = e->key_a;
     uint64_t* ends = e->key_b;
-    k_list_bounds<<<ceil_div(m, kScanTile), kScanThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, m, tptr, ends,
-                                                                         next_look(e));
-    count_launch(e);
-    if ((rc = check_launch(e, "k_list_bounds")) || (rc = want_lists(e, done)) || !*done ||
+    if ((rc = launch_chained(e, "k_list_bounds", e->chained ? k_list_bounds<true> : k_list_bounds<false>,
+                             ceil_div(m, kScanTile), kScanThreads, 0, e->sup, e->rnd, e->tr, m, tptr, ends,
+                             next_look(e))) || (rc = want_lists(e, done)) || !*done ||
         (rc = fill_lists(e, tptr, ends)))
         return rc;
     ListParams P;

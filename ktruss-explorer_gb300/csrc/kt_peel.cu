@@ -808,12 +808,14 @@ __device__ void count_passes(const uint32_t* __restrict__ size, const uint32_t* 
     }
 }
 
+template <bool kChained>
 __global__ void __launch_bounds__(kThreads) k_emit_truss(const uint32_t* __restrict__ entry_eid, uint64_t entries,
                                                          const uint32_t* __restrict__ tr, uint32_t* __restrict__ out,
                                                          uint32_t* __restrict__ k_max,
                                                          const uint32_t* __restrict__ round_size,
                                                          const uint32_t* __restrict__ round_level, uint32_t cap_rounds,
                                                          uint32_t m, uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(entry_eid, tr, out, k_max, round_size, round_level, ctrl);
     if (failed(ctrl)) return;  // the same for the whole launch
     if (blockIdx.x == 0 && ctrl[kPRounds] < cap_rounds)
         count_passes(round_size, round_level, ctrl[kPRounds], m, ctrl);
@@ -822,8 +824,10 @@ __global__ void __launch_bounds__(kThreads) k_emit_truss(const uint32_t* __restr
     if (i == 0 && k_max) *k_max = ctrl[kPKmax];
 }
 
+template <bool kChained>
 __global__ void k_emit_keep(const uint32_t* __restrict__ entry_eid, uint64_t entries, const uint32_t* __restrict__ rnd,
                             uint8_t* __restrict__ out, const uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(entry_eid, rnd, out, ctrl);
     if (failed(ctrl)) return;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < entries) out[i] = rnd[entry_eid[i]] == 0 ? 1 : 0;
@@ -1027,10 +1031,9 @@ int peel_single_k(kt_engine* e, uint32_t k) {
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max) {
     int rc;
     if (e->entries) {
-        k_emit_truss<<<grid_for(e->entries), kThreads, 0, e->stream>>>(
-            e->entry_eid, e->entries, e->tr, d_out, d_k_max, e->round_size, e->round_level, e->cap_rounds, e->m, e->ctrl);
-        count_launch(e);
-        return check_launch(e, "k_emit_truss");
+        return launch_chained(e, "k_emit_truss", e->chained ? k_emit_truss<true> : k_emit_truss<false>,
+                              grid_for(e->entries), kThreads, 0, e->entry_eid, e->entries, e->tr, d_out, d_k_max,
+                              e->round_size, e->round_level, e->cap_rounds, e->m, e->ctrl);
     }
     if (d_k_max && (rc = check_cuda(cudaMemsetAsync(d_k_max, 0, sizeof(uint32_t), e->stream), "clear k_max"))) return rc;
     return KT_OK;
@@ -1050,9 +1053,8 @@ int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, 
 
 int emit_keep(kt_engine* e, uint8_t* d_keep) {
     if (!e->entries) return KT_OK;
-    k_emit_keep<<<grid_for(e->entries), kThreads, 0, e->stream>>>(e->entry_eid, e->entries, e->rnd, d_keep, e->ctrl);
-    count_launch(e);
-    return check_launch(e, "k_emit_keep");
+    return launch_chained(e, "k_emit_keep", e->chained ? k_emit_keep<true> : k_emit_keep<false>,
+                          grid_for(e->entries), kThreads, 0, e->entry_eid, e->entries, e->rnd, d_keep, e->ctrl);
 }
 
 // Reads the control block (unless the call left it in h_ctrl) after the stream has drained; fills the

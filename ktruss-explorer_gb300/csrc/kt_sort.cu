@@ -33,6 +33,7 @@ constexpr int kSmallThreads = 256, kSmallItems = (int)kSmallTile / kSmallThreads
 // Digit counts of all passes for keys that are there already.
 __global__ void __launch_bounds__(256) k_digit_counts(const uint64_t* __restrict__ keys, uint64_t n, unsigned shift,
                                                       unsigned passes, uint32_t* __restrict__ counts) {
+    after_previous(keys, counts);
     __shared__ uint32_t h[kMaxDigitPasses * kDigits];
     digit_counts_clear(h, passes);
     for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
                                                          uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
                                                          uint64_t n, unsigned shift,
                                                          const uint32_t* __restrict__ counts, Look L) {
+    if (kThreads * kItems == (int)kSmallTile) after_previous(kin, vin, kout, vout, counts);
     extern __shared__ __align__(16) unsigned char raw[];
     PassSmem<kThreads, kItems>& S = *reinterpret_cast<PassSmem<kThreads, kItems>*>(raw);
     constexpr int kWarps = kThreads / 32;
@@ -209,6 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
 __global__ void k_session(uint32_t* __restrict__ ctrl, uint32_t ctrl_words, uint32_t n, uint32_t* __restrict__ deg,
                           uint32_t deg_words, uint4* __restrict__ words, uint64_t quads, uint32_t* __restrict__ counts,
                           uint32_t count_words) {
+    after_previous(ctrl, deg, words, counts);
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = tid; i < ctrl_words; i += step) ctrl[i] = i == kCtrlBigRow || i == kCtrlTinyRow ? n : 0u;
     for (uint64_t i = tid; i < deg_words; i += step) deg[i] = 0;
@@ -220,11 +223,16 @@ template <int kThreads, int kItems, bool kVals>
 int launch_pass(kt_engine* e, const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, uint64_t n,
                 unsigned shift, const uint32_t* counts, const Look& L) {
     const int smem = (int)sizeof(PassSmem<kThreads, kItems>);
-    int rc = check_cuda(cudaFuncSetAttribute(k_radix_pass<kThreads, kItems, kVals>,
+    int rc = KT_OK;
+    if (smem > 48 * 1024)
+        rc = check_cuda(cudaFuncSetAttribute(k_radix_pass<kThreads, kItems, kVals>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                         "shared memory of k_radix_pass");
     if (rc) return rc;
     const uint64_t tiles = (n + kThreads * kItems - 1) / (kThreads * kItems);
+    if (kThreads * kItems == (int)kSmallTile)
+        return launch_chained(e, "k_radix_pass", k_radix_pass<kThreads, kItems, kVals>, (uint32_t)tiles, kThreads, smem,
+                              kin, vin, kout, vout, n, shift, counts, L);
     k_radix_pass<kThreads, kItems, kVals><<<(uint32_t)tiles, kThreads, smem, e->stream>>>(kin, vin, kout, vout, n, shift,
                                                                                          counts, L);
     count_launch(e);
@@ -233,16 +241,17 @@ int launch_pass(kt_engine* e, const uint64_t* kin, const uint32_t* vin, uint64_t
 
 }  // namespace
 
-int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words) {
+int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words, uint64_t keys) {
+    // Small graphs: their kernels are no longer than a launch takes (R-MAT of 2^20 vertices gains nothing, and
+    // the pointers that a chained kernel launders cost its build 8 %).  Not on a caller's own stream.
+    e->chained = e->lists_allowed && keys <= kSmallSort && n <= kSmallSort;
     if (words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
     e->look_tag = e->look_count = 0;
     e->ctrl_fresh = false;
     const uint64_t work = std::max<uint64_t>(words / 2, std::max<uint32_t>(deg_words, kCountWords));
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((work + 255) / 256, (uint64_t)e->num_sms * 8);
-    k_session<<<blocks, 256, 0, e->stream>>>(e->ctrl, kCtrlWords, n, e->deg, deg_words,
-                                             reinterpret_cast<uint4*>(e->look), words / 2, e->digit_counts, kCountWords);
-    count_launch(e);
-    return check_launch(e, "k_session");
+    return launch_chained(e, "k_session", k_session, blocks, 256, 0, e->ctrl, kCtrlWords, n, e->deg, deg_words,
+                          reinterpret_cast<uint4*>(e->look), words / 2, e->digit_counts, kCountWords);
 }
 
 Look next_look(kt_engine* e) {
@@ -258,9 +267,7 @@ uint32_t* next_counts(kt_engine* e, unsigned passes) {
 
 int count_digits(kt_engine* e, const uint64_t* keys, uint64_t n, unsigned shift, unsigned passes, uint32_t* counts) {
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((n + 1023) / 1024, (uint64_t)e->num_sms * 8);
-    k_digit_counts<<<blocks, 256, 0, e->stream>>>(keys, n, shift, passes, counts);
-    count_launch(e);
-    return check_launch(e, "k_digit_counts");
+    return launch_chained(e, "k_digit_counts", k_digit_counts, blocks, 256, 0, keys, n, shift, passes, counts);
 }
 
 int radix_passes(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b, uint32_t* val_b, uint64_t n,

@@ -192,6 +192,7 @@ __device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
 
 template <int G, bool kFill, bool kPruned = false>
 __global__ void __launch_bounds__(kThreads) k_support(Graph g, Credits c) {
+    after_previous();
     if (skip<kPruned>(g)) return;
     edge_body<G, kFill, kPruned>(g, c);
 }
@@ -473,8 +474,10 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
 
 // sup += supx, what it was into ycount, the sum of all supports (three per triangle), and the number of
 // supports below `limit` (a single-k call's first frontier).
+template <bool kChained>
 __global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __restrict__ supx,
                                 uint32_t* __restrict__ ycount, uint32_t m, uint32_t limit, uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(sup, supx, ycount, ctrl);
     if (failed(ctrl)) return;
     uint64_t s = 0;
     uint32_t low = 0;
@@ -498,8 +501,10 @@ __global__ void k_merge_support(uint32_t* __restrict__ sup, const uint32_t* __re
 // that the peel kernel would have left.
 // Bound: memory, 12 bytes an edge, and for small graphs its own latency.  R-MAT 20 (15 M edges)
 // 0.024 ms, 7.4 TB/s as the supports lie in L2 (merging the credits and the peel kernel's one round: 0.70 ms).
+template <bool kChained>
 __global__ void __launch_bounds__(kThreads) k_truss3(uint32_t* __restrict__ sup, uint32_t* __restrict__ rnd,
                                                      uint32_t m, PeelLog log, uint32_t* __restrict__ ctrl) {
+    if (kChained) after_previous(sup, rnd, ctrl);
     __shared__ unsigned long long s_sum;
     __shared__ uint32_t s_low;
     if (__syncthreads_or(failed(ctrl))) return;
@@ -661,19 +666,17 @@ int count_support(kt_engine* e) {
     const uint32_t G = e->sched.support_group ? e->sched.support_group : 8;
     const uint32_t blocks = edge_blocks(e, G);
     switch (G) {
-        case 4: k_support<4, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
-        case 16: k_support<16, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
-        case 32: k_support<32, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
-        default: k_support<8, false><<<blocks, kThreads, 0, e->stream>>>(g, c); break;
+        case 4: rc = launch_chained(e, "k_support", k_support<4, false>, blocks, kThreads, 0, g, c); break;
+        case 16: rc = launch_chained(e, "k_support", k_support<16, false>, blocks, kThreads, 0, g, c); break;
+        case 32: rc = launch_chained(e, "k_support", k_support<32, false>, blocks, kThreads, 0, g, c); break;
+        default: rc = launch_chained(e, "k_support", k_support<8, false>, blocks, kThreads, 0, g, c); break;
     }
-    count_launch(e);
-    return check_launch(e, "k_support");
+    return rc;
 }
 
 int merge_support(kt_engine* e, uint32_t limit) {
-    k_merge_support<<<(uint32_t)e->num_sms * 4, kThreads, 0, e->stream>>>(e->sup, e->rnd, e->tr, e->m, limit, e->ctrl);
-    count_launch(e);
-    return check_launch(e, "k_merge_support");
+    return launch_chained(e, "k_merge_support", e->chained ? k_merge_support<true> : k_merge_support<false>,
+                          (uint32_t)e->num_sms * 4, kThreads, 0, e->sup, e->rnd, e->tr, e->m, limit, e->ctrl);
 }
 
 int truss3(kt_engine* e) {
@@ -681,9 +684,8 @@ int truss3(kt_engine* e) {
                       e->level_k, e->level_alive, e->level_ns, e->level_front, e->cap_levels};
     const uint32_t blocks =
         (uint32_t)std::min<uint64_t>(((uint64_t)e->m + 4 * kThreads - 1) / (4 * kThreads), (uint64_t)e->num_sms * 8);
-    k_truss3<<<blocks, kThreads, 0, e->stream>>>(e->sup, e->rnd, e->m, log, e->ctrl);
-    count_launch(e);
-    return check_launch(e, "k_truss3");
+    return launch_chained(e, "k_truss3", e->chained ? k_truss3<true> : k_truss3<false>, blocks, kThreads, 0, e->sup,
+                          e->rnd, e->m, log, e->ctrl);
 }
 
 // The first round of a single-k call whose frontier (supports below `limit`) is a recount round: the
@@ -729,10 +731,9 @@ int recount_pruned(kt_engine* e, uint32_t limit, uint32_t percent, PrunedCount* 
     k_middle_plan<true><<<(e->n + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(g, items_of(e), nullptr, e->ctrl);
     count_launch(e);
     if ((rc = check_launch(e, "k_middle_plan")) || (rc = launch_middle<false, true>(e, g, c))) return rc;
-    k_support<8, false, true><<<edge_blocks(e, 8), kThreads, 0, e->stream>>>(g, c);
-    count_launch(e);
+    rc = launch_chained(e, "k_support", k_support<8, false, true>, edge_blocks(e, 8), kThreads, 0, g, c);
     *out = PrunedCount{percent, new_id, count};
-    return check_launch(e, "k_support");
+    return rc;
 }
 
 int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends) {
@@ -748,9 +749,7 @@ int fill_lists(kt_engine* e, const uint64_t* tptr, uint64_t* ends) {
         count_launch(e);
         if ((rc = check_launch(e, "k_rows"))) return rc;
     }
-    k_support<8, true><<<edge_blocks(e, 8), kThreads, 0, e->stream>>>(g, c);
-    count_launch(e);
-    return check_launch(e, "k_support");
+    return launch_chained(e, "k_support", k_support<8, true>, edge_blocks(e, 8), kThreads, 0, g, c);
 }
 
 }  // namespace kt
