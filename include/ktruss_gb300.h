@@ -173,12 +173,13 @@ typedef struct kt_stats {
     float peel_phase_ms[6];      /* peel kernel time by phase (init, level scan, frontier
                                     collection, row compaction, mark, process), barrier to
                                     barrier, as seen by its first block                        */
-    float peel_kernel_ms;        /* CUDA-event time of the peel kernel launch alone            */
+    float peel_kernel_ms;        /* CUDA-event time of the peel kernel launch alone (0 for k <= 3,
+                                    which need none)                                           */
     float select_ms;             /* learned selector: statistics, features and inference, one
                                     launch (0 without a selector); part of last_ms             */
-    uint64_t walk_entries;       /* adjacency entries in the rows of all queued edges: the
-                                    decrement work (a round that recounts instead does not walk
-                                    its queued rows)                                          */
+    uint64_t walk_entries;       /* entries of the triangle lists, or of the adjacency rows, of all
+                                    queued edges: the decrement work (a round that recounts
+                                    instead does not walk its queued rows)                    */
     float copy_in_ms;            /* host-buffer calls (kt_decompose, kt_decompose_batch): device
                                     time of the input copies host -> device                   */
     float copy_out_ms;           /*   and of the output copies device -> host (plus the emit
@@ -190,9 +191,13 @@ typedef struct kt_stats {
 /* Schedule of the engine's kernels (no counterpart in the reference, whose tuning knobs are the
  * -b/-t block and tile sizes).  Every schedule gives the same result; only the time differs. */
 typedef struct kt_schedule {
-    uint32_t support_group;    /* support count: lanes per oriented edge (4, 8, 16 or 32), or 0
-                                  for the vertex-centric count with shared-memory hash tables   */
-    uint32_t chunk_width;      /* row entries per peel work chunk (lanes per chunk): 8, 16 or 32  */
+    uint32_t support_group;    /* support count: lanes per oriented edge (4, 8, 16 or 32) where it is
+                                  counted edge by edge, or 0 to count every vertex with
+                                  shared-memory tables (graphs of 2^18 edges or more count the
+                                  vertices that pay for a table that way with any group)        */
+    uint32_t chunk_width;      /* row entries per work chunk of the walking peel (lanes per
+                                  chunk): 8, 16 or 32.  This and the fields below have no effect
+                                  on decompositions from triangle lists                          */
     uint32_t compact_percent;  /* compact the adjacency rows at a level start once the alive
                                   edges are below this percentage of the count at the last
                                   compaction: 1..99, or 0 = never                                */
@@ -200,7 +205,9 @@ typedef struct kt_schedule {
                                   the alive edges removes it at once and recounts the support of
                                   the surviving edges from scratch (the reference's full
                                   recount) instead of decrementing it per destroyed triangle
-                                  (its affected-edge recount, made exact): 1..100, or 0 = never */
+                                  (its affected-edge recount, made exact): 1..100, or 0 = never.
+                                  The first round of a single-k call on 2^20 edges or more
+                                  recounts from 7/10 of it on                                    */
     uint32_t peel_blocks;      /* peel kernel blocks per SM: 1 (64 registers a thread), 2 (32
                                   registers, twice the warps: hides DRAM latency once the graph
                                   outgrows L2), or 0 = 2 when the oriented CSR of a single graph
@@ -216,7 +223,8 @@ int kt_engine_destroy(kt_engine* engine);
 /* Returns the engine's cudaStream_t (as void*). */
 void* kt_engine_stream(kt_engine* engine);
 /* Pre-allocates the device workspace for graphs up to these sizes, so that later calls of at
- * most this size do not allocate. */
+ * most this size do not allocate - but for the triangle lists of graphs of more than 32,768 edges,
+ * whose size their triangles decide: the first decomposition that needs more of them allocates. */
 int kt_engine_reserve(kt_engine* engine, uint32_t max_nodes, uint64_t max_entries);
 /* Device-resident decomposition.  d_src/d_dst: num_entries entries on the engine's device
  * (symmetric simple graph, both directions).  d_truss_per_entry: num_entries outputs.
