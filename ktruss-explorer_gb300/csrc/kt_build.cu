@@ -14,8 +14,8 @@
 //      the neighbour's oriented row, which also proves the input symmetric (k_entry_eid).
 //
 // Scans and radix passes are one kernel each (kt_look.cuh).  A small graph's build is bound by its
-// launches: G(4096, 16/4095) takes 12 instead of 43, chained, 0.064 ms instead of 0.238; R-MAT 16 0.21 instead of
-// 0.42 ms, R-MAT 20 2.6 instead of 3.05 ms (the sort's five passes 1.3 ms of it).
+// launches: G(4096, 16/4095) takes 12 instead of 43, chained, 0.064 ms instead of 0.238; R-MAT 16 0.20 instead of
+// 0.42 ms, R-MAT 20 2.53 instead of 3.05 ms (the sort's five passes 1.3 ms of it).
 //
 // Layout in HBM (n vertices, m undirected edges, all uint32):
 //   s_ptr[n+1], s_len[n], s_split[n]   symmetric rows (lower ranks, then higher ranks)
@@ -169,11 +169,29 @@ __global__ void __launch_bounds__(kThreads) k_edge_keys(const uint32_t* __restri
     digit_counts_flush(h, passes, counts);
 }
 
+// A tile's sorted keys in shared memory, key[1] on, with the one before it (~0 in front of the first) and the
+// one after it (past the last entry: ~0, then 0).  Ends with a __syncthreads.  Kept here over the look-back instead
+// of in registers, 2,048 threads fit an SM: k_csr over 30 M keys 0.235 -> 0.195 ms.
+__device__ __forceinline__ void stage_keys(uint64_t* key, const uint64_t* __restrict__ keys, uint64_t entries,
+                                           uint32_t tile) {
+    const uint64_t t0 = (uint64_t)tile * kFlagTile;
+#pragma unroll
+    for (uint32_t s = 0; s < kFlagSteps; ++s) {
+        const uint32_t i = s * kFlagThreads + threadIdx.x;
+        key[1 + i] = t0 + i < entries ? keys[t0 + i] : t0 + i == entries ? ~0ull : 0ull;
+    }
+    if (threadIdx.x == 0) {
+        key[0] = t0 > 0 ? keys[t0 - 1] : ~0ull;
+        key[1 + kFlagTile] = t0 + kFlagTile < entries ? keys[t0 + kFlagTile] : ~0ull;
+    }
+    __syncthreads();
+}
+
 // One pass over the sorted entry keys builds both CSRs: columns, the duplicate check, where each
 // row's higher-rank part starts, and - by a scan of the higher-rank entries - their oriented
 // positions, which are the edge ids.  A row's oriented start is the scan at its first entry.
 template <bool kChained>
-__global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
+__global__ void __launch_bounds__(kFlagThreads, 4) k_csr(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb,
                                                       uint32_t n, uint32_t m, uint32_t* __restrict__ s_col,
                                                       uint32_t* __restrict__ s_eid, uint32_t* __restrict__ s_split,
                                                       uint32_t* __restrict__ o_ptr, uint32_t* __restrict__ o_col,
@@ -181,27 +199,24 @@ __global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict
                                                       Look L) {
     if (kChained) after_previous(keys, s_col, s_eid, s_split, o_ptr, o_col, e_src, fence);
     __shared__ FlagSmem S;
+    __shared__ uint64_t key[kFlagTile + 2];  // the tile's, one before and one after
     const uint32_t tile = look_tile(L, &S.tile);
     if (tile == kNoTile) return;
     const uint64_t p0 = (uint64_t)tile * kFlagTile + threadIdx.x;
     const uint64_t mask = (1ull << vb) - 1;
     const uint32_t warp = threadIdx.x >> 5;
-    uint64_t key[kFlagSteps];
     uint32_t fwd = 0;  // bit s: the entry of step s is a higher-rank one
+    stage_keys(key, keys, entries, tile);
 #pragma unroll
     for (uint32_t s = 0; s < kFlagSteps; ++s) {
-        const uint64_t p = p0 + s * kFlagThreads;
-        key[s] = p < entries ? keys[p] : 0ull;
-    }
-#pragma unroll
-    for (uint32_t s = 0; s < kFlagSteps; ++s) {
-        const bool f = (uint32_t)(key[s] & mask) > (uint32_t)(key[s] >> vb);
+        const uint64_t k = key[1 + s * kFlagThreads + threadIdx.x];
+        const bool f = (uint32_t)(k & mask) > (uint32_t)(k >> vb);
         fwd |= (uint32_t)f << s;
         const uint32_t b = __ballot_sync(kFullMask, f);
         if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
     }
     __syncthreads();
-    flag_sums<true>(S, L, tile);
+    flag_sums(S, L, tile);
     uint32_t err = 0;
 #pragma unroll
     for (uint32_t s = 0; s < kFlagSteps; ++s) {
@@ -210,8 +225,8 @@ __global__ void __launch_bounds__(kFlagThreads) k_csr(const uint64_t* __restrict
         const uint64_t j = S.prefix + S.before[s * kFlagWarps + warp] +
                            __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
         if (p < entries) {
-            const uint64_t k = key[s];
-            const uint64_t prev = p > 0 ? keys[p - 1] : ~0ull, next = p + 1 < entries ? keys[p + 1] : ~0ull;
+            const uint64_t* const at = key + 1 + s * kFlagThreads + threadIdx.x;
+            const uint64_t k = *at, prev = at[-1], next = at[1];
             const uint32_t row = (uint32_t)(k >> vb), col = (uint32_t)(k & mask);
             const bool first = p == 0 || (uint32_t)(prev >> vb) != row;
             const bool last = p + 1 == entries || (uint32_t)(next >> vb) != row;
@@ -414,60 +429,65 @@ __device__ __forceinline__ bool canon_first(const uint64_t* __restrict__ keys, u
     return (*key >> vb) != (*key & ((1ull << vb) - 1)) && (p == 0 || keys[p - 1] != *key);
 }
 
-// Unique edges before each tile, and all of them into the control block.
+// Unique edges, into the control block.  (16.8 M keys: 37 us, and k_canon_emit, which numbers them by
+// look-back, 119; with the look-back here, where the tiles finish almost together, 83 and 90.)
 __global__ void __launch_bounds__(kFlagThreads) k_canon_count(const uint64_t* __restrict__ keys, uint64_t entries,
-                                                              unsigned vb, uint32_t* __restrict__ tile_start, Look L) {
-    after_previous(keys, tile_start);
-    __shared__ FlagSmem S;
-    const uint32_t tile = look_tile(L, &S.tile);
-    if (tile == kNoTile) return;
+                                                              unsigned vb, uint32_t* __restrict__ ctrl) {
+    after_previous(keys, ctrl);
+    __shared__ uint32_t s_count;
+    if (threadIdx.x == 0) s_count = 0;
+    if (__syncthreads_or(timed_out(ctrl))) return;
+    uint32_t count = 0;
+    for (uint64_t p0 = (uint64_t)blockIdx.x * kFlagTile + threadIdx.x; p0 < entries;
+         p0 += (uint64_t)gridDim.x * kFlagTile) {
 #pragma unroll
-    for (uint32_t s = 0; s < kFlagSteps; ++s) {
-        uint64_t key;
-        const bool f =
-            canon_first(keys, entries, vb, (uint64_t)tile * kFlagTile + s * kFlagThreads + threadIdx.x, &key);
-        const uint32_t b = __ballot_sync(kFullMask, f);
-        if (lane_id() == 0) S.before[s * kFlagWarps + (threadIdx.x >> 5)] = __popc(b);
+        for (uint32_t s = 0; s < kFlagSteps; ++s) {
+            uint64_t key;
+            count += canon_first(keys, entries, vb, p0 + s * kFlagThreads, &key);
+        }
     }
+    count = __reduce_add_sync(kFullMask, count);
+    if (lane_id() == 0 && count) atomicAdd(&s_count, count);
     __syncthreads();
-    flag_sums<true>(S, L, tile);
-    if (threadIdx.x == 0) {
-        tile_start[tile] = (uint32_t)S.prefix;
-        if (tile == gridDim.x - 1) L.ctrl[kCtrlTriLo] = (uint32_t)(S.prefix + S.total);
-    }
+    if (threadIdx.x == 0 && s_count) atomicAdd(ctrl + kCtrlTriLo, s_count);
 }
 
 // Unique edge j goes to j as (lo, hi) and to u + j as (hi, lo), where u is their number; nothing is
 // written unless all 2u entries fit.
-__global__ void __launch_bounds__(kFlagThreads) k_canon_emit(const uint64_t* __restrict__ keys, uint64_t entries,
-                                                             unsigned vb, const uint32_t* __restrict__ tile_start,
-                                                             uint64_t capacity, uint32_t* __restrict__ src_out,
+__global__ void __launch_bounds__(kFlagThreads, 4) k_canon_emit(const uint64_t* __restrict__ keys, uint64_t entries,
+                                                             unsigned vb, uint64_t capacity,
+                                                             uint32_t* __restrict__ src_out,
                                                              uint32_t* __restrict__ dst_out, Look L) {
-    after_previous(keys, tile_start, src_out, dst_out);
+    after_previous(keys, src_out, dst_out);
     __shared__ FlagSmem S;
+    __shared__ uint64_t key[kFlagTile + 2];
     const uint64_t u = L.ctrl[kCtrlTriLo];
-    if (__syncthreads_or(2 * u > capacity || timed_out(L.ctrl))) return;
+    if (__syncthreads_or(2 * u > capacity)) return;
+    const uint32_t tile = look_tile(L, &S.tile);
+    if (tile == kNoTile) return;
     const uint32_t warp = threadIdx.x >> 5;
-    uint64_t key[kFlagSteps];
+    const uint64_t mask = (1ull << vb) - 1;
     uint32_t first = 0;
+    stage_keys(key, keys, entries, tile);
 #pragma unroll
     for (uint32_t s = 0; s < kFlagSteps; ++s) {
-        const bool f = canon_first(keys, entries, vb, (uint64_t)blockIdx.x * kFlagTile + s * kFlagThreads + threadIdx.x,
-                                   &key[s]);
+        const uint32_t i = s * kFlagThreads + threadIdx.x;
+        const uint64_t k = key[1 + i];
+        const bool f = (uint64_t)tile * kFlagTile + i < entries && k != key[i] && (k >> vb) != (k & mask);
         first |= (uint32_t)f << s;
         const uint32_t b = __ballot_sync(kFullMask, f);
         if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
     }
     __syncthreads();
-    flag_sums<false>(S, L, blockIdx.x);
-    const uint32_t start = tile_start[blockIdx.x];
+    flag_sums(S, L, tile);
 #pragma unroll
     for (uint32_t s = 0; s < kFlagSteps; ++s) {
         const bool f = first >> s & 1u;
         const uint64_t j =
-            start + S.before[s * kFlagWarps + warp] + __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
+            S.prefix + S.before[s * kFlagWarps + warp] + __popc(__ballot_sync(kFullMask, f) & lanemask_lt());
         if (f) {
-            const uint32_t lo = (uint32_t)(key[s] >> vb), hi = (uint32_t)(key[s] & ((1ull << vb) - 1));
+            const uint64_t k = key[1 + s * kFlagThreads + threadIdx.x];
+            const uint32_t lo = (uint32_t)(k >> vb), hi = (uint32_t)(k & mask);
             src_out[j] = lo;
             dst_out[j] = hi;
             src_out[u + j] = hi;
@@ -488,7 +508,6 @@ int symmetrize(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
     if ((n > e->cap_nodes || entries > e->cap_entries) &&
         (rc = reserve(e, n > e->cap_nodes ? n : e->cap_nodes, entries > e->cap_entries ? entries : e->cap_entries)))
         return rc;
-    cudaStream_t st = e->stream;
     const unsigned vb = bits_for(n > 1 ? n : 2), passes = (2 * vb + 7) / 8;
     if ((rc = begin_session(e, n, 0, look_words(entries), entries))) return rc;
     uint32_t* counts = next_counts(e, passes);
@@ -497,12 +516,11 @@ int symmetrize(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint6
     int in_b = 0;
     if ((rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, entries, 0, passes, counts, &in_b))) return rc;
     const uint64_t* keys = in_b ? e->key_b : e->key_a;
-    uint32_t* tile_start = reinterpret_cast<uint32_t*>(in_b ? e->key_a : e->key_b);  // the sort's other buffer
     const uint32_t tiles = ceil_div(entries, kFlagTile);
-    if ((rc = launch_chained(e, "k_canon_count", k_canon_count, tiles, kFlagThreads, 0, keys, entries, vb,
-                             tile_start, next_look(e)))) return rc;
-    if ((rc = launch_chained(e, "k_canon_emit", k_canon_emit, tiles, kFlagThreads, 0, keys, entries, vb, tile_start,
-                             capacity, d_src_out, d_dst_out, next_look(e))) || (rc = sync_and_check(e))) return rc;
+    if ((rc = launch_chained(e, "k_canon_count", k_canon_count, std::min(tiles, (uint32_t)e->num_sms * 4), kFlagThreads,
+                             0, keys, entries, vb, e->ctrl))) return rc;
+    if ((rc = launch_chained(e, "k_canon_emit", k_canon_emit, tiles, kFlagThreads, 0, keys, entries, vb, capacity,
+                             d_src_out, d_dst_out, next_look(e))) || (rc = sync_and_check(e))) return rc;
     const uint32_t u = e->h_ctrl[kCtrlTriLo];
     *num_out = 2ull * u;
     if (2ull * u > capacity)
@@ -563,7 +581,6 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     e->sched_on_device = false;  // a call with a selector sets it after the build
     e->vb = bits_for(n > 1 ? n : 2);
     const unsigned vb = e->vb;
-    cudaStream_t st = e->stream;
     int rc = begin_session(e, n, n, std::max(look_words(n), look_words(entries)), entries);
     if (rc) return rc;
     if (n == 0) return entries ? fail(KT_ERR_INVALID_ARG, "entries given for a graph with 0 vertices") : KT_OK;

@@ -189,8 +189,7 @@ struct FlagSmem {
 };
 
 // Turns the counts in S.before into exclusive sums (after a __syncthreads by the caller; ends with
-// one).  With kLook the tile's prefix over all tiles comes from its predecessors.
-template <bool kLook>
+// one).  The tile's prefix over all tiles comes from its predecessors.
 __device__ __forceinline__ void flag_sums(FlagSmem& S, const Look& L, uint32_t tile) {
     constexpr uint32_t kPer = kFlagSteps * kFlagWarps / 32;
     const uint32_t lane = lane_id();
@@ -214,7 +213,7 @@ __device__ __forceinline__ void flag_sums(FlagSmem& S, const Look& L, uint32_t t
             at += c[i];
         }
         const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-        const uint64_t p = kLook ? look_back(L, tile, total) : 0;
+        const uint64_t p = look_back(L, tile, total);
         if (lane == 0) {
             S.prefix = p;
             S.total = total;

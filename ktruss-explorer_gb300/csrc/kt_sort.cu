@@ -9,7 +9,7 @@
 //
 // Bound: the serial chain of a tile (ticket, loads, counts, ranks, look-back, runs) at half occupancy, 64
 // registers, issue active 47 % - and for small inputs the launches.  A pass over 30 M keys with values
-// takes 0.26 ms, 2.8 TB/s of keys and values (0.31 ms when the counts were published after the ranks
+// takes 0.255 ms, 2.8 TB/s of keys and values (0.31 ms when the counts were published after the ranks
 // and a tile's places were added up from three tables; histogram, scan and scatter kernels: 0.33 ms); a
 // pass over 64,000 entries is one launch instead of four.
 
@@ -72,17 +72,18 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
     const uint32_t tile = look_tile(L, &S.tile);
     if (tile == kNoTile) return;
     const uint64_t tbase = (uint64_t)tile * (kThreads * kItems);
-    const uint64_t wbase = tbase + (uint64_t)warp * (32 * kItems);
+    const uint32_t left = (uint32_t)min((uint64_t)(kThreads * kItems), n - tbase);  // keys of the tile
+    const uint32_t p0 = warp * (32 * kItems) + lane;  // this lane's first one
     uint64_t key[kItems];
 #pragma unroll
     for (int s = 0; s < kItems; ++s) {
-        const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
-        key[s] = idx < n ? kin[idx] : 0ull;
+        const uint32_t p = p0 + (uint32_t)s * 32;
+        key[s] = p < left ? kin[tbase + p] : 0ull;
     }
     // the counts first: the tile's successors wait for them, not for its ranks
 #pragma unroll
     for (int s = 0; s < kItems; ++s)
-        if (wbase + (uint32_t)s * 32 + lane < n) atomicAdd(&S.wh[warp][(uint32_t)(key[s] >> shift) & 255u], 1u);
+        if (p0 + (uint32_t)s * 32 < left) atomicAdd(&S.wh[warp][(uint32_t)(key[s] >> shift) & 255u], 1u);
     __syncthreads();
     uint32_t count = 0, all = 0;  // keys of digit threadIdx.x in the tile, and in all tiles
     uint32_t x = 0, y = 0;
@@ -128,36 +129,43 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
         }
     }
     __syncthreads();
-    // the leader of each set of equal digits claims its places, step after step, without waiting for
-    // the atomics' results in between
-    uint32_t first[kItems], rk[kItems];
+    // the leader of each set of equal digits claims its places, four steps at a time, without waiting for
+    // the atomics' results in between (all twelve at once spill: symmetrize 0.93 ms, 0.90 in fours)
+    static_assert(kItems % 4 == 0, "steps in groups of four");
+    uint32_t rk[kItems];
 #pragma unroll
-    for (int s = 0; s < kItems; ++s) {
-        const bool valid = wbase + (uint32_t)s * 32 + lane < n;
-        const uint32_t d = valid ? ((uint32_t)(key[s] >> shift) & 255u) : 256u;
-        // lanes with the same digit, bit by bit (match.any instead of the eight ballots made the warps
-        // wait on its result: short-scoreboard stalls 11 against 2 cycles an instruction)
-        uint32_t peers = __ballot_sync(kFullMask, valid);
-        peers = valid ? peers : 0u;
+    for (int s0 = 0; s0 < kItems; s0 += 4) {
+        uint32_t first[4];
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const uint32_t ones = __ballot_sync(kFullMask, d >> b & 1u);
-            peers &= (d >> b & 1u) ? ones : ~ones;
+        for (int q = 0; q < 4; ++q) {
+            const int s = s0 + q;
+            const bool valid = p0 + (uint32_t)s * 32 < left;
+            const uint32_t d = valid ? ((uint32_t)(key[s] >> shift) & 255u) : 256u;
+            // lanes with the same digit, bit by bit (match.any instead of the eight ballots made the
+            // warps wait on its result: short-scoreboard stalls 11 against 2 cycles an instruction)
+            uint32_t peers = __ballot_sync(kFullMask, valid);
+            peers = valid ? peers : 0u;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const uint32_t ones = __ballot_sync(kFullMask, d >> b & 1u);
+                peers &= (d >> b & 1u) ? ones : ~ones;
+            }
+            const uint32_t leader = __ffs(peers) - 1;
+            first[q] = 0;
+            if (valid && lane == leader) first[q] = atomicAdd(&S.wh[warp][d], __popc(peers));
+            __syncwarp();
+            rk[s] = leader << 8 | __popc(peers & lanemask_lt());
         }
-        const uint32_t leader = __ffs(peers) - 1;
-        first[s] = 0;
-        if (valid && lane == leader) first[s] = atomicAdd(&S.wh[warp][d], __popc(peers));
-        __syncwarp();
-        rk[s] = leader << 8 | __popc(peers & lanemask_lt());
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            rk[s0 + q] = __shfl_sync(kFullMask, first[q], rk[s0 + q] >> 8) + (rk[s0 + q] & 255u);
     }
 #pragma unroll
-    for (int s = 0; s < kItems; ++s) rk[s] = __shfl_sync(kFullMask, first[s], rk[s] >> 8) + (rk[s] & 255u);
-#pragma unroll
     for (int s = 0; s < kItems; ++s) {
-        const uint64_t idx = wbase + (uint32_t)s * 32 + lane;
-        if (idx < n) {
+        const uint32_t p = p0 + (uint32_t)s * 32;
+        if (p < left) {
             S.key[rk[s]] = key[s];
-            if (kVals) S.val[rk[s]] = vin ? vin[idx] : (uint32_t)idx;
+            if (kVals) S.val[rk[s]] = vin ? vin[tbase + p] : (uint32_t)tbase + p;
         }
     }
     // the owners look back, four predecessors at a time
@@ -195,8 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
     }
     __syncthreads();
     if (!S.ok) return;
-    const uint32_t valid = (uint32_t)min((uint64_t)(kThreads * kItems), n - tbase);
-    for (uint32_t i = threadIdx.x; i < valid; i += kThreads) {
+    for (uint32_t i = threadIdx.x; i < left; i += kThreads) {
         const uint64_t k = S.key[i];
         const uint64_t pos = S.goff[(uint32_t)(k >> shift) & 255u] + i;  // modulo 2^32
         if ((uint32_t)pos < n) {

@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_prune(Graph whole, const uint3
         if (lane_id() == 0) S.before[s * kFlagWarps + warp] = __popc(b);
     }
     __syncthreads();
-    flag_sums<true>(S, L, tile);
+    flag_sums(S, L, tile);
 #pragma unroll
     for (uint32_t s = 0; s < kFlagSteps; ++s) {
         const uint64_t j = j0 + s * kFlagThreads;
