@@ -56,6 +56,7 @@ enum : uint32_t {
     kPruneFront = 116,  // single-k: edges whose counted support is too small (the first round's frontier)
     kPruneLeft = 117,   //   the others, when these were counted again (recount_pruned)
     kPruneT0 = 118,     //   u64 (words 118..119): when that began
+    kListLocal = 118,   // decompositions: u64, list entries of edges in near-cliques (k_list_bounds)
     kPrunePlan = 120,   //   items, bases and cursor of its plan
     kCtrlWords = 128,
 };

@@ -663,13 +663,16 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
 }
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
-// total, three per triangle) and ends.
+// total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
+// of whose endpoint's neighbours are common ones: near-cliques (want_lists).
 template <bool kChained>
 __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restrict__ sup,
                                                               const uint32_t* __restrict__ supx,
                                                               uint32_t* __restrict__ ycount, uint32_t m,
                                                               uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
-                                                              Look L) {
+                                                              const uint32_t* __restrict__ rows,
+                                                              const uint32_t* __restrict__ e_src,
+                                                              const uint32_t* __restrict__ o_col, Look L) {
     if (kChained) after_previous(sup, supx, ycount, tptr, ends);
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
@@ -699,13 +702,15 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
     }
     static_assert(kScanItems == 4, "four supports a thread");
     uint64_t end;
-    uint64_t at = tile_scan<uint64_t>(L, tile, (uint64_t)v[0] + v[1] + v[2] + v[3], ws, &s_prefix, &end);
+    uint64_t at = tile_scan<uint64_t>(L, tile, (uint64_t)v[0] + v[1] + v[2] + v[3], ws, &s_prefix, &end), local = 0;
 #pragma unroll
     for (uint32_t i = 0; i < kScanItems; ++i) {
         if (j0 + i < m) {
             tptr[j0 + i] = at;
             at += v[i];
             ends[j0 + i] = at;
+            if (rows && 16 * (uint64_t)(v[i] + 1) >= 15 * (uint64_t)min(rows[e_src[j0 + i]], rows[o_col[j0 + i]]))
+                local += v[i];
             if (j0 + i == m - 1) {
                 tptr[m] = at;
                 L.ctrl[kCtrlTriLo] = (uint32_t)at;
@@ -713,21 +718,31 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
             }
         }
     }
+    if (!rows) return;
+    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(kFullMask, local, o);
+    if (lane_id() == 0 && local)
+        atomicAdd(reinterpret_cast<unsigned long long*>(L.ctrl + kListLocal), (unsigned long long)local);
 }
 
 }  // namespace
 
-// Most list entries per edge on average (three per triangle) with which the lists are made.  Denser
-// graphs spend more on writing the lists than the walks cost them, the more so as their last rounds
-// remove most edges at once, which a recount round of the walking peel gets for little.  Whole
-// decomposition, lists / walks: R-MAT 16 of edge factor 16 (52 entries an edge) 6.3 / 10.0 ms,
-// G(3000, 0.2) (120) 5.2 / 8.6 ms, R-MAT 14 of edge factor 64 (134) 8.7 / 13.0 ms; past the line
-// R-MAT 18 of edge factor 64 (261) 139 / 126 ms, R-MAT 16 of edge factor 128 (334) 72 / 66 ms,
-// R-MAT 18 of edge factor 128 (480) 450 / 322 ms.
-#ifndef KT_LIST_PER_EDGE
-#define KT_LIST_PER_EDGE 192
-#endif
-constexpr uint64_t kMaxListPerEdge = KT_LIST_PER_EDGE;
+// Most list entries per edge on average (three per triangle) with which the lists are made: writing them
+// costs more than the walks in denser graphs.  Whole decomposition, lists / walks: R-MAT 16 of edge
+// factor 16 (52 entries an edge) 5.3 / 9.8 ms, G(3000, 0.2) (120) 3.7 / 7.9, R-MAT 18 of edge factor 64
+// (261) 88 / 116, R-MAT 16 of edge factor 128 (334) 50 / 62, G(3000, 0.4) (479) 18.6 / 20.3, R-MAT 18 of
+// edge factor 128 (480) 255 / 291; past the line G(8000, 0.3) (719) 186 / 201, but G(3000, 0.5) (749)
+// 34 / 20 and G(3000, 0.9) (2,429) 203 / 38.
+constexpr uint64_t kMaxListPerEdge = 512;
+
+// Near-cliques go in a few rounds that remove most edges at once, which a recount round of the walking
+// peel gets for little.  A graph of kCliqueEdges edges (the lists of smaller ones cost at most half a
+// millisecond) with kCliqueEntries or more entries an edge walks if more than three
+// quarters of them belong to edges with 15/16 or more of their shorter row in triangles: disjoint
+// cliques of 100 vertices 2.1 / 0.65 ms, of 400 10.7 / 1.5 ms, G(200000, 16/n) with cliques of 300-500
+// vertices 4.8 / 3.8 ms; cliques of 20 (18 entries an edge) 0.53 / 0.44 ms, cliques of 50 with a
+// tenth of the edges rewired (35; not near-cliques) 1.6 / 2.6 ms.
+constexpr uint64_t kCliqueEntries = 32;
+constexpr uint32_t kCliqueEdges = 1u << 18;
 
 // Graphs of up to this many edges take lists whatever their density: m edges have at most
 // (sqrt(2) / 3) m^1.5 triangles, so a buffer of 8.4 M entries (67 MB) holds their lists and the call
@@ -753,12 +768,14 @@ bool grow_lists(kt_engine* e, uint64_t entries) {
     return true;
 }
 
+bool small_lists(const kt_engine* e) { return e->m <= kSmallLists && most_entries(e->m) <= e->list_cap; }
+
 // Whether the current graph takes lists; waits for its triangle count unless it is small, and sizes the
 // list buffer.
 int want_lists(kt_engine* e, bool* use) {
     *use = false;
     int rc;
-    if (e->m <= kSmallLists && most_entries(e->m) <= e->list_cap) {
+    if (small_lists(e)) {
         *use = true;
         return KT_OK;
     }
@@ -766,9 +783,11 @@ int want_lists(kt_engine* e, bool* use) {
     if (!e->trusted) {
         if ((rc = sync_and_check(e))) return rc;
         total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
+        const uint64_t local = (uint64_t)e->h_ctrl[kListLocal + 1] << 32 | e->h_ctrl[kListLocal];
+        if (e->m >= kCliqueEdges && total >= kCliqueEntries * e->m && local > total / 4 * 3) total = ~0ull;  // walks
         e->list_entries = total;
     }
-    if (total > kMaxListPerEdge * e->m) return KT_OK;
+    if (total / kMaxListPerEdge > e->m) return KT_OK;
     if (total > e->list_cap) {
         if (e->trusted) return KT_OK;
         const uint64_t want = total + total / 16;
@@ -797,6 +816,7 @@ int peel_lists(kt_engine* e, bool* done) {
     uint64_t* ends = e->key_b;
     if ((rc = launch_chained(e, "k_list_bounds", e->chained ? k_list_bounds<true> : k_list_bounds<false>,
                              ceil_div(m, kScanTile), kScanThreads, 0, e->sup, e->rnd, e->tr, m, tptr, ends,
+                             m < kCliqueEdges ? nullptr : e->s_len, e->e_src, e->o_col,
                              next_look(e))) || (rc = want_lists(e, done)) || !*done ||
         (rc = fill_lists(e, tptr, ends)))
         return rc;
