@@ -571,7 +571,9 @@ int build_graph(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint
     if (entries & 1) return fail(KT_ERR_NOT_SYMMETRIC, "odd number of entries (%llu): every edge needs both directions",
                                  (unsigned long long)entries);
     if (entries >= 0xffffffffull) return fail(KT_ERR_TOO_LARGE, "more than 2^32-2 entries");
-    if (n > e->cap_nodes || entries > e->cap_entries) {
+    // (an engine that has done nothing, or whose reservation failed, has no workspace: the session's kernels
+    // write to it for an empty graph too)
+    if (n > e->cap_nodes || entries > e->cap_entries || !e->look) {
         int rc = reserve(e, n > e->cap_nodes ? n : e->cap_nodes, entries > e->cap_entries ? entries : e->cap_entries);
         if (rc) return rc;
     }

@@ -252,7 +252,7 @@ int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words, 
     // Small graphs: their kernels are no longer than a launch takes (R-MAT of 2^20 vertices gains nothing, and
     // the pointers that a chained kernel launders cost its build 8 %).  Not on a caller's own stream.
     e->chained = e->lists_allowed && keys <= kSmallSort && n <= kSmallSort;
-    if (words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
+    if (!e->look || words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
     e->look_tag = e->look_count = 0;
     e->ctrl_fresh = false;
     const uint64_t work = std::max<uint64_t>(words / 2, std::max<uint32_t>(deg_words, kCountWords));
