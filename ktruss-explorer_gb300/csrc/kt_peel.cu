@@ -849,6 +849,12 @@ __device__ __forceinline__ uint32_t graph_of(const uint32_t* __restrict__ offset
     return lo - 1;
 }
 
+// Clears the graphs' k_max, unless the batch was refused: its error is in the control block, not yet read.
+__global__ void k_clear_kmax(uint32_t* __restrict__ kmax, uint32_t num_graphs, const uint32_t* __restrict__ ctrl) {
+    const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < num_graphs && !failed(ctrl)) kmax[g] = 0;
+}
+
 // Per-graph k_max of a batch: entry i belongs to the graph whose vertex range holds its source;
 // an entry whose endpoints lie in different graphs sets kErrCrossGraph.  Each warp walks its own
 // contiguous span of entries 32 at a time and keeps, per lane, the maximum of the graph it is in;
@@ -1041,7 +1047,9 @@ int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max) {
 
 int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, const uint32_t* d_offsets,
                     uint32_t num_graphs, const uint32_t* d_truss, uint32_t* d_kmax) {
-    int rc = check_cuda(cudaMemsetAsync(d_kmax, 0, sizeof(uint32_t) * num_graphs, e->stream), "clear k_max");
+    k_clear_kmax<<<grid_for(num_graphs), kThreads, 0, e->stream>>>(d_kmax, num_graphs, e->ctrl);
+    count_launch(e);
+    int rc = check_launch(e, "k_clear_kmax");
     if (rc || !e->entries) return rc;
     // a grid of eight blocks a SM; each warp takes a contiguous span of the entries
     const uint64_t blocks = std::min<uint64_t>(grid_for(e->entries), (uint64_t)e->num_sms * 8);
