@@ -266,6 +266,8 @@ int kt_engine_ktruss(kt_engine* engine, const uint32_t* d_src, const uint32_t* d
  * first replay captures the call's device pipeline (build, support count, peel, output) into a
  * CUDA graph without the input checks the call already made; later replays launch that graph.
  * A different call, a new schedule or selector, or a larger reservation drops the graph.
+ * (Contents that did change are not looked for; a graph whose triangle lists no longer fit the call's
+ * buffer is KT_ERR_INVALID_ARG.)
  * Statistics afterwards: everything but the per-phase times (0); last_ms is the replay's. */
 int kt_engine_replay(kt_engine* engine, int sync);
 /* How the next replay runs: 0 nothing to replay yet or not captured yet, 1 one launch of the

@@ -20,6 +20,7 @@ enum : uint32_t {
     kErrTimeout = 1u << 4,     // a bounded grid-barrier wait expired
     kErrRunaway = 1u << 5,     // the peel loop exceeded its round or level bound
     kErrCrossGraph = 1u << 6,  // a batch entry joins two different graphs
+    kErrListSpace = 1u << 7,   // a repeated call's triangle lists outgrew their buffer
 };
 
 // Layout of the device control block (uint32 words unless noted).

@@ -112,7 +112,7 @@ void remember(kt_engine* e, const kt_engine::LastCall& c) {
         l.truss != c.truss || l.k_max != c.k_max || l.k != c.k || l.keep != c.keep)
         drop_replay(e);
     e->last = c;
-    e->last.list_entries = e->list_entries;
+    e->last.list_need = e->list_need;
 }
 
 void forget(kt_engine* e) {

@@ -92,7 +92,7 @@ struct kt_engine {
     uint64_t ingest_words = 0;             //   (own allocation, made by the first ingest)
     uint2* lists = nullptr;        // triangle lists of a decomposition (own allocation, kt_lists.cu)
     uint64_t list_cap = 0;         //   entries it holds
-    uint64_t list_entries = 0;     //   entries of the last call (three per triangle)
+    uint64_t list_need = 0;        //   entries that the current call's lists need (0: it walks rows)
     bool lists_allowed = false;    //   kt_engine_create sets it; the allocation-free path never does
 
     // Current graph.
@@ -129,7 +129,7 @@ struct kt_engine {
         uint32_t* k_max = nullptr;
         uint32_t k = 0;
         uint8_t* keep = nullptr;
-        uint64_t list_entries = 0;           // triangle list entries the call counted
+        uint64_t list_need = 0;              // list buffer that the call needed (0: it walked rows)
     } last;
     cudaGraphExec_t replay = nullptr;
     bool replay_direct = false;      // the pipeline could not be captured: replays launch it directly

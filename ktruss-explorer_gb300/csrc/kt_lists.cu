@@ -40,9 +40,9 @@
 // 4.2 -> 3.5.
 
 #include <algorithm>
-#include <cmath>
 
 #include "kt_engine.h"
+#include "kt_list_rule.h"
 #include "kt_look.cuh"
 
 namespace kt {
@@ -664,7 +664,8 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
-// of whose endpoint's neighbours are common ones: near-cliques (want_lists).
+// of whose endpoint's neighbours are common ones: near-cliques (want_lists).  More than `cap` entries, what
+// the buffer of a call holds that does not wait for the total, are an error: nothing is written to it.
 template <bool kChained>
 __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restrict__ sup,
                                                               const uint32_t* __restrict__ supx,
@@ -672,7 +673,8 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
                                                               uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
                                                               const uint32_t* __restrict__ rows,
                                                               const uint32_t* __restrict__ e_src,
-                                                              const uint32_t* __restrict__ o_col, Look L) {
+                                                              const uint32_t* __restrict__ o_col, uint64_t cap,
+                                                              Look L) {
     if (kChained) after_previous(sup, supx, ycount, tptr, ends);
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
@@ -715,6 +717,7 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
                 tptr[m] = at;
                 L.ctrl[kCtrlTriLo] = (uint32_t)at;
                 L.ctrl[kCtrlTriHi] = (uint32_t)(at >> 32);
+                if (at > cap) atomicOr(&L.ctrl[kCtrlError], kErrListSpace);
             }
         }
     }
@@ -744,15 +747,7 @@ constexpr uint64_t kMaxListPerEdge = 512;
 constexpr uint64_t kCliqueEntries = 32;
 constexpr uint32_t kCliqueEdges = 1u << 18;
 
-// Graphs of up to this many edges take lists whatever their density: m edges have at most
-// (sqrt(2) / 3) m^1.5 triangles, so a buffer of 8.4 M entries (67 MB) holds their lists and the call
-// need not wait for the triangle count.
-constexpr uint32_t kSmallLists = 1u << 15;
-
 namespace {
-
-// At least three times the triangles that m edges can form.
-uint64_t most_entries(uint64_t m) { return (uint64_t)(1.41422 * (double)m * std::sqrt((double)m)) + 64; }
 
 bool grow_lists(kt_engine* e, uint64_t entries) {
     if (e->lists) cudaFree(e->lists);
@@ -768,35 +763,25 @@ bool grow_lists(kt_engine* e, uint64_t entries) {
     return true;
 }
 
-bool small_lists(const kt_engine* e) { return e->m <= kSmallLists && most_entries(e->m) <= e->list_cap; }
-
-// Whether the current graph takes lists; waits for its triangle count unless it is small, and sizes the
-// list buffer.
+// Whether the current graph takes lists: reads its triangle count and sizes the list buffer.
 int want_lists(kt_engine* e, bool* use) {
     *use = false;
     int rc;
-    if (small_lists(e)) {
-        *use = true;
-        return KT_OK;
-    }
-    uint64_t total = e->last.list_entries;  // a trusted run repeats a call that counted them
-    if (!e->trusted) {
-        if ((rc = sync_and_check(e))) return rc;
-        total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
-        const uint64_t local = (uint64_t)e->h_ctrl[kListLocal + 1] << 32 | e->h_ctrl[kListLocal];
-        if (e->m >= kCliqueEdges && total >= kCliqueEntries * e->m && local > total / 4 * 3) total = ~0ull;  // walks
-        e->list_entries = total;
-    }
+    if ((rc = sync_and_check(e))) return rc;
+    const uint64_t total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
+    const uint64_t local = (uint64_t)e->h_ctrl[kListLocal + 1] << 32 | e->h_ctrl[kListLocal];
+    if (e->m >= kCliqueEdges && total >= kCliqueEntries * e->m && local > total / 4 * 3) return KT_OK;
     if (total / kMaxListPerEdge > e->m) return KT_OK;
-    if (total > e->list_cap) {
-        if (e->trusted) return KT_OK;
-        const uint64_t want = total + total / 16;
+    const uint64_t need = std::max<uint64_t>(total, 1);
+    if (need > e->list_cap) {
+        const uint64_t want = total + total / 16 + 1;
         drop_replay(e);
         size_t free_bytes = 0, all_bytes = 0;
         if ((rc = check_cuda(cudaMemGetInfo(&free_bytes, &all_bytes), "free device memory"))) return rc;
         if (want * sizeof(uint2) > (free_bytes + e->list_cap * sizeof(uint2)) / 2) return KT_OK;  // walk rows instead
         if (!grow_lists(e, want)) return KT_OK;
     }
+    e->list_need = need;
     *use = true;
     return KT_OK;
 }
@@ -814,11 +799,16 @@ int peel_lists(kt_engine* e, bool* done) {
     // the sort's key buffers are free after the build: list starts, and ends for the fill
     uint64_t* tptr = e->key_a;
     uint64_t* ends = e->key_b;
+    // a repeated call does what the call did; a small graph's lists fit whatever it is: neither waits
+    const bool small = !e->trusted && small_lists(m, e->list_cap);
+    if (e->trusted) e->list_need = repeat_lists(e->last.list_need, e->list_cap) ? e->last.list_need : 0;
+    else e->list_need = small ? most_entries(m) : 0;
+    *done = e->list_need != 0;
     if ((rc = launch_chained(e, "k_list_bounds", e->chained ? k_list_bounds<true> : k_list_bounds<false>,
                              ceil_div(m, kScanTile), kScanThreads, 0, e->sup, e->rnd, e->tr, m, tptr, ends,
                              m < kCliqueEdges ? nullptr : e->s_len, e->e_src, e->o_col,
-                             next_look(e))) || (rc = want_lists(e, done)) || !*done ||
-        (rc = fill_lists(e, tptr, ends)))
+                             *done ? e->list_cap : ~0ull, next_look(e))) ||
+        (!e->trusted && !small && (rc = want_lists(e, done))) || !*done || (rc = fill_lists(e, tptr, ends)))
         return rc;
     ListParams P;
     P.tri = e->lists;

@@ -1095,6 +1095,7 @@ int finish_stats(kt_engine* e) {
     const uint32_t err = e->h_ctrl[kCtrlError];
     if (err & kErrTimeout) return fail(KT_ERR_TIMEOUT, "a grid barrier wait of the peel kernel expired");
     if (err & kErrRunaway) return fail(KT_ERR_INTERNAL, "the peel kernel exceeded its round or level bound");
+    if (err & kErrListSpace) return fail(KT_ERR_INVALID_ARG, "the repeated call's input has changed since the call");
     if (err & kErrCrossGraph) return fail(KT_ERR_INVALID_ARG, "a batch entry joins vertices of two different graphs");
     const uint64_t m = e->m;
     e->stats.triangles = ((uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo]) / 3;

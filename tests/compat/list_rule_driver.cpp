@@ -1,0 +1,19 @@
+// Prints what kt_list_rule.h decides: lines "most m", "small m cap", "repeat need cap".
+#include <cstdio>
+#include <cstring>
+
+#include "kt_list_rule.h"
+
+int main() {
+    char op[16];
+    unsigned long long a, b = 0;
+    while (scanf("%15s %llu", op, &a) == 2) {
+        if (!strcmp(op, "most")) {
+            printf("%llu\n", (unsigned long long)kt::most_entries(a));
+            continue;
+        }
+        if (scanf("%llu", &b) != 1) return 1;
+        printf("%d\n", !strcmp(op, "small") ? kt::small_lists(a, b) : kt::repeat_lists(a, b));
+    }
+    return 0;
+}
