@@ -223,9 +223,23 @@ int kt_engine_destroy(kt_engine* engine);
 /* Returns the engine's cudaStream_t (as void*). */
 void* kt_engine_stream(kt_engine* engine);
 /* Pre-allocates the device workspace for graphs up to these sizes, so that later calls of at
- * most this size do not allocate - but for the triangle lists of graphs of more than 32,768 edges,
- * whose size their triangles decide: the first decomposition that needs more of them allocates. */
+ * most this size do not allocate - but for the triangle lists (kt_engine_set_list_limit). */
 int kt_engine_reserve(kt_engine* engine, uint32_t max_nodes, uint64_t max_entries);
+/* Device memory of the triangle lists, which decompositions peel from where they fit (single-k calls
+ * and kt_decompose_noalloc use none).  They take 24 bytes a triangle (an R-MAT graph of 15 M edges 9 GB,
+ * one of 60 M edges 43 GB), and a sixteenth more is allocated.  A reservation takes the 67 MB (less for a
+ * smaller one) that hold the lists of any graph of up to 32,768 edges; larger graphs' lists are allocated
+ * by the first decomposition that needs more, if that is at most half of the device memory then free.  The
+ * engine keeps its largest buffer for later calls and gives it back when it needs the memory for another
+ * of its arrays, when the limit is set below the buffer's size, and when it is destroyed.  A decomposition
+ * whose lists do not fit walks adjacency rows, without an error and with the same result, at 1.4 to 2.7
+ * times the time of a graph that would take lists (R-MAT 22 278 against 175 ms, R-MAT 20 67 against 38, a
+ * Watts-Strogatz graph of 10 M edges 17.1 against 6.3).
+ * bytes: the most that the buffer may take, at once and later (default: UINT64_MAX).  0: no lists; calls
+ * within the reservation allocate nothing. */
+int kt_engine_set_list_limit(kt_engine* engine, uint64_t bytes);
+/* The limit, and the bytes that the engine holds now (either pointer may be NULL). */
+int kt_engine_get_list_limit(kt_engine* engine, uint64_t* bytes, uint64_t* held);
 /* Device-resident decomposition.  d_src/d_dst: num_entries entries on the engine's device
  * (symmetric simple graph, both directions).  d_truss_per_entry: num_entries outputs.
  * d_k_max: one uint32 on the device.  Work is enqueued on the engine stream; the call
@@ -320,6 +334,9 @@ int kt_last_stats(kt_stats* stats);
  * kt_decompose_batch). */
 int kt_set_schedule(const kt_schedule* schedule);
 int kt_get_schedule(kt_schedule* schedule);
+/* List limit of that engine, which lives as long as the process (kt_engine_set_list_limit). */
+int kt_set_list_limit(uint64_t bytes);
+int kt_get_list_limit(uint64_t* bytes, uint64_t* held);
 /* The autotuner's built-in grid of schedules: support_group {4, 8, 16} x chunk_width
  * {8, 16, 32} x compact_percent {0, 85} x recount_percent {0, 50}, peel_blocks 0 (36).  Writes
  * min(36, cap) schedules to `out` (may be NULL) and returns 36. */

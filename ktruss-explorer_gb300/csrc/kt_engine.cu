@@ -135,7 +135,7 @@ int reserve(kt_engine* e, uint32_t max_nodes, uint64_t max_entries) {
     }
     const size_t bytes = carve(e, nullptr, max_nodes, max_entries, true);
     void* p = nullptr;
-    if ((rc = check_cuda(cudaMalloc(&p, bytes), "allocate engine workspace"))) {
+    if ((rc = check_cuda(alloc_device(e, &p, bytes), "allocate engine workspace"))) {
         e->cap_nodes = 0;
         e->cap_entries = 0;
         return rc;
@@ -447,6 +447,28 @@ int kt_engine_reserve(kt_engine* e, uint32_t max_nodes, uint64_t max_entries) {
     return kt::reserve(e, max_nodes, max_entries);
 }
 
+int kt_engine_set_list_limit(kt_engine* e, uint64_t bytes) {
+    kt::clear_error();
+    if (!e) return fail(KT_ERR_INVALID_ARG, "kt_engine_set_list_limit: null engine");
+    int rc = check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
+    if (rc) return rc;
+    e->list_limit = bytes;
+    if (e->list_cap * sizeof(uint2) > bytes) {
+        if ((rc = check_cuda(cudaStreamSynchronize(e->stream), "synchronize"))) return rc;
+        kt::free_lists(e);
+    }
+    if (e->arena) kt::reserve_small_lists(e, e->cap_entries / 2);
+    return KT_OK;
+}
+
+int kt_engine_get_list_limit(kt_engine* e, uint64_t* bytes, uint64_t* held) {
+    kt::clear_error();
+    if (!e) return fail(KT_ERR_INVALID_ARG, "kt_engine_get_list_limit: null engine");
+    if (bytes) *bytes = e->list_limit;
+    if (held) *held = e->list_cap * sizeof(uint2);
+    return KT_OK;
+}
+
 int kt_engine_decompose(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_t num_entries,
                         uint32_t num_nodes, uint32_t* d_truss, uint32_t* d_k_max, int sync) {
     if (!e) return fail(KT_ERR_INVALID_ARG, "kt_engine_decompose: null engine");
@@ -586,6 +608,22 @@ int kt_set_schedule(const kt_schedule* s) {
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(g_default_mu);
     return kt_engine_set_schedule(e, s);
+}
+
+int kt_set_list_limit(uint64_t bytes) {
+    kt_engine* e = nullptr;
+    int rc = default_engine(&e);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lock(g_default_mu);
+    return kt_engine_set_list_limit(e, bytes);
+}
+
+int kt_get_list_limit(uint64_t* bytes, uint64_t* held) {
+    kt_engine* e = nullptr;
+    int rc = default_engine(&e);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lock(g_default_mu);
+    return kt_engine_get_list_limit(e, bytes, held);
 }
 
 int kt_get_schedule(kt_schedule* s) {
@@ -826,7 +864,8 @@ int kt_decompose_batch(const uint32_t* src, const uint32_t* dst, uint64_t num_en
         if (e->aux) cudaFree(e->aux);
         e->aux = nullptr;
         e->aux_words = 0;
-        if ((rc = check_cuda(cudaMalloc(&e->aux, sizeof(uint32_t) * need), "allocate batch staging"))) return rc;
+        if ((rc = check_cuda(kt::alloc_device(e, (void**)&e->aux, sizeof(uint32_t) * need), "allocate batch staging")))
+            return rc;
         e->aux_words = need;
     }
     uint32_t* d_off = e->aux;

@@ -92,6 +92,7 @@ struct kt_engine {
     uint64_t ingest_words = 0;             //   (own allocation, made by the first ingest)
     uint2* lists = nullptr;        // triangle lists of a decomposition (own allocation, kt_lists.cu)
     uint64_t list_cap = 0;         //   entries it holds
+    uint64_t list_limit = ~0ull;   //   bytes it may take (kt_engine_set_list_limit)
     uint64_t list_need = 0;        //   entries that the current call's lists need (0: it walks rows)
     bool lists_allowed = false;    //   kt_engine_create sets it; the allocation-free path never does
 
@@ -241,6 +242,9 @@ int peel_single_k(kt_engine* e, uint32_t k);
 int peel_lists(kt_engine* e, bool* done);
 // A list buffer for graphs of up to max_edges whose lists are made without reading the triangle count.
 void reserve_small_lists(kt_engine* e, uint64_t max_edges);
+void free_lists(kt_engine* e);
+// cudaMalloc for the engine's other arrays: gives the list buffer back if there is no memory left.
+cudaError_t alloc_device(kt_engine* e, void** p, size_t bytes);
 int emit_truss_per_entry(kt_engine* e, uint32_t* d_out, uint32_t* d_k_max);
 int emit_keep(kt_engine* e, uint8_t* d_keep);
 int emit_graph_kmax(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, const uint32_t* d_offsets,

@@ -343,7 +343,8 @@ int parse_tsv(kt_engine* e, const char* d_text, uint64_t bytes, uint32_t* d_src,
         if (e->ingest) cudaFree(e->ingest);
         e->ingest = nullptr;
         e->ingest_words = 0;
-        if ((rc = check_cuda(cudaMalloc(&e->ingest, sizeof(unsigned long long) * words), "allocate ingest scratch")))
+        if ((rc = check_cuda(alloc_device(e, (void**)&e->ingest, sizeof(unsigned long long) * words),
+                             "allocate ingest scratch")))
             return rc;
         e->ingest_words = words;
     }
@@ -431,7 +432,7 @@ int kt_engine_read_tsv(kt_engine* e, const char* path, uint32_t* d_src, uint32_t
     char* d = nullptr;
     if (!rc && sz > 0) {
         if (!(rc = check_cuda(cudaMallocHost(&h, (size_t)sz), "allocate pinned staging")) &&
-            !(rc = check_cuda(cudaMalloc(&d, (size_t)sz), "allocate device text"))) {
+            !(rc = check_cuda(kt::alloc_device(e, (void**)&d, (size_t)sz), "allocate device text"))) {
             if (fread(h, 1, (size_t)sz, fp) != (size_t)sz) rc = fail(KT_ERR_IO, "short read on %s", path);
             if (!rc) rc = check_cuda(cudaMemcpyAsync(d, h, (size_t)sz, cudaMemcpyHostToDevice, e->stream), "H2D");
         }

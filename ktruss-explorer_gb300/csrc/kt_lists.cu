@@ -750,9 +750,7 @@ constexpr uint32_t kCliqueEdges = 1u << 18;
 namespace {
 
 bool grow_lists(kt_engine* e, uint64_t entries) {
-    if (e->lists) cudaFree(e->lists);
-    e->lists = nullptr;
-    e->list_cap = 0;
+    free_lists(e);
     void* p = nullptr;
     if (cudaMalloc(&p, entries * sizeof(uint2)) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -774,11 +772,11 @@ int want_lists(kt_engine* e, bool* use) {
     if (total / kMaxListPerEdge > e->m) return KT_OK;
     const uint64_t need = std::max<uint64_t>(total, 1);
     if (need > e->list_cap) {
-        const uint64_t want = total + total / 16 + 1;
-        drop_replay(e);
+        const uint64_t want = buffer_entries(total, e->list_limit);
+        if (want == 0) return KT_OK;  // walk rows instead
         size_t free_bytes = 0, all_bytes = 0;
         if ((rc = check_cuda(cudaMemGetInfo(&free_bytes, &all_bytes), "free device memory"))) return rc;
-        if (want * sizeof(uint2) > (free_bytes + e->list_cap * sizeof(uint2)) / 2) return KT_OK;  // walk rows instead
+        if (want * sizeof(uint2) > (free_bytes + e->list_cap * sizeof(uint2)) / 2) return KT_OK;
         if (!grow_lists(e, want)) return KT_OK;
     }
     e->list_need = need;
@@ -788,9 +786,25 @@ int want_lists(kt_engine* e, bool* use) {
 
 }  // namespace
 
+void free_lists(kt_engine* e) {
+    if (!e->lists) return;
+    drop_replay(e);  // a captured pipeline may point to them
+    cudaFree(e->lists);  // (waits for the device)
+    e->lists = nullptr;
+    e->list_cap = 0;
+}
+
 void reserve_small_lists(kt_engine* e, uint64_t max_edges) {
     const uint64_t want = most_entries(std::min<uint64_t>(max_edges, kSmallLists));
-    if (e->lists_allowed && want > e->list_cap) grow_lists(e, want);
+    if (e->lists_allowed && want > e->list_cap && want <= e->list_limit / sizeof(uint2)) grow_lists(e, want);
+}
+
+cudaError_t alloc_device(kt_engine* e, void** p, size_t bytes) {
+    cudaError_t err = cudaMalloc(p, bytes);
+    if (err != cudaErrorMemoryAllocation || !e->lists) return err;
+    (void)cudaGetLastError();
+    free_lists(e);
+    return cudaMalloc(p, bytes);
 }
 
 int peel_lists(kt_engine* e, bool* done) {

@@ -183,7 +183,8 @@ int ktruss_tiled(kt_engine* e, uint32_t k, bool recount_all, bool capped) {
         if (e->tile_off) cudaFree(e->tile_off);
         e->tile_off = nullptr;
         e->tile_off_words = 0;
-        if ((rc = check_cuda(cudaMalloc(&e->tile_off, sizeof(uint32_t) * (words ? words : 1)), "allocate tile table")))
+        if ((rc = check_cuda(alloc_device(e, (void**)&e->tile_off, sizeof(uint32_t) * (words ? words : 1)),
+                             "allocate tile table")))
             return rc;
         e->tile_off_words = words;
     }

@@ -137,6 +137,9 @@ def lib() -> ctypes.CDLL:
         L.kt_engine_stream.argtypes = [_VP]
         L.kt_engine_stream.restype = _VP
         L.kt_engine_reserve.argtypes = [_VP, ctypes.c_uint32, ctypes.c_uint64]
+        for p, f in (([_VP], "kt_engine_%s_list_limit"), ([], "kt_%s_list_limit")):
+            getattr(L, f % "set").argtypes = p + [ctypes.c_uint64]
+            getattr(L, f % "get").argtypes = p + [ctypes.POINTER(ctypes.c_uint64)] * 2
         L.kt_engine_decompose.argtypes = [_VP, _VP, _VP, ctypes.c_uint64, ctypes.c_uint32, _VP, _VP, ctypes.c_int]
         L.kt_engine_ktruss.argtypes = [_VP, _VP, _VP, ctypes.c_uint64, ctypes.c_uint32, ctypes.c_uint32, _VP,
                                        ctypes.c_int]
@@ -364,6 +367,15 @@ def verify(truss: COOGraph, config: Config) -> None:
     _check(lib().kt_verify(ctypes.byref(t), ctypes.byref(cfg)))
 
 
+_NO_LIMIT = (1 << 64) - 1
+
+
+def _list_limit(get) -> tuple:
+    limit, held = ctypes.c_uint64(0), ctypes.c_uint64(0)
+    _check(get(ctypes.byref(limit), ctypes.byref(held)))
+    return (None if limit.value == _NO_LIMIT else limit.value), held.value
+
+
 class Engine:
     """Device-resident engine: graph and outputs stay in HBM (pointers are device addresses)."""
 
@@ -389,6 +401,15 @@ class Engine:
 
     def reserve(self, max_nodes: int, max_entries: int) -> None:
         _check(lib().kt_engine_reserve(self._h, max_nodes, max_entries))
+
+    def set_list_limit(self, max_bytes: Optional[int] = None) -> None:
+        """Most device memory that the triangle lists of decompositions may take (None: no limit but half
+        of the free memory; 0: no lists).  A buffer above it is given back at once."""
+        _check(lib().kt_engine_set_list_limit(self._h, _NO_LIMIT if max_bytes is None else max_bytes))
+
+    def list_limit(self) -> tuple:
+        """(limit or None, bytes held now) of the triangle lists."""
+        return _list_limit(lambda *a: lib().kt_engine_get_list_limit(self._h, *a))
 
     def decompose(self, d_src: int, d_dst: int, num_entries: int, num_nodes: int, d_truss: int,
                   d_k_max: int = 0, sync: bool = True) -> None:
@@ -612,6 +633,16 @@ def get_schedule() -> Schedule:
     s = Schedule()
     _check(lib().kt_get_schedule(ctypes.byref(s)))
     return s
+
+
+def set_list_limit(max_bytes: Optional[int] = None) -> None:
+    """Engine.set_list_limit for the engine behind the host-buffer calls."""
+    _check(lib().kt_set_list_limit(_NO_LIMIT if max_bytes is None else max_bytes))
+
+
+def list_limit() -> tuple:
+    """Engine.list_limit of the engine behind the host-buffer calls."""
+    return _list_limit(lib().kt_get_list_limit)
 
 
 def schedule_grid() -> list:

@@ -1,4 +1,5 @@
-// Prints what kt_list_rule.h decides: lines "most m", "small m cap", "repeat need cap".
+// Prints what kt_list_rule.h decides: lines "most m", "small m cap", "repeat need cap",
+// "buffer total limit".
 #include <cstdio>
 #include <cstring>
 
@@ -13,6 +14,10 @@ int main() {
             continue;
         }
         if (scanf("%llu", &b) != 1) return 1;
+        if (!strcmp(op, "buffer")) {
+            printf("%llu\n", (unsigned long long)kt::buffer_entries(a, b));
+            continue;
+        }
         printf("%d\n", !strcmp(op, "small") ? kt::small_lists(a, b) : kt::repeat_lists(a, b));
     }
     return 0;

@@ -49,3 +49,10 @@ def test_a_repeated_call_without_its_buffer_walks(ask):
     # the buffer it had, a larger one, a smaller one, none; a call that walked
     assert ask(("repeat", 100, 100), ("repeat", 100, 101), ("repeat", 100, 99), ("repeat", 1, 0), ("repeat", 0, 0),
                ("repeat", 0, 100)) == [1, 1, 0, 0, 0, 0]
+
+
+def test_buffers_keep_to_the_limit(ask):
+    none = (1 << 64) - 1
+    cases = [(0, none, 1), (0, 8, 1), (0, 7, 0), (0, 0, 0), (15, none, 15), (16, none, 17), (16, 17 * 8, 17),
+             (16, 17 * 8 - 1, 16), (16, 16 * 8, 16), (16, 16 * 8 - 1, 0), (5 << 30, none, (5 << 30) + (5 << 26))]
+    assert ask(*[("buffer", t, limit) for t, limit, _ in cases]) == [want for *_, want in cases]
