@@ -347,7 +347,11 @@ uint32_t kt_schedule_grid(kt_schedule* out, uint32_t cap);
  * events; the CSR build does not depend on the schedule).  candidates: num_candidates schedules,
  * or NULL for the built-in grid.  ms (optional): the least time of each candidate.  On return the
  * engine runs with the fastest schedule, also written to *best (optional).  Callers tune on a
- * sample of the graphs they will run and reuse the schedule for the rest. */
+ * sample of the graphs they will run and reuse the schedule for the rest.  One run before the
+ * candidates' is not timed.  A graph that is decomposed from triangle lists has one time for all
+ * candidates of a support group, as the other fields do not act on it; of these candidates the one
+ * with the engine's own chunk width, compaction, recount and peel blocks is kept (else the first),
+ * for the calls on which they do act.  kt_engine_set_list_limit(engine, 0) tunes the row walks. */
 int kt_engine_autotune(kt_engine* engine, const uint32_t* d_src, const uint32_t* d_dst, uint64_t num_entries,
                        uint32_t num_nodes, const kt_schedule* candidates, uint32_t num_candidates,
                        uint32_t repeats, float* ms, kt_schedule* best);
@@ -399,7 +403,9 @@ int kt_engine_read_tsv(kt_engine* engine, const char* path, uint32_t* d_src, uin
  * the autotuner's grid: the variant (support_group x chunk_width x compact_percent, 18 classes)
  * and the recount switch (recount_percent 50 or 0).  It is trained on timings of the grid's 36
  * schedules (kt_engine_autotune with ms output) measured on graphs like the ones it will see.
- * Every schedule gives the same truss numbers: a wrong prediction only costs time. */
+ * Every schedule gives the same truss numbers: a wrong prediction only costs time.  Of a
+ * decomposition from triangle lists it decides the support group alone; train it on timings of the
+ * row walks (kt_engine_set_list_limit(engine, 0)), where all of a schedule acts. */
 #define KT_SELECTOR_FEATURES 16
 #define KT_SELECTOR_VARIANTS 18
 #define KT_SELECTOR_SCHEDULES 36

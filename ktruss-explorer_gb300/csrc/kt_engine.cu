@@ -663,30 +663,47 @@ int autotune(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uint64_
     const kt_schedule saved = e->sched;
     int rc = check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
     if (rc) return rc;
+    // support count and peel of one run (the rows are compacted in place while peeling, so every run
+    // builds the CSR again)
+    const auto run = [&](float* t) {
+        int rc;
+        if ((rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes, true)) || (rc = record(e, e->ev_built)) ||
+            (rc = kt::count_support(e)) || (rc = kt::peel_decompose(e)) || (rc = record(e, e->ev_stop)) ||
+            (rc = check_cuda(cudaEventSynchronize(e->ev_stop), "synchronize")) ||
+            (rc = check_cuda(cudaEventElapsedTime(t, e->ev_built, e->ev_stop), "elapsed time")))
+            return rc;
+        return kt::finish_stats(e);
+    };
+    // what but the support group a schedule says has no effect on a decomposition from lists
+    const auto same_walks = [](const kt_schedule& a, const kt_schedule& b) {
+        return a.chunk_width == b.chunk_width && a.compact_percent == b.compact_percent &&
+               a.recount_percent == b.recount_percent && a.peel_blocks == b.peel_blocks;
+    };
     uint32_t best_i = 0;
-    float best_ms = 0;
+    std::vector<float> times(num_candidates);
     e->batch_call = batch;  // the peel's launch shape follows the call being tuned
-    for (uint32_t i = 0; i < num_candidates; ++i) {
+    float first = 0;
+    rc = run(&first);  // not counted: it makes the list buffer, and shows whether the graph takes lists
+    const bool lists = e->m != 0 && e->list_need != 0;
+    for (uint32_t i = 0; i < num_candidates && !rc; ++i) {
         if ((rc = kt_engine_set_schedule(e, &candidates[i]))) break;
-        float t_min = 0;
-        for (uint32_t r = 0; r < repeats && !rc; ++r) {
-            // the rows are compacted in place while peeling, so every run builds the CSR again
-            if ((rc = kt::build_graph(e, d_src, d_dst, num_entries, num_nodes, true)) || (rc = record(e, e->ev_built)) ||
-                (rc = kt::count_support(e)) || (rc = kt::peel_decompose(e)) || (rc = record(e, e->ev_stop)) ||
-                (rc = check_cuda(cudaEventSynchronize(e->ev_stop), "synchronize")))
-                break;
-            float t = 0;
-            if ((rc = check_cuda(cudaEventElapsedTime(&t, e->ev_built, e->ev_stop), "elapsed time")) ||
-                (rc = kt::finish_stats(e)))
-                break;
-            t_min = r == 0 || t < t_min ? t : t_min;
+        uint32_t same = 0;  // an earlier candidate that ran the same kernels
+        while (same < i && !(lists && candidates[same].support_group == candidates[i].support_group)) ++same;
+        if (same < i) {
+            times[i] = times[same];
+        } else {
+            for (uint32_t r = 0; r < repeats && !rc; ++r) {
+                float t = 0;
+                if (!(rc = run(&t))) times[i] = r == 0 || t < times[i] ? t : times[i];
+            }
         }
         if (rc) break;
-        if (ms) ms[i] = t_min;
-        if (i == 0 || t_min < best_ms) {
-            best_ms = t_min;
+        if (ms) ms[i] = times[i];
+        const kt_schedule& b = candidates[best_i];
+        if (i == 0 || times[i] < times[best_i] ||
+            (lists && candidates[i].support_group == b.support_group && same_walks(candidates[i], saved) &&
+             !same_walks(b, saved)))
             best_i = i;
-        }
     }
     e->batch_call = false;
     if (rc) {

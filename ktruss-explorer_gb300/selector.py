@@ -9,7 +9,7 @@
 `collect` generates seeded graphs - Erdos-Renyi, R-MAT scale 12-18, Barabasi-Albert, random
 geometric (unit square, radius for an average degree of 8-64) and graphs with planted cliques -
 and for each records the selector's 16 features (computed by the library on the device) and the
-device time of all 36 schedules of the autotuner's grid (kt_engine_autotune).  `evaluate` trains
+device time of all 36 schedules of the autotuner's grid (kt_engine_autotune), walking rows.  `evaluate` trains
 the network with the library's CUDA kernels on the training set and reports, on the held-out
 set, the time of its choices against the exhaustively tuned best and the default schedule.
 The data in data/ were measured on a GB300.
@@ -96,6 +96,7 @@ def collect(count: int, seed: int, device: int = 0, repeats: int = 1, log=None, 
 
     torch.cuda.set_device(device)
     eng = kt.Engine(device)
+    eng.set_list_limit(0)  # time the row walks: peeling from triangle lists, only the support group acts
     grid = kt.schedule_grid()
     feats = np.zeros((count, kt.SELECTOR_FEATURES), np.float32)
     times = np.zeros((count, kt.SELECTOR_SCHEDULES), np.float32)
