@@ -53,6 +53,7 @@ enum : uint32_t {
     kPAliveSum = 82,   // u64 (words 82..83): the alive edges they see
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
+    kListLeast = 84,   // decompositions: complement of the least support (k_list_bounds)
     // words 88-115: the list peel (kt_lists.cu)
     kPruneFront = 116,  // single-k: edges whose counted support is too small (the first round's frontier)
     kPruneLeft = 117,   //   the others, when these were counted again (recount_pruned)

@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
-// of whose endpoint's neighbours are common ones: near-cliques (want_lists).  More than `cap` entries, what
+// of whose endpoint's neighbours are common ones, near-cliques, and the least support (walks_rows).  More than `cap` entries, what
 // the buffer of a call holds that does not wait for the total, are an error: nothing is written to it.
 template <bool kChained>
 __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restrict__ sup,
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
                                                               const uint32_t* __restrict__ e_src,
                                                               const uint32_t* __restrict__ o_col, uint64_t cap,
                                                               Look L) {
-    if (kChained) after_previous(sup, supx, ycount, tptr, ends);
+    if (kChained) after_previous(sup, supx, ycount, tptr, ends, rows, e_src, o_col);
     __shared__ uint64_t ws[33], s_prefix;
     __shared__ uint32_t s_tile;
     if (__syncthreads_or(failed(L.ctrl))) return;
@@ -722,30 +722,20 @@ __global__ void __launch_bounds__(kScanThreads) k_list_bounds(uint32_t* __restri
         }
     }
     if (!rows) return;
+    if (m < kCliqueEdges) {
+        uint32_t least = ~0u;
+#pragma unroll
+        for (uint32_t i = 0; i < kScanItems; ++i)
+            if (j0 + i < m) least = min(least, v[i]);
+        least = __reduce_min_sync(kFullMask, least);
+        if (lane_id() == 0) atomicMax(L.ctrl + kListLeast, ~least);
+    }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(kFullMask, local, o);
     if (lane_id() == 0 && local)
         atomicAdd(reinterpret_cast<unsigned long long*>(L.ctrl + kListLocal), (unsigned long long)local);
 }
 
 }  // namespace
-
-// Most list entries per edge on average (three per triangle) with which the lists are made: writing them
-// costs more than the walks in denser graphs.  Whole decomposition, lists / walks: R-MAT 16 of edge
-// factor 16 (52 entries an edge) 5.3 / 9.8 ms, G(3000, 0.2) (120) 3.7 / 7.9, R-MAT 18 of edge factor 64
-// (261) 88 / 116, R-MAT 16 of edge factor 128 (334) 50 / 62, G(3000, 0.4) (479) 18.6 / 20.3, R-MAT 18 of
-// edge factor 128 (480) 255 / 291; past the line G(8000, 0.3) (719) 186 / 201, but G(3000, 0.5) (749)
-// 34 / 20 and G(3000, 0.9) (2,429) 203 / 38.
-constexpr uint64_t kMaxListPerEdge = 512;
-
-// Near-cliques go in a few rounds that remove most edges at once, which a recount round of the walking
-// peel gets for little.  A graph of kCliqueEdges edges (the lists of smaller ones cost at most half a
-// millisecond) with kCliqueEntries or more entries an edge walks if more than three
-// quarters of them belong to edges with 15/16 or more of their shorter row in triangles: disjoint
-// cliques of 100 vertices 2.1 / 0.65 ms, of 400 10.7 / 1.5 ms, G(200000, 16/n) with cliques of 300-500
-// vertices 4.8 / 3.8 ms; cliques of 20 (18 entries an edge) 0.53 / 0.44 ms, cliques of 50 with a
-// tenth of the edges rewired (35; not near-cliques) 1.6 / 2.6 ms.
-constexpr uint64_t kCliqueEntries = 32;
-constexpr uint32_t kCliqueEdges = 1u << 18;
 
 namespace {
 
@@ -768,8 +758,7 @@ int want_lists(kt_engine* e, bool* use) {
     if ((rc = sync_and_check(e))) return rc;
     const uint64_t total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
     const uint64_t local = (uint64_t)e->h_ctrl[kListLocal + 1] << 32 | e->h_ctrl[kListLocal];
-    if (e->m >= kCliqueEdges && total >= kCliqueEntries * e->m && local > total / 4 * 3) return KT_OK;
-    if (total / kMaxListPerEdge > e->m) return KT_OK;
+    if (walks_rows(e->m, total, local, ~e->h_ctrl[kListLeast])) return KT_OK;
     const uint64_t need = std::max<uint64_t>(total, 1);
     if (need > e->list_cap) {
         const uint64_t want = buffer_entries(total, e->list_limit);
@@ -820,7 +809,7 @@ int peel_lists(kt_engine* e, bool* done) {
     *done = e->list_need != 0;
     if ((rc = launch_chained(e, "k_list_bounds", e->chained ? k_list_bounds<true> : k_list_bounds<false>,
                              ceil_div(m, kScanTile), kScanThreads, 0, e->sup, e->rnd, e->tr, m, tptr, ends,
-                             m < kCliqueEdges ? nullptr : e->s_len, e->e_src, e->o_col,
+                             m <= kSmallLists ? nullptr : e->s_len, e->e_src, e->o_col,
                              *done ? e->list_cap : ~0ull, next_look(e))) ||
         (!e->trusted && !small && (rc = want_lists(e, done))) || !*done || (rc = fill_lists(e, tptr, ends)))
         return rc;

@@ -1,5 +1,5 @@
 // Prints what kt_list_rule.h decides: lines "most m", "small m cap", "repeat need cap",
-// "buffer total limit".
+// "buffer total limit", "walks m total local least".
 #include <cstdio>
 #include <cstring>
 
@@ -14,6 +14,13 @@ int main() {
             continue;
         }
         if (scanf("%llu", &b) != 1) return 1;
+        unsigned long long c = 0;
+        if (!strcmp(op, "walks")) {
+            unsigned least = 0;
+            if (scanf("%llu %u", &c, &least) != 2) return 1;
+            printf("%d\n", kt::walks_rows(a, b, c, least));
+            continue;
+        }
         if (!strcmp(op, "buffer")) {
             printf("%llu\n", (unsigned long long)kt::buffer_entries(a, b));
             continue;

@@ -1,6 +1,6 @@
-"""The host rules of the triangle lists' buffer (csrc/kt_list_rule.h), built for the host: its size for
-uncounted graphs covers every graph of that many edges, and a repeated call whose buffer was lost or shrank
-walks rows instead of writing to it."""
+"""The rules of the triangle lists (csrc/kt_list_rule.h), built for the host: the buffer for uncounted graphs
+covers every graph of that many edges, a repeated call whose buffer was lost or shrank walks rows instead of
+writing to it, buffers keep to their limit, and which graphs walk."""
 import math
 import os
 import shutil
@@ -56,3 +56,29 @@ def test_buffers_keep_to_the_limit(ask):
     cases = [(0, none, 1), (0, 8, 1), (0, 7, 0), (0, 0, 0), (15, none, 15), (16, none, 17), (16, 17 * 8, 17),
              (16, 17 * 8 - 1, 16), (16, 16 * 8, 16), (16, 16 * 8 - 1, 0), (5 << 30, none, (5 << 30) + (5 << 26))]
     assert ask(*[("buffer", t, limit) for t, limit, _ in cases]) == [want for *_, want in cases]
+
+
+def _cliques(size, count):
+    m = count * math.comb(size, 2)
+    return m, (size - 2) * m
+
+
+def test_which_graphs_walk(ask):
+    near = [(c, (*_cliques(*c), _cliques(*c)[1], 0), walks) for c, walks in [
+        ((500, 2), 1), ((400, 1), 1), ((200, 6), 1), ((100, 26), 0), ((60, 140), 0), ((60, 160), 1), ((20, 1500), 0),
+        ((514, 3), 1), ((516, 1), 1)]]
+    for (c, _, walks), got in zip(near, ask(*[("walks", *q) for _, q, _ in near])):
+        assert got == walks, c
+    total = 1 << 25
+    assert ask(("walks", 200000, total, total, 0), ("walks", 200000, total, total - total // 256, 0),
+               ("walks", 200000, total, total - total // 256 - 1, 0), ("walks", 200000, 1 << 24, 1 << 24, 0),
+               ("walks", 200000, (1 << 24) - 1, (1 << 24) - 1, 0), ("walks", 1 << 18, 1 << 23, 1 << 23, 0),
+               ("walks", 1 << 18, (1 << 23) - 1, (1 << 23) - 1, 0), ("walks", 1 << 18, 1 << 24, 3 << 22, 0),
+               ("walks", 1 << 18, 1 << 24, (3 << 22) + 1, 0)) == [1, 1, 0, 1, 0, 1, 0, 0, 1]
+    # density; dense and even
+    m = 50000
+    assert ask(("walks", m, 512 * m + 511, 0, 0), ("walks", m, 512 * (m + 1), 0, 0), ("walks", 40000, 0, 0, 0),
+               ("walks", 1 << 18, (512 << 18) + 511, 0, 400), ("walks", 1 << 18, 512 * ((1 << 18) + 1), 0, 0),
+               ("walks", m, 400 * m, 0, 320), ("walks", m, 400 * m, 0, 319), ("walks", m, 320 * m, 0, 320),
+               ("walks", m, 320 * (m + 1), 0, 260), ("walks", m, 320 * (m + 1), 0, 250),
+               ("walks", 1 << 18, 400 << 18, 0, 400)) == [0, 1, 0, 0, 1, 1, 0, 0, 1, 0, 0]
