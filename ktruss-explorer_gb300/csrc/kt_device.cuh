@@ -26,8 +26,10 @@ enum : uint32_t {
 // Layout of the device control block (uint32 words unless noted).
 enum : uint32_t {
     kCtrlError = 0,
-    // words 1-9, 12, 13 and 26-27 are unused; 21-24 hold the support plan during the count
+    kMidPlan = 21,      // [4] plan of the vertex-centric count: items, bases, cursors of count and fill
     kCtrlVariantChanged = 25,  // a variant pass deleted an edge
+    kRowItems = 26,     // the fill's row blocks: rows, and the next one
+    kRowCursor = 27,
     kCtrlTriLo = 10,      // 64-bit triangle counter (lo, hi)
     kCtrlTriHi = 11,
     kCtrlBigRow = 14,     // first rank whose symmetric row is long (block-wide compaction)
@@ -54,14 +56,36 @@ enum : uint32_t {
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
     kListLeast = 84,   // decompositions: complement of the least support (k_list_bounds)
-    // words 88-115: the list peel (kt_lists.cu)
-    kPruneFront = 116,  // single-k: edges whose counted support is too small (the first round's frontier)
-    kPruneLeft = 117,   //   the others, when these were counted again (recount_pruned)
-    kPruneT0 = 118,     //   u64 (words 118..119): when that began
-    kListLocal = 118,   // decompositions: u64, list entries of edges in near-cliques (k_list_bounds)
-    kPrunePlan = 120,   //   items, bases and cursor of its plan
+    kListLocal = 86,   //   u64, list entries of edges in near-cliques
+    kLRing = 88,       // [4] barrier slots of the list peel, kLSlotWords each (kt_lists.cu)
+    kPruneFront = 120,  // single-k: edges whose counted support is too small (the first round's frontier)
+    kPruneLeft = 121,   //   the others, when these were counted again (recount_pruned)
+    kPruneT0 = 122,     //   u64 (words 122..123): when that began
+    kPrunePlan = 124,   //   [3] items, bases and cursor of its plan
     kCtrlWords = 128,
 };
+constexpr uint32_t kLSlotWords = 8;
+
+// The map above, word for word: no two share one, and what is read 8 or 16 bytes at a time is aligned.
+struct CtrlRange {
+    uint32_t first, words, align;
+};
+constexpr CtrlRange kCtrlMap[] = {
+    {kCtrlError, 1, 1}, {kCtrlTriLo, 2, 2}, {kCtrlBigRow, 1, 1}, {kCtrlTinyRow, 1, 1}, {kPBarCount, 2, 2},
+    {kPKmax, 1, 1}, {kPRounds, 1, 1}, {kPLevels, 1, 1}, {kMidPlan, 4, 1}, {kCtrlVariantChanged, 1, 1},
+    {kRowItems, 1, 1}, {kRowCursor, 1, 1}, {kPBigCount, 4, 1}, {kPLAlive, 4, 1}, {kPLMin, 4, 1}, {kPLMinId, 4, 1},
+    {kPCompactions, 1, 1}, {kPPhaseNs, 12, 2}, {kPEdges, 4, 1}, {kPChunks, 8, 2}, {kPWalk, 2, 2}, {kPSched, 4, 1},
+    {kPPasses, 1, 1}, {kPAliveSum, 2, 2}, {kListLeast, 1, 1}, {kListLocal, 2, 2}, {kLRing, 4 * kLSlotWords, 4},
+    {kPruneFront, 1, 1}, {kPruneLeft, 1, 1}, {kPruneT0, 2, 2}, {kPrunePlan, 3, 1}};
+constexpr bool ctrl_map_holds() {
+    uint32_t next = 0;
+    for (const CtrlRange& r : kCtrlMap) {  // in ascending order
+        if (r.first < next || r.first % r.align) return false;
+        next = r.first + r.words;
+    }
+    return next <= kCtrlWords && kCtrlTriHi == kCtrlTriLo + 1;
+}
+static_assert(ctrl_map_holds(), "control words overlap, are out of order or are misaligned");
 
 // Kernels that the host chains (launch_chained) start while their predecessor still runs: its tail hides
 // their launch.  They wait here, before they touch memory, until it is done and its writes are visible;

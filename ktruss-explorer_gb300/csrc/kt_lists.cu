@@ -60,12 +60,10 @@ constexpr uint32_t kNotLoaded = 0xffffffffu;
 constexpr uint32_t kPrefetch = 1u << 16;  // chunks of a frontier whose entries are prefetched to L2 (16 MB):
                                           // R-MAT 20 peel kernel 20.9 -> 20.3 ms
 
-// Control words of this kernel (beyond the words it shares with the walking peel): a ring of four
-// barrier slots, each {u64 arrivals << 32 | edges queued, u64 global chunks, overflowed edges,
-// minimum support, smallest alive edge id, unused}.
-constexpr uint32_t kLRing = 96, kLSlotWords = 8;
+// A barrier slot of the ring at kLRing: {u64 arrivals << 32 | edges queued, u64 global chunks, overflowed
+// edges, minimum support, smallest alive edge id, unused}.
 constexpr uint32_t kLChunks = 2, kLBig = 4, kLMin = 5, kLMinId = 6;
-static_assert(kLRing + 4 * kLSlotWords <= kCtrlWords, "control block holds the list peel's words");
+static_assert(kLMinId < kLSlotWords && kLSlotWords == 8, "a slot is two 16-byte words");
 
 struct ListParams {
     const uint2* __restrict__ tri;       // per list entry: the triangle's other two edges

@@ -69,10 +69,8 @@ constexpr uint32_t kRowFactor = 6;
 constexpr uint32_t kMidMinEdges = 1u << 18;
 constexpr uint32_t kPruneMin = 1u << 19, kPruneEarly = 1u << 20;  // edges (see recount_pruned)
 constexpr uint32_t kEmpty = 0xffffffffu;
-// control words of the plan, zero since the build
-constexpr uint32_t kMidPlan = 21;  // items, bases, count cursor, fill cursor
+// words of a plan (kMidPlan, kPrunePlan), zero since the build: items, bases, count cursor, fill cursor
 constexpr uint32_t kPlanBases = 1, kPlanCursor = 2;
-constexpr uint32_t kRowItems = 26, kRowCursor = 27;
 
 struct Graph {
     const uint32_t* ctrl;
