@@ -319,12 +319,13 @@ int kt_engine_level_log(kt_engine* engine, uint32_t* k, uint32_t* alive, uint32_
 int kt_engine_set_schedule(kt_engine* engine, const kt_schedule* schedule);
 int kt_engine_get_schedule(kt_engine* engine, kt_schedule* schedule);
 
-/* Wait limit of the peel kernel's grid barriers (no counterpart in the reference, whose loop is
+/* Wait limit of the device's waits - the peel kernels' grid barriers, and the look-back of the sorts'
+ * and scans' tiles (no counterpart in the reference, whose loop is
  * driven from the host): every wait is bounded by base_ns plus ns_per_unit for each unit of work
- * the wait can legitimately cover - each row entry slot of the work chunks queued for the round
- * that the barrier closes (row entries rounded up to whole chunks),
- * each edge (twice) for a level phase - after which the kernel returns KT_ERR_TIMEOUT instead of
- * waiting forever.  Defaults: 10 s and 8 ns.  base_ns must be at least 1 microsecond. */
+ * the wait can legitimately cover - each row or list entry slot of the work chunks queued for the round
+ * that the barrier closes (entries rounded up to whole chunks),
+ * each edge (twice) for a level phase, each entry or vertex for a look-back - after which the kernel
+ * returns KT_ERR_TIMEOUT instead of waiting forever.  Defaults: 10 s and 8 ns.  base_ns must be at least 1 microsecond. */
 int kt_engine_set_wait_limit(kt_engine* engine, uint64_t base_ns, uint32_t ns_per_unit);
 int kt_engine_get_wait_limit(kt_engine* engine, uint64_t* base_ns, uint32_t* ns_per_unit);
 /* Statistics of the last call of the host-buffer entry points (kt_ktruss, kt_decompose,
@@ -445,6 +446,11 @@ int kt_engine_set_selector(kt_engine* engine, kt_selector* selector);
  * with a wait limit of timeout_ns (at most 5 s).  Returns KT_ERR_TIMEOUT when the wait expired
  * and the kernel returned as designed; the engine stays usable afterwards. */
 int kt_engine_selftest_barrier_timeout(kt_engine* engine, uint64_t timeout_ns);
+/* The same for each kind of device wait: the walking peel's grid barrier, the list peel's, and the
+ * look-back of sorts and scans (a tile whose predecessor never runs), after which the kernels that
+ * would use what it left must write nothing (else KT_ERR_INTERNAL). */
+enum { KT_WAIT_GRID_BARRIER = 0, KT_WAIT_LIST_BARRIER = 1, KT_WAIT_LOOK_BACK = 2 };
+int kt_engine_selftest_wait_timeout(kt_engine* engine, int wait, uint64_t timeout_ns);
 
 /* Decomposition that allocates nothing (no counterpart in the reference).  For callers that
  * cannot let a library allocate device memory: programs whose device memory is owned by one

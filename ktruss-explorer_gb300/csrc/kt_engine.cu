@@ -774,14 +774,22 @@ int kt_engine_features(kt_engine* e, const uint32_t* d_src, const uint32_t* d_ds
     return check_cuda(cudaStreamSynchronize(e->stream), "synchronize");
 }
 
-int kt_engine_selftest_barrier_timeout(kt_engine* e, uint64_t timeout_ns) {
-    if (!e) return fail(KT_ERR_INVALID_ARG, "kt_engine_selftest_barrier_timeout: null engine");
+int kt_engine_selftest_wait_timeout(kt_engine* e, int wait, uint64_t timeout_ns) {
+    if (!e) return fail(KT_ERR_INVALID_ARG, "kt_engine_selftest_wait_timeout: null engine");
     if (timeout_ns == 0 || timeout_ns > 5000000000ull)
         return fail(KT_ERR_INVALID_ARG, "timeout must be in (0, 5 s]");
+    if (wait < KT_WAIT_GRID_BARRIER || wait > KT_WAIT_LOOK_BACK)
+        return fail(KT_ERR_INVALID_ARG, "kt_engine_selftest_wait_timeout: unknown wait %d", wait);
     int rc = check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
     if (rc) return rc;
     e->stats_ready = true;  // the probe leaves no peel statistics behind
-    return kt::barrier_timeout_probe(e, timeout_ns);
+    return wait == KT_WAIT_GRID_BARRIER   ? kt::barrier_timeout_probe(e, timeout_ns)
+           : wait == KT_WAIT_LIST_BARRIER ? kt::list_timeout_probe(e, timeout_ns)
+                                          : kt::look_timeout_probe(e, timeout_ns);
+}
+
+int kt_engine_selftest_barrier_timeout(kt_engine* e, uint64_t timeout_ns) {
+    return kt_engine_selftest_wait_timeout(e, KT_WAIT_GRID_BARRIER, timeout_ns);
 }
 
 int kt_engine_round_log(kt_engine* e, uint32_t* size, uint32_t* level, uint32_t* ns, uint32_t cap,

@@ -65,6 +65,7 @@ struct kt_engine {
     uint64_t look_cap = 0;
     uint32_t* digit_counts = nullptr;
     uint32_t look_tag = 0, look_count = 0;
+    uint64_t look_limit_ns = 0;  // longest look-back wait of the session
     // Control block (device) and its pinned host mirror.
     uint32_t* ctrl = nullptr;
     uint32_t* h_ctrl = nullptr;
@@ -257,8 +258,11 @@ int graph_features(kt_engine* e, const float* d_params);
 int select_schedule(kt_engine* e);
 // Reads the peel's control block and round log (stream must be drained); reports timeouts.
 int finish_stats(kt_engine* e);
-// Launches a grid barrier that cannot complete and returns the status it reports.
+// Launches a grid barrier (kt_peel.cu), a barrier of the list peel (kt_lists.cu) or look-backs of a radix pass
+// and of a scan (kt_sort.cu) that cannot complete and returns the status they report.
 int barrier_timeout_probe(kt_engine* e, uint64_t timeout_ns);
+int list_timeout_probe(kt_engine* e, uint64_t timeout_ns);
+int look_timeout_probe(kt_engine* e, uint64_t timeout_ns);
 // kt_variants.cu: single-k truss by count-and-delete passes (undirected capped counts; tiled
 // counts); edge states in e->rnd, so emit_keep applies.  Synchronous (one read per pass).
 int ktruss_undirected(kt_engine* e, uint32_t k, bool recount_all, uint32_t group);

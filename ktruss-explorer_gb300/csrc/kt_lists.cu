@@ -264,8 +264,9 @@ __device__ __forceinline__ void flush(const ListParams& P, ListShared& S, uint32
 
 // Grid barrier `epoch` (counted from 0) on ring slot epoch & 3, which was zero when the epoch
 // began: the block's queued edges are added to the slot's first word together with its arrival.
-// Bounded like grid_barrier (`units`: the work it covers).  Delivers the phase's frontier in S.front (kScan: and the minima).
-template <bool kScan>
+// Bounded like grid_barrier (`units`: the work it covers).  Delivers the phase's frontier in S.front (kScan: and
+// the minima).  kAbsent: blocks that never arrive (the self-test's).
+template <bool kScan, uint32_t kAbsent = 0>
 __device__ __forceinline__ bool list_barrier(const ListParams& P, ListShared& S, uint32_t epoch, uint64_t units) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -280,7 +281,7 @@ __device__ __forceinline__ bool list_barrier(const ListParams& P, ListShared& S,
                 : "=l"(bar), "=l"(chunks)
                 : "l"(slot)
                 : "memory");
-            if ((uint32_t)(bar >> 32) == gridDim.x) break;
+            if ((uint32_t)(bar >> 32) == gridDim.x + kAbsent) break;
             if ((++spins & 31u) == 0) {
                 if (spins == 32) t0 = global_ns();
                 if (ld_acquire(P.ctrl + kCtrlError) & kErrTimeout) { ok = 0; break; }
@@ -660,6 +661,14 @@ __global__ void __launch_bounds__(kListThreads, 1) k_peel_lists(const __grid_con
     }
 }
 
+// Self-test: a barrier that one block never reaches; *passed counts the blocks that got past it.
+__global__ void k_list_barrier_probe(const __grid_constant__ ListParams P, uint32_t* passed) {
+    __shared__ ListShared S;
+    if (threadIdx.x == 0) S.queued = 0;
+    __syncthreads();
+    if (list_barrier<false, 1>(P, S, 0, 0) && threadIdx.x == 0) atomicAdd(passed, 1u);
+}
+
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
 // of whose endpoint's neighbours are common ones, near-cliques, and the least support (walks_rows).  More than `cap` entries, what
@@ -845,6 +854,25 @@ int peel_lists(kt_engine* e, bool* done) {
     if (rc || !timed) return rc;
     e->peel_timed = true;
     return check_cuda(cudaEventRecord(e->ev_peel1, e->stream), "record event");
+}
+
+int list_timeout_probe(kt_engine* e, uint64_t timeout_ns) {
+    e->ctrl_fresh = false;
+    int rc = check_cuda(cudaMemsetAsync(e->ctrl, 0, sizeof(uint32_t) * kCtrlWords, e->stream), "clear control block");
+    if (rc) return rc;
+    ListParams P{};
+    P.ctrl = e->ctrl;
+    P.wait_base_ns = timeout_ns;
+    uint32_t* passed = e->ctrl + kPRounds;
+    void* args[] = {&P, &passed};
+    if ((rc = check_cuda(cudaLaunchCooperativeKernel((const void*)k_list_barrier_probe, dim3(2), dim3(32), args, 0,
+                                                     e->stream), "cooperative launch of k_list_barrier_probe")))
+        return rc;
+    count_launch(e);
+    rc = sync_and_check(e);
+    if (rc != KT_ERR_TIMEOUT || e->h_ctrl[kPRounds])
+        return rc && rc != KT_ERR_TIMEOUT ? rc : fail(KT_ERR_INTERNAL, "list barrier probe: the wait did not expire");
+    return fail(KT_ERR_TIMEOUT, "list barrier probe: wait expired as intended");
 }
 
 }  // namespace kt

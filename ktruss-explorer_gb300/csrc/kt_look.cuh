@@ -4,15 +4,14 @@
 // Each tile publishes its aggregate, adds up its predecessors' words backwards until it meets an
 // inclusive one, and publishes its own inclusive prefix.  A word is flag << 62 | tag << 56 | value:
 // every launch of a session has a tag of its own, so the words of earlier launches need no clearing.
-// Every wait is bounded: past kLookLimitNs it sets kErrTimeout and gives up, and every kernel that
-// would index by what such a launch left behind returns at once when it sees that bit.
+// Every wait is bounded: past the session's limit (kt_engine_set_wait_limit) it sets kErrTimeout and gives
+// up, and every kernel that would index by what such a launch left behind returns at once when it sees that bit.
 #pragma once
 
 #include "kt_device.cuh"
 
 namespace kt {
 
-constexpr uint64_t kLookLimitNs = 10ull * 1000 * 1000 * 1000;
 constexpr uint64_t kLookValue = (1ull << 56) - 1;
 constexpr uint32_t kLookTags = 32;  // launches of one session
 enum : uint64_t { kLookAggregate = 1, kLookInclusive = 2 };
@@ -22,6 +21,7 @@ struct Look {
     uint32_t* tickets;  // one per tag
     uint32_t* ctrl;
     uint32_t tag;
+    uint64_t limit_ns;
 };
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
@@ -48,12 +48,12 @@ __device__ __forceinline__ bool timed_out(const uint32_t* ctrl) { return __ldca(
 struct LookWait {
     uint32_t spins = 0;
     uint64_t t0 = 0;
-    __device__ __forceinline__ bool again(uint32_t* ctrl) {
+    __device__ __forceinline__ bool again(const Look& L) {
         if ((++spins & 63u) == 0) {
             if (spins == 64) t0 = global_ns();
-            if (ld_acquire(ctrl + kCtrlError) & kErrTimeout) return false;
-            if (global_ns() - t0 > kLookLimitNs) {
-                atomicOr(ctrl + kCtrlError, kErrTimeout);
+            if (ld_acquire(L.ctrl + kCtrlError) & kErrTimeout) return false;
+            if (global_ns() - t0 > L.limit_ns) {
+                atomicOr(L.ctrl + kCtrlError, kErrTimeout);
                 return false;
             }
         }
@@ -86,7 +86,7 @@ __device__ __forceinline__ uint64_t look_back(const Look& L, uint32_t tile, uint
         const uint32_t incl = __ballot_sync(kFullMask, look_valid(w, L.tag) && (w >> 62) == kLookInclusive);
         const uint32_t first = incl ? __ffs(incl) - 1 : 31;  // the last word to add
         if ((~valid & (0xffffffffu >> (31 - first))) != 0) {
-            if (!__all_sync(kFullMask, wait.again(L.ctrl))) break;
+            if (!__all_sync(kFullMask, wait.again(L))) break;
             continue;
         }
         uint64_t v = lane <= first ? (uint64_t)w & kLookValue : 0;

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <utility>
+#include <vector>
 
 #include "kt_engine.h"
 #include "kt_look.cuh"
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_radix_pass(const 
                     }
                 }
                 t -= used;
-                if (!done && used == 0 && !wait.again(L.ctrl)) {
+                if (!done && used == 0 && !wait.again(L)) {
                     S.ok = 0;
                     break;
                 }
@@ -226,6 +227,18 @@ __global__ void k_session(uint32_t* __restrict__ ctrl, uint32_t ctrl_words, uint
     for (uint64_t i = tid; i < count_words; i += step) counts[i] = 0;
 }
 
+// Self-test: takes a tile's number without running it, so that the next tile's look-back runs out.
+__global__ void k_drop_tile(Look L) { atomicAdd(L.tickets + L.tag, 1u); }
+
+// Self-test: one block's look-back as in a scan.
+__global__ void k_look_probe(Look L, uint32_t* __restrict__ prefix) {
+    __shared__ uint32_t s_tile;
+    const uint32_t tile = look_tile(L, &s_tile);
+    if (tile == kNoTile) return;
+    const uint64_t p = look_back(L, tile, 1);
+    if (threadIdx.x == 0) *prefix = (uint32_t)p;
+}
+
 template <int kThreads, int kItems, bool kVals>
 int launch_pass(kt_engine* e, const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, uint64_t n,
                 unsigned shift, const uint32_t* counts, const Look& L) {
@@ -254,6 +267,7 @@ int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words, 
     e->chained = e->lists_allowed && keys <= kSmallSort && n <= kSmallSort;
     if (!e->look || words > e->look_cap) return fail(KT_ERR_INTERNAL, "look-back scratch too small");
     e->look_tag = e->look_count = 0;
+    e->look_limit_ns = e->wait_base_ns + e->wait_ns_per_unit * std::max<uint64_t>(keys, n);
     e->ctrl_fresh = false;
     const uint64_t work = std::max<uint64_t>(words / 2, std::max<uint32_t>(deg_words, kCountWords));
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((work + 255) / 256, (uint64_t)e->num_sms * 8);
@@ -263,7 +277,7 @@ int begin_session(kt_engine* e, uint32_t n, uint32_t deg_words, uint64_t words, 
 
 Look next_look(kt_engine* e) {
     ++e->look_tag;
-    return Look{e->look, e->digit_counts + kLookTags * 256, e->ctrl, e->look_tag};
+    return Look{e->look, e->digit_counts + kLookTags * 256, e->ctrl, e->look_tag, e->look_limit_ns};
 }
 
 uint32_t* next_counts(kt_engine* e, unsigned passes) {
@@ -300,6 +314,43 @@ int radix_passes(kt_engine* e, uint64_t* key_a, uint32_t* val_a, uint64_t* key_b
         *result_in_b ^= 1;
     }
     return KT_OK;
+}
+
+int look_timeout_probe(kt_engine* e, uint64_t timeout_ns) {
+    constexpr uint64_t kKeys = 2 * kSmallTile;
+    int rc;
+    if ((!e->look || e->cap_entries < kKeys) &&
+        (rc = reserve(e, e->cap_nodes, std::max<uint64_t>(e->cap_entries, kKeys))))
+        return rc;
+    std::vector<uint64_t> out(kKeys);
+    for (int scan = 0; scan < 2; ++scan) {
+        if ((rc = begin_session(e, 0, 0, look_words(kKeys), kKeys))) return rc;
+        e->look_limit_ns = timeout_ns;
+        if ((rc = check_cuda(cudaMemsetAsync(e->key_a, 0, kKeys * 8, e->stream), "clear keys")) ||
+            (rc = check_cuda(cudaMemsetAsync(e->key_b, 0xff, kKeys * 8, e->stream), "mark keys")))
+            return rc;
+        // tile 1 waits for a tile 0 that nobody runs, with every other kernel of the session behind it
+        const Look L = next_look(e);
+        k_drop_tile<<<1, 1, 0, e->stream>>>(L);
+        if (scan)
+            k_look_probe<<<1, 32, 0, e->stream>>>(L, reinterpret_cast<uint32_t*>(e->key_a));
+        else
+            k_radix_pass<kSmallThreads, kSmallItems, false>
+                <<<1, kSmallThreads, (int)sizeof(PassSmem<kSmallThreads, kSmallItems>), e->stream>>>(
+                    e->key_a, nullptr, e->key_b, nullptr, kKeys, 0, next_counts(e, 1), L);
+        count_launch(e, 2);
+        int in_b = 0;
+        if ((rc = check_launch(e, "look-back probe")) ||
+            (rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, kKeys, 0, 1, next_counts(e, 1), &in_b)) ||
+            (rc = check_cuda(cudaMemcpyAsync(out.data(), e->key_b, kKeys * 8, cudaMemcpyDeviceToHost, e->stream),
+                             "read keys")))
+            return rc;
+        rc = sync_and_check(e);
+        if (rc != KT_ERR_TIMEOUT) return rc ? rc : fail(KT_ERR_INTERNAL, "look-back probe: the wait did not expire");
+        for (const uint64_t k : out)
+            if (k != ~0ull) return fail(KT_ERR_INTERNAL, "look-back probe: keys written after the wait expired");
+    }
+    return fail(KT_ERR_TIMEOUT, "look-back probe: waits expired as intended");
 }
 
 }  // namespace kt

@@ -148,6 +148,7 @@ def lib() -> ctypes.CDLL:
         L.kt_engine_stats.argtypes = [_VP, ctypes.POINTER(Stats)]
         L.kt_last_stats.argtypes = [ctypes.POINTER(Stats)]
         L.kt_engine_selftest_barrier_timeout.argtypes = [_VP, ctypes.c_uint64]
+        L.kt_engine_selftest_wait_timeout.argtypes = [_VP, ctypes.c_int, ctypes.c_uint64]
         L.kt_engine_decompose_batch.argtypes = [_VP, _VP, _VP, ctypes.c_uint64, ctypes.c_uint32, _VP, ctypes.c_uint32,
                                                 _VP, _VP, ctypes.c_int]
         L.kt_decompose_batch.argtypes = [_U32P, _U32P, ctypes.c_uint64, ctypes.c_uint32, _U32P, ctypes.c_uint32,
@@ -454,7 +455,7 @@ class Engine:
         return v
 
     def set_wait_limit(self, base_ns: int, ns_per_unit: int = 8) -> None:
-        """Bound of every peel barrier wait: base_ns plus ns_per_unit per unit of covered work."""
+        """Bound of every device wait: base_ns plus ns_per_unit per unit of covered work."""
         _check(lib().kt_engine_set_wait_limit(self._h, base_ns, ns_per_unit))
 
     def wait_limit(self) -> tuple:
@@ -524,6 +525,11 @@ class Engine:
     def selftest_barrier_timeout(self, timeout_ns: int) -> int:
         """Status of a grid barrier that cannot complete (KT_ERR_TIMEOUT = 11 when correct)."""
         return lib().kt_engine_selftest_barrier_timeout(self._h, timeout_ns)
+
+    def selftest_wait_timeout(self, wait: str, timeout_ns: int) -> int:
+        """The same for a "grid barrier", "list barrier" or "look-back"."""
+        kind = ("grid barrier", "list barrier", "look-back").index(wait)
+        return lib().kt_engine_selftest_wait_timeout(self._h, kind, timeout_ns)
 
     def round_log(self, cap: int = 1 << 20) -> dict:
         """Frontier size, level and device nanoseconds of each peel round of the last call."""
