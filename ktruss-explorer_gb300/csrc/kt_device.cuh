@@ -21,6 +21,7 @@ enum : uint32_t {
     kErrRunaway = 1u << 5,     // the peel loop exceeded its round or level bound
     kErrCrossGraph = 1u << 6,  // a batch entry joins two different graphs
     kErrListSpace = 1u << 7,   // a repeated call's triangle lists outgrew their buffer
+    kErrRoundLog = 1u << 8,    // a decomposition's round log is inconsistent
 };
 
 // Layout of the device control block (uint32 words unless noted).
@@ -187,6 +188,13 @@ __host__ __device__ __forceinline__ uint32_t fenced_lower_bound(const uint32_t* 
         hi = e;
     }
     return lo + lower_bound_u32(a + lo, hi - lo, t);
+}
+
+// Whether a logged round of level k that removes `size` of `alive` edges may follow one of level `before` (2 for
+// the first) in a decomposition up to k_max.
+__host__ __device__ __forceinline__ bool round_follows(uint32_t k, uint32_t before, uint32_t k_max, uint32_t size,
+                                                       uint32_t alive) {
+    return k >= 3 && k >= before && k <= k_max + 1 && size != 0 && size <= alive;
 }
 
 // An error of the call so far: kernels that index by what the build made return at once (the host

@@ -769,7 +769,7 @@ __global__ void k_barrier_probe(uint32_t* ctrl, uint64_t timeout_ns) {
 // the alive edges they see: level 3 is one pass over all m edges; each level k >= 4 up to k_max+1
 // takes one pass per removing round plus a final one, each seeing the edges alive at its start;
 // levels that remove nothing take one pass each.  One block; counting along in the peel kernels
-// instead cost their rounds 1-3 %.
+// instead cost their rounds 1-3 %.  A log that no decomposition leaves behind is an error.
 __device__ void count_passes(const uint32_t* __restrict__ size, const uint32_t* __restrict__ level, uint32_t rounds,
                              uint32_t m, uint32_t* __restrict__ ctrl) {
     __shared__ uint32_t removed[kThreads];
@@ -784,8 +784,13 @@ __device__ void count_passes(const uint32_t* __restrict__ size, const uint32_t* 
     uint32_t alive = m;
     for (uint32_t t = 0; t < threadIdx.x; ++t) alive -= removed[t];
     unsigned long long passes = threadIdx.x == 0 ? 1 : 0, seen = threadIdx.x == 0 ? m : 0;
+    const uint32_t k_max = ctrl[kPKmax];
     for (uint32_t i = a; i < b; ++i) {
         const uint32_t k = level[i], before = i > 1 ? level[i - 1] : 2u;
+        if (!round_follows(k, before, k_max, size[i], alive)) {
+            atomicOr(&ctrl[kCtrlError], kErrRoundLog);
+            break;
+        }
         const uint32_t next = before + 1 > 4 ? before + 1 : 4u;  // the first level after the last one
         if (before != k && k > next) {
             passes += k - next;
@@ -1095,6 +1100,7 @@ int finish_stats(kt_engine* e) {
     const uint32_t err = e->h_ctrl[kCtrlError];
     if (err & kErrTimeout) return fail(KT_ERR_TIMEOUT, "a grid barrier wait of the peel kernel expired");
     if (err & kErrRunaway) return fail(KT_ERR_INTERNAL, "the peel kernel exceeded its round or level bound");
+    if (err & kErrRoundLog) return fail(KT_ERR_INTERNAL, "inconsistent round log");
     if (err & kErrListSpace) return fail(KT_ERR_INVALID_ARG, "the repeated call's input has changed since the call");
     if (err & kErrCrossGraph) return fail(KT_ERR_INVALID_ARG, "a batch entry joins vertices of two different graphs");
     const uint64_t m = e->m;
