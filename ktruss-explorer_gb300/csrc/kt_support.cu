@@ -18,10 +18,10 @@
 // shorter of tail and row is walked, the longer binary-searched; x and y are credited with global
 // atomics, j once per group.
 //
-// The lists are written by a second pass over the triangles (kFill), in list order of locality:
-// scattered eight-byte writes into lists of many GB are bound by the DRAM's random accesses (R-MAT 20,
-// 1.1 G entries: 18.0 ms with the edge-centric pass alone, 24.6 ms with the vertex-centric one),
-// so three kernels write what is next to each other:
+// The lists are written by a second pass over the triangles (kFill), in list order of locality: eight-byte
+// writes scattered over lists of many GB reach the DRAM in pieces of 32 bytes (R-MAT 20, 1.1 G entries:
+// 18.0 ms with the edge-centric pass alone, 24.6 ms with the vertex-centric one; R-MAT 18 3.8 GB written for
+// 1.8 GB of entries), so three kernels write what is next to each other:
 //   k_middle  the entries of y for vertex-centric v: all in v's row.  An item's part of y's list was
 //             claimed by the count, whose addition to `sup` returned where it starts (bases); all
 //             other credits go to a second array (supx), so the claimed parts come first in a list;
@@ -34,7 +34,10 @@
 // waits for the longest tail).  k_middle issues in 84 % of the cycles, L1 70 % (bank conflicts of the
 // probes), DRAM 5 %.  A filter of the row's columns in front of the table: 3.9-4.2 ms; lookups queued up
 // to full warps, by binary search in the row: 5.0 ms.  Fill 18.0 -> 13.0 ms and 114 -> 76 ms, its DRAM
-// writes on R-MAT 18 3.8 -> 2.1 GB for 1.8 GB of entries.
+// writes on R-MAT 18 3.8 -> 2.1 GB.  It is no longer bound by memory (R-MAT 19, 4.5 GB of entries): k_middle
+// issues in 48 % of the cycles, between loads (long scoreboard 8.4 of 24 stall cycles an instruction) and the
+// barriers of a batch (5.5), with DRAM at 18 % and L2 at 42 % (each entry is a 32-byte sector there); k_rows is
+// bound by its instructions, 75 %.
 
 #include <algorithm>
 
@@ -60,7 +63,6 @@ constexpr uint32_t kMidItemIn = 256;           // in-edges per work item (more f
 // Rows of kRowMin entries or more get a block of the fill: R-MAT 22 76.4 ms at 128, 79.8 at 64, 79.9
 // at 256; whole warps stream their rows (half warps: 81.0).
 constexpr uint32_t kRowMin = 128;
-constexpr int kRowGroup = 32;
 // A row is streamed through the table unless it is this many times longer than the tail that could
 // be searched in it instead (R-MAT 22: 76.4 ms at 6, 77.6 at 3, 78.8 at 12, 82.0 streaming always).
 constexpr uint32_t kRowFactor = 6;
@@ -372,19 +374,18 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
 // The fill's row blocks: for the rows u of kRowMin entries or more, the list entries of j and x of
 // the triangles whose middle vertex is vertex-centric (their y entries are k_middle's).  Both lie
 // in u's own row, so a block with the row hashed into shared memory and a cursor per row position
-// writes them without global atomics, into lists that are next to each other.  Groups of lanes
-// stream the rows N+(v) through the table - or, where v's row is much longer than u's tail above v,
-// search the tail's entries in it.
+// writes them without global atomics, into lists that are next to each other.  Warps stream the rows
+// N+(v) through the table - or, where v's row is much longer than u's tail above v, search the tail's
+// entries in it.
+// Bound: instructions, issue active 75 % (R-MAT 19; DRAM 17 %, L2 36 %).
 __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, const uint32_t* __restrict__ rows,
                                                          uint32_t* __restrict__ ctrl) {
     __shared__ uint2 key[kMidSlots / 2];  // (as in k_middle)
     __shared__ uint16_t at[kMidSlots];
     __shared__ uint32_t cur[kMidRow];  // next list entry, from the start of the row's lists
     __shared__ uint32_t s_row;
-    constexpr int G = kRowGroup;
-    const uint32_t lane = lane_id(), glane = lane & (G - 1);
-    const uint32_t gmask = (G == 32) ? kFullMask : (((1u << G) - 1) << (lane & ~(uint32_t)(G - 1)));
-    const uint32_t group = threadIdx.x / G, n_rows = failed(ctrl) ? 0u : ctrl[kRowItems];
+    constexpr uint32_t kWarps = kMidThreads / 32;
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, n_rows = failed(ctrl) ? 0u : ctrl[kRowItems];
     for (;;) {
         if (threadIdx.x == 0) {
             const uint32_t t = atomicAdd(ctrl + kRowCursor, 1u);
@@ -418,53 +419,52 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
             }
         }
         __syncthreads();
-        // positions group, group + groups, ...: the group's lanes load the rows of the next G together
-        constexpr uint32_t kGroups = kMidThreads / G;
-        for (uint32_t i0 = group; i0 + 1 < row; i0 += kGroups * G) {
+        // positions warp, warp + kWarps, ...: the lanes load the rows of the next 32 together
+        for (uint32_t i0 = warp; i0 + 1 < row; i0 += kWarps * 32) {
             uint32_t lb0 = 0, lb1 = 0;
-            if (i0 + glane * kGroups + 1 < row) {
-            const uint32_t v = g.o_col[r0 + i0 + glane * kGroups];
-            lb0 = g.o_ptr[v];
-            lb1 = g.o_ptr[v + 1];
-            if (lb0 != lb1 && !vertex_centric(g, v, lb1 - lb0)) lb1 = lb0;
+            if (i0 + lane * kWarps + 1 < row) {
+                const uint32_t v = g.o_col[r0 + i0 + lane * kWarps];
+                lb0 = g.o_ptr[v];
+                lb1 = g.o_ptr[v + 1];
+                if (lb0 != lb1 && !vertex_centric(g, v, lb1 - lb0)) lb1 = lb0;
             }
-            for (int l = 0; l < G; ++l) {
-            const uint32_t i = i0 + l * kGroups;
-            const uint32_t b0 = __shfl_sync(gmask, lb0, l, G), b1 = __shfl_sync(gmask, lb1, l, G), tail = row - 1 - i;
-            if (b0 == b1) continue;
-            const bool stream = b1 - b0 <= kRowFactor * tail;
-            const uint32_t p0 = stream ? b0 : r0 + i + 1, p1 = stream ? b1 : r0 + row;
-            uint32_t w_next = p0 + glane < p1 ? g.o_col[p0 + glane] : kEmpty;
-            for (uint32_t q0 = p0; q0 < p1; q0 += G) {
-                const uint32_t p = q0 + glane, w = w_next;
-                w_next = p + G < p1 ? g.o_col[p + G] : kEmpty;
-                uint32_t pos = kEmpty, y = p;  // x = r0 + pos
-                if (w != kEmpty) {
-                    if (stream) {
-                        uint32_t h = (w * 0x9E3779B1u) >> shift;
-                        uint2 k = key[h];
-                        while (k.x != w && k.y != w && k.y != kEmpty) k = key[h = (h + 1) & mask];
-                        if (k.x == w || k.y == w) pos = at[2 * h + (k.y == w)];
-                    } else {
-                        y = b0 + lower_bound_u32(g.o_col + b0, b1 - b0, w);
-                        if (y < b1 && g.o_col[y] == w) pos = p - r0;
+            for (int l = 0; l < 32; ++l) {
+                const uint32_t i = i0 + l * kWarps, tail = row - 1 - i;
+                const uint32_t b0 = __shfl_sync(kFullMask, lb0, l), b1 = __shfl_sync(kFullMask, lb1, l);
+                if (b0 == b1) continue;
+                const bool stream = b1 - b0 <= kRowFactor * tail;
+                const uint32_t p0 = stream ? b0 : r0 + i + 1, p1 = stream ? b1 : r0 + row;
+                uint32_t w_next = p0 + lane < p1 ? g.o_col[p0 + lane] : kEmpty;
+                for (uint32_t q0 = p0; q0 < p1; q0 += 32) {
+                    const uint32_t p = q0 + lane, w = w_next;
+                    w_next = p + 32 < p1 ? g.o_col[p + 32] : kEmpty;
+                    uint32_t pos = kEmpty, y = p;  // x = r0 + pos
+                    if (w != kEmpty) {
+                        if (stream) {
+                            uint32_t h = (w * 0x9E3779B1u) >> shift;
+                            uint2 k = key[h];
+                            while (k.x != w && k.y != w && k.y != kEmpty) k = key[h = (h + 1) & mask];
+                            if (k.x == w || k.y == w) pos = at[2 * h + (k.y == w)];
+                        } else {
+                            y = b0 + lower_bound_u32(g.o_col + b0, b1 - b0, w);
+                            if (y < b1 && g.o_col[y] == w) pos = p - r0;
+                        }
+                    }
+                    const uint32_t hits = __ballot_sync(kFullMask, pos != kEmpty);
+                    if (hits) {
+                        const uint32_t first = __ffs(hits) - 1;
+                        uint32_t own = 0;
+                        if (lane == first) own = atomicAdd(&cur[i], __popc(hits));
+                        own = __shfl_sync(kFullMask, own, first);
+                        if (pos != kEmpty) {
+                            c.tri[(wide ? __ldg(c.tptr + r0 + i) : row_at) + own + __popc(hits & lanemask_lt())] =
+                                make_uint2(r0 + pos, y);
+                            c.tri[(wide ? __ldg(c.tptr + r0 + pos) : row_at) + atomicAdd(&cur[pos], 1u)] =
+                                make_uint2(r0 + i, y);
+                        }
                     }
                 }
-                const uint32_t hits = __ballot_sync(gmask, pos != kEmpty) & gmask;
-                if (hits) {
-                    const uint32_t first = __ffs(hits) - 1;
-                    uint32_t own = 0;
-                    if (lane == first) own = atomicAdd(&cur[i], __popc(hits));
-                    own = __shfl_sync(gmask, own, first);
-                    if (pos != kEmpty) {
-                        c.tri[(wide ? __ldg(c.tptr + r0 + i) : row_at) + own + __popc(hits & lanemask_lt())] =
-                            make_uint2(r0 + pos, y);
-                        c.tri[(wide ? __ldg(c.tptr + r0 + pos) : row_at) + atomicAdd(&cur[pos], 1u)] =
-                            make_uint2(r0 + i, y);
-                    }
-                }
             }
-          }
         }
         __syncthreads();
     }
