@@ -1031,7 +1031,11 @@ def run_ours(args, world, rank, local):
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "kernel": peel_kernel, "achieved": pk_gbs, "peak": hbm,
                          "peak_kind": hbm_kind, "unit": "GB/s", "frac": pk_gbs / hbm,
+                         "basis": "bytes that the reference's full-recount schedule streams for the same "
+                                  "decomposition; what this kernel moves itself is traffic, traffic_frac of the peak",
                          "traffic": traffic.get(peel_kernel), "traffic_source": traffic_note,
+                         "traffic_frac": (traffic[peel_kernel] / (pk_ms * 1e-3) / 1e9 / hbm
+                                          if traffic.get(peel_kernel) else None),
                          "algorithmic_bytes": plain_bytes, "kernel_ms": pk_ms, "passes": passes,
                          "alive_sum": alive_sum, "passes_source": "oracle fixture" if fx else "engine round log"},
             "roofline_support": {"bound": "hbm", "kernel": "k_middle + k_support", "achieved": sup_gbs, "peak": hbm,
