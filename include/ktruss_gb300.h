@@ -192,9 +192,10 @@ typedef struct kt_stats {
  * -b/-t block and tile sizes).  Every schedule gives the same result; only the time differs. */
 typedef struct kt_schedule {
     uint32_t support_group;    /* support count: lanes per oriented edge (4, 8, 16 or 32) where it is
-                                  counted edge by edge, or 0 to count every vertex with
-                                  shared-memory tables (graphs of 2^18 edges or more count the
-                                  vertices that pay for a table that way with any group)        */
+                                  counted edge by edge, or 0 for shared-memory tables at every
+                                  vertex with 16 lower and 16 higher neighbours (graphs of 2^18
+                                  edges or more count the vertices that pay for a table that way
+                                  with any group)                                               */
     uint32_t chunk_width;      /* row entries per work chunk of the walking peel (lanes per
                                   chunk): 8, 16 or 32.  This and the fields below have no effect
                                   on decompositions from triangle lists                          */

@@ -6,7 +6,7 @@
 // o_col[j+1 .. o_ptr[u+1]), holds u's neighbours above v; the triangles of j are the tail's members
 // that are also in v's row N+(v).  Two ways to test them, chosen by the middle vertex v:
 //
-// Vertex-centric (k_middle): vertices with at least kMidIn in-edges and a row of at most kMidRow
+// Vertex-centric (k_middle): vertices with at least kMidIn in-edges and a row of kMidOut to kMidRow
 // entries.  A block hashes N+(v) into shared memory (column -> row position, in buckets of two, at most a
 // quarter to a half full) and streams the tails of a range of v's in-edges (the lower half of v's
 // symmetric row) through it: one or two shared-memory probes per entry instead of a binary search.  The
@@ -66,6 +66,10 @@ constexpr uint32_t kRowMin = 128;
 // A row is streamed through the table unless it is this many times longer than the tail that could
 // be searched in it instead (R-MAT 22: 76.4 ms at 6, 77.6 at 3, 78.8 at 12, 82.0 streaming always).
 constexpr uint32_t kRowFactor = 6;
+// With support group 0, at least kAllIn in-edges and row entries: R-MAT 20 count 3.65 ms (4.27 from one on, 3.72
+// from 8), a batch of shorter rows, Watts-Strogatz of 4 M edges, 0.25 ms (1.69, 0.80), a path of 200,000 vertices
+// 0.02 ms (0.48; a block a vertex).
+constexpr uint32_t kAllIn = 16;
 // Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save
 // (R-MAT 14 with 220,000 edges counts in 0.05 ms).
 constexpr uint32_t kMidMinEdges = 1u << 18;
@@ -613,7 +617,7 @@ __global__ void k_prune_rows(Graph whole, uint32_t percent, const uint32_t* __re
 Graph graph_of(const kt_engine* e) {
     // the choice must be the same in the count and in the fill of one call
     const bool hash_all = !e->sched_on_device && e->sched.support_group == 0;
-    const uint32_t mid_in = hash_all ? 1u : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? 1u : kMidOut;
+    const uint32_t mid_in = hash_all ? kAllIn : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? kAllIn : kMidOut;
     return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out,
                  kMidPlan, 0, nullptr};
 }
