@@ -105,7 +105,8 @@ struct kt_engine {
 
     kt_schedule sched{8, 32, 85, 50, 0};  // kernel schedule (kt_engine_set_schedule)
     kt_variant variant{KT_DIRECTED_BY_DEGREE, KT_FORMAT_COOCSR, KT_RECOUNT_ALL, 512, 8, 8};  // single-k calls
-    bool orient_by_index = false;      // the current build orients by vertex id (KT_DIRECTED_BY_INDEX)
+    bool orient_by_index = false;      // the next build orients by vertex id (KT_DIRECTED_BY_INDEX)
+    bool by_index = false;             // the current graph is oriented by vertex id
     uint32_t variant_passes = 0;       // passes of the last undirected or tiled single-k call
     uint64_t wait_base_ns = 10ull * 1000 * 1000 * 1000;  // peel barrier wait limit: base ...
     uint64_t wait_ns_per_unit = 8;                        // ... plus per unit of covered work

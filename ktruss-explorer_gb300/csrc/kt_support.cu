@@ -70,6 +70,14 @@ constexpr uint32_t kRowFactor = 6;
 // from 8), a batch of shorter rows, Watts-Strogatz of 4 M edges, 0.25 ms (1.69, 0.80), a path of 200,000 vertices
 // 0.02 ms (0.48; a block a vertex).
 constexpr uint32_t kAllIn = 16;
+// Oriented by vertex id, a hub's row can be any length, and its tails then cost more than the search of
+// v's row in them: the in-edges whose tail is more than kMidTail times v's row stay edge-centric.  R-MAT 20 count,
+// hubs first, 43.4 ms (46.4 edge-centric, 52.5 without the limit; 44.7 at 2, 45.3 at 16), ids shuffled 32.7
+// (38.9, 35.5).  Graphs of fewer than kMidMinById edges and 128 neighbours a vertex, or of 16 a vertex, stay
+// edge-centric altogether: R-MAT 15 0.52 ms (0.70), of edge factor 28 1.15 (1.39), R-MAT 18 of edge factor 4 0.94
+// (1.07); above, R-MAT 16 1.22 (1.21), shuffled 1.05 (0.96), G(2000, 0.3) 0.80 (0.45).  By degree no limit holds.
+constexpr uint32_t kMidTail = 4;
+constexpr uint32_t kMidMinById = 3u << 18;
 // Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save
 // (R-MAT 14 with 220,000 edges counts in 0.05 ms).
 constexpr uint32_t kMidMinEdges = 1u << 18;
@@ -89,7 +97,8 @@ struct Graph {
     const uint32_t* __restrict__ s_eid;
     uint32_t n, m;
     uint32_t mid_in;   // vertices with this many in-edges are vertex-centric (0: none) ...
-    uint32_t mid_out;  // ... if their row has this many entries
+    uint32_t mid_out;  // ... if their row has this many entries,
+    uint32_t mid_tail; // for the in-edges whose tail is at most this many times the row
     uint32_t plan;     // first control word of the plan
     // The edges left by a first round (recount_pruned): o_ptr, o_col and e_src are theirs, m is the
     // edges of the whole graph, which s_ptr .. s_eid describe; new_id[j] is what became of edge j.
@@ -126,6 +135,11 @@ __device__ __forceinline__ bool skip(const Graph& g) {
     return failed(g.ctrl) || (kPruned && !pruned_first(g.ctrl, g.m, g.percent));
 }
 
+// Whether the triangles of an in-edge of v are found at v: its tail has `tail` entries.
+__device__ __forceinline__ bool at_middle(const Graph& g, uint32_t v, uint32_t row, uint32_t tail) {
+    return vertex_centric(g, v, row) && tail <= (uint64_t)g.mid_tail * row;
+}
+
 // Rows long enough for a row block of the fill (k_rows).
 __device__ __forceinline__ bool row_block(uint32_t row) { return row >= kRowMin && row <= kMidRow; }
 
@@ -144,7 +158,7 @@ __device__ __forceinline__ void edge_body(const Graph& g, const Credits& c) {
         const uint32_t b0 = g.o_ptr[v], b1 = g.o_ptr[v + 1];
         const uint32_t na = a1 - a0, nb = b1 - b0;
         if (!na || !nb) continue;  // the same for the whole group
-        const bool middle = vertex_centric(g, v, nb);
+        const bool middle = at_middle(g, v, nb, na);
         if (middle && (!kFill || row_block(a1 - g.o_ptr[u]))) continue;
         uint32_t cnt = 0;
         // iterate the shorter list, search the longer
@@ -294,6 +308,7 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
                 j = g.s_eid[p];
                 if (kPruned) j = g.new_id[j];
                 if (!kPruned || !(j & kGone)) len = g.o_ptr[g.s_col[p] + 1] - (j + 1);  // (else no tail)
+                if (len > (uint64_t)g.mid_tail * row) len = 0;  // k_support's
             }
             uint32_t incl = len;
 #pragma unroll
@@ -617,9 +632,11 @@ __global__ void k_prune_rows(Graph whole, uint32_t percent, const uint32_t* __re
 Graph graph_of(const kt_engine* e) {
     // the choice must be the same in the count and in the fill of one call
     const bool hash_all = !e->sched_on_device && e->sched.support_group == 0;
-    const uint32_t mid_in = hash_all ? kAllIn : e->m >= kMidMinEdges ? kMidIn : 0u, mid_out = hash_all ? kAllIn : kMidOut;
+    const uint64_t m = e->m, n = e->n;
+    const bool pays = m >= kMidMinEdges && (!e->by_index || (m >= 8 * n && (m >= kMidMinById || m >= 64 * n)));
+    const uint32_t mid_in = hash_all ? kAllIn : pays ? kMidIn : 0u, mid_out = hash_all ? kAllIn : kMidOut;
     return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out,
-                 kMidPlan, 0, nullptr};
+                 e->by_index ? kMidTail : 0xffffffffu, kMidPlan, 0, nullptr};
 }
 
 // The items lie in the first chunk buffer, the claims in the second, the rows in the first queue:
