@@ -114,8 +114,7 @@ __global__ void __launch_bounds__(kScanThreads) k_rank_rows(const uint64_t* __re
             len[i] = (uint32_t)(key >> vb);
             rank[key & mask] = (uint32_t)p;
             s_len[p] = len[i];
-            if (kByIndex && p == 0) L.ctrl[kCtrlTinyRow] = 0;  // rows in no order: a warp for each
-            if (!kByIndex) {
+            if (!kByIndex) {  // (by vertex id rows are in no order of length: no marks)
                 if (len[i] >= kBigRow && (p == 0 || before < kBigRow)) L.ctrl[kCtrlBigRow] = (uint32_t)p;
                 if (len[i] > kTinyRow && (p == 0 || before <= kTinyRow)) L.ctrl[kCtrlTinyRow] = (uint32_t)p;
                 before = len[i];

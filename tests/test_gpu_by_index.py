@@ -1,5 +1,6 @@
 """Support counts of graphs oriented by vertex id, where hubs have long rows and tails: on both sides of the
-lines that choose how an edge is counted, with both support schedules and after a packed first round."""
+lines that choose how an edge is counted, with both support schedules and after a packed first round, whose
+rows are in no order of length."""
 import numpy as np
 import pytest
 
@@ -34,6 +35,10 @@ GRAPHS = {
     "er1500": lambda: kt.gen_er(1500, 0.3, 5),                           # small, but 450 neighbours a vertex
     "hub_tails": lambda: _hub_tails(70, 9000),
     "sparse": lambda: kt.gen_er(300000, 2e-5, 6),                        # six neighbours a vertex
+    # a first round that removes all edges, or all but a clique, from rows of a few entries in no order
+    "tree": lambda: (800001, (np.arange(1, 800001) // 4).astype(np.uint32), np.arange(1, 800001, dtype=np.uint32)),
+    "tree_clique": lambda: kt.plant_cliques(600001, (np.arange(1, 600001) // 4).astype(np.uint32),
+                                            np.arange(1, 600001, dtype=np.uint32), 2, 12, 30, 7),
 }
 
 
