@@ -363,11 +363,13 @@ __global__ void k_tile_keys(const uint32_t* __restrict__ src, const uint32_t* __
     if (err && lane_id() == 0) atomicOr(&ctrl[kCtrlError], err);
 }
 
-// Sorted keys back to entries: the source from the row, the destination from the key.
+// Sorted keys back to entries: the source from the row, the destination from the key.  (An input error is read
+// only behind this kernel and the next, which write nothing then.)
 __global__ void k_tile_entries(const uint64_t* __restrict__ keys, uint64_t entries, uint32_t T, uint32_t ts,
-                               unsigned vb, uint32_t* __restrict__ src_out, uint32_t* __restrict__ dst_out) {
+                               unsigned vb, uint32_t* __restrict__ src_out, uint32_t* __restrict__ dst_out,
+                               const uint32_t* __restrict__ ctrl) {
     const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < entries) {
+    if (p < entries && !failed(ctrl)) {
         const uint64_t key = keys[p];
         const uint64_t row = key >> vb;
         const uint64_t tile = row / ts;  // src tile * T + dst tile
@@ -378,9 +380,9 @@ __global__ void k_tile_entries(const uint64_t* __restrict__ keys, uint64_t entri
 
 // tile_src_ptr[r] = first sorted position whose row is >= r (rows + 1 offsets).
 __global__ void k_tile_ptr(const uint64_t* __restrict__ keys, uint64_t entries, unsigned vb, uint64_t rows,
-                           uint32_t* __restrict__ ptr) {
+                           uint32_t* __restrict__ ptr, const uint32_t* __restrict__ ctrl) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r > rows) return;
+    if (r > rows || failed(ctrl)) return;
     uint64_t lo = 0, len = entries;
     while (len > 0) {
         const uint64_t half = len >> 1;
@@ -548,18 +550,19 @@ int tiled_coocsr(kt_engine* e, const uint32_t* d_src, const uint32_t* d_dst, uin
     if (entries) {
         k_tile_keys<<<grid_for(entries), kThreads, 0, st>>>(d_src, d_dst, entries, n, T, ts, vb, e->key_a, e->ctrl);
         count_launch(e);
-        if ((rc = check_launch(e, "k_tile_keys")) || (rc = sync_and_check(e))) return rc;
+        if ((rc = check_launch(e, "k_tile_keys"))) return rc;
         const unsigned passes = (rb + vb + 7) / 8;
         uint32_t* counts = next_counts(e, passes);
         if ((rc = count_digits(e, e->key_a, entries, 0, passes, counts)) ||
             (rc = radix_passes(e, e->key_a, nullptr, e->key_b, nullptr, entries, 0, passes, counts, &in_b)))
             return rc;
         k_tile_entries<<<grid_for(entries), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, entries, T, ts, vb,
-                                                              d_src_out, d_dst_out);
+                                                              d_src_out, d_dst_out, e->ctrl);
         count_launch(e);
         if ((rc = check_launch(e, "k_tile_entries"))) return rc;
     }
-    k_tile_ptr<<<grid_for(rows + 1), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, entries, vb, rows, d_tile_src_ptr);
+    k_tile_ptr<<<grid_for(rows + 1), kThreads, 0, st>>>(in_b ? e->key_b : e->key_a, entries, vb, rows, d_tile_src_ptr,
+                                                       e->ctrl);
     count_launch(e);
     if ((rc = check_launch(e, "k_tile_ptr"))) return rc;
     return sync_and_check(e);
