@@ -208,7 +208,7 @@ typedef struct kt_schedule {
                                   recount) instead of decrementing it per destroyed triangle
                                   (its affected-edge recount, made exact): 1..100, or 0 = never.
                                   The first round of a single-k call on 2^20 edges or more
-                                  recounts from 7/10 of it on                                    */
+                                  recounts from 7/10 of it on (directed by degree)               */
     uint32_t peel_blocks;      /* peel kernel blocks per SM: 1 (64 registers a thread), 2 (32
                                   registers, twice the warps: hides DRAM latency once the graph
                                   outgrows L2), or 0 = 2 when the oriented CSR of a single graph

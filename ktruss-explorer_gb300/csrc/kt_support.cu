@@ -718,13 +718,15 @@ int truss3(kt_engine* e) {
 // frontier of 30-32 % of an R-MAT graph's edges takes 3.9 ms walked and 3.7 here (15 M edges), 0.80 and
 // 0.81 (3.7 M); 26 %: 2.8 and 3.9, 0.55 and 0.88; 41 %: 7.5 and 3.5, 1.2 and 0.73.  Below 2^20 edges it is the
 // share itself (400,000 edges: 40 % 0.10 and 0.14 ms, 48 % 0.135 and 0.125), and below 2^19 the peel's: the five
-// launches that return cost a call 0.02 ms, 4 % of one on 400,000 edges whose frontier is smaller.
+// launches that return cost a call 0.02 ms, 4 % of one on 400,000 edges whose frontier is smaller.  By vertex id,
+// where the count itself costs ten times as much, it is the share too: R-MAT 21 of 12 M edges, k = 5, 48 % 5.4 ms
+// walked and 12.5 here; R-MAT 20, k = 20, 53 % 25.7 walked, 58.6 recounted by the peel kernel, 20.9 here.
 // The peel finds new ids in e->tr and the new counts in key_b (3 m words on); the sort keys are free
 // after the build.
 int recount_pruned(kt_engine* e, uint32_t limit, uint32_t percent, PrunedCount* out) {
     *out = PrunedCount{0, nullptr, nullptr};
     if (percent == 0 || e->m < kPruneMin || e->sched_on_device) return KT_OK;
-    if (e->m >= kPruneEarly) percent = std::max(1u, percent * 7 / 10);
+    if (e->m >= kPruneEarly && !e->by_index) percent = std::max(1u, percent * 7 / 10);
     int rc;
     const Graph whole = graph_of(e);
     uint32_t* o_ptr = reinterpret_cast<uint32_t*>(e->key_a);  // n + 1 words of 2 max(n, entries)

@@ -65,3 +65,35 @@ def test_by_index_counts(name):
                 triangles.add(eng.stats().triangles)
     assert len(triangles) == 1
     eng.close()
+
+
+def test_first_rounds_below_the_recount_share():
+    """A first round of seven tenths of the recount share or more is counted again over the packed survivors by
+    degree, and walked by vertex id, where counting costs more; from the share on both are packed."""
+    torch = pytest.importorskip("torch")
+    n, u, v = kt.gen_rmat(16, 24, 0.57, 0.19, 0.19, 4)
+    u, v = u[: 1 << 20], v[: 1 << 20]
+    src, dst = both_directions(u, v)
+    eng = kt.Engine(0)
+    d_src, d_dst = (torch.from_numpy(np.ascontiguousarray(x).view(np.int32)).cuda() for x in (src, dst))
+    keep = torch.empty(len(src), dtype=torch.uint8, device="cuda")
+    got = {}
+    for directedness in ("directed-by-degree", "directed-by-index"):
+        eng.set_variant(directedness=directedness)
+        eng.set_schedule(8, 32, 85, 0)
+        eng.ktruss(d_src.data_ptr(), d_dst.data_ptr(), len(src), n, 12, keep.data_ptr())
+        want = keep.cpu().numpy()
+        share = 100 * int(eng.round_log()["size"][0]) // len(u)
+        assert 5 < share < 90
+        for percent in (share, share + 1, share * 10 // 7 - 1, min(100, share * 10 // 7 + 2)):
+            eng.set_schedule(8, 32, 85, percent)
+            keep.fill_(7)
+            torch.cuda.synchronize()
+            eng.ktruss(d_src.data_ptr(), d_dst.data_ptr(), len(src), n, 12, keep.data_ptr())
+            assert np.array_equal(keep.cpu().numpy(), want)
+            got[directedness, percent > share, percent * 7 // 10 > share] = eng.stats().peel_phase_ms[4] > 0
+    # peel_phase_ms[4]: time in rounds that count again
+    assert got["directed-by-degree", False, False] and got["directed-by-index", False, False]
+    assert got["directed-by-degree", True, False] and not got["directed-by-index", True, False]
+    assert not got["directed-by-degree", True, True] and not got["directed-by-index", True, True]
+    eng.close()
