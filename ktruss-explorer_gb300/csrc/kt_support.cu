@@ -70,12 +70,13 @@ constexpr uint32_t kRowFactor = 6;
 // from 8), a batch of shorter rows, Watts-Strogatz of 4 M edges, 0.25 ms (1.69, 0.80), a path of 200,000 vertices
 // 0.02 ms (0.48; a block a vertex).
 constexpr uint32_t kAllIn = 16;
-// Oriented by vertex id, a hub's row can be any length, and its tails then cost more than the search of
-// v's row in them: the in-edges whose tail is more than kMidTail times v's row stay edge-centric.  R-MAT 20 count,
-// hubs first, 43.4 ms (46.4 edge-centric, 52.5 without the limit; 44.7 at 2, 45.3 at 16), ids shuffled 32.7
-// (38.9, 35.5).  Graphs of fewer than kMidMinById edges and 128 neighbours a vertex, or of 16 a vertex, stay
+// A tail much longer than v's row costs more than the search of the row in it: the in-edges whose tail is more
+// than kMidTail times v's row stay edge-centric.  K(2000, 2000) with a clique of 100 vertices, count 2.19 ms (2.11
+// edge-centric, 5.20 without the limit; 2.21 at 2, 2.40 at 8, 3.79 at 16); R-MAT 20 3.83 (3.88 without).  By vertex id,
+// where a hub's row can be any length, R-MAT 20, hubs first, 43.4 ms (46.4, 52.5; 44.7 at 2, 45.3 at 16), ids
+// shuffled 32.7 (38.9, 35.5); graphs of fewer than kMidMinById edges and 128 neighbours a vertex, or of 16 a vertex, stay
 // edge-centric altogether: R-MAT 15 0.52 ms (0.70), of edge factor 28 1.15 (1.39), R-MAT 18 of edge factor 4 0.94
-// (1.07); above, R-MAT 16 1.22 (1.21), shuffled 1.05 (0.96), G(2000, 0.3) 0.80 (0.45).  By degree no limit holds.
+// (1.07); above, R-MAT 16 1.22 (1.21), shuffled 1.05 (0.96), G(2000, 0.3) 0.80 (0.45).
 constexpr uint32_t kMidTail = 4;
 constexpr uint32_t kMidMinById = 3u << 18;
 // Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save
@@ -97,8 +98,7 @@ struct Graph {
     const uint32_t* __restrict__ s_eid;
     uint32_t n, m;
     uint32_t mid_in;   // vertices with this many in-edges are vertex-centric (0: none) ...
-    uint32_t mid_out;  // ... if their row has this many entries,
-    uint32_t mid_tail; // for the in-edges whose tail is at most this many times the row
+    uint32_t mid_out;  // ... if their row has this many entries
     uint32_t plan;     // first control word of the plan
     // The edges left by a first round (recount_pruned): o_ptr, o_col and e_src are theirs, m is the
     // edges of the whole graph, which s_ptr .. s_eid describe; new_id[j] is what became of edge j.
@@ -137,7 +137,7 @@ __device__ __forceinline__ bool skip(const Graph& g) {
 
 // Whether the triangles of an in-edge of v are found at v: its tail has `tail` entries.
 __device__ __forceinline__ bool at_middle(const Graph& g, uint32_t v, uint32_t row, uint32_t tail) {
-    return vertex_centric(g, v, row) && tail <= (uint64_t)g.mid_tail * row;
+    return vertex_centric(g, v, row) && tail <= kMidTail * row;  // (rows of at most kMidRow)
 }
 
 // Rows long enough for a row block of the fill (k_rows).
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kMidThreads, 1536 / kMidThreads) k_middle(Grap
                 j = g.s_eid[p];
                 if (kPruned) j = g.new_id[j];
                 if (!kPruned || !(j & kGone)) len = g.o_ptr[g.s_col[p] + 1] - (j + 1);  // (else no tail)
-                if (len > (uint64_t)g.mid_tail * row) len = 0;  // k_support's
+                if (len > kMidTail * row) len = 0;  // k_support's
             }
             uint32_t incl = len;
 #pragma unroll
@@ -441,11 +441,12 @@ __global__ void __launch_bounds__(kMidThreads, 6) k_rows(Graph g, Credits c, con
         // positions warp, warp + kWarps, ...: the lanes load the rows of the next 32 together
         for (uint32_t i0 = warp; i0 + 1 < row; i0 += kWarps * 32) {
             uint32_t lb0 = 0, lb1 = 0;
-            if (i0 + lane * kWarps + 1 < row) {
-                const uint32_t v = g.o_col[r0 + i0 + lane * kWarps];
+            const uint32_t mine = i0 + lane * kWarps;
+            if (mine + 1 < row) {
+                const uint32_t v = g.o_col[r0 + mine];
                 lb0 = g.o_ptr[v];
                 lb1 = g.o_ptr[v + 1];
-                if (lb0 != lb1 && !vertex_centric(g, v, lb1 - lb0)) lb1 = lb0;
+                if (lb0 != lb1 && !at_middle(g, v, lb1 - lb0, row - 1 - mine)) lb1 = lb0;
             }
             for (int l = 0; l < 32; ++l) {
                 const uint32_t i = i0 + l * kWarps, tail = row - 1 - i;
@@ -636,7 +637,7 @@ Graph graph_of(const kt_engine* e) {
     const bool pays = m >= kMidMinEdges && (!e->by_index || (m >= 8 * n && (m >= kMidMinById || m >= 64 * n)));
     const uint32_t mid_in = hash_all ? kAllIn : pays ? kMidIn : 0u, mid_out = hash_all ? kAllIn : kMidOut;
     return Graph{e->ctrl, e->o_ptr, e->o_col, e->e_src, e->s_ptr, e->s_split, e->s_col, e->s_eid, e->n, e->m, mid_in, mid_out,
-                 e->by_index ? kMidTail : 0xffffffffu, kMidPlan, 0, nullptr};
+                 kMidPlan, 0, nullptr};
 }
 
 // The items lie in the first chunk buffer, the claims in the second, the rows in the first queue:
