@@ -56,7 +56,8 @@ enum : uint32_t {
     kPAliveSum = 82,   // u64 (words 82..83): the alive edges they see
     kPSched = 76,      // [4] schedule chosen on the device by the learned selector: support group,
                        //     chunk width, compaction and recount percentages (kept by the peel's init)
-    kListLeast = 84,   // decompositions: complement of the least support (k_list_bounds)
+    kListLeast = 84,   // decompositions: complement of the least support but 0 (k_list_bounds)
+    kListWith = 85,    //   edges in triangles
     kListLocal = 86,   //   u64, list entries of edges in near-cliques
     kLRing = 88,       // [4] barrier slots of the list peel, kLSlotWords each (kt_lists.cu)
     kPruneFront = 120,  // single-k: edges whose counted support is too small (the first round's frontier)
@@ -76,7 +77,7 @@ constexpr CtrlRange kCtrlMap[] = {
     {kPKmax, 1, 1}, {kPRounds, 1, 1}, {kPLevels, 1, 1}, {kMidPlan, 4, 1}, {kCtrlVariantChanged, 1, 1},
     {kRowItems, 1, 1}, {kRowCursor, 1, 1}, {kPBigCount, 4, 1}, {kPLAlive, 4, 1}, {kPLMin, 4, 1}, {kPLMinId, 4, 1},
     {kPCompactions, 1, 1}, {kPPhaseNs, 12, 2}, {kPEdges, 4, 1}, {kPChunks, 8, 2}, {kPWalk, 2, 2}, {kPSched, 4, 1},
-    {kPPasses, 1, 1}, {kPAliveSum, 2, 2}, {kListLeast, 1, 1}, {kListLocal, 2, 2}, {kLRing, 4 * kLSlotWords, 4},
+    {kPPasses, 1, 1}, {kPAliveSum, 2, 2}, {kListLeast, 1, 1}, {kListWith, 1, 1}, {kListLocal, 2, 2}, {kLRing, 4 * kLSlotWords, 4},
     {kPruneFront, 1, 1}, {kPruneLeft, 1, 1}, {kPruneT0, 2, 2}, {kPrunePlan, 3, 1}};
 constexpr bool ctrl_map_holds() {
     uint32_t next = 0;

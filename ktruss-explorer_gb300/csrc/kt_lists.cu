@@ -671,7 +671,7 @@ __global__ void k_list_barrier_probe(const __grid_constant__ ListParams P, uint3
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
-// of whose endpoint's neighbours are common ones, near-cliques, and the least support (walks_rows).  More
+// of whose endpoint's neighbours are common ones, near-cliques, the edges in triangles and their least support (walks_rows).  More
 // than `cap` entries, what the buffer of a call holds that does not wait for the total, are an error:
 // nothing is written to it.  Two blocks an SM: with one, R-MAT 20 takes 0.04 ms more.
 template <bool kChained>
@@ -685,7 +685,11 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_list_bounds(uint32_t* __res
                                                                  Look L) {
     if (kChained) after_previous(sup, supx, ycount, tptr, ends, rows, e_src, o_col);
     __shared__ uint64_t ws[33], s_prefix;
-    __shared__ uint32_t s_tile;
+    __shared__ uint32_t s_tile, s_with, s_least;
+    if (threadIdx.x == 0) {
+        s_with = 0;
+        s_least = ~0u;
+    }
     if (__syncthreads_or(failed(L.ctrl))) return;
     const uint32_t tile = look_tile(L, &s_tile);
     if (tile == kNoTile) return;
@@ -730,13 +734,22 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_list_bounds(uint32_t* __res
         }
     }
     if (!rows) return;
-    if (m < kCliqueEdges) {
-        uint32_t least = ~0u;
+    uint32_t with = 0, least = ~0u;
 #pragma unroll
-        for (uint32_t i = 0; i < kScanItems; ++i)
-            if (j0 + i < m) least = min(least, v[i]);
-        least = __reduce_min_sync(kFullMask, least);
-        if (lane_id() == 0) atomicMax(L.ctrl + kListLeast, ~least);
+    for (uint32_t i = 0; i < kScanItems; ++i) {
+        with += v[i] != 0;
+        least = v[i] ? min(least, v[i]) : least;
+    }
+    with = __reduce_add_sync(kFullMask, with);
+    least = __reduce_min_sync(kFullMask, least);
+    if (lane_id() == 0) {
+        atomicAdd(&s_with, with);
+        atomicMin(&s_least, least);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_with) {
+        atomicAdd(L.ctrl + kListWith, s_with);
+        atomicMax(L.ctrl + kListLeast, ~s_least);
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(kFullMask, local, o);
     if (lane_id() == 0 && local)
@@ -766,7 +779,7 @@ int want_lists(kt_engine* e, bool* use) {
     if ((rc = sync_and_check(e))) return rc;
     const uint64_t total = (uint64_t)e->h_ctrl[kCtrlTriHi] << 32 | e->h_ctrl[kCtrlTriLo];
     const uint64_t local = (uint64_t)e->h_ctrl[kListLocal + 1] << 32 | e->h_ctrl[kListLocal];
-    if (walks_rows(e->m, total, local, ~e->h_ctrl[kListLeast])) return KT_OK;
+    if (walks_rows(e->m, e->h_ctrl[kListWith], total, local, ~e->h_ctrl[kListLeast])) return KT_OK;
     const uint64_t need = std::max<uint64_t>(total, 1);
     if (need > e->list_cap) {
         const uint64_t want = buffer_entries(total, e->list_limit);
@@ -817,7 +830,7 @@ int peel_lists(kt_engine* e, bool* done) {
     *done = e->list_need != 0;
     if ((rc = launch_chained(e, "k_list_bounds", e->chained ? k_list_bounds<true> : k_list_bounds<false>,
                              ceil_div(m, kScanTile), kScanThreads, 0, e->sup, e->rnd, e->tr, m, tptr, ends,
-                             m <= kSmallLists ? nullptr : e->s_len, e->e_src, e->o_col,
+                             e->trusted || small ? nullptr : e->s_len, e->e_src, e->o_col,
                              *done ? e->list_cap : ~0ull, next_look(e))) ||
         (!e->trusted && !small && (rc = want_lists(e, done))) || !*done || (rc = fill_lists(e, tptr, ends)))
         return rc;

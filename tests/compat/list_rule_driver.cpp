@@ -1,5 +1,5 @@
 // Prints what kt_list_rule.h decides: lines "most m", "small m cap", "repeat need cap",
-// "buffer total limit", "walks m total local least".
+// "buffer total limit", "walks m with total local least".
 #include <cstdio>
 #include <cstring>
 
@@ -16,9 +16,10 @@ int main() {
         if (scanf("%llu", &b) != 1) return 1;
         unsigned long long c = 0;
         if (!strcmp(op, "walks")) {
+            unsigned long long local = 0;
             unsigned least = 0;
-            if (scanf("%llu %u", &c, &least) != 2) return 1;
-            printf("%d\n", kt::walks_rows(a, b, c, least));
+            if (scanf("%llu %llu %u", &c, &local, &least) != 3) return 1;
+            printf("%d\n", kt::walks_rows(a, b, c, local, least));
             continue;
         }
         if (!strcmp(op, "buffer")) {

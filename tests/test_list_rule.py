@@ -64,21 +64,29 @@ def _cliques(size, count):
 
 
 def test_which_graphs_walk(ask):
-    near = [(c, (*_cliques(*c), _cliques(*c)[1], 0), walks) for c, walks in [
+    def walks(*graphs):  # (edges, list entries, near-cliques' entries, least support[, edges in triangles])
+        return ask(*[("walks", g[0], g[4] if len(g) > 4 else g[0], *g[1:4]) for g in graphs])
+
+    near = [(c, (*_cliques(*c), _cliques(*c)[1], 0), walk) for c, walk in [
         ((500, 2), 1), ((400, 1), 1), ((200, 6), 1), ((100, 26), 0), ((60, 140), 0), ((60, 160), 1), ((20, 1500), 0),
         ((514, 3), 1), ((516, 1), 1)]]
-    for (c, _, walks), got in zip(near, ask(*[("walks", *q) for _, q, _ in near])):
-        assert got == walks, c
+    for (c, _, walk), got in zip(near, walks(*[g for _, g, _ in near])):
+        assert got == walk, c
     total = 1 << 25
-    assert ask(("walks", 200000, total, total, 0), ("walks", 200000, total, total - total // 256, 0),
-               ("walks", 200000, total, total - total // 256 - 1, 0), ("walks", 200000, 1 << 24, 1 << 24, 0),
-               ("walks", 200000, (1 << 24) - 1, (1 << 24) - 1, 0), ("walks", 1 << 18, 1 << 23, 1 << 23, 0),
-               ("walks", 1 << 18, (1 << 23) - 1, (1 << 23) - 1, 0), ("walks", 1 << 18, 1 << 24, 3 << 22, 0),
-               ("walks", 1 << 18, 1 << 24, (3 << 22) + 1, 0)) == [1, 1, 0, 1, 0, 1, 0, 0, 1]
+    assert walks((200000, total, total, 0), (200000, total, total - total // 256, 0),
+                 (200000, total, total - total // 256 - 1, 0), (200000, 1 << 24, 1 << 24, 0),
+                 (200000, (1 << 24) - 1, (1 << 24) - 1, 0), (1 << 18, 1 << 23, 1 << 23, 0),
+                 (1 << 18, (1 << 23) - 1, (1 << 23) - 1, 0), (1 << 18, 1 << 24, 3 << 22, 0),
+                 (1 << 18, 1 << 24, (3 << 22) + 1, 0)) == [1, 1, 0, 1, 0, 1, 0, 0, 1]
     # density; dense and even
     m = 50000
-    assert ask(("walks", m, 512 * m + 511, 0, 0), ("walks", m, 512 * (m + 1), 0, 0), ("walks", 40000, 0, 0, 0),
-               ("walks", 1 << 18, (512 << 18) + 511, 0, 400), ("walks", 1 << 18, 512 * ((1 << 18) + 1), 0, 0),
-               ("walks", m, 400 * m, 0, 320), ("walks", m, 400 * m, 0, 319), ("walks", m, 320 * m, 0, 320),
-               ("walks", m, 320 * (m + 1), 0, 260), ("walks", m, 320 * (m + 1), 0, 250),
-               ("walks", 1 << 18, 400 << 18, 0, 400)) == [0, 1, 0, 0, 1, 1, 0, 0, 1, 0, 0]
+    assert walks((m, 512 * m + 511, 0, 0), (m, 512 * (m + 1), 0, 0), (40000, 0, 0, 0, 0),
+                 (1 << 18, (512 << 18) + 511, 0, 400), (1 << 18, 512 * ((1 << 18) + 1), 0, 0),
+                 (m, 400 * m, 0, 320), (m, 400 * m, 0, 319), (m, 320 * m, 0, 320),
+                 (m, 320 * (m + 1), 0, 260), (m, 320 * (m + 1), 0, 250),
+                 (1 << 18, 400 << 18, 0, 400)) == [0, 1, 0, 0, 1, 1, 0, 0, 1, 0, 0]
+    # edges in no triangle do not thin an even graph out
+    assert walks((10 * m, 512 * m + 511, 0, 512, m), (10 * m, 512 * (m + 1), 0, 350, m),
+                 (10 * m, 512 * (m + 1), 0, 341, m), (200000, 400 * m, 0, 320, m), (200000, 400 * m, 0, 319, m),
+                 (10 * m, 400 * m, 0, 400, m), (10 * m, 512 * 10 * m + 511, 0, 0, m),
+                 (10 * m, 512 * (10 * m + 1), 0, 0, m)) == [0, 1, 0, 1, 0, 0, 0, 1]
