@@ -326,7 +326,8 @@ int kt_engine_get_schedule(kt_engine* engine, kt_schedule* schedule);
  * the wait can legitimately cover - each row or list entry slot of the work chunks queued for the round
  * that the barrier closes (entries rounded up to whole chunks),
  * each edge (twice) for a level phase, each entry or vertex for a look-back - after which the kernel
- * returns KT_ERR_TIMEOUT instead of waiting forever.  Defaults: 10 s and 8 ns.  base_ns must be at least 1 microsecond. */
+ * returns KT_ERR_TIMEOUT instead of waiting forever.  Defaults: 10 s and 8 ns.  base_ns must be at
+ * least 1 microsecond. */
 int kt_engine_set_wait_limit(kt_engine* engine, uint64_t base_ns, uint32_t ns_per_unit);
 int kt_engine_get_wait_limit(kt_engine* engine, uint64_t* base_ns, uint32_t* ns_per_unit);
 /* Statistics of the last call of the host-buffer entry points (kt_ktruss, kt_decompose,

@@ -77,8 +77,8 @@ constexpr CtrlRange kCtrlMap[] = {
     {kPKmax, 1, 1}, {kPRounds, 1, 1}, {kPLevels, 1, 1}, {kMidPlan, 4, 1}, {kCtrlVariantChanged, 1, 1},
     {kRowItems, 1, 1}, {kRowCursor, 1, 1}, {kPBigCount, 4, 1}, {kPLAlive, 4, 1}, {kPLMin, 4, 1}, {kPLMinId, 4, 1},
     {kPCompactions, 1, 1}, {kPPhaseNs, 12, 2}, {kPEdges, 4, 1}, {kPChunks, 8, 2}, {kPWalk, 2, 2}, {kPSched, 4, 1},
-    {kPPasses, 1, 1}, {kPAliveSum, 2, 2}, {kListLeast, 1, 1}, {kListWith, 1, 1}, {kListLocal, 2, 2}, {kLRing, 4 * kLSlotWords, 4},
-    {kPruneFront, 1, 1}, {kPruneLeft, 1, 1}, {kPruneT0, 2, 2}, {kPrunePlan, 3, 1}};
+    {kPPasses, 1, 1}, {kPAliveSum, 2, 2}, {kListLeast, 1, 1}, {kListWith, 1, 1}, {kListLocal, 2, 2},
+    {kLRing, 4 * kLSlotWords, 4}, {kPruneFront, 1, 1}, {kPruneLeft, 1, 1}, {kPruneT0, 2, 2}, {kPrunePlan, 3, 1}};
 constexpr bool ctrl_map_holds() {
     uint32_t next = 0;
     for (const CtrlRange& r : kCtrlMap) {  // in ascending order

@@ -39,15 +39,15 @@ constexpr uint64_t kCliqueTotal = 1u << 24, kCliqueRest = 256;
 // 1.62 / 1.48, G(700, 0.84) (494, 0.90) 2.47 / 1.85, G(900, 0.6) (323, 0.81) 2.33 / 2.16; with fewer entries
 // G(600, 0.7) (293) 1.29 / 1.46, G(724, 0.66) (314) 1.63 / 1.71; where supports differ, of Barabasi-Albert graphs
 // of 700 vertices (493, 0.45) 12.2 / 21.6, of geometric ones (348, 0.41) 5.7 / 10.3, of cliques of 500 with a tenth
-// of the edges rewired (391, 0.03) 3.1 / 3.9.  (Between 2^18 and 2^19 edges it would be the same: G(900, 0.75) 3.2 / 2.0,
-// G(1200, 0.65) 5.1 / 3.6.)
+// of the edges rewired (391, 0.03) 3.1 / 3.9.  (Between 2^18 and 2^19 edges it would be the same: G(900, 0.75)
+// 3.2 / 2.0, G(1200, 0.65) 5.1 / 3.6.)
 constexpr uint64_t kEvenPerEdge = 320;
 // Edges in no triangle go first and cost either way nothing: evenness is that of the others, which also walk past
-// kMaxListPerEdge entries an edge of theirs if the least support is two thirds of the mean.  K(4000, 2500) with a clique
-// of 600 vertices (143 entries an edge, 867 an edge in triangles, 0.69 of the mean) 35 / 19 ms, a tree of 4 M edges
-// beside a clique of 600 (26, 598, 1) 2.9 / 2.3, beside G(1500, 0.7) (121, 734, 0.86) 11.5 / 10.4, beside G(3000, 0.5)
-// (269, 749, 0.8) 33 / 35; uneven: beside a Barabasi-Albert graph of 3,000 vertices (299, 874) 95 / 150, beside a
-// geometric one of 4,000 (177, 590) 39 / 59.
+// kMaxListPerEdge entries an edge of theirs if the least support is two thirds of the mean.  K(4000, 2500) with
+// a clique of 600 vertices (143 entries an edge, 867 an edge in triangles, 0.69 of the mean) 35 / 19 ms, a tree of
+// 4 M edges beside a clique of 600 (26, 598, 1) 2.9 / 2.3, beside G(1500, 0.7) (121, 734, 0.86) 11.5 / 10.4, beside
+// G(3000, 0.5) (269, 749, 0.8) 33 / 35; uneven: beside a Barabasi-Albert graph of 3,000 vertices (299, 874) 95 / 150,
+// beside a geometric one of 4,000 (177, 590) 39 / 59.
 
 // Whether a graph of m edges, `with` of them in triangles, and `total` list entries walks its rows; `local` of the
 // entries are near-cliques' and `least` is the least support but 0.

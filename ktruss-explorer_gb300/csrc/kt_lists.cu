@@ -671,14 +671,15 @@ __global__ void k_list_barrier_probe(const __grid_constant__ ListParams P, uint3
 
 // sup += supx, what it was into ycount (the claimed part of each list), list starts (tptr[m] is the
 // total, three per triangle) and ends.  With rows (symmetric row lengths), also the entries of edges most
-// of whose endpoint's neighbours are common ones, near-cliques, the edges in triangles and their least support (walks_rows).  More
-// than `cap` entries, what the buffer of a call holds that does not wait for the total, are an error:
-// nothing is written to it.  Two blocks an SM: with one, R-MAT 20 takes 0.04 ms more.
+// of whose endpoint's neighbours are common ones, near-cliques, the edges in triangles and their least
+// support (walks_rows).  More than `cap` entries, what the buffer of a call holds that does not wait for the
+// total, are an error: nothing is written to it.  Two blocks an SM: with one, R-MAT 20 takes 0.04 ms more.
 template <bool kChained>
 __global__ void __launch_bounds__(kScanThreads, 2) k_list_bounds(uint32_t* __restrict__ sup,
                                                                  const uint32_t* __restrict__ supx,
                                                                  uint32_t* __restrict__ ycount, uint32_t m,
-                                                                 uint64_t* __restrict__ tptr, uint64_t* __restrict__ ends,
+                                                                 uint64_t* __restrict__ tptr,
+                                                                 uint64_t* __restrict__ ends,
                                                                  const uint32_t* __restrict__ rows,
                                                                  const uint32_t* __restrict__ e_src,
                                                                  const uint32_t* __restrict__ o_col, uint64_t cap,

@@ -78,9 +78,9 @@ constexpr uint32_t kAllIn = 16;
 // than kMidTail times v's row stay edge-centric.  K(2000, 2000) with a clique of 100 vertices, count 2.19 ms (2.11
 // edge-centric, 5.20 without the limit; 2.21 at 2, 2.40 at 8, 3.79 at 16); R-MAT 20 3.83 (3.88 without).  By vertex id,
 // where a hub's row can be any length, R-MAT 20, hubs first, 43.4 ms (46.4, 52.5; 44.7 at 2, 45.3 at 16), ids
-// shuffled 32.7 (38.9, 35.5); graphs of fewer than kMidMinById edges and 128 neighbours a vertex, or of 16 a vertex, stay
-// edge-centric altogether: R-MAT 15 0.52 ms (0.70), of edge factor 28 1.15 (1.39), R-MAT 18 of edge factor 4 0.94
-// (1.07); above, R-MAT 16 1.22 (1.21), shuffled 1.05 (0.96), G(2000, 0.3) 0.80 (0.45).
+// shuffled 32.7 (38.9, 35.5); graphs of fewer than kMidMinById edges and 128 neighbours a vertex, or than 16 a
+// vertex, stay edge-centric altogether: R-MAT 15 0.52 ms (0.70), of edge factor 28 1.15 (1.39), R-MAT 18 of edge
+// factor 4 0.94 (1.07); above, R-MAT 16 1.22 (1.21), shuffled 1.05 (0.96), G(2000, 0.3) 0.80 (0.45).
 constexpr uint32_t kMidTail = 4;
 constexpr uint32_t kMidMinById = 3u << 18;
 // Smaller graphs are counted edge by edge: the plan and the extra launches cost more than they save

@@ -61,7 +61,8 @@ def test_by_index_counts(name):
                 keep.fill_(7)
                 torch.cuda.synchronize()
                 eng.ktruss(d_src.data_ptr(), d_dst.data_ptr(), len(src), n, k, keep.data_ptr())
-                assert np.array_equal(keep.cpu().numpy(), (ref["truss"] >= k).astype(np.uint8)), (directedness, group, k)
+                want = (ref["truss"] >= k).astype(np.uint8)
+                assert np.array_equal(keep.cpu().numpy(), want), (directedness, group, k)
                 triangles.add(eng.stats().triangles)
     assert len(triangles) == 1
     eng.close()

@@ -1,5 +1,6 @@
 """Graphs of fewer than 2^18 edges on both sides of the rules that send them to the walks: near-cliques by
-their list entries and by what lies beside them, others by their density and evenness.  The truss numbers are the oracle's, a replay goes the same way."""
+their list entries and by what lies beside them, others by their density and evenness.  The truss numbers
+are the oracle's, a replay goes the same way."""
 import numpy as np
 import pytest
 
